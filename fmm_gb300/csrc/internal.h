@@ -156,6 +156,9 @@ struct Workspace {
     int wred_p = -1;  // order of the reduced weights in wred computed from this call's moments (-1: none)
     // direct sum: scaled multipoles and partial sums
     DevBuf dsmc, partial;
+    // FP64 near field: source rows and per-slice sums (not `partial`: the
+    // sampled direct sum runs beside it on another stream)
+    DevBuf near_rows, near_part;
     // second stream (the learned selector's sampled direct sum overlaps the tree phases)
     cudaStream_t aux = nullptr;
     // host entry points: the multipoles and exclusions are copied on `copy`

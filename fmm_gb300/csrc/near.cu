@@ -3,15 +3,23 @@
 // Reference: particle_fields (src/fmm.F90:623-747) and particle_fields_direct
 // (src/fmm.F90:749-824).  Both loop over target particles and call
 // multipole_field on a vector of sources, moving excluded sources to
-// R = (1e10, 1e10, 1e10).  Here the hot loops evaluate every source except the
-// target itself, and a separate per-target pass fixes up the (few) excluded
-// partners: it subtracts their contribution again and, in reference mode,
-// adds the contribution at R = (1e10, 1e10, 1e10) that the reference keeps
-// (a small potential term, src/fmm.F90:714-720).
+// R = (1e10, 1e10, 1e10).  The kernels here do the same pair by pair: a warp
+// holds one target, its lanes take consecutive sources, and a source that the
+// target excludes (itself included, where it lists itself) is evaluated at
+// R = (1e10, 1e10, 1e10) in reference mode (a small potential term,
+// src/fmm.F90:714-720) and passed over in mask mode.
+//
+// The pairs are bound by FP64 issue (pair_f64.cuh): a warp instruction takes a
+// scheduler's FP64 pipe 64 cycles, so index arithmetic, exclusion tests and
+// loads (14 doubles per pair, about 1 TB/s from L1 and L2) are hidden behind
+// it.  What the layout has to give is full lanes and an even spread over the
+// 4 x 152 schedulers: with the sources across the lanes no leaf or system size
+// leaves lanes idle beyond a target's last step, and a warp per target (and
+// source slice, where there are few targets) makes thousands of equal items.
 #include <algorithm>
 
 #include "internal.h"
-#include "pair.cuh"
+#include "pair_f64.cuh"
 #include "dispatch.cuh"
 
 namespace fmm {
@@ -45,6 +53,24 @@ __global__ void k_scale_mp(int64_t n, int dim, const double* __restrict__ mp, do
     for (int c = 0; c < dim; ++c) out[(size_t)c * n + k] = cSrcCoef[c] * mp[(size_t)c * n + k];
 }
 
+// Near rows (pair_f64.cuh) of quadrupole sources: the contraction coefficients
+// (scaled: already folded in), off-diagonal second moments halved, and the
+// trace of the second moments as row 10.
+__global__ void k_near_rows(int64_t n, bool scaled, const double* __restrict__ mp, double* __restrict__ out) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    double tr = 0.0;
+#pragma unroll
+    for (int c = 0; c < 10; ++c) {
+        double v = mp[(size_t)c * n + k];
+        if (!scaled) v *= cSrcCoef[c];
+        if (c == 4 || c == 7 || c == 9) tr += v;
+        if (c == 5 || c == 6 || c == 8) v *= 0.5;
+        out[(size_t)c * n + k] = v;
+    }
+    out[(size_t)10 * n + k] = tr;
+}
+
 // Particle data in key-sorted order (coordinates, damping, scaled multipoles).
 __global__ void k_gather(int64_t n, int dim, const uint32_t* __restrict__ perm, const double* __restrict__ X,
                          const double* __restrict__ mp, const double* __restrict__ damp, double* __restrict__ sx,
@@ -60,166 +86,138 @@ __global__ void k_gather(int64_t n, int dim, const uint32_t* __restrict__ perm, 
     for (int c = 0; c < dim; ++c) smc[(size_t)c * n + k] = cSrcCoef[c] * mp[(size_t)c * n + o];
 }
 
-// P2P: one warp per target leaf.  A leaf's targets are taken 32 at a time;
-// when a chunk has g <= 16 targets (g rounded up to a power of two), the warp
-// splits into 32/g groups that walk disjoint subsets of the sources, and the
-// groups are summed with shuffles at the end, so few lanes idle.
+// The target's exclusion list: its first kExRegs entries in registers (0:
+// unused slot, which no 1-based index equals), the rest read where needed.
+constexpr int kExRegs = 4;
+struct ExList {
+    int e[kExRegs];
+    const int32_t* more;
+    int64_t n;
+    int exw;
+    __device__ __forceinline__ ExList(const int32_t* __restrict__ excl, int exw_, int64_t n_, int64_t i)
+        : more(excl + i), n(n_), exw(exw_) {
+#pragma unroll
+        for (int w = 0; w < kExRegs; ++w) e[w] = w < exw ? excl[(size_t)w * n + i] : 0;
+    }
+    __device__ __forceinline__ bool has(int j1) const {
+        bool x = false;
+#pragma unroll
+        for (int w = 0; w < kExRegs; ++w) x |= e[w] == j1;
+        for (int w = kExRegs; w < exw; ++w) x |= more[(size_t)w * n] == j1;
+        return x;
+    }
+};
+
+// P2P: a warp per target particle and source slice (blockIdx.y of gridDim.y),
+// its lanes over the concatenated particles of the target leaf's near list
+// (each lane walks the list on its own).  Totals go to out[slice][f][particle].
 // IMG: the lists are those of a periodic image (t.shift, t.central): sources
-// sit at x_j + shift, the self pair counts unless the image is the central
-// one, and the result is added to fs (src/fmm.F90:704-736).
+// sit at x_j + shift, the self pair and the exclusions count only in the
+// central image (src/fmm.F90:704-736).
+// 66,666 water molecules, Thole, f = 2 (4.6e8 pairs): 294 ms with a warp per
+// target leaf (targets across the lanes) and the tensor contraction.
 template <int M, int F, bool IMG>
 __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* __restrict__ sx,
                                                  const double* __restrict__ sy, const double* __restrict__ sz,
-                                                 const double* __restrict__ sd, const double* __restrict__ smc,
-                                                 int64_t n, int damp, double* __restrict__ fs) {
-    constexpr int NF = nT(F), NM = nT(M);
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+                                                 const double* __restrict__ sd, const double* __restrict__ rows,
+                                                 int64_t n, int damp, int excl_mode, int exw,
+                                                 const int32_t* __restrict__ excl, double* __restrict__ out) {
+    constexpr int NF = nT(F), NR = near_row_count(M, F);
+    const int64_t tgt = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (w >= t.num_leaves) return;
-    const int leaf = t.leaves[w];
-    const int s0 = t.start[leaf], cnt = t.count[leaf];
-    const int q0 = t.near_off[leaf], q1 = t.near_off[leaf + 1];
-    for (int chunk = 0; chunk < cnt; chunk += 32) {
-        const int nt = min(32, cnt - chunk);
-        int g = 1;
-        while (g < nt) g <<= 1;
-        const int ngr = 32 / g;
-        const int tl = lane & (g - 1), grp = lane / g;
-        const bool valid = tl < nt;
-        const int tgt = s0 + chunk + (valid ? tl : 0);
-        const double xt = sx[tgt], yt = sy[tgt], zt = sz[tgt], dt = sd[tgt];
-        double acc[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) acc[f] = 0.0;
-        if (valid) {
-            for (int q = q0; q < q1; ++q) {
-                const int j = t.near_src[q];
-                const int js = t.start[j], je = js + t.count[j];
-                for (int k = js + grp; k < je; k += ngr) {
-                    if (k == tgt && (!IMG || t.central)) continue;
-                    double mc[NM];
-#pragma unroll
-                    for (int s = 0; s < NM; ++s) mc[s] = smc[(size_t)s * n + k];
-                    if (IMG)
-                        pair_field<M, F, double>(xt - (sx[k] + t.shift[0]), yt - (sy[k] + t.shift[1]),
-                                                 zt - (sz[k] + t.shift[2]), dt * sd[k], damp, mc, acc);
-                    else
-                        pair_field<M, F, double>(xt - sx[k], yt - sy[k], zt - sz[k], dt * sd[k], damp, mc, acc);
-                }
-            }
-        }
-        for (int off = g; off < 32; off <<= 1) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], off);
-        }
-        if (grp == 0 && valid) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                if (IMG)
-                    fs[(size_t)f * n + tgt] += acc[f];
-                else
-                    fs[(size_t)f * n + tgt] = acc[f];
-            }
-        }
-    }
-}
-
-// Direct sum: 128 targets per block, sources streamed through shared memory
-// in tiles of 128; blockIdx.y splits the sources, partial sums per split.
-template <int M, int F>
-__global__ void __launch_bounds__(128) k_direct_f64(int64_t n, const int64_t* __restrict__ targets, int64_t ntgt,
-                                                    const double* __restrict__ X, const double* __restrict__ mc,
-                                                    const double* __restrict__ damp, int damp_type, int64_t chunk,
-                                                    double* __restrict__ partial) {
-    constexpr int NF = nT(F), NM = nT(M);
-    constexpr int TILE = 128;
-    __shared__ double shx[TILE], shy[TILE], shz[TILE], shd[TILE], shm[NM][TILE];
-    const int64_t ti = blockIdx.x * (int64_t)TILE + threadIdx.x;
-    const bool valid = ti < ntgt;
-    const int64_t i = valid ? (targets ? targets[ti] : ti) : 0;
-    const double xi = X[i], yi = X[n + i], zi = X[2 * n + i];
-    const double di = damp ? damp[i] : 0.0;
+    if (tgt >= n) return;
+    const int leaf = t.leaf_of[tgt];
+    const double xt = sx[tgt], yt = sy[tgt], zt = sz[tgt], dt = sd[tgt];
+    const bool here = !IMG || t.central;  // exclusions and the self pair count
+    const ExList ex(excl, here ? exw : 0, n, (int64_t)t.perm[tgt]);
     double acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.0;
-    const int64_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    for (int64_t jt = j0; jt < j1; jt += TILE) {
-        const int64_t j = jt + threadIdx.x;
-        if (j < j1) {
-            shx[threadIdx.x] = X[j];
-            shy[threadIdx.x] = X[n + j];
-            shz[threadIdx.x] = X[2 * n + j];
-            shd[threadIdx.x] = damp ? damp[j] : 0.0;
-#pragma unroll
-            for (int s = 0; s < NM; ++s) shm[s][threadIdx.x] = mc[(size_t)s * n + j];
+    const int q1 = t.near_off[leaf + 1], step = 32 * (int)gridDim.y;
+    int q = t.near_off[leaf] - 1, js = 0, jc = 0;
+    for (int off = lane + 32 * (int)blockIdx.y;; off += step) {
+        while (off >= jc) {
+            off -= jc;
+            if (++q >= q1) break;
+            const int j = t.near_src[q];
+            js = t.start[j];
+            jc = t.count[j];
         }
-        __syncthreads();
-        const int lim = (int)min((int64_t)TILE, j1 - jt);
-        for (int k = 0; k < lim; ++k) {
-            if (jt + k == i) continue;
-            double m[NM];
-#pragma unroll
-            for (int s = 0; s < NM; ++s) m[s] = shm[s][k];
-            pair_field<M, F, double>(xi - shx[k], yi - shy[k], zi - shz[k], di * shd[k], damp_type, m, acc);
+        if (q >= q1) break;
+        const int k = js + off;
+        double dx, dy, dz;
+        if (IMG) {
+            dx = xt - (sx[k] + t.shift[0]);
+            dy = yt - (sy[k] + t.shift[1]);
+            dz = zt - (sz[k] + t.shift[2]);
+        } else {
+            dx = xt - sx[k];
+            dy = yt - sy[k];
+            dz = zt - sz[k];
         }
-        __syncthreads();
-    }
-    if (valid) {
+        if (here) {
+            const bool out_of = ex.has((int)t.perm[k] + 1);
+            if (excl_mode == 0) {
+                if (out_of) dx = dy = dz = 1e10;
+            } else if (out_of || k == tgt) {
+                continue;
+            }
+        }
+        double mc[NR];
 #pragma unroll
-        for (int f = 0; f < NF; ++f) partial[((size_t)blockIdx.y * NF + f) * ntgt + ti] = acc[f];
+        for (int s = 0; s < NR; ++s) mc[s] = rows[(size_t)s * n + k];
+        pair_field_f64<M, F>(dx, dy, dz, dt * sd[k], damp, mc, acc);
     }
+    int f;
+    if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * n + tgt] = acc[0];
 }
 
-// Direct sum for a few targets: one block per (target, source split), the
-// block's threads stride over the sources; block reduction of the partial
-// field into partial[split][f][target].
+// Slices of k_p2p_f64 (and, for periodic images, the sum over images) into
+// the sorted field.
+__global__ void k_p2p_slices(int64_t total, int slices, const double* __restrict__ part, bool add,
+                             double* __restrict__ fs) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    double s = add ? fs[e] : 0.0;
+    for (int k = 0; k < slices; ++k) s += part[(size_t)k * total + e];
+    fs[e] = s;
+}
+
+// Direct sum: a warp per target and slice of `chunk` sources (blockIdx.y), the
+// sources across the lanes; totals go to out[slice][f][target].
 template <int M, int F>
-__global__ void __launch_bounds__(128) k_direct_few(int64_t n, const int64_t* __restrict__ targets, int64_t ntgt,
-                                                    const double* __restrict__ X, const double* __restrict__ mc,
-                                                    const double* __restrict__ damp, int damp_type, int64_t chunk,
-                                                    double* __restrict__ partial) {
-    constexpr int NF = nT(F), NM = nT(M);
-    __shared__ double red[NF][4];
-    const int64_t ti = blockIdx.x;
+__global__ void __launch_bounds__(128) k_direct_f64(int64_t n, const int64_t* __restrict__ targets, int64_t ntgt,
+                                                    const double* __restrict__ X, const double* __restrict__ rows,
+                                                    const double* __restrict__ damp, int damp_type, int excl_mode,
+                                                    int exw, const int32_t* __restrict__ excl, int64_t chunk,
+                                                    double* __restrict__ out) {
+    constexpr int NF = nT(F), NR = near_row_count(M, F);
+    const int64_t ti = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (ti >= ntgt) return;
     const int64_t i = targets ? targets[ti] : ti;
     const double xi = X[i], yi = X[n + i], zi = X[2 * n + i];
     const double di = damp ? damp[i] : 0.0;
+    const ExList ex(excl, exw, n, i);
     double acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.0;
     const int64_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-        if (j == i) continue;
-        double m[NM];
+    for (int64_t j = j0 + lane; j < j1; j += 32) {
+        double dx = xi - X[j], dy = yi - X[n + j], dz = zi - X[2 * n + j];
+        const bool out_of = ex.has((int)j + 1);
+        if (excl_mode == 0) {
+            if (out_of) dx = dy = dz = 1e10;
+        } else if (out_of || j == i) {
+            continue;
+        }
+        double mc[NR];
 #pragma unroll
-        for (int s = 0; s < NM; ++s) m[s] = mc[(size_t)s * n + j];
-        pair_field<M, F, double>(xi - X[j], yi - X[n + j], zi - X[2 * n + j], di * (damp ? damp[j] : 0.0), damp_type,
-                                 m, acc);
+        for (int s = 0; s < NR; ++s) mc[s] = rows[(size_t)s * n + j];
+        pair_field_f64<M, F>(dx, dy, dz, di * (damp ? damp[j] : 0.0), damp_type, mc, acc);
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        double v = acc[f];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[f][w] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < NF) {
-        const int f = threadIdx.x;
-        partial[((size_t)blockIdx.y * NF + f) * ntgt + ti] = (red[f][0] + red[f][1]) + (red[f][2] + red[f][3]);
-    }
-}
-
-__global__ void k_direct_reduce(int64_t ntgt, int nf, int ks, const double* __restrict__ partial,
-                                const int64_t* __restrict__ targets, int64_t ld, double* __restrict__ field) {
-    const int64_t ti = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (ti >= ntgt) return;
-    const int64_t i = targets ? ti : ti;
-    for (int f = 0; f < nf; ++f) {
-        double s = 0.0;
-        for (int k = 0; k < ks; ++k) s += partial[((size_t)k * nf + f) * ntgt + ti];
-        field[(size_t)f * ld + i] = s;
-    }
+    int f;
+    if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * ntgt + ti] = acc[0];
 }
 
 __device__ __forceinline__ bool is_near_leaf(const int32_t* near_off, const int32_t* near_src, int li, int lj) {
@@ -234,29 +232,23 @@ __device__ __forceinline__ bool is_near_leaf(const int32_t* near_off, const int3
     return a < near_off[li + 1] && near_src[a] == lj;
 }
 
-// Exclusion fix-up, one thread per particle (original index i).  With a tree
-// (FMM) the field is indexed by sorted position and "near" means the partner's
-// leaf is in the near list of the target's leaf; without one (direct sum) every
-// partner was evaluated by the hot loop.
+// Mask mode: the far field holds the undamped contribution of excluded
+// partners whose leaf is not in the near list of the target's leaf (the
+// near-field kernels pass over the others); this takes it out again.  One
+// thread per particle (original index i, field in sorted order).
 template <int M, int F>
-__global__ void k_excl_fix(int64_t n, int64_t ntgt, const int64_t* __restrict__ targets, const double* __restrict__ X,
-                           const double* __restrict__ mc, int exw, const int32_t* __restrict__ excl,
-                           const double* __restrict__ damp, int damp_type, int excl_mode,
-                           const int32_t* __restrict__ pos_of, const int32_t* __restrict__ leaf_of,
-                           const int32_t* __restrict__ near_off, const int32_t* __restrict__ near_src,
-                           double* __restrict__ field, int64_t ld, int near_masked) {
+__global__ void k_excl_fix(int64_t n, const double* __restrict__ X, const double* __restrict__ mc, int exw,
+                           const int32_t* __restrict__ excl, const int32_t* __restrict__ pos_of,
+                           const int32_t* __restrict__ leaf_of, const int32_t* __restrict__ near_off,
+                           const int32_t* __restrict__ near_src, double* __restrict__ field) {
     constexpr int NF = nT(F), NM = nT(M);
-    const int64_t ti = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (ti >= ntgt) return;
-    const int64_t i = targets ? targets[ti] : ti;
-    const bool fmm = pos_of != nullptr;
-    const int64_t ki = fmm ? pos_of[i] : ti;
-    const double xi = X[i], yi = X[n + i], zi = X[2 * n + i];
-    const double di = damp ? damp[i] : 0.0;
-    double add[NF], sub[NF];
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t ki = pos_of[i];
+    double sub[NF];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) add[f] = sub[f] = 0.0;
-    bool self_listed = false;
+    for (int f = 0; f < NF; ++f) sub[f] = 0.0;
+    bool any = false;
     for (int w = 0; w < exw; ++w) {
         const int e = excl[(size_t)w * n + i];
         if (e == 0) continue;
@@ -265,34 +257,17 @@ __global__ void k_excl_fix(int64_t n, int64_t ntgt, const int64_t* __restrict__ 
             if (excl[(size_t)w2 * n + i] == e) dup = true;
         if (dup) continue;
         const int64_t j = e - 1;
-        if (j == i) {
-            self_listed = true;
-            continue;
-        }
+        if (j == i || is_near_leaf(near_off, near_src, leaf_of[ki], leaf_of[pos_of[j]])) continue;
         double m[NM];
 #pragma unroll
         for (int s = 0; s < NM; ++s) m[s] = mc[(size_t)s * n + j];
-        const double a = di * (damp ? damp[j] : 0.0);
-        const bool near = fmm ? is_near_leaf(near_off, near_src, leaf_of[ki], leaf_of[pos_of[j]]) : true;
-        if (near) {
-            if (near_masked) continue;  // the near-field kernel already skipped this pair
-            pair_field_cold<M, F, double>(xi - X[j], yi - X[n + j], zi - X[2 * n + j], a, damp_type, m, sub);
-            if (excl_mode == 0) pair_field_cold<M, F, double>(1e10, 1e10, 1e10, a, damp_type, m, add);
-        } else if (excl_mode == 1) {
-            pair_field_cold<M, F, double>(xi - X[j], yi - X[n + j], zi - X[2 * n + j], 0.0, DAMP_NONE, m, sub);
-        }
+        pair_field_cold<M, F, double>(X[i] - X[j], X[n + i] - X[n + j], X[2 * n + i] - X[2 * n + j], 0.0, DAMP_NONE, m,
+                                      sub);
+        any = true;
     }
-    if (excl_mode == 0) {
-        double m[NM];
+    if (!any) return;
 #pragma unroll
-        for (int s = 0; s < NM; ++s) m[s] = mc[(size_t)s * n + i];
-        if (self_listed)
-            pair_field_cold<M, F, double>(1e10, 1e10, 1e10, di * di, damp_type, m, add);
-        else  // the reference evaluates the self pair at R = 0 (non-finite result)
-            pair_field_cold<M, F, double>(0.0, 0.0, 0.0, di * di, damp_type, m, add);
-    }
-#pragma unroll
-    for (int f = 0; f < NF; ++f) field[(size_t)f * ld + ki] += add[f] - sub[f];
+    for (int f = 0; f < NF; ++f) field[(size_t)f * n + ki] -= sub[f];
 }
 
 __global__ void k_scatter(int64_t n, int nf, const uint32_t* __restrict__ perm, const double* __restrict__ fs,
@@ -314,37 +289,36 @@ int launch_direct_f64(Workspace& ws, const Particles& P, int field_order, const 
     const int64_t n = P.n;
     if (!d_targets) ntgt = n;
     const int nf = nT(field_order);
-    FMM_TRY(ws.dsmc.ensure(sizeof(double) * (size_t)n * P.dim));  // own buffer: may overlap the FMM phases
-    double* mc = ws.dsmc.as<double>();
+    // own buffer: may overlap the FMM phases
+    FMM_TRY(ws.dsmc.ensure(sizeof(double) * (size_t)n * near_row_count(m, field_order)));
+    double* rows = ws.dsmc.as<double>();
     count_launches(1);
-    k_scale_mp<<<grid_for(n, 256), 256, 0, st>>>(n, P.dim, P.mp, mc);
-    // few targets (sampled checks): a block per target and source split
-    const bool few = ntgt <= 64;
-    const int64_t tblocks = few ? ntgt : (ntgt + 127) / 128;
-    int64_t ks = std::max<int64_t>(1, ((few ? 16LL : 8LL) * num_sms() + tblocks - 1) / tblocks);
-    ks = std::min<int64_t>(ks, std::max<int64_t>(1, n / (few ? 1024 : 256)));
+    if (near_row_count(m, field_order) > P.dim)
+        k_near_rows<<<grid_for(n, 128), 128, 0, st>>>(n, false, P.mp, rows);
+    else
+        k_scale_mp<<<grid_for(n, 128), 128, 0, st>>>(n, P.dim, P.mp, rows);
+    // Slices: 16 items per scheduler where the sum is long enough, at least
+    // one step of 32 sources each (300 targets: 10 slices of one step; 4096: 2
+    // of 64 steps; from 10,000 on one slice, written straight to the field)
+    const int64_t steps = (n + 31) / 32;
+    const int64_t per = std::max<int64_t>(1, ntgt * steps / (16LL * 4 * num_sms()));
+    int64_t ks = (steps + per - 1) / per;
+    if (split_cap > 0) ks = std::min<int64_t>(ks, 4LL * split_cap);
     ks = std::min<int64_t>(ks, 65535);
-    if (split_cap > 0) ks = std::min<int64_t>(ks, split_cap);
-    const int64_t chunk = (n + ks - 1) / ks;
-    FMM_TRY(ws.partial.ensure(sizeof(double) * (size_t)ks * nf * ntgt));
-    dim3 grid((unsigned)tblocks, (unsigned)ks);
-    if (few) {
-        FMM_MF_SWITCH_F64(m, field_order, (k_direct_few<MM, FF><<<grid, 128, 0, st>>>(n, d_targets, ntgt, P.x, mc, P.damp,
-                                                                                   P.damp_type, chunk,
-                                                                                   ws.partial.as<double>())));
-    } else {
-        FMM_MF_SWITCH_F64(m, field_order, (k_direct_f64<MM, FF><<<grid, 128, 0, st>>>(n, d_targets, ntgt, P.x, mc,
-                                                                                   P.damp, P.damp_type, chunk,
-                                                                                   ws.partial.as<double>())));
+    const int64_t chunk = (steps + ks - 1) / ks * 32;
+    ks = (n + chunk - 1) / chunk;
+    double* out = d_field;
+    if (ks > 1) {
+        FMM_TRY(ws.partial.ensure(sizeof(double) * (size_t)ks * nf * ntgt));
+        out = ws.partial.as<double>();
     }
-    count_launches(1);
-    k_direct_reduce<<<grid_for(ntgt, 256), 256, 0, st>>>(ntgt, nf, (int)ks, ws.partial.as<double>(), nullptr, ntgt,
-                                                         d_field);
-    if (P.exw > 0 || md.excl_mode == 0) {
-        FMM_MF_SWITCH_F64(m, field_order,
-                      (k_excl_fix<MM, FF><<<grid_for(ntgt, 128), 128, 0, st>>>(
-                          n, ntgt, d_targets, P.x, mc, P.exw, P.excl, P.damp, P.damp_type, md.excl_mode, nullptr,
-                          nullptr, nullptr, nullptr, d_field, ntgt, 0)));
+    const dim3 grid(grid_for(ntgt, 4), (unsigned)ks);
+    FMM_MF_SWITCH_F64(m, field_order,
+                      (k_direct_f64<MM, FF><<<grid, 128, 0, st>>>(n, d_targets, ntgt, P.x, rows, P.damp, P.damp_type,
+                                                                  md.excl_mode, P.exw, P.excl, chunk, out)));
+    if (ks > 1) {
+        count_launches(1);
+        k_p2p_slices<<<grid_for(ntgt * nf, 128), 128, 0, st>>>(ntgt * nf, (int)ks, out, false, d_field);
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -370,25 +344,42 @@ int gather_sorted(Workspace& ws, const Particles& P, const TreeDev& t, cudaStrea
 
 int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int field_order, const Modes& md,
                    cudaStream_t st, bool image) {
-    (void)md;
     const int m = dim_to_order(P.dim);
     if (!near_orders_supported(m, field_order)) return FMM_ENOTSUP;
     const int64_t n = P.n;
     const int nf = nT(field_order);
     FMM_TRY(ws.fsorted.ensure(sizeof(double) * (size_t)n * nf));
-    const unsigned blocks = grid_for((int64_t)t.num_leaves * 32, 128);
+    const double* rows = ws.smc.as<double>();
+    if (near_row_count(m, field_order) > P.dim) {
+        FMM_TRY(ws.near_rows.ensure(sizeof(double) * (size_t)n * near_row_count(m, field_order)));
+        count_launches(1);
+        k_near_rows<<<grid_for(n, 128), 128, 0, st>>>(n, true, ws.smc.as<double>(), ws.near_rows.as<double>());
+        rows = ws.near_rows.as<double>();
+    }
+    // slices of the near lists while there are fewer than 16 targets per
+    // scheduler (a near list holds many steps of 32 sources)
+    const int ks = (int)std::max<int64_t>(1, std::min<int64_t>(8, 16LL * 4 * num_sms() / n));
+    const bool part = image || ks > 1;
+    double* out = ws.fsorted.as<double>();
+    if (part) {
+        FMM_TRY(ws.near_part.ensure(sizeof(double) * (size_t)ks * nf * n));
+        out = ws.near_part.as<double>();
+    }
+    const dim3 grid(grid_for(n, 4), (unsigned)ks);
     if (image) {
         FMM_MF_SWITCH_F64(m, field_order,
-                      (k_p2p_f64<MM, FF, true><<<blocks, 128, 0, st>>>(t, ws.sx.as<double>(), ws.sy.as<double>(),
-                                                                       ws.sz.as<double>(), ws.sd.as<double>(),
-                                                                       ws.smc.as<double>(), n, P.damp_type,
-                                                                       ws.fsorted.as<double>())));
+                      (k_p2p_f64<MM, FF, true><<<grid, 128, 0, st>>>(
+                          t, ws.sx.as<double>(), ws.sy.as<double>(), ws.sz.as<double>(), ws.sd.as<double>(), rows, n,
+                          P.damp_type, md.excl_mode, P.exw, P.excl, out)));
     } else {
         FMM_MF_SWITCH_F64(m, field_order,
-                      (k_p2p_f64<MM, FF, false><<<blocks, 128, 0, st>>>(t, ws.sx.as<double>(), ws.sy.as<double>(),
-                                                                        ws.sz.as<double>(), ws.sd.as<double>(),
-                                                                        ws.smc.as<double>(), n, P.damp_type,
-                                                                        ws.fsorted.as<double>())));
+                      (k_p2p_f64<MM, FF, false><<<grid, 128, 0, st>>>(
+                          t, ws.sx.as<double>(), ws.sy.as<double>(), ws.sz.as<double>(), ws.sd.as<double>(), rows, n,
+                          P.damp_type, md.excl_mode, P.exw, P.excl, out)));
+    }
+    if (part) {
+        count_launches(1);
+        k_p2p_slices<<<grid_for(n * nf, 128), 128, 0, st>>>(n * nf, ks, out, image, ws.fsorted.as<double>());
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -396,14 +387,13 @@ int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
 
 int launch_excl_correction(Workspace& ws, const Particles& P, const TreeDev* t, int field_order, const Modes& md,
                            double* d_field, cudaStream_t st) {
+    if (md.excl_mode == 0 || P.exw == 0) return FMM_OK;  // reference mode leaves far partners in
     const int m = dim_to_order(P.dim);
     const int64_t n = P.n;
     const double* mc_orig = ws.smc.as<double>() + (size_t)n * P.dim;
     FMM_MF_SWITCH_F64(m, field_order,
                   (k_excl_fix<MM, FF><<<grid_for(n, 128), 128, 0, st>>>(
-                      n, n, nullptr, P.x, mc_orig, P.exw, P.excl, P.damp, P.damp_type, md.excl_mode, t->pos_of,
-                      t->leaf_of, t->near_off, t->near_src, d_field, n,
-                      (md.precision == 1 || md.precision == 2) ? 1 : 0)));
+                      n, P.x, mc_orig, P.exw, P.excl, t->pos_of, t->leaf_of, t->near_off, t->near_src, d_field)));
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
