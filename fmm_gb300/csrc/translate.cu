@@ -440,6 +440,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_p2m(const TreeDev t, const dou
         typename O::Acc sum;
 #pragma unroll
         for (int sidx = 0; sidx < NM; ++sidx) {
+            if (sidx >= nq) break;  // moments above the expansion order reach no output
             const int sc = comp[sidx], qx = ux_(sc), qy = uy_(sc), qz = uz_(sc);
             if (qx <= tx && qy <= ty && qz <= tz) sum.add(A[pk_index(tx - qx, ty - qy, tz - qz) * NM + sidx]);
         }
