@@ -1,9 +1,15 @@
 // Reference-mode M2L (FP64): the reference's own closed-form tensors with the
-// int32 Cnij table (src/tensors_recursive.F90:29-135) over the full Cartesian
-// bases, L_f(i) += sum_s (-1)^(|s|+1) M'_s(j) T_{s+f}(c_i - c_j)
-// (src/fmm.F90:826-882), with M'_s = M_s / s! the scaled moments of
-// translate.cu.  The exact-coefficient modes use the reduced-basis M2L
-// (m2l.cu, m2l_gemm.cu) instead.
+// int32 Cnij table (src/tensors_recursive.F90:29-135), L_f(i) += sum_s
+// (-1)^(|s|+1) M'_s(j) T_{s+f}(c_i - c_j) (src/fmm.F90:826-882), with M'_s =
+// M_s / s! the scaled moments of translate.cu.
+//
+// Up to order 2p = 10 no coefficient wraps: the closed form is the exact tensor
+// up to rounding, and the reduced-basis M2L of the exact modes (m2l.cu,
+// m2l_gemm.cu) gives the reference's result.  Above, the tensors are not
+// harmonic; they are evaluated once per displacement group and multiplied over
+// all Cartesian components (m2l_gemm.cu, m2l_tc64.cuh), or per pair where the
+// groups hold a pair or two each (k_m2l_f64).  66,666 water molecules, p = 6
+// (9.3e5 far pairs): 136.7 ms when every pair had its own closed form.
 #include <algorithm>
 #include <vector>
 
@@ -271,7 +277,65 @@ int ensure_ref_terms(Workspace& ws, int N, cudaStream_t st) {
     return FMM_OK;
 }
 
-int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md, bool accumulate, cudaStream_t st) {
+namespace {
+
+// Whether the reference's int32 coefficients of order N are the exact ones:
+// they reach 2^31 first at N = 11.
+constexpr int kExactRefOrder = 10;
+
+// Warp per displacement group: the closed-form tensor at the displacement in
+// units of the coarser cell's half-width, the group's order and unit ratios.
+__global__ void k_group_tensor_ref(int ng, const int32_t* __restrict__ gstart, const int32_t* __restrict__ svals,
+                                   const int32_t* __restrict__ tgt, const TreeDev t, int p, int ldT,
+                                   const int32_t* __restrict__ term_off, const uchar4* __restrict__ term_abc,
+                                   const double* __restrict__ term_c, double* __restrict__ gT,
+                                   int32_t* __restrict__ gq, float2* __restrict__ gab) {
+    extern __shared__ double smem[];
+    const int N = 2 * p, nqT = nT(N);
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double* TA = smem + wib * (nqT + 4 * (N + 1));
+    double* gsh = TA + nqT;
+    double* yp = gsh + (N + 1);
+    double* zp = yp + (N + 1);
+    double* ir = zp + (N + 1);
+    const int g = blockIdx.x * (blockDim.x >> 5) + wib;
+    if (g >= ng) return;
+    const int pos0 = svals[gstart[g]];
+    const int i = tgt[pos0], j = t.far_src[pos0];
+    const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
+    const double X = __dsub_rn(t.cx[i], __dadd_rn(t.cx[j], t.shift[0])) / hc;
+    const double Y = __dsub_rn(t.cy[i], __dadd_rn(t.cy[j], t.shift[1])) / hc;
+    const double Z = __dsub_rn(t.cz[i], __dadd_rn(t.cz[j], t.shift[2])) / hc;
+    const double* T = warp_tensor(X, Y, Z, N, 1, nullptr, TA, nullptr, gsh, yp, zp, ir, term_off, term_abc, term_c,
+                                  lane);
+    for (int c = lane; c < nqT; c += 32) gT[(size_t)g * ldT + c] = T[c];
+    if (lane == 0) {
+        gq[g] = p;
+        gab[g] = make_float2((float)(hi / hc), (float)(hj / hc));
+    }
+}
+
+}  // namespace
+
+int launch_group_tensor_ref(Workspace& ws, const TreeDev& t, int ng, const int32_t* tgt, int p, int ldT,
+                            cudaStream_t st) {
+    const int N = 2 * p;
+    FMM_TRY(ensure_ref_terms(ws, N, st));
+    const size_t per_warp = sizeof(double) * (nT(N) + 4 * (N + 1));
+    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (100 * 1024) / per_warp));
+    FMM_TRY(set_smem((const void*)k_group_tensor_ref, wpb * per_warp));
+    count_launches(1);
+    k_group_tensor_ref<<<grid_for(ng, wpb), 32 * wpb, wpb * per_warp, st>>>(
+        ng, ws.m2l_gstart.as<int32_t>(), ws.m2l_vals2.as<int32_t>(), tgt, t, p, ldT, ws.term_off.as<int32_t>(),
+        ws.term_abc.as<uchar4>(), ws.term_c.as<double>(), ws.m2l_T.as<double>(), ws.m2l_gq.as<int32_t>(),
+        ws.m2l_gab.as<float2>());
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
+// M2L pair by pair on the CUDA cores (FP64), ref or exact tensors.
+static int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md, bool accumulate,
+                               cudaStream_t st) {
     const int nq = nT(p), N = 2 * p, nqT = nT(N);
     FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nq));
     const int ref = md.coef_mode == 0 ? 1 : 0;
@@ -288,9 +352,16 @@ int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md,
     return FMM_OK;
 }
 
-int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st) {
-    if (md.coef_mode != 0) return launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, st);
-    return launch_m2l_pairwise(ws, t, p, md, false, st);
+int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st, bool accumulate) {
+    int rc;
+    if (md.coef_mode != 0 || 2 * p <= kExactRefOrder) {
+        rc = launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, st, accumulate);
+    } else {
+        FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nT(p)));
+        rc = (ws.reuse_structure && ws.m2l_pairwise) ? FMM_ENOTSUP
+                                                     : launch_m2l_grouped(ws, t, p, false, st, true, accumulate);
+    }
+    return rc == FMM_ENOTSUP ? launch_m2l_pairwise(ws, t, p, md, accumulate, st) : rc;
 }
 
 // ---------------------------------------------------------------- periodic

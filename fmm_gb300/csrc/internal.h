@@ -144,7 +144,7 @@ struct Workspace {
     DevBuf sel_budget;  // per node: log10 error budget of far pairs with that target, then its field scale
     // grouped M2L
     DevBuf m2l_tgt, m2l_keys, m2l_keys2, m2l_vals, m2l_vals2, m2l_ukeys, m2l_cnt, m2l_gstart, m2l_tcnt, m2l_toff,
-        m2l_tasks, m2l_T, m2l_gq, m2l_gab, m2l_wsc, m2l_out, m2l_wsplit, m2l_gop, m2l_gopoff, m2l_rowbase;
+        m2l_tasks, m2l_T, m2l_gq, m2l_gab, m2l_wsc, m2l_out, m2l_wsplit, m2l_gop, m2l_gopoff, m2l_rowbase, m2l_gexp;
     // sorted particle data
     DevBuf sx, sy, sz, smc, sd;
     DevBuf f32buf;   // FP32 particle records of the mixed-precision near field
@@ -252,17 +252,22 @@ int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
                    cudaStream_t st, bool image = false);
 // df: P2M sums in double-float (FP32 pipe) instead of FP64 (mixed path)
 int launch_p2m_m2m(Workspace& ws, const Particles& P, const TreeDev& t, int p, cudaStream_t st, bool df = false);
-int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st);
-// M2L pair by pair on the CUDA cores (FP64), ref or exact tensors, honouring
-// t.shift; accumulate adds into the local expansions instead of writing them.
-int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md, bool accumulate, cudaStream_t st);
+// M2L into the local expansions, honouring t.shift; accumulate adds to them
+// instead of writing them.
+int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st, bool accumulate = false);
+// Reference mode: the closed-form tensor of every displacement group of the
+// grouped M2L (all components of order <= 2p, ldT entries a group), with the
+// group's order and unit ratios.
+int launch_group_tensor_ref(Workspace& ws, const TreeDev& t, int ng, const int32_t* tgt, int p, int ldT,
+                            cudaStream_t st);
 // Periodic boxes: lattice sum beyond the 27 images into the root's local
 // expansion and the surface (dipole) term into the sorted field d_fs;
 // *d_levels receives the number of lattice levels used.
 int launch_periodic_lattice(Workspace& ws, const TreeDev& t, int p, int f, const Modes& md, const Box9& H,
                             double* d_fs, int* d_levels, cudaStream_t st);
-int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st);
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st);
+int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool accumulate = false);
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full = false,
+                       bool accumulate = false);
 int launch_reduce_moments(Workspace& ws, const TreeDev& t, int p, cudaStream_t st);
 // selector.cu
 int selector_node_norms(Workspace& ws, const TreeDev& t, int P, const double* d_sorted_damp, cudaStream_t st);

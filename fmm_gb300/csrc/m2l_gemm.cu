@@ -9,10 +9,14 @@
 // the group's displacement, computed once per group in FP64), and the group's
 // pairs are the columns of one product C = G W.  FP32 products run on the
 // tensor cores (tcgen05, kind::tf32 with operands split into two TF32 parts,
-// three products per term, FP32 accumulators in tensor memory); FP64
-// products, and FP32 ones on request, on the CUDA cores as register-tiled
-// blocks.  Per-pair columns go to a buffer in target-sorted order and are
-// summed per target with compensated sums.
+// three products per term, FP32 accumulators in tensor memory), FP64 products
+// too, in fixed point (m2l_tc64.cuh), and either on request on the CUDA cores
+// as register-tiled blocks.  Per-pair columns go to a buffer in target-sorted
+// order and are summed per target with compensated sums.
+//
+// Where the reference's 32-bit tensor coefficients wrap (orders 2p > 10), its
+// tensors are not harmonic: the FP64 product then runs over all Cartesian
+// components (`full`), with the reference's closed form once per group.
 //
 // Units: per-node weights w'_s = w^_s / h_j^|s|, per-target locals
 // L'_f = h_i^(|f|+1) L_f, tensor T(D_c) at the displacement in units of the
@@ -28,6 +32,7 @@
 
 #include "internal.h"
 #include "m2l_basis.cuh"
+#include "m2l_tc64.cuh"
 #include "umma.cuh"
 
 namespace fmm {
@@ -40,6 +45,7 @@ constexpr int kFallback = 63;            // key code of pairs without a grid dis
 // Key layout (46 bits, so the radix sort needs 6 digit passes): level
 // difference + 31 (6 bits) | order (4) | Dx, Dy, Dz + kDOff (12 bits each).
 constexpr int kKeyBits = 46;
+constexpr int kKeyBitsLevel = 51;        // with the target's depth above (displaced sources)
 constexpr int64_t kDOff = 1 << 11;       // offset of the 12-bit displacement fields
 constexpr int kTaskCols = 512;           // pairs (columns) per product block
 constexpr int kGemmThreads = 128;        // 16 row groups x 8 column groups
@@ -85,7 +91,10 @@ __global__ void k_scale_weights(int M, int nr, int ld, const double* __restrict_
 // pipe; its error (a few 1e-8 relative of the displacement, up to ~1e-4 cell
 // units at the largest encodable displacement) stays far below the 1e-3
 // tolerance of the integer test.  Without them, FP64 with a 1e-6 tolerance.
-__global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restrict__ tgt, int p, int oclass,
+// level: the sources are displaced by a periodic image's shift, which is the
+// same for all pairs but not in units of their cells, so only pairs of one
+// level share an operator.
+__global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restrict__ tgt, int p, int oclass, bool level,
                            const float4* __restrict__ chi, const float4* __restrict__ clo,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -127,7 +136,8 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
     uint64_t key;
     if (grid)
         key = ((uint64_t)(dl + 31) << 40) | ((uint64_t)oc << 36) | ((uint64_t)((int64_t)rx + kDOff) << 24) |
-              ((uint64_t)((int64_t)ry + kDOff) << 12) | (uint64_t)((int64_t)rz + kDOff);
+              ((uint64_t)((int64_t)ry + kDOff) << 12) | (uint64_t)((int64_t)rz + kDOff) |
+              (level ? (uint64_t)t.depth[i] << kKeyBits : 0);
     else
         key = ((uint64_t)kFallback << 40) | (uint64_t)q;
     keys[q] = key;
@@ -164,7 +174,9 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_
         q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
     for (int off = 16; off > 0; off >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, off));
     const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
-    const double X = (t.cx[i] - t.cx[j]) / hc, Y = (t.cy[i] - t.cy[j]) / hc, Z = (t.cz[i] - t.cz[j]) / hc;
+    // (the source cells of a periodic image are displaced by t.shift)
+    const double X = (t.cx[i] - (t.cx[j] + t.shift[0])) / hc, Y = (t.cy[i] - (t.cy[j] + t.shift[1])) / hc,
+                 Z = (t.cz[i] - (t.cz[j] + t.shift[2])) / hc;
     const int Nq = 2 * q;
     const double r2 = X * X + Y * Y + Z * Z;
     const double rinv = 1.0 / sqrt(r2), rinv2 = rinv * rinv;
@@ -210,8 +222,16 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_
 }
 
 // Tasks of up to `cols` pairs of one group: counts, then (group, first
-// column).  cols < 0: tensor-core tasks of kTcPairs pairs and one operator
-// half each, (group, 2 x first column + half).
+// column).  Tensor-core tasks (cols kTcTasks: kTcPairs pairs and one operator
+// half each, (group, 2 x first column + half); kD64Tasks, kD64FullTasks: the
+// FP64 products' kD64Pairs pairs and one part, (group, 4 x first column + part)).
+constexpr int kTcTasks = -1, kD64Tasks = -2, kD64FullTasks = -3;
+
+__device__ __forceinline__ int task_pairs(int cols) { return cols > 0 ? cols : (cols == kTcTasks ? kTcPairs : kD64Pairs); }
+__device__ __forceinline__ int task_parts(int cols, int q) {
+    return cols > 0 ? 1 : (cols == kTcTasks ? tc_halves(q) : d64_parts(q, cols == kD64FullTasks));
+}
+
 __global__ void k_task_counts(int ng, int cols, const int32_t* __restrict__ gq, const int32_t* __restrict__ gstart,
                               int32_t* __restrict__ tcnt) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -220,21 +240,17 @@ __global__ void k_task_counts(int ng, int cols, const int32_t* __restrict__ gq, 
         tcnt[g] = 0;
         return;
     }
-    const int n = gstart[g + 1] - gstart[g];
-    tcnt[g] = cols > 0 ? (n + cols - 1) / cols : (n + kTcPairs - 1) / kTcPairs * tc_halves(gq[g]);
+    const int n = gstart[g + 1] - gstart[g], w = task_pairs(cols);
+    tcnt[g] = (n + w - 1) / w * task_parts(cols, gq[g]);
 }
 
 __global__ void k_fill_tasks(int ng, int cols, const int32_t* __restrict__ gq, const int32_t* __restrict__ gstart,
                              const int32_t* __restrict__ toff, int2* __restrict__ tasks) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
-    const int n = toff[g + 1] - toff[g];
-    if (cols > 0) {
-        for (int k = 0; k < n; ++k) tasks[toff[g] + k] = make_int2(g, k * cols);
-    } else {
-        const int h = tc_halves(gq[g]);
-        for (int k = 0; k < n; ++k) tasks[toff[g] + k] = make_int2(g, 2 * kTcPairs * (k / h) + k % h);
-    }
+    const int n = toff[g + 1] - toff[g], w = task_pairs(cols), h = task_parts(cols, gq[g]);
+    const int mul = cols > 0 ? 1 : (cols == kTcTasks ? 2 : 4);
+    for (int k = 0; k < n; ++k) tasks[toff[g] + k] = make_int2(g, mul * w * (k / h) + k % h);
 }
 
 // Shared-memory plan of the product kernel (elements of R unless noted).
@@ -415,8 +431,8 @@ __device__ __forceinline__ void gemm_task(const GemmSmem<R, CPT>& L, char* sm, i
 // row of (q+1)^2 rounded up to kRowUnit entries (32 bytes in FP32, one DRAM
 // sector) per pair in group order.
 constexpr int kRowUnit = 8;
-__host__ __device__ __forceinline__ int row_len(int q) {
-    return ((q + 1) * (q + 1) + kRowUnit - 1) / kRowUnit * kRowUnit;
+__host__ __device__ __forceinline__ int row_len(int q, bool full = false) {
+    return (d64_rows(q, full) + kRowUnit - 1) / kRowUnit * kRowUnit;
 }
 
 // tcols: pairs per task (at most kTaskCols); tasks of order < qmin are left
@@ -550,21 +566,21 @@ __global__ void k_split_weights(int64_t total, int nr, int ldw, int ldk, const f
 }
 
 // Rows of each group in units of kRowUnit entries (scanned into rowbase).
-__global__ void k_row_sizes(int ng, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
+__global__ void k_row_sizes(int ng, bool full, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
                             int32_t* __restrict__ rsz) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g > ng) return;
-    rsz[g] = g < ng ? (gstart[g + 1] - gstart[g]) * (row_len(gq[g]) / kRowUnit) : 0;
+    rsz[g] = g < ng ? (gstart[g + 1] - gstart[g]) * (row_len(gq[g], full) / kRowUnit) : 0;
 }
 
 // Row of every far pair, indexed in target order (svals maps group order to
 // target order), in units of kRowUnit entries.  Warp per group.
-__global__ void k_row_offsets(int ng, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
+__global__ void k_row_offsets(int ng, bool full, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
                               const int32_t* __restrict__ rowbase, const int32_t* __restrict__ svals,
                               int32_t* __restrict__ roff) {
     const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= ng) return;
-    const int lane = threadIdx.x & 31, u = row_len(gq[g]) / kRowUnit;
+    const int lane = threadIdx.x & 31, u = row_len(gq[g], full) / kRowUnit;
     for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32) roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
 }
 
@@ -856,17 +872,19 @@ struct Sum<double> {
     __device__ __forceinline__ double value() const { return v; }
 };
 
-// Block per target, thread per reduced component: compensated sum of the
+// Block per target, thread per component of the basis: compensated sum of the
 // target's pair rows (stored in group order; roff gives each target-order
-// pair's row in units of kRowUnit entries; a pair of order q contributes its first
-// (q+1)^2 entries; eight loads in flight), back to physical units, into the
-// reduced components of the local expansion.
-template <typename R>
-__global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p, const R* __restrict__ out,
-                                                 const int32_t* __restrict__ roff, double* __restrict__ loc) {
+// pair's row in units of kRowUnit entries; a pair of order q contributes its
+// first rows(q) entries; eight loads in flight), back to physical units, into
+// (accumulate: added to) the basis' components of the local expansion.
+template <typename R, bool full>
+__global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p, bool accumulate,
+                                                 const R* __restrict__ out, const int32_t* __restrict__ roff,
+                                                 double* __restrict__ loc) {
     const int i = blockIdx.x;
-    const int nr = (p + 1) * (p + 1);
+    const int nr = d64_rows(p, full);
     const int q0 = t.far_off[i], q1 = t.far_off[i + 1];
+    if (accumulate && q0 == q1) return;
     const double ih = 1.0 / t.r[i];
     double* L = loc + (size_t)i * nT(p);
     for (int f = threadIdx.x; f < nr; f += blockDim.x) {
@@ -878,24 +896,25 @@ __global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p, const R
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int qq = t.far_ord ? min((int)t.far_ord[q + u], p) : p;
-                v[u] = f < (qq + 1) * (qq + 1) ? out[(size_t)roff[q + u] * kRowUnit + f] : (R)0;
+                v[u] = f < d64_rows(qq, full) ? out[(size_t)roff[q + u] * kRowUnit + f] : (R)0;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) acc.add(v[u]);
         }
         for (; q < q1; ++q) {
             const int qq = t.far_ord ? min((int)t.far_ord[q], p) : p;
-            if (f < (qq + 1) * (qq + 1)) acc.add(out[(size_t)roff[q] * kRowUnit + f]);
+            if (f < d64_rows(qq, full)) acc.add(out[(size_t)roff[q] * kRowUnit + f]);
         }
-        const int c = qcomp(f);
+        const int c = d64_comp(f, full);
         const int k = c >> 24;
         double s = ih;
         for (int e = 0; e < k; ++e) s *= ih;
-        L[pidx(c & 0xff, (c >> 8) & 0xff, (c >> 16) & 0xff)] = acc.value() * s;
+        double* o = L + (full ? f : pidx(c & 0xff, (c >> 8) & 0xff, (c >> 16) & 0xff));
+        *o = accumulate ? *o + acc.value() * s : acc.value() * s;
     }
 }
 
-// FP32 products on the CUDA cores instead of the tensor cores
+// Products on the CUDA cores instead of the tensor cores
 // (FMM_GB300_M2L_PRODUCT=cuda; read at every call).
 bool product_on_cuda_cores() {
     const char* e = std::getenv("FMM_GB300_M2L_PRODUCT");
@@ -907,23 +926,52 @@ bool product_on_cuda_cores() {
 // learned selector's mixed orders).
 constexpr int kOrderClass = 2;
 
-constexpr double kMinGroupPairs = 16.0;    // mean far pairs per displacement group for the grouped products
+// Mean far pairs per displacement group for the grouped products.  FP64: the
+// tensor-core product of one group costs about what the per-pair kernel takes
+// for one or two pairs (order 10: 33 ns against 44 ns a pair at the FP64 peak).
+constexpr double kMinGroupPairs = 16.0, kMinGroupPairs64 = 2.0;
+// Result rows of the full basis: above this the reference-mode M2L runs pair
+// by pair, which needs no rows.
+constexpr double kFullRowBytes = 64e9;
 constexpr double kOperatorBytes = 16e9;  // TF32 operator parts of one batch of groups
 
+// Split operators of the groups of one batch.
+int launch_operators(Workspace& ws, bool tc, bool full, int ldT, int ldr, const M2lBatch& b, int64_t base,
+                     cudaStream_t st) {
+    count_launches(1);
+    if (tc) {
+        k_group_operator<<<(unsigned)(b.g1 - b.g0), 256, 0, st>>>(ldT, ws.m2l_T.as<float>(), ws.m2l_gq.as<int32_t>(),
+                                                                  ws.m2l_gab.as<float2>(), ws.m2l_gopoff.as<int64_t>(),
+                                                                  b.g0, base, ws.m2l_gop.as<float>());
+    } else {
+        k_operator64<<<(unsigned)(b.g1 - b.g0), 256, sizeof(double) * ldT, st>>>(
+            full, ldT, ws.m2l_T.as<double>(), ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>(),
+            ws.m2l_gopoff.as<int64_t>(), b.g0, base, ldr, ws.m2l_gop.as<uint4>(), ws.m2l_gexp.as<int>());
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
 template <typename R, int CPT>
-int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
-    const int M = t.num_nodes, nr = (p + 1) * (p + 1), N = 2 * p, nTr = rbase(N + 1);
+int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, bool accumulate) {
+    const int M = t.num_nodes, nr = d64_rows(p, full), N = 2 * p, nTr = full ? nT(N) : rbase(N + 1);
     const bool tc = sizeof(R) == 4 && !product_on_cuda_cores();
-    const int cols = tc ? -1 : kTaskCols;  // -1: tensor-core tasks (256 pairs, one operator half)
+    const bool tc64 = sizeof(R) == 8 && (full || !product_on_cuda_cores());
+    const int cols = tc ? kTcTasks : (tc64 ? (full ? kD64FullTasks : kD64Tasks) : kTaskCols);
     const int64_t nf = t.nfar;
     const int ldw = wsc_ld<R>(nr);
     const int ldk = (nr + 15) / 16 * 16;
     const int ldT = nTr;
+    const int wchunks = d64_chunks(p, full);
     const int32_t* roff = nullptr;  // row of each far pair (target order), units of 32 entries
     if (nf > 0 && !ws.reuse_structure) {
         // structure: displacement groups, their tensors and operators, tasks
         // and result rows (geometry only; kept for replays)
         ws.m2l_pairwise = false;
+        if (full && (double)nf * row_len(p, true) * sizeof(R) > kFullRowBytes) {
+            ws.m2l_pairwise = true;
+            return FMM_ENOTSUP;
+        }
         FMM_TRY(ws.m2l_tgt.ensure(sizeof(int32_t) * nf));
         FMM_TRY(ws.m2l_keys.ensure(sizeof(uint64_t) * nf));
         FMM_TRY(ws.m2l_keys2.ensure(sizeof(uint64_t) * nf));
@@ -932,7 +980,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         FMM_TRY(ws.m2l_ukeys.ensure(sizeof(uint64_t) * nf));
         FMM_TRY(ws.m2l_cnt.ensure(sizeof(int32_t) * (nf + 1)));
         FMM_TRY(ws.m2l_gstart.ensure(sizeof(int32_t) * (nf + 1)));
-        FMM_TRY(ws.m2l_wsc.ensure(sizeof(R) * (size_t)M * ldw));
+        if (!tc64) FMM_TRY(ws.m2l_wsc.ensure(sizeof(R) * (size_t)M * ldw));
         FMM_TRY(ws.counters.ensure(sizeof(unsigned long long) * 32));
         int32_t* tgt = ws.m2l_tgt.as<int32_t>();
         count_launches(1);
@@ -940,13 +988,15 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         count_launches(1);
         // FP32 node data where the mixed path prepared it
         const float4* chi = (sizeof(R) == 4 && ws.f32node_ok) ? ws.f32node.as<float4>() : nullptr;
-        k_m2l_keys<<<grid_for(nf, 256), 256, 0, st>>>(nf, t, tgt, p, kOrderClass, chi, chi ? chi + M : nullptr,
+        const bool level = t.shift[0] != 0.0 || t.shift[1] != 0.0 || t.shift[2] != 0.0;
+        const int kbits = level ? kKeyBitsLevel : kKeyBits;
+        k_m2l_keys<<<grid_for(nf, 256), 256, 0, st>>>(nf, t, tgt, p, kOrderClass, level, chi, chi ? chi + M : nullptr,
                                                        ws.m2l_keys.as<uint64_t>(), ws.m2l_vals.as<int32_t>());
         // sort by key, run-length encode into groups
         int* d_nruns = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 14);
         size_t tb1 = 0, tb2 = 0, tb3 = 0;
         cub::DeviceRadixSort::SortPairs(nullptr, tb1, ws.m2l_keys.as<uint64_t>(), ws.m2l_keys2.as<uint64_t>(),
-                                        ws.m2l_vals.as<int32_t>(), ws.m2l_vals2.as<int32_t>(), (int)nf, 0, kKeyBits, st);
+                                        ws.m2l_vals.as<int32_t>(), ws.m2l_vals2.as<int32_t>(), (int)nf, 0, kbits, st);
         cub::DeviceRunLengthEncode::Encode(nullptr, tb2, ws.m2l_keys2.as<uint64_t>(), ws.m2l_ukeys.as<uint64_t>(),
                                            ws.m2l_cnt.as<int32_t>(), d_nruns, (int)nf, st);
         cub::DeviceScan::ExclusiveSum(nullptr, tb3, ws.m2l_cnt.as<int32_t>(), ws.m2l_gstart.as<int32_t>(),
@@ -954,7 +1004,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         FMM_TRY(ws.cub_tmp.ensure(std::max(tb1, std::max(tb2, tb3))));
         FMM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.p, tb1, ws.m2l_keys.as<uint64_t>(),
                                                      ws.m2l_keys2.as<uint64_t>(), ws.m2l_vals.as<int32_t>(),
-                                                     ws.m2l_vals2.as<int32_t>(), (int)nf, 0, kKeyBits, st));
+                                                     ws.m2l_vals2.as<int32_t>(), (int)nf, 0, kbits, st));
         FMM_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(ws.cub_tmp.p, tb2, ws.m2l_keys2.as<uint64_t>(),
                                                         ws.m2l_ukeys.as<uint64_t>(), ws.m2l_cnt.as<int32_t>(),
                                                         d_nruns, (int)nf, st));
@@ -965,7 +1015,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         // displacement groups of a few pairs each (irregular trees, mixed
         // orders) leave the products' columns empty and multiply the
         // per-group operators: the per-pair kernel is then the faster one
-        if ((double)nf < kMinGroupPairs * (double)ng) {
+        if ((double)nf < (tc64 ? kMinGroupPairs64 : kMinGroupPairs) * (double)ng) {
             ws.m2l_pairwise = true;
             return FMM_ENOTSUP;
         }
@@ -979,7 +1029,9 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         FMM_TRY(ws.m2l_T.ensure(sizeof(R) * (size_t)ng * ldT));
         FMM_TRY(ws.m2l_gq.ensure(sizeof(int32_t) * ng));
         FMM_TRY(ws.m2l_gab.ensure(sizeof(float2) * ng));
-        {
+        if (full) {
+            FMM_TRY(launch_group_tensor_ref(ws, t, ng, tgt, p, ldT, st));
+        } else {
             const int wpb = 4;
             const size_t sm = sizeof(double) * (nTr + (size_t)wpb * (2 * nTr + N + 1));
             if (sm > 48 * 1024)
@@ -1008,14 +1060,14 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         FMM_TRY(ws.m2l_rowbase.ensure(sizeof(int32_t) * (ng + 1)));
         int32_t* rowbase = ws.m2l_rowbase.as<int32_t>();
         count_launches(1);
-        k_row_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
+        k_row_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
                                                             rowbase);
         size_t tb7 = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tb7, rowbase, rowbase, ng + 1, st);
         FMM_TRY(ws.cub_tmp.ensure(tb7));
         FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws.cub_tmp.p, tb7, rowbase, rowbase, ng + 1, st));
         count_launches(1);
-        k_row_offsets<<<grid_for(ng, 8), 256, 0, st>>>(ng, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
+        k_row_offsets<<<grid_for(ng, 8), 256, 0, st>>>(ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
                                                         rowbase, ws.m2l_vals2.as<int32_t>(),
                                                         reinterpret_cast<int32_t*>(ws.m2l_keys.p));
         int hcnt[2] = {0, 0};  // tasks, rows (units of 32 entries)
@@ -1028,8 +1080,11 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         count_launches(1);
         k_fill_tasks<<<grid_for(ng, 256), 256, 0, st>>>(ng, cols, ws.m2l_gq.as<int32_t>(), ws.m2l_gstart.as<int32_t>(),
                                                         ws.m2l_toff.as<int32_t>(), ws.m2l_tasks.as<int2>());
-        if (tc) {
-            FMM_TRY(ws.m2l_wsplit.ensure(sizeof(float) * 2 * (size_t)M * ldk));
+        if (tc || tc64) {
+            // tensor-core operands: per node the weights, per group the operator
+            FMM_TRY(ws.m2l_wsplit.ensure(tc ? sizeof(float) * 2 * (size_t)M * ldk
+                                            : (size_t)M * (wchunks * kDig * kD64K * 2 + sizeof(int))));
+            if (tc64) FMM_TRY(ws.m2l_gexp.ensure(sizeof(int) * (size_t)ng * nr));
             // source node per sorted pair (into the free unsorted-values buffer)
             count_launches(1);
             k_pair_sources<<<grid_for(nf, 256), 256, 0, st>>>(nf, ws.m2l_vals2.as<int32_t>(), t.far_src,
@@ -1037,13 +1092,16 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
             FMM_TRY(ws.m2l_gopoff.ensure(sizeof(int64_t) * (ng + 1)));
             int64_t* goff = ws.m2l_gopoff.as<int64_t>();
             count_launches(1);
-            k_gop_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, ws.m2l_gq.as<int32_t>(), goff);
+            if (tc)
+                k_gop_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, ws.m2l_gq.as<int32_t>(), goff);
+            else
+                k_op64_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, full, ws.m2l_gq.as<int32_t>(), goff);
             size_t tb6 = 0;
             cub::DeviceScan::ExclusiveSum(nullptr, tb6, goff, goff, ng + 1, st);
             FMM_TRY(ws.cub_tmp.ensure(tb6));
             FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws.cub_tmp.p, tb6, goff, goff, ng + 1, st));
-            // TF32 parts of the operators (per group, at each group's order),
-            // in batches of consecutive groups of at most kOperatorBytes: one
+            // split operators (per group, at each group's order; offsets in
+            // floats, FP64: in 16-byte units), in batches of consecutive groups of at most kOperatorBytes: one
             // batch is built here once; several are built, each before the
             // product over its tasks, at every evaluation
             std::vector<int64_t> hgoff((size_t)ng + 1);
@@ -1052,7 +1110,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
             FMM_CUDA_TRY(cudaMemcpyAsync(htoff.data(), ws.m2l_toff.as<int32_t>(), sizeof(int32_t) * (ng + 1),
                                          cudaMemcpyDeviceToHost, st));
             FMM_CUDA_TRY(cudaStreamSynchronize(st));
-            const int64_t cap = (int64_t)(kOperatorBytes / sizeof(float));
+            const size_t unit = tc ? sizeof(float) : sizeof(uint4);
+            const int64_t cap = (int64_t)(kOperatorBytes / unit);
             ws.m2l_batches.clear();
             int64_t biggest = 0;
             for (int g0 = 0; g0 < ng;) {
@@ -1062,13 +1121,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
                 biggest = std::max(biggest, hgoff[g1] - hgoff[g0]);
                 g0 = g1;
             }
-            FMM_TRY(ws.m2l_gop.ensure(sizeof(float) * std::max<int64_t>(1, biggest)));
-            if (ws.m2l_batches.size() == 1) {
-                count_launches(1);
-                k_group_operator<<<(unsigned)ng, 256, 0, st>>>(ldT, reinterpret_cast<const float*>(ws.m2l_T.p),
-                                                               ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>(), goff,
-                                                               0, 0, ws.m2l_gop.as<float>());
-            }
+            FMM_TRY(ws.m2l_gop.ensure(unit * std::max<int64_t>(1, biggest)));
+            if (ws.m2l_batches.size() == 1) FMM_TRY(launch_operators(ws, tc, full, ldT, nr, ws.m2l_batches[0], 0, st));
         }
         ws.m2l_ng = ng;
         ws.m2l_ntasks = ntasks;
@@ -1078,16 +1132,29 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
         const int ntasks = ws.m2l_ntasks;
         const int32_t* rowbase = ws.m2l_rowbase.as<int32_t>();
         roff = reinterpret_cast<const int32_t*>(ws.m2l_keys.p);
-        count_launches(1);
-        k_scale_weights<R><<<grid_for(M, 4), 128, 0, st>>>(M, nr, ldw, ws.wred.as<double>(), t.r, ws.m2l_wsc.as<R>());
-        int* d_err = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 13);
-        if (tc) {
-            // TF32 parts of the weights (per node)
+        if (!tc64) {
             count_launches(1);
-            k_split_weights<<<grid_for((int64_t)M * ldk, 256), 256, 0, st>>>(
-                (int64_t)M * ldk, nr, ldw, ldk, reinterpret_cast<const float*>(ws.m2l_wsc.p), ws.m2l_wsplit.as<float>());
-            FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)TcSmem::bytes));
+            k_scale_weights<R><<<grid_for(M, 4), 128, 0, st>>>(M, nr, ldw, ws.wred.as<double>(), t.r,
+                                                               ws.m2l_wsc.as<R>());
+        }
+        int* d_err = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 13);
+        if (tc || tc64) {
+            // TF32 parts or digits of the weights (per node)
+            int* wexp = nullptr;
+            count_launches(1);
+            if (tc) {
+                k_split_weights<<<grid_for((int64_t)M * ldk, 256), 256, 0, st>>>(
+                    (int64_t)M * ldk, nr, ldw, ldk, reinterpret_cast<const float*>(ws.m2l_wsc.p),
+                    ws.m2l_wsplit.as<float>());
+                FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)TcSmem::bytes));
+            } else {
+                wexp = reinterpret_cast<int*>(ws.m2l_wsplit.as<uint4>() + (size_t)M * wchunks * kDig * 2);
+                k_weights64<<<grid_for(M, 4), 128, 0, st>>>(M, p, full, full ? ws.mom.as<double>() : ws.wred.as<double>(),
+                                                            t.r, ws.m2l_wsplit.as<uint4>(), wexp);
+                FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)D64Smem::bytes));
+            }
             int dev = 0, sms = 0;
             FMM_CUDA_TRY(cudaGetDevice(&dev));
             FMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1098,21 +1165,24 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
             }
             const bool many = ws.m2l_batches.size() > 1;
             for (const M2lBatch& b : ws.m2l_batches) {
-                if (many) {
-                    count_launches(1);
-                    k_group_operator<<<(unsigned)(b.g1 - b.g0), 256, 0, st>>>(
-                        ldT, reinterpret_cast<const float*>(ws.m2l_T.p), ws.m2l_gq.as<int32_t>(),
-                        ws.m2l_gab.as<float2>(), ws.m2l_gopoff.as<int64_t>(), b.g0, b.gop_base, ws.m2l_gop.as<float>());
-                }
+                if (many) FMM_TRY(launch_operators(ws, tc, full, ldT, nr, b, b.gop_base, st));
                 const int nt = b.t1 - b.t0;
                 if (nt <= 0) continue;
                 const int grid = std::max(1, std::min(nt, sms));  // one block per SM (all tensor memory)
                 count_launches(1);
-                k_m2l_tc<<<(unsigned)grid, kTcThreads, TcSmem::bytes, st>>>(
-                    ws.m2l_tasks.as<int2>() + b.t0, nt, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
-                    ws.m2l_gopoff.as<int64_t>(), many ? b.gop_base : 0, ws.m2l_gop.as<float>(),
-                    ws.m2l_vals.as<int32_t>(), ws.m2l_wsplit.as<float>(), ldk, reinterpret_cast<float*>(ws.m2l_out.p),
-                    rowbase, d_err);
+                if (tc)
+                    k_m2l_tc<<<(unsigned)grid, kTcThreads, TcSmem::bytes, st>>>(
+                        ws.m2l_tasks.as<int2>() + b.t0, nt, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
+                        ws.m2l_gopoff.as<int64_t>(), many ? b.gop_base : 0, ws.m2l_gop.as<float>(),
+                        ws.m2l_vals.as<int32_t>(), ws.m2l_wsplit.as<float>(), ldk,
+                        reinterpret_cast<float*>(ws.m2l_out.p), rowbase, d_err);
+                else
+                    k_m2l_tc64<<<(unsigned)grid, kD64Threads, D64Smem::bytes, st>>>(
+                        ws.m2l_tasks.as<int2>() + b.t0, nt, full, ws.m2l_gstart.as<int32_t>(),
+                        ws.m2l_gq.as<int32_t>(), ws.m2l_gopoff.as<int64_t>(), many ? b.gop_base : 0,
+                        ws.m2l_gop.as<uint4>(), nr, ws.m2l_gexp.as<int>(), ws.m2l_vals.as<int32_t>(),
+                        ws.m2l_wsplit.as<uint4>(), wchunks, wexp, reinterpret_cast<double*>(ws.m2l_out.p), rowbase,
+                        kRowUnit, d_err);
             }
             if (ws.product_timed) cudaEventRecord(ws.ev[9], st);
             // the product's error flag is read with the call's final copies
@@ -1133,24 +1203,33 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st) {
             if (ws.product_timed) cudaEventRecord(ws.ev[9], st);
         }
     }
+    if (nf == 0 && accumulate) return FMM_OK;
     count_launches(1);
     if (nf == 0) FMM_TRY(ws.m2l_out.ensure(sizeof(R) * kRowUnit));
-    // one output per thread: (p+1)^2 rounded up to whole warps (192 at p = 12)
-    k_m2l_sum<R><<<(unsigned)M, (unsigned)std::min(256, (nr + 31) / 32 * 32), 0, st>>>(t, p, ws.m2l_out.as<R>(), roff,
-                                                                                     ws.loc.as<double>());
+    // one output per thread: the basis rounded up to whole warps (192 at p = 12)
+    const unsigned sum_threads = (unsigned)std::min(256, (nr + 31) / 32 * 32);
+    if (sizeof(R) == 8 && full)
+        k_m2l_sum<double, true><<<(unsigned)M, sum_threads, 0, st>>>(t, p, accumulate, ws.m2l_out.as<double>(), roff,
+                                                                     ws.loc.as<double>());
+    else
+        k_m2l_sum<R, false><<<(unsigned)M, sum_threads, 0, st>>>(t, p, accumulate, ws.m2l_out.as<R>(), roff,
+                                                                 ws.loc.as<double>());
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
 
 }  // namespace
 
-// Grouped reduced-basis M2L into the reduced components of ws.loc (the
-// weights ws.wred must be current).  FP32 products for `fp32`, else FP64;
-// returns FMM_ENOTSUP where the FP64 operator does not fit shared memory.
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st) {
-    if (fp32) return grouped<float, 8>(ws, t, p, st);
-    if (GemmSmem<double, 4>(p).bytes > 227 * 1024) return FMM_ENOTSUP;
-    return grouped<double, 4>(ws, t, p, st);
+// Grouped M2L into (accumulate: added to) the local expansions ws.loc: the
+// reduced components from the weights ws.wred (which must be current), in FP32
+// products for `fp32`, else FP64; or (full) all Cartesian components in FP64
+// with the reference's wrapped tensors.  Returns FMM_ENOTSUP where the pairs
+// should be evaluated one by one.
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full,
+                       bool accumulate) {
+    if (fp32) return grouped<float, 8>(ws, t, p, st, false, accumulate);
+    if (!full && product_on_cuda_cores() && GemmSmem<double, 4>(p).bytes > 227 * 1024) return FMM_ENOTSUP;
+    return grouped<double, 4>(ws, t, p, st, full, accumulate);
 }
 
 }  // namespace fmm
