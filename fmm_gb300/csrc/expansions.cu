@@ -370,63 +370,74 @@ int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStre
 // (M'_t = M_t / t!): S_0 is the root's with its charge removed (the
 // reference forces charge neutrality), and S_l = S_(l-1) plus the 26 copies
 // of S_(l-1) shifted by H (3^(l-1) a), a != 0, in the reference's order of a.
-// One block; S_0 .. S_(L-1) are written to S (L x nq).
-__global__ void k_lattice_moments(int p, int L, const double* __restrict__ root_mom, const Box9 H,
-                                  double* __restrict__ S) {
+// One block with a warp per copy (each copy's moments, then per component the
+// sum over the copies in order): the levels are a serial chain, and so were the
+// copies when one after another went through the block (14 us each, 18.5 ms for
+// 50 levels at p = 5).
+//
+// The levels run in batches [l0, l1): the sum stops after the first level whose
+// contribution is below the threshold (a cubic cell's after about six), and
+// the kernels of the later batches return at once when *stop is set.
+constexpr int kLatticeCopies = 26;
+
+__global__ void __launch_bounds__(32 * kLatticeCopies) k_lattice_moments(int p, int l0, int l1,
+                                                                         const int* __restrict__ stop,
+                                                                         const double* __restrict__ root_mom,
+                                                                         const Box9 H, double* __restrict__ S) {
     extern __shared__ double sh[];
+    if (*stop) return;
     const int nq = nT(p), P1 = p + 1;
     double* src = sh;
-    double* dst = src + nq;
-    double* e = dst + nq;  // scaled powers d^u / u! per axis, 3 x (p + 1)
+    double* part = src + nq;                  // copies x nq
+    double* e = part + kLatticeCopies * nq;   // scaled powers d^u / u! per copy and axis
     for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-        const double v = q == 0 ? 0.0 : root_mom[q];
+        const double v = l0 > 0 ? S[(size_t)(l0 - 1) * nq + q] : (q == 0 ? 0.0 : root_mom[q]);
         src[q] = v;
-        S[q] = v;
+        if (l0 == 0) S[q] = v;
     }
-    __syncthreads();
     double three_l = 1.0;
-    for (int l = 1; l < L; ++l) {
+    for (int l = 1; l < l0; ++l) three_l *= 3.0;
+    for (int l = max(l0, 1); l < l1; ++l) {
         three_l *= 3.0;  // 3^l, exact
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) dst[q] = src[q];
-        __syncthreads();
-        for (int ai = -1; ai <= 1; ++ai)
-            for (int aj = -1; aj <= 1; ++aj)
-                for (int ak = -1; ak <= 1; ++ak) {
-                    if (ai == 0 && aj == 0 && ak == 0) continue;
-                    if (threadIdx.x < 3) {
-                        const int ax = threadIdx.x;
-                        // d_aijk = matmul(H, a 3^l) / 3 (fmm.F90:920-923)
-                        const double v = __dadd_rn(__dadd_rn(__dmul_rn(H.h[ax], ai * three_l),
-                                                             __dmul_rn(H.h[3 + ax], aj * three_l)),
-                                                   __dmul_rn(H.h[6 + ax], ak * three_l));
-                        const double d = __ddiv_rn(v, 3.0);
-                        double pw = 1.0, fact = 1.0;
-                        for (int u = 0; u <= p; ++u) {
-                            e[ax * P1 + u] = pw / fact;
-                            pw *= d;
-                            fact *= (double)(u + 1);
-                        }
-                    }
-                    __syncthreads();
-                    for (int t = threadIdx.x; t < nq; t += blockDim.x) {
-                        const int tx = comp_x(t), ty = comp_y(t), tz = comp_z(t), to = tx + ty + tz;
-                        double acc = 0.0;
-                        for (int so = 0; so <= to; ++so)
-                            for (int sx = min(so, tx); sx >= 0; --sx)
-                                for (int sy = min(so - sx, ty); sy >= 0; --sy) {
-                                    const int sz = so - sx - sy;
-                                    if (sz > tz) continue;
-                                    acc += e[tx - sx] * e[P1 + ty - sy] * e[2 * P1 + tz - sz] * src[pidx(sx, sy, sz)];
-                                }
-                        dst[t] += acc;
-                    }
-                    __syncthreads();
-                }
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            src[q] = dst[q];
-            S[(size_t)l * nq + q] = dst[q];
+        if (threadIdx.x < 3 * kLatticeCopies) {
+            const int ax = threadIdx.x % 3;
+            int k = threadIdx.x / 3;
+            if (k >= 13) ++k;  // skip a = 0 (index 13 of the 27 in i,j,k order)
+            const int ai = k / 9 - 1, aj = (k / 3) % 3 - 1, ak = k % 3 - 1;
+            // d_aijk = matmul(H, a 3^l) / 3 (fmm.F90:920-923)
+            const double v = __dadd_rn(__dadd_rn(__dmul_rn(H.h[ax], ai * three_l), __dmul_rn(H.h[3 + ax], aj * three_l)),
+                                       __dmul_rn(H.h[6 + ax], ak * three_l));
+            const double d = __ddiv_rn(v, 3.0);
+            double pw = 1.0, fact = 1.0;
+            for (int u = 0; u <= p; ++u) {
+                e[threadIdx.x * P1 + u] = pw / fact;
+                pw *= d;
+                fact *= (double)(u + 1);
+            }
         }
         __syncthreads();
+        const int c = threadIdx.x >> 5;
+        const double* ec = e + 3 * c * P1;
+        for (int t = threadIdx.x & 31; t < nq; t += 32) {
+            const int tx = comp_x(t), ty = comp_y(t), tz = comp_z(t), to = tx + ty + tz;
+            double acc = 0.0;
+            for (int so = 0; so <= to; ++so)
+                for (int sx = min(so, tx); sx >= 0; --sx)
+                    for (int sy = min(so - sx, ty); sy >= 0; --sy) {
+                        const int sz = so - sx - sy;
+                        if (sz > tz) continue;
+                        acc += ec[tx - sx] * ec[P1 + ty - sy] * ec[2 * P1 + tz - sz] * src[pidx(sx, sy, sz)];
+                    }
+            part[c * nq + t] = acc;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+            double v = src[q];
+            for (int k = 0; k < kLatticeCopies; ++k) v += part[k * nq + q];
+            src[q] = v;
+            S[(size_t)l * nq + q] = v;
+        }
+        // (the next level's powers touch neither src nor part)
     }
 }
 
@@ -439,12 +450,14 @@ __global__ void k_lattice_moments(int p, int L, const double* __restrict__ root_
 // results rescaled by the matching powers of two, so the recursion's r^-(4p+1)
 // does not underflow at the far levels; ref mode follows the reference's
 // closed form unscaled.
-constexpr int kLatticeSlices = 16;
+constexpr int kLatticeSlices = 16;  // (the order of the copies' sum)
 
-__global__ void k_lattice_m2l(int p, int L, int ref, const double* __restrict__ S, const Box9 H,
+__global__ void k_lattice_m2l(int p, int l0, const int* __restrict__ stop, int ref, const double* __restrict__ S,
+                              const Box9 H,
                               const int32_t* __restrict__ term_off, const uchar4* __restrict__ term_abc,
                               const double* __restrict__ term_c, double* __restrict__ C) {
     extern __shared__ double smem[];
+    if (*stop) return;
     const int nq = nT(p), N = 2 * p, nqT = nT(N);
     int* comp = reinterpret_cast<int*>(smem);
     double* base = smem + (nqT + 1) / 2 + 1;
@@ -459,7 +472,7 @@ __global__ void k_lattice_m2l(int p, int L, int ref, const double* __restrict__ 
     double* zp = yp + (N + 1);
     double* ir = zp + (N + 1);
     fill_comp(comp, nqT);
-    const int l = blockIdx.x + 1, slice = blockIdx.y;
+    const int l = l0 + blockIdx.x + 1, slice = blockIdx.y;
     const int ksc = ref ? 0 : (int)floor(l * 1.5849625007211563);  // log2(3)
     const double* Sl = S + (size_t)(l - 1) * nq;
     for (int s = lane; s < nq; s += 32) {
@@ -521,13 +534,14 @@ __global__ void k_lattice_m2l(int p, int L, int ref, const double* __restrict__ 
 // stops after the first level whose contribution (without its first
 // component) has a norm below tol, as the reference does (fmm.F90:944-950);
 // levels_used receives the number of levels added.
-__global__ void k_lattice_apply(int nq, int L, const double* __restrict__ C, double* __restrict__ loc_root,
-                                double tol, int* levels_used) {
+__global__ void k_lattice_apply(int nq, int l0, int l1, const double* __restrict__ C, double* __restrict__ loc_root,
+                                double tol, int* levels_used, int* stop_flag) {
     __shared__ double lev[kMaxNPL * 32];
     __shared__ int stop;
     const int lane = threadIdx.x;
-    int used = 0;
-    for (int l = 0; l < L; ++l) {
+    if (*stop_flag) return;
+    int used = l0;
+    for (int l = l0; l < l1; ++l) {
         for (int f = lane; f < nq; f += 32) {
             double v = 0.0;
             for (int sl = 0; sl < kLatticeSlices; ++sl) v += C[((size_t)l * kLatticeSlices + sl) * nq + f];
@@ -558,7 +572,10 @@ __global__ void k_lattice_apply(int nq, int L, const double* __restrict__ C, dou
         ++used;
         if (stop) break;
     }
-    if (lane == 0) *levels_used = used;
+    if (lane == 0) {
+        *levels_used = used;
+        *stop_flag = stop;
+    }
 }
 
 // Surface term of the periodic sum (src/fmm.F90:954-979), on the field in
@@ -599,28 +616,30 @@ int launch_periodic_lattice(Workspace& ws, const TreeDev& t, int p, int f, const
     const int nq = nT(p), N = 2 * p, nqT = nT(N);
     const int ref = md.coef_mode == 0 ? 1 : 0;
     if (ref) FMM_TRY(ensure_ref_terms(ws, N, st));
-    FMM_TRY(ws.lattice.ensure(sizeof(double) * ((size_t)L * nq + (size_t)L * kLatticeSlices * nq)));
+    FMM_TRY(ws.lattice.ensure(sizeof(double) * ((size_t)L * nq + (size_t)L * kLatticeSlices * nq) + sizeof(int)));
     double* S = ws.lattice.as<double>();
     double* C = S + (size_t)L * nq;
+    int* stop = reinterpret_cast<int*>(C + (size_t)L * kLatticeSlices * nq);
+    FMM_CUDA_TRY(cudaMemsetAsync(stop, 0, sizeof(int), st));
     const double* root_mom = ws.mom.as<double>();  // the root is node 0
-    {
-        const size_t sm = sizeof(double) * (2 * nq + 3 * (p + 1));
-        FMM_TRY(set_smem((const void*)k_lattice_moments, sm));
-        count_launches(1);
-        k_lattice_moments<<<1, 256, sm, st>>>(p, L, root_mom, H, S);
+    const size_t sm_mom = sizeof(double) * ((size_t)(1 + kLatticeCopies) * nq + 3 * kLatticeCopies * (p + 1));
+    FMM_TRY(set_smem((const void*)k_lattice_moments, sm_mom));
+    const int per_warp = 2 * nqT + nq + 5 * (N + 1);
+    const int nw = (int)std::max<size_t>(1, std::min<size_t>(4, (100 * 1024) / (sizeof(double) * (per_warp + nq))));
+    const size_t sm = comp_bytes(nqT) + sizeof(double) * nw * (per_warp + nq);
+    FMM_TRY(set_smem((const void*)k_lattice_m2l, sm));
+    // batches of levels: cubic cells stop within the first, skewed ones run all
+    constexpr int kFirst = 8;
+    for (int l0 = 0; l0 < L; l0 = l0 == 0 ? kFirst : L) {
+        const int l1 = l0 == 0 ? kFirst : L;
+        count_launches(3);
+        k_lattice_moments<<<1, 32 * kLatticeCopies, sm_mom, st>>>(p, l0, l1, stop, root_mom, H, S);
+        k_lattice_m2l<<<dim3(l1 - l0, kLatticeSlices), 32 * nw, sm, st>>>(p, l0, stop, ref, S, H,
+                                                                           ws.term_off.as<int32_t>(),
+                                                                           ws.term_abc.as<uchar4>(),
+                                                                           ws.term_c.as<double>(), C);
+        k_lattice_apply<<<1, 32, 0, st>>>(nq, l0, l1, C, ws.loc.as<double>(), 1.0e-8, d_levels, stop);
     }
-    {
-        const int per_warp = 2 * nqT + nq + 5 * (N + 1);
-        int nw = (int)std::max<size_t>(1, std::min<size_t>(4, (100 * 1024) / (sizeof(double) * (per_warp + nq))));
-        const size_t sm = comp_bytes(nqT) + sizeof(double) * nw * (per_warp + nq);
-        FMM_TRY(set_smem((const void*)k_lattice_m2l, sm));
-        count_launches(1);
-        k_lattice_m2l<<<dim3(L, kLatticeSlices), 32 * nw, sm, st>>>(p, L, ref, S, H, ws.term_off.as<int32_t>(),
-                                                                     ws.term_abc.as<uchar4>(),
-                                                                     ws.term_c.as<double>(), C);
-    }
-    count_launches(1);
-    k_lattice_apply<<<1, 32, 0, st>>>(nq, L, C, ws.loc.as<double>(), 1.0e-8, d_levels);
     count_launches(1);
     k_dipole_fix<<<grid_for(t.n, 256), 256, 0, st>>>(t.n, f, ws.sx.as<double>(), ws.sy.as<double>(),
                                                       ws.sz.as<double>(), root_mom, H, ref, d_fs);
