@@ -47,7 +47,7 @@ void Workspace::release_buffers(bool keep_selector) {
                      &sz,        &smc,       &sd,          &fsorted,    &mom,        &loc,        &partial,
                      &term_off,  &term_abc,  &term_c, &f32buf, &wred, &far_ord, &sel_norms, &sel_params, &sel_scratch, &sysbuf,
                      &m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
-                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part};
+                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
     for (DevBuf* b : all)
         if (!(keep_selector && b == &sel_params)) b->release();
     if (!keep_selector) sel_ready = false;
@@ -360,52 +360,34 @@ double sampled_rms(const std::vector<double>& F, const std::vector<double>& R, i
     return std::sqrt(acc / ntgt);
 }
 
-// Periodic boxes (box != null): the 27 images of src/fmm.F90:156-175 in the
-// reference's order (a_x outer, a_z inner), each with its own interaction
-// lists built from (root, root + H a) (fmm.F90:337-343), its near field with
-// the exclusions applied only in the central image (fmm.F90:660-736) and its
-// M2L (fmm.F90:861-878); then the lattice sum beyond the images and the
-// surface term (fmm.F90:884-979), before L2L and L2P.  FP64 and the fixed
+// Periodic boxes (box != null): the 27 images of src/fmm.F90:156-175 as
+// displaced copies of the tree's nodes (build_images), so that one list build
+// (from (root, root + H a) for every a, fmm.F90:337-343), one near field (with
+// the exclusions applied only in the central image, fmm.F90:660-736) and one
+// M2L (fmm.F90:861-878) cover them; then the lattice sum beyond the images and
+// the surface term (fmm.F90:884-979), before L2L and L2P.  FP64 and the fixed
 // acceptance rule only.
 int run_periodic(Workspace& ws, const Particles& P, int p, int f, const Modes& md, const TreeParams& tpl, TreeDev& t,
                  const Box9& box, cudaStream_t st, int* levels, unsigned long long* d_hist) {
-    const int64_t n = P.n;
-    const int nf = nT(f), nq = nT(p);
-    FMM_TRY(ws.fsorted.ensure(sizeof(double) * (size_t)n * nf));
-    FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nq));
-    FMM_CUDA_TRY(cudaMemsetAsync(ws.fsorted.p, 0, sizeof(double) * (size_t)n * nf, st));
-    FMM_CUDA_TRY(cudaMemsetAsync(ws.loc.p, 0, sizeof(double) * (size_t)t.num_nodes * nq, st));
-    int64_t nfar = 0, nnear = 0, npp = 0;
-    for (int ai = -1; ai <= 1; ++ai)
-        for (int aj = -1; aj <= 1; ++aj)
-            for (int ak = -1; ak <= 1; ++ak) {
-                // displacement = matmul(box_matrix, a) (fmm.F90:355, 662)
-                for (int c = 0; c < 3; ++c)
-                    t.shift[c] = (box.h[c] * ai + box.h[3 + c] * aj) + box.h[6 + c] * ak;
-                t.central = (ai == 0 && aj == 0 && ak == 0) ? 1 : 0;
-                FMM_TRY(build_lists(ws, t, tpl, st));
-                if (t.nfar > 0 && t.far_ord) {  // far pairs per order, summed over the images
-                    count_launches(1);
-                    k_order_hist<<<(unsigned)std::min<int64_t>(1024, (t.nfar + 255) / 256), 256, 0, st>>>(
-                        t.nfar, t.far_ord, d_hist);
-                }
-                FMM_TRY(launch_p2p_f64(ws, P, t, f, md, st, true));
-                if (t.central) FMM_TRY(launch_excl_correction(ws, P, &t, f, md, ws.fsorted.as<double>(), st));
-                FMM_TRY(launch_m2l(ws, t, p, md, st, true));
-                nfar += t.nfar;
-                nnear += t.nnear;
-                npp += t.near_particle_pairs;
-            }
-    t.shift[0] = t.shift[1] = t.shift[2] = 0.0;
-    t.central = 1;
+    TreeDev ti;
+    FMM_TRY(build_images(ws, t, box, &ti, st));
+    FMM_TRY(build_lists(ws, ti, tpl, st));
+    if (ti.nfar > 0 && ti.far_ord) {  // far pairs per order
+        count_launches(1);
+        k_order_hist<<<(unsigned)std::min<int64_t>(1024, (ti.nfar + 255) / 256), 256, 0, st>>>(ti.nfar, ti.far_ord,
+                                                                                               d_hist);
+    }
+    FMM_TRY(launch_p2p_f64(ws, P, ti, f, md, st));
+    FMM_TRY(launch_excl_correction(ws, P, &ti, f, md, ws.fsorted.as<double>(), st));
+    FMM_TRY(launch_m2l(ws, ti, p, md, st));
     int* d_levels = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 15);
     FMM_TRY(launch_periodic_lattice(ws, t, p, f, md, box, ws.fsorted.as<double>(), d_levels, st));
     FMM_TRY(launch_l2l_l2p(ws, P, t, p, f, false, st));
     FMM_CUDA_TRY(cudaMemcpyAsync(levels, d_levels, sizeof(int), cudaMemcpyDeviceToHost, st));
     FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    t.nfar = nfar;
-    t.nnear = nnear;
-    t.near_particle_pairs = npp;
+    t.nfar = ti.nfar;
+    t.nnear = ti.nnear;
+    t.near_particle_pairs = ti.near_particle_pairs;
     return FMM_OK;
 }
 
@@ -563,8 +545,7 @@ int run_fmm(Workspace& ws, const Particles& P, double theta, int ncrit, int p, i
     cudaEventRecord(ws.ev[6], st);
     // far pairs per expansion order (outside the timed phases)
     unsigned long long hist[16] = {0};
-    // (periodic boxes: summed image by image; t.nfar is then the total over
-    // the images while t.far_ord holds only the last image's pairs)
+    // (periodic boxes: counted with the images' lists)
     if (!box && t.nfar > 0 && t.far_ord) {
         count_launches(1);
         k_order_hist<<<(unsigned)std::min<int64_t>(1024, (t.nfar + 255) / 256), 256, 0, st>>>(t.nfar, t.far_ord,

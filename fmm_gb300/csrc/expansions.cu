@@ -133,7 +133,7 @@ __device__ double* warp_tensor(double X, double Y, double Z, int N, int ref, con
 
 __global__ void k_m2l_f64(const TreeDev t, const double* __restrict__ mom, double* __restrict__ loc, int p, int ref,
                           const int32_t* __restrict__ term_off, const uchar4* __restrict__ term_abc,
-                          const double* __restrict__ term_c, int accumulate) {
+                          const double* __restrict__ term_c) {
     extern __shared__ double smem[];
     const int nq = nT(p), N = 2 * p, nqT = nT(N);
     int* comp = reinterpret_cast<int*>(smem);
@@ -161,12 +161,11 @@ __global__ void k_m2l_f64(const TreeDev t, const double* __restrict__ mom, doubl
     for (int r = 0; r < kMaxNPL; ++r) acc[r] = 0.0;
     for (int q = q0; q < q1; ++q) {
         const int j = t.far_src[q];
-        // the source cell of a periodic image is displaced by t.shift (0 otherwise)
-        const double X = __dsub_rn(cxi, __dadd_rn(t.cx[j], t.shift[0]));
-        const double Y = __dsub_rn(cyi, __dadd_rn(t.cy[j], t.shift[1]));
-        const double Z = __dsub_rn(czi, __dadd_rn(t.cz[j], t.shift[2]));
+        const double X = __dsub_rn(cxi, t.cx[j]);
+        const double Y = __dsub_rn(cyi, t.cy[j]);
+        const double Z = __dsub_rn(czi, t.cz[j]);
         for (int s = lane; s < nq; s += 32) {
-            const double v = mom[(size_t)j * nq + s];
+            const double v = mom[(size_t)src_node(t, j) * nq + s];
             ms[s] = ((order_of(s) + 1) % 2) ? -v : v;  // (-1)^(|s|+1) M'_s
         }
         double* T = warp_tensor(X, Y, Z, N, ref, comp, TA, TB, gsh, yp, zp, ir, term_off, term_abc, term_c, lane);
@@ -188,10 +187,7 @@ __global__ void k_m2l_f64(const TreeDev t, const double* __restrict__ mom, doubl
 #pragma unroll
     for (int r = 0; r < kMaxNPL; ++r) {
         const int fq = lane + 32 * r;
-        if (fq < nq) {
-            double* L = loc + (size_t)i * nq + fq;
-            *L = accumulate ? *L + acc[r] : acc[r];
-        }
+        if (fq < nq) loc[(size_t)i * nq + fq] = acc[r];
     }
 }
 
@@ -303,9 +299,7 @@ __global__ void k_group_tensor_ref(int ng, const int32_t* __restrict__ gstart, c
     const int pos0 = svals[gstart[g]];
     const int i = tgt[pos0], j = t.far_src[pos0];
     const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
-    const double X = __dsub_rn(t.cx[i], __dadd_rn(t.cx[j], t.shift[0])) / hc;
-    const double Y = __dsub_rn(t.cy[i], __dadd_rn(t.cy[j], t.shift[1])) / hc;
-    const double Z = __dsub_rn(t.cz[i], __dadd_rn(t.cz[j], t.shift[2])) / hc;
+    const double X = (t.cx[i] - t.cx[j]) / hc, Y = (t.cy[i] - t.cy[j]) / hc, Z = (t.cz[i] - t.cz[j]) / hc;
     const double* T = warp_tensor(X, Y, Z, N, 1, nullptr, TA, nullptr, gsh, yp, zp, ir, term_off, term_abc, term_c,
                                   lane);
     for (int c = lane; c < nqT; c += 32) gT[(size_t)g * ldT + c] = T[c];
@@ -334,8 +328,7 @@ int launch_group_tensor_ref(Workspace& ws, const TreeDev& t, int ng, const int32
 }
 
 // M2L pair by pair on the CUDA cores (FP64), ref or exact tensors.
-static int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md, bool accumulate,
-                               cudaStream_t st) {
+static int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st) {
     const int nq = nT(p), N = 2 * p, nqT = nT(N);
     FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nq));
     const int ref = md.coef_mode == 0 ? 1 : 0;
@@ -347,21 +340,21 @@ static int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Mod
     count_launches(1);
     k_m2l_f64<<<grid_for(t.num_nodes, wpb), 32 * wpb, sm, st>>>(t, ws.mom.as<double>(), ws.loc.as<double>(), p, ref,
                                                                 ws.term_off.as<int32_t>(), ws.term_abc.as<uchar4>(),
-                                                                ws.term_c.as<double>(), accumulate ? 1 : 0);
+                                                                ws.term_c.as<double>());
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
 
-int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st, bool accumulate) {
+int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st) {
     int rc;
     if (md.coef_mode != 0 || 2 * p <= kExactRefOrder) {
-        rc = launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, st, accumulate);
+        rc = launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, st);
     } else {
         FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nT(p)));
         rc = (ws.reuse_structure && ws.m2l_pairwise) ? FMM_ENOTSUP
-                                                     : launch_m2l_grouped(ws, t, p, false, st, true, accumulate);
+                                                     : launch_m2l_grouped(ws, t, p, false, st, true);
     }
-    return rc == FMM_ENOTSUP ? launch_m2l_pairwise(ws, t, p, md, accumulate, st) : rc;
+    return rc == FMM_ENOTSUP ? launch_m2l_pairwise(ws, t, p, md, st) : rc;
 }
 
 // ---------------------------------------------------------------- periodic

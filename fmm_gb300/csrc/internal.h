@@ -58,11 +58,19 @@ struct TreeDev {
     // range, CSR by target leaf like the near list
     int64_t ncorr = 0;
     int32_t *corr_off = nullptr, *corr_src = nullptr;
-    // periodic boxes: the lists in use are those of the image whose source
-    // cells are displaced by `shift`; `central` is 0 for the 26 other images
-    double shift[3] = {0.0, 0.0, 0.0};
-    int central = 1;
+    // periodic boxes (build_images): the node arrays hold every node nimg = 27
+    // times, image a's copies from a x num_nodes on with their centres displaced
+    // by its shift (image 0: the central cell, the tree itself).  Targets are
+    // nodes of image 0, sources of any.
+    int nimg = 1;
+    const double* img_shift = nullptr;  // 3 per image
 };
+
+#ifdef __CUDACC__
+// The tree's node of a source (its image's copy in periodic boxes), and the image.
+__device__ __forceinline__ int src_node(const TreeDev& t, int j) { return t.nimg > 1 ? j % t.num_nodes : j; }
+__device__ __forceinline__ int src_image(const TreeDev& t, int j) { return t.nimg > 1 ? j / t.num_nodes : 0; }
+#endif
 
 // A 3x3 box matrix, column-major (the reference's box_matrix(3,3)).
 struct Box9 {
@@ -104,6 +112,8 @@ struct TreeParams {
 double damping_range(int damp, double a, int nmax, double eps);
 int build_tree(Workspace& ws, const double* d_coords, int64_t n, const TreeParams& tp, TreeDev& t, cudaStream_t st);
 int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st);
+// The tree with its 27 periodic images as sources (out: see TreeDev::nimg).
+int build_images(Workspace& ws, const TreeDev& t, const Box9& H, TreeDev* out, cudaStream_t st);
 // Smallest damping factor of n particles (device array), 0 if none is positive.
 double min_damping_factor(Workspace& ws, const double* d_damp, int64_t n, cudaStream_t st);
 
@@ -152,6 +162,7 @@ struct Workspace {
     DevBuf fsorted;
     // expansions
     DevBuf mom, loc, wred;
+    DevBuf images;   // periodic boxes: node arrays of the images
     DevBuf lattice;  // periodic boxes (level multipoles and contributions), QM/MM classification scratch
     int wred_p = -1;  // order of the reduced weights in wred computed from this call's moments (-1: none)
     // direct sum: scaled multipoles and partial sums
@@ -246,15 +257,12 @@ int launch_direct_scale_f32(Workspace& ws, const Particles& P, const TreeDev& t,
 
 // FMM phases (near.cu / expansions.cu)
 int gather_sorted(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st);
-// image: the lists are a periodic image's (t.shift, t.central) and the near
-// field is added to ws.fsorted instead of written.
 int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int field_order, const Modes& md,
-                   cudaStream_t st, bool image = false);
+                   cudaStream_t st);
 // df: P2M sums in double-float (FP32 pipe) instead of FP64 (mixed path)
 int launch_p2m_m2m(Workspace& ws, const Particles& P, const TreeDev& t, int p, cudaStream_t st, bool df = false);
-// M2L into the local expansions, honouring t.shift; accumulate adds to them
-// instead of writing them.
-int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st, bool accumulate = false);
+// M2L into the local expansions.
+int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st);
 // Reference mode: the closed-form tensor of every displacement group of the
 // grouped M2L (all components of order <= 2p, ldT entries a group), with the
 // group's order and unit ratios.
@@ -265,9 +273,8 @@ int launch_group_tensor_ref(Workspace& ws, const TreeDev& t, int ng, const int32
 // *d_levels receives the number of lattice levels used.
 int launch_periodic_lattice(Workspace& ws, const TreeDev& t, int p, int f, const Modes& md, const Box9& H,
                             double* d_fs, int* d_levels, cudaStream_t st);
-int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool accumulate = false);
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full = false,
-                       bool accumulate = false);
+int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st);
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full = false);
 int launch_reduce_moments(Workspace& ws, const TreeDev& t, int p, cudaStream_t st);
 // selector.cu
 int selector_node_norms(Workspace& ws, const TreeDev& t, int P, const double* d_sorted_damp, cudaStream_t st);

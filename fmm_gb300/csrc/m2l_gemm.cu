@@ -45,7 +45,7 @@ constexpr int kFallback = 63;            // key code of pairs without a grid dis
 // Key layout (46 bits, so the radix sort needs 6 digit passes): level
 // difference + 31 (6 bits) | order (4) | Dx, Dy, Dz + kDOff (12 bits each).
 constexpr int kKeyBits = 46;
-constexpr int kKeyBitsLevel = 51;        // with the target's depth above (displaced sources)
+constexpr int kKeyBitsImages = 56;       // with the target's depth and the source's image (5 bits each) above
 constexpr int64_t kDOff = 1 << 11;       // offset of the 12-bit displacement fields
 constexpr int kTaskCols = 512;           // pairs (columns) per product block
 constexpr int kGemmThreads = 128;        // 16 row groups x 8 column groups
@@ -91,15 +91,15 @@ __global__ void k_scale_weights(int M, int nr, int ld, const double* __restrict_
 // pipe; its error (a few 1e-8 relative of the displacement, up to ~1e-4 cell
 // units at the largest encodable displacement) stays far below the 1e-3
 // tolerance of the integer test.  Without them, FP64 with a 1e-6 tolerance.
-// level: the sources are displaced by a periodic image's shift, which is the
-// same for all pairs but not in units of their cells, so only pairs of one
-// level share an operator.
-__global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restrict__ tgt, int p, int oclass, bool level,
+// Sources in periodic images are displaced by their image's shift, the same in
+// bohr but not in units of their cells: only pairs of one image and one level
+// share an operator.
+__global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restrict__ tgt, int p, int oclass,
                            const float4* __restrict__ chi, const float4* __restrict__ clo,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= nfar) return;
-    const int i = tgt[q], j = t.far_src[q];
+    const int i = tgt[q], j = src_node(t, t.far_src[q]);
     const int ord = t.far_ord ? min((int)t.far_ord[q], p) : p;
     // half-widths are the root's divided by powers of two: 1/h times an
     // integer multiple of h stays within rounding of that integer
@@ -137,7 +137,7 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
     if (grid)
         key = ((uint64_t)(dl + 31) << 40) | ((uint64_t)oc << 36) | ((uint64_t)((int64_t)rx + kDOff) << 24) |
               ((uint64_t)((int64_t)ry + kDOff) << 12) | (uint64_t)((int64_t)rz + kDOff) |
-              (level ? (uint64_t)t.depth[i] << kKeyBits : 0);
+              (t.nimg > 1 ? (uint64_t)(t.depth[i] | (src_image(t, t.far_src[q]) << 5)) << kKeyBits : 0);
     else
         key = ((uint64_t)kFallback << 40) | (uint64_t)q;
     keys[q] = key;
@@ -174,9 +174,7 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_
         q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
     for (int off = 16; off > 0; off >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, off));
     const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
-    // (the source cells of a periodic image are displaced by t.shift)
-    const double X = (t.cx[i] - (t.cx[j] + t.shift[0])) / hc, Y = (t.cy[i] - (t.cy[j] + t.shift[1])) / hc,
-                 Z = (t.cz[i] - (t.cz[j] + t.shift[2])) / hc;
+    const double X = (t.cx[i] - t.cx[j]) / hc, Y = (t.cy[i] - t.cy[j]) / hc, Z = (t.cz[i] - t.cz[j]) / hc;
     const int Nq = 2 * q;
     const double r2 = X * X + Y * Y + Z * Z;
     const double rinv = 1.0 / sqrt(r2), rinv2 = rinv * rinv;
@@ -273,8 +271,8 @@ struct GemmSmem {
         off_T = o;
         o += sizeof(R) * nTr;
         o = (o + 15) & ~(size_t)15;
-        off_col = o;  // the task's pair positions and source nodes
-        o += sizeof(int) * 2 * kTaskCols;
+        off_col = o;  // the source nodes of the task's pairs
+        o += sizeof(int) * kTaskCols;
         off_G = o;
         o += sizeof(R) * (size_t)((nrmax + VS - 1) / VS * VS) * rmmax;
         bytes = o;
@@ -334,8 +332,7 @@ __device__ __forceinline__ void load_rows(const R* p, R (&v)[RT]) {
 // needs no block barrier.
 template <typename R, int RT, int CPT>
 __device__ __forceinline__ void gemm_task(const GemmSmem<R, CPT>& L, char* sm, int c_begin, int tcols, int nrq,
-                                          int cnt, int gs,
-                                          const int32_t* __restrict__ svals, const int32_t* __restrict__ far_src,
+                                          int cnt, int gs, const int32_t* __restrict__ psrc,
                                           const R* __restrict__ wsc, int ldw, R* __restrict__ gout, int ldo) {
     constexpr int TN = GemmSmem<R, CPT>::TN;
     constexpr int VS = GemmSmem<R, CPT>::VS;
@@ -348,16 +345,11 @@ __device__ __forceinline__ void gemm_task(const GemmSmem<R, CPT>& L, char* sm, i
     const R* bpow = apow + 16;
     const R* Tsh = reinterpret_cast<const R*>(sm + L.off_T);
     R* G = reinterpret_cast<R*>(sm + L.off_G);
-    int* cpos = reinterpret_cast<int*>(sm + L.off_col);
-    int* csrc = cpos + kTaskCols;
+    int* csrc = reinterpret_cast<int*>(sm + L.off_col);
     const int nrv = (nrq + VS - 1) / VS * VS;
     const int c_end = min(cnt, c_begin + tcols);
-    // the task's columns: pair positions and source nodes (loaded once)
-    for (int i = tid; i < c_end - c_begin; i += kGemmThreads) {
-        const int pos = svals[gs + c_begin + i];
-        cpos[i] = pos;
-        csrc[i] = far_src[pos];
-    }
+    // the task's columns: source nodes (loaded once)
+    for (int i = tid; i < c_end - c_begin; i += kGemmThreads) csrc[i] = psrc[gs + c_begin + i];
     // operator G^T (s-major, RM rows per s; rows f >= nrq and s >= nrq zero)
     for (int e = tid; e < nrv * RM; e += kGemmThreads) {
         const int s = e / RM, f = e - s * RM;
@@ -443,8 +435,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_m2l_gemm(const int2* __restric
                                                            const int32_t* __restrict__ gstart,
                                                            const int32_t* __restrict__ gq,
                                                            const float2* __restrict__ gab, const R* __restrict__ gT,
-                                                           int ldT, const int32_t* __restrict__ svals,
-                                                           const int32_t* __restrict__ far_src,
+                                                           int ldT, const int32_t* __restrict__ psrc,
                                                            const R* __restrict__ wsc, R* __restrict__ out,
                                                            const int32_t* __restrict__ rowbase) {
     extern __shared__ __align__(16) char sm_gemm[];
@@ -477,7 +468,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_m2l_gemm(const int2* __restric
     switch (rt) {
 #define FMM_GEMM_CASE(K)                                                                                     \
     case K:                                                                                                  \
-        gemm_task<R, K, CPT>(L, sm_gemm, task.y, tcols, nrq, cnt, gs, svals, far_src, wsc, wsc_ld<R>(nr),     \
+        gemm_task<R, K, CPT>(L, sm_gemm, task.y, tcols, nrq, cnt, gs, psrc, wsc, wsc_ld<R>(nr),     \
                              out + (size_t)rowbase[g] * kRowUnit, row_len(q));                                      \
         break;
         FMM_GEMM_CASE(1)
@@ -584,11 +575,11 @@ __global__ void k_row_offsets(int ng, bool full, const int32_t* __restrict__ gst
     for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32) roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
 }
 
-// Source node of every far pair in group order: psrc[k] = far_src[svals[k]].
-__global__ void k_pair_sources(int64_t nf, const int32_t* __restrict__ svals, const int32_t* __restrict__ far_src,
+// Source node of every far pair in group order.
+__global__ void k_pair_sources(int64_t nf, const int32_t* __restrict__ svals, const TreeDev t,
                                int32_t* __restrict__ psrc) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < nf) psrc[k] = far_src[svals[k]];
+    if (k < nf) psrc[k] = src_node(t, t.far_src[svals[k]]);
 }
 
 // Size in floats of a group's split operator (halves x chunks x (hi + lo) x
@@ -876,15 +867,14 @@ struct Sum<double> {
 // target's pair rows (stored in group order; roff gives each target-order
 // pair's row in units of kRowUnit entries; a pair of order q contributes its
 // first rows(q) entries; eight loads in flight), back to physical units, into
-// (accumulate: added to) the basis' components of the local expansion.
+// the basis' components of the local expansion.
 template <typename R, bool full>
-__global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p, bool accumulate,
+__global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p,
                                                  const R* __restrict__ out, const int32_t* __restrict__ roff,
                                                  double* __restrict__ loc) {
     const int i = blockIdx.x;
     const int nr = d64_rows(p, full);
     const int q0 = t.far_off[i], q1 = t.far_off[i + 1];
-    if (accumulate && q0 == q1) return;
     const double ih = 1.0 / t.r[i];
     double* L = loc + (size_t)i * nT(p);
     for (int f = threadIdx.x; f < nr; f += blockDim.x) {
@@ -909,8 +899,7 @@ __global__ void __launch_bounds__(256) k_m2l_sum(const TreeDev t, int p, bool ac
         const int k = c >> 24;
         double s = ih;
         for (int e = 0; e < k; ++e) s *= ih;
-        double* o = L + (full ? f : pidx(c & 0xff, (c >> 8) & 0xff, (c >> 16) & 0xff));
-        *o = accumulate ? *o + acc.value() * s : acc.value() * s;
+        L[full ? f : pidx(c & 0xff, (c >> 8) & 0xff, (c >> 16) & 0xff)] = acc.value() * s;
     }
 }
 
@@ -953,7 +942,7 @@ int launch_operators(Workspace& ws, bool tc, bool full, int ldT, int ldr, const 
 }
 
 template <typename R, int CPT>
-int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, bool accumulate) {
+int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) {
     const int M = t.num_nodes, nr = d64_rows(p, full), N = 2 * p, nTr = full ? nT(N) : rbase(N + 1);
     const bool tc = sizeof(R) == 4 && !product_on_cuda_cores();
     const bool tc64 = sizeof(R) == 8 && (full || !product_on_cuda_cores());
@@ -988,9 +977,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         count_launches(1);
         // FP32 node data where the mixed path prepared it
         const float4* chi = (sizeof(R) == 4 && ws.f32node_ok) ? ws.f32node.as<float4>() : nullptr;
-        const bool level = t.shift[0] != 0.0 || t.shift[1] != 0.0 || t.shift[2] != 0.0;
-        const int kbits = level ? kKeyBitsLevel : kKeyBits;
-        k_m2l_keys<<<grid_for(nf, 256), 256, 0, st>>>(nf, t, tgt, p, kOrderClass, level, chi, chi ? chi + M : nullptr,
+        const int kbits = t.nimg > 1 ? kKeyBitsImages : kKeyBits;
+        k_m2l_keys<<<grid_for(nf, 256), 256, 0, st>>>(nf, t, tgt, p, kOrderClass, chi, chi ? chi + M : nullptr,
                                                        ws.m2l_keys.as<uint64_t>(), ws.m2l_vals.as<int32_t>());
         // sort by key, run-length encode into groups
         int* d_nruns = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 14);
@@ -1080,15 +1068,14 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         count_launches(1);
         k_fill_tasks<<<grid_for(ng, 256), 256, 0, st>>>(ng, cols, ws.m2l_gq.as<int32_t>(), ws.m2l_gstart.as<int32_t>(),
                                                         ws.m2l_toff.as<int32_t>(), ws.m2l_tasks.as<int2>());
+        // source node per sorted pair (into the free unsorted-values buffer)
+        count_launches(1);
+        k_pair_sources<<<grid_for(nf, 256), 256, 0, st>>>(nf, ws.m2l_vals2.as<int32_t>(), t, ws.m2l_vals.as<int32_t>());
         if (tc || tc64) {
             // tensor-core operands: per node the weights, per group the operator
             FMM_TRY(ws.m2l_wsplit.ensure(tc ? sizeof(float) * 2 * (size_t)M * ldk
                                             : (size_t)M * (wchunks * kDig * kD64K * 2 + sizeof(int))));
             if (tc64) FMM_TRY(ws.m2l_gexp.ensure(sizeof(int) * (size_t)ng * nr));
-            // source node per sorted pair (into the free unsorted-values buffer)
-            count_launches(1);
-            k_pair_sources<<<grid_for(nf, 256), 256, 0, st>>>(nf, ws.m2l_vals2.as<int32_t>(), t.far_src,
-                                                              ws.m2l_vals.as<int32_t>());
             FMM_TRY(ws.m2l_gopoff.ensure(sizeof(int64_t) * (ng + 1)));
             int64_t* goff = ws.m2l_gopoff.as<int64_t>();
             count_launches(1);
@@ -1198,21 +1185,19 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
             count_launches(1);
             k_m2l_gemm<R, CPT><<<(unsigned)ntasks, kGemmThreads, L.bytes, st>>>(
                 ws.m2l_tasks.as<int2>(), cols, 0, p, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
-                ws.m2l_gab.as<float2>(), ws.m2l_T.as<R>(), ldT, ws.m2l_vals2.as<int32_t>(), t.far_src,
-                ws.m2l_wsc.as<R>(), ws.m2l_out.as<R>(), rowbase);
+                ws.m2l_gab.as<float2>(), ws.m2l_T.as<R>(), ldT, ws.m2l_vals.as<int32_t>(), ws.m2l_wsc.as<R>(), ws.m2l_out.as<R>(), rowbase);
             if (ws.product_timed) cudaEventRecord(ws.ev[9], st);
         }
     }
-    if (nf == 0 && accumulate) return FMM_OK;
     count_launches(1);
     if (nf == 0) FMM_TRY(ws.m2l_out.ensure(sizeof(R) * kRowUnit));
     // one output per thread: the basis rounded up to whole warps (192 at p = 12)
     const unsigned sum_threads = (unsigned)std::min(256, (nr + 31) / 32 * 32);
     if (sizeof(R) == 8 && full)
-        k_m2l_sum<double, true><<<(unsigned)M, sum_threads, 0, st>>>(t, p, accumulate, ws.m2l_out.as<double>(), roff,
+        k_m2l_sum<double, true><<<(unsigned)M, sum_threads, 0, st>>>(t, p, ws.m2l_out.as<double>(), roff,
                                                                      ws.loc.as<double>());
     else
-        k_m2l_sum<R, false><<<(unsigned)M, sum_threads, 0, st>>>(t, p, accumulate, ws.m2l_out.as<R>(), roff,
+        k_m2l_sum<R, false><<<(unsigned)M, sum_threads, 0, st>>>(t, p, ws.m2l_out.as<R>(), roff,
                                                                  ws.loc.as<double>());
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -1220,16 +1205,14 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
 
 }  // namespace
 
-// Grouped M2L into (accumulate: added to) the local expansions ws.loc: the
-// reduced components from the weights ws.wred (which must be current), in FP32
-// products for `fp32`, else FP64; or (full) all Cartesian components in FP64
-// with the reference's wrapped tensors.  Returns FMM_ENOTSUP where the pairs
-// should be evaluated one by one.
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full,
-                       bool accumulate) {
-    if (fp32) return grouped<float, 8>(ws, t, p, st, false, accumulate);
+// Grouped M2L into the local expansions ws.loc: the reduced components from the
+// weights ws.wred (which must be current), in FP32 products for `fp32`, else
+// FP64; or (full) all Cartesian components in FP64 with the reference's wrapped
+// tensors.  Returns FMM_ENOTSUP where the pairs should be evaluated one by one.
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full) {
+    if (fp32) return grouped<float, 8>(ws, t, p, st, false);
     if (!full && product_on_cuda_cores() && GemmSmem<double, 4>(p).bytes > 227 * 1024) return FMM_ENOTSUP;
-    return grouped<double, 4>(ws, t, p, st, full, accumulate);
+    return grouped<double, 4>(ws, t, p, st, full);
 }
 
 }  // namespace fmm

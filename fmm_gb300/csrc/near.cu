@@ -111,9 +111,9 @@ struct ExList {
 // P2P: a warp per target particle and source slice (blockIdx.y of gridDim.y),
 // its lanes over the concatenated particles of the target leaf's near list
 // (each lane walks the list on its own).  Totals go to out[slice][f][particle].
-// IMG: the lists are those of a periodic image (t.shift, t.central): sources
-// sit at x_j + shift, the self pair and the exclusions count only in the
-// central image (src/fmm.F90:704-736).
+// IMG: the sources are cells of the periodic images: their particles sit at
+// x_j + the image's shift, and the self pair and the exclusions count only in
+// the central image (src/fmm.F90:704-736).
 // 66,666 water molecules, Thole, f = 2 (4.6e8 pairs): 294 ms with a warp per
 // target leaf (targets across the lanes) and the tensor contraction.
 template <int M, int F, bool IMG>
@@ -128,13 +128,12 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
     if (tgt >= n) return;
     const int leaf = t.leaf_of[tgt];
     const double xt = sx[tgt], yt = sy[tgt], zt = sz[tgt], dt = sd[tgt];
-    const bool here = !IMG || t.central;  // exclusions and the self pair count
-    const ExList ex(excl, here ? exw : 0, n, (int64_t)t.perm[tgt]);
+    const ExList ex(excl, exw, n, (int64_t)t.perm[tgt]);
     double acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.0;
     const int q1 = t.near_off[leaf + 1], step = 32 * (int)gridDim.y;
-    int q = t.near_off[leaf] - 1, js = 0, jc = 0;
+    int q = t.near_off[leaf] - 1, js = 0, jc = 0, img = 0;
     for (int off = lane + 32 * (int)blockIdx.y;; off += step) {
         while (off >= jc) {
             off -= jc;
@@ -142,20 +141,22 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
             const int j = t.near_src[q];
             js = t.start[j];
             jc = t.count[j];
+            if (IMG) img = src_image(t, j);
         }
         if (q >= q1) break;
         const int k = js + off;
         double dx, dy, dz;
         if (IMG) {
-            dx = xt - (sx[k] + t.shift[0]);
-            dy = yt - (sy[k] + t.shift[1]);
-            dz = zt - (sz[k] + t.shift[2]);
+            const double* sh = t.img_shift + 3 * img;
+            dx = xt - (sx[k] + sh[0]);
+            dy = yt - (sy[k] + sh[1]);
+            dz = zt - (sz[k] + sh[2]);
         } else {
             dx = xt - sx[k];
             dy = yt - sy[k];
             dz = zt - sz[k];
         }
-        if (here) {
+        if (!IMG || img == 0) {
             const bool out_of = ex.has((int)t.perm[k] + 1);
             if (excl_mode == 0) {
                 if (out_of) dx = dy = dz = 1e10;
@@ -172,13 +173,11 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
     if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * n + tgt] = acc[0];
 }
 
-// Slices of k_p2p_f64 (and, for periodic images, the sum over images) into
-// the sorted field.
-__global__ void k_p2p_slices(int64_t total, int slices, const double* __restrict__ part, bool add,
-                             double* __restrict__ fs) {
+// Sum of the slices.
+__global__ void k_p2p_slices(int64_t total, int slices, const double* __restrict__ part, double* __restrict__ fs) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
-    double s = add ? fs[e] : 0.0;
+    double s = 0.0;
     for (int k = 0; k < slices; ++k) s += part[(size_t)k * total + e];
     fs[e] = s;
 }
@@ -318,7 +317,7 @@ int launch_direct_f64(Workspace& ws, const Particles& P, int field_order, const 
                                                                   md.excl_mode, P.exw, P.excl, chunk, out)));
     if (ks > 1) {
         count_launches(1);
-        k_p2p_slices<<<grid_for(ntgt * nf, 128), 128, 0, st>>>(ntgt * nf, (int)ks, out, false, d_field);
+        k_p2p_slices<<<grid_for(ntgt * nf, 128), 128, 0, st>>>(ntgt * nf, (int)ks, out, d_field);
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -343,7 +342,7 @@ int gather_sorted(Workspace& ws, const Particles& P, const TreeDev& t, cudaStrea
 }
 
 int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int field_order, const Modes& md,
-                   cudaStream_t st, bool image) {
+                   cudaStream_t st) {
     const int m = dim_to_order(P.dim);
     if (!near_orders_supported(m, field_order)) return FMM_ENOTSUP;
     const int64_t n = P.n;
@@ -359,14 +358,13 @@ int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     // slices of the near lists while there are fewer than 16 targets per
     // scheduler (a near list holds many steps of 32 sources)
     const int ks = (int)std::max<int64_t>(1, std::min<int64_t>(8, 16LL * 4 * num_sms() / n));
-    const bool part = image || ks > 1;
     double* out = ws.fsorted.as<double>();
-    if (part) {
+    if (ks > 1) {
         FMM_TRY(ws.near_part.ensure(sizeof(double) * (size_t)ks * nf * n));
         out = ws.near_part.as<double>();
     }
     const dim3 grid(grid_for(n, 4), (unsigned)ks);
-    if (image) {
+    if (t.nimg > 1) {
         FMM_MF_SWITCH_F64(m, field_order,
                       (k_p2p_f64<MM, FF, true><<<grid, 128, 0, st>>>(
                           t, ws.sx.as<double>(), ws.sy.as<double>(), ws.sz.as<double>(), ws.sd.as<double>(), rows, n,
@@ -377,9 +375,9 @@ int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
                           t, ws.sx.as<double>(), ws.sy.as<double>(), ws.sz.as<double>(), ws.sd.as<double>(), rows, n,
                           P.damp_type, md.excl_mode, P.exw, P.excl, out)));
     }
-    if (part) {
+    if (ks > 1) {
         count_launches(1);
-        k_p2p_slices<<<grid_for(n * nf, 128), 128, 0, st>>>(n * nf, ks, out, image, ws.fsorted.as<double>());
+        k_p2p_slices<<<grid_for(n * nf, 128), 128, 0, st>>>(n * nf, ks, out, ws.fsorted.as<double>());
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;

@@ -374,11 +374,11 @@ __global__ void k_list_iter(const int2* __restrict__ in, int nin, int2* __restri
     if (!skip) {
         i = in[q].x;
         j = in[q].y;
-        // delta = c_i - (c_j + displacement) (fmm.F90:357-358); the
-        // displacement is that of the periodic image (0 without one)
-        const double dx = __dsub_rn(t.cx[i], __dadd_rn(t.cx[j], t.shift[0]));
-        const double dy = __dsub_rn(t.cy[i], __dadd_rn(t.cy[j], t.shift[1]));
-        const double dz = __dsub_rn(t.cz[i], __dadd_rn(t.cz[j], t.shift[2]));
+        // delta = c_i - (c_j + displacement) (fmm.F90:357-358); a periodic
+        // image's nodes hold the displaced centre
+        const double dx = __dsub_rn(t.cx[i], t.cx[j]);
+        const double dy = __dsub_rn(t.cy[i], t.cy[j]);
+        const double dz = __dsub_rn(t.cz[i], t.cz[j]);
         const double r = norm2_3(dx, dy, dz);
         ri = t.rmax[i];
         rj = t.rmax[j];
@@ -534,6 +534,26 @@ __global__ void k_near_pair_count(int64_t m, const uint64_t* __restrict__ sorted
     __shared__ typename BR::TempStorage tmp;
     unsigned long long b = BR(tmp).Sum(s);
     if (threadIdx.x == 0) atomicAdd(out, b);
+}
+
+// Copies of the M nodes for every periodic image (see TreeDev::nimg).
+__global__ void k_images(int64_t total, int M, const TreeDev t, const double* __restrict__ shift, TreeDev o) {
+    const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (v >= total) return;
+    const int img = (int)(v / M), k = (int)(v - (int64_t)img * M);
+    o.cx[v] = __dadd_rn(t.cx[k], shift[3 * img]);
+    o.cy[v] = __dadd_rn(t.cy[k], shift[3 * img + 1]);
+    o.cz[v] = __dadd_rn(t.cz[k], shift[3 * img + 2]);
+    o.r[v] = t.r[k];
+    o.rmax[v] = t.rmax[k];
+    o.start[v] = t.start[k];
+    o.count[v] = t.count[k];
+    o.depth[v] = t.depth[k];
+    o.is_leaf[v] = t.is_leaf[k];
+    for (int c = 0; c < 8; ++c) {
+        const int ch = t.child[8 * (size_t)k + c];
+        o.child[8 * v + c] = ch >= 0 ? ch + img * M : -1;
+    }
 }
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
@@ -776,6 +796,38 @@ double min_damping_factor(Workspace& ws, const double* d, int64_t n, cudaStream_
     return h >= 1e299 ? 0.0 : h;
 }
 
+int build_images(Workspace& ws, const TreeDev& t, const Box9& H, TreeDev* out, cudaStream_t st) {
+    const int M = t.num_nodes;
+    const int64_t V = 27LL * M;
+    if (V > INT32_MAX) return FMM_ENOTSUP;
+    FMM_TRY(ws.images.ensure(sizeof(double) * (27 * 3 + 5 * (size_t)V) + sizeof(int32_t) * 12 * (size_t)V));
+    double* d = ws.images.as<double>();
+    double h[27 * 3] = {0.0, 0.0, 0.0};
+    int k = 1;  // image 0 is the central cell
+    for (int ai = -1; ai <= 1; ++ai)
+        for (int aj = -1; aj <= 1; ++aj)
+            for (int ak = -1; ak <= 1; ++ak) {
+                if (ai == 0 && aj == 0 && ak == 0) continue;
+                // displacement = matmul(box_matrix, a) (fmm.F90:355, 662)
+                for (int c = 0; c < 3; ++c) h[3 * k + c] = (H.h[c] * ai + H.h[3 + c] * aj) + H.h[6 + c] * ak;
+                ++k;
+            }
+    FMM_CUDA_TRY(cudaMemcpyAsync(d, h, sizeof(h), cudaMemcpyHostToDevice, st));
+    *out = t;
+    out->nimg = 27;
+    out->img_shift = d;
+    double** da[5] = {&out->cx, &out->cy, &out->cz, &out->r, &out->rmax};
+    for (int a = 0; a < 5; ++a) *da[a] = d + 27 * 3 + (size_t)a * V;
+    int32_t* i = reinterpret_cast<int32_t*>(d + 27 * 3 + 5 * (size_t)V);
+    int32_t** ia[4] = {&out->start, &out->count, &out->depth, &out->is_leaf};
+    for (int a = 0; a < 4; ++a) *ia[a] = i + (size_t)a * V;
+    out->child = i + 4 * (size_t)V;
+    count_launches(1);
+    k_images<<<grid_for(V, 256), 256, 0, st>>>(V, M, t, d, *out);
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
 int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st) {
     const int M = t.num_nodes;
     // capacities: pair counts grow like theta^-3; never below what the
@@ -796,12 +848,13 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
         FMM_TRY(ws.far_pairs.ensure(sizeof(uint64_t) * cap_far));
         FMM_TRY(ws.near_pairs.ensure(sizeof(uint64_t) * cap_near));
         if (corr) FMM_TRY(ws.corr_pairs.ensure(sizeof(uint64_t) * cap_corr));
-        const int2 root = make_int2(0, 0);
-        FMM_CUDA_TRY(cudaMemcpyAsync(ws.front_a.p, &root, sizeof(int2), cudaMemcpyHostToDevice, st));
+        int2 root[27];
+        for (int a = 0; a < t.nimg; ++a) root[a] = make_int2(0, a * M);
+        FMM_CUDA_TRY(cudaMemcpyAsync(ws.front_a.p, root, sizeof(int2) * t.nimg, cudaMemcpyHostToDevice, st));
         // frontier, far, near, overflow flag, network evaluations, correction pairs
         unsigned long long h[6] = {0, 0, 0, 0, 0, 0};
         FMM_CUDA_TRY(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, st));
-        int64_t nin = 1;
+        int64_t nin = t.nimg;
         int64_t candidates = 0;
         int2* fin = ws.front_a.as<int2>();
         int2* fout = ws.front_b.as<int2>();
