@@ -45,9 +45,9 @@ void Workspace::release_buffers(bool keep_selector) {
                      &node_val2, &counters,  &scalars,     &front_a,    &front_b,    &far_pairs,  &near_pairs,
                      &far_sorted, &near_sorted, &node_dfs, &far_src,    &near_src,   &sx,         &sy,
                      &sz,        &smc,       &sd,          &fsorted,    &mom,        &loc,        &partial,
-                     &term_off,  &term_abc,  &term_c, &f32buf, &wred, &far_ord, &sel_norms, &sel_params, &sel_scratch, &sysbuf,
+                     &term_off,  &term_abc,  &term_c, &f32buf, &f32sel, &wred, &far_ord, &sel_norms, &sel_params, &sel_scratch, &sysbuf,
                      &m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
-                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
+                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &f32x2c, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
     for (DevBuf* b : all)
         if (!(keep_selector && b == &sel_params)) b->release();
     if (!keep_selector) sel_ready = false;
@@ -452,7 +452,7 @@ int run_fmm(Workspace& ws, const Particles& P, double theta, int ncrit, int p, i
     }
     FMM_TRY(gather_sorted(ws, P, t, st));
     const bool f32_near = md.precision == 1 || md.precision == 2;
-    if (f32_near || learned) FMM_TRY(prepare_f32_records(ws, P, t, st));
+    if (f32_near || learned) FMM_TRY(prepare_f32_records(ws, P, t, f32_near, learned, st));
     FMM_TRY(launch_p2m_m2m(ws, P, t, p, st, md.precision != 0));
     if (learned) {
         FMM_TRY(launch_reduce_moments(ws, t, p, st));
@@ -848,7 +848,7 @@ int plan_numeric(PlanImpl& pl) {
     if (pl.direct) return launch_direct_f64(ws, P, pl.f, pl.md, ws.out_field.as<double>(), st);
     ws.product_err = nullptr;
     FMM_TRY(gather_sorted(ws, P, t, st));
-    if (pl.f32_near) FMM_TRY(prepare_f32_records(ws, P, t, st));
+    if (pl.f32_near) FMM_TRY(prepare_f32_records(ws, P, t, true, false, st));
     FMM_TRY(launch_p2m_m2m(ws, P, t, pl.p, st, pl.md.precision != 0));
     if (pl.f32_near)
         FMM_TRY(launch_p2p_f32(ws, P, t, pl.f, st));

@@ -158,6 +158,7 @@ struct Workspace {
     // sorted particle data
     DevBuf sx, sy, sz, smc, sd;
     DevBuf f32buf;   // FP32 particle records of the mixed-precision near field
+    DevBuf f32sel;   // the selector's, relative to the leaf centres
     DevBuf f32node;  // node centres as FP32 hi/lo pairs
     DevBuf fsorted;
     // expansions
@@ -169,7 +170,7 @@ struct Workspace {
     DevBuf dsmc, partial;
     // FP64 near field: source rows and per-slice sums (not `partial`: the
     // sampled direct sum runs beside it on another stream)
-    DevBuf near_rows, near_part;
+    DevBuf near_rows, near_part;  // (near_part also holds the FP32 near field's slices)
     // second stream (the learned selector's sampled direct sum overlaps the tree phases)
     cudaStream_t aux = nullptr;
     // host entry points: the multipoles and exclusions are copied on `copy`
@@ -204,6 +205,7 @@ struct Workspace {
     DevBuf leaf_ext;          // damping correction: per leaf (particle extent, smallest damping factor)
     DevBuf p2p_pad;      // packed near field: padded leaf starts (node-indexed), odd-leaf flags and their scan
     DevBuf f32x2;        // packed near field: interleaved source records of padded leaves
+    DevBuf f32x2c;       // the damping-correction list's
     int m2l_ng = 0, m2l_ntasks = 0;  // grouped M2L structure of the last evaluation
     bool m2l_pairwise = false;       // the last structure chose the per-pair M2L kernel
     std::vector<M2lBatch> m2l_batches;  // operator batches of the last structure
@@ -244,16 +246,15 @@ struct Modes {
 // used when the sum runs beside other work on a second stream).
 int launch_direct_f64(Workspace& ws, const Particles& P, int field_order, const Modes& md, double* d_field,
                       cudaStream_t st, int64_t ntgt = 0, const int64_t* d_targets = nullptr, int split_cap = 0);
-// FP32 particle records and node centres of the mixed-precision near field
-// (near_f32.cu; after gather_sorted).
-int prepare_f32_records(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st);
+// FP32 particle records of the mixed-precision near field and of the selector,
+// and node centres (near_f32.cu; after gather_sorted).
+int prepare_f32_records(Workspace& ws, const Particles& P, const TreeDev& t, bool near, bool selector,
+                        cudaStream_t st);
 // Per leaf: particle extent from the leaf centre and smallest damping factor
-// (ws.leaf_ext, from the FP32 records), for the damping correction.
+// (ws.leaf_ext, from the selector's records), for the damping correction.
 int launch_leaf_extent(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st);
-// FP32 field estimate at a few targets (exclusions masked) from those
-// records, into d_out (ntgt x nT(field_order), FP64, column-major).
-int launch_direct_scale_f32(Workspace& ws, const Particles& P, const TreeDev& t, int field_order, double* d_out,
-                            cudaStream_t st, int64_t ntgt, const int64_t* d_targets);
+// out[e] = sum over the slices of part[slice][e], e < total.
+int sum_slices(int64_t total, int slices, const double* part, double* out, cudaStream_t st);
 
 // FMM phases (near.cu / expansions.cu)
 int gather_sorted(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st);

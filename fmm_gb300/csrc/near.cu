@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
     if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * n + tgt] = acc[0];
 }
 
-// Sum of the slices.
-__global__ void k_p2p_slices(int64_t total, int slices, const double* __restrict__ part, double* __restrict__ fs) {
+// out[e] = sum over the slices of part[slice][e].
+__global__ void k_sum_slices(int64_t total, int slices, const double* __restrict__ part, double* __restrict__ fs) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
     double s = 0.0;
@@ -281,6 +281,13 @@ __global__ void k_scatter(int64_t n, int nf, const uint32_t* __restrict__ perm, 
 
 bool near_orders_supported(int m, int f) { return m >= 0 && m <= 3 && f >= 0 && f <= 3; }
 
+int sum_slices(int64_t total, int slices, const double* part, double* out, cudaStream_t st) {
+    count_launches(1);
+    k_sum_slices<<<grid_for(total, 128), 128, 0, st>>>(total, slices, part, out);
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
 int launch_direct_f64(Workspace& ws, const Particles& P, int field_order, const Modes& md, double* d_field,
                       cudaStream_t st, int64_t ntgt, const int64_t* d_targets, int split_cap) {
     const int m = dim_to_order(P.dim);
@@ -315,10 +322,7 @@ int launch_direct_f64(Workspace& ws, const Particles& P, int field_order, const 
     FMM_MF_SWITCH_F64(m, field_order,
                       (k_direct_f64<MM, FF><<<grid, 128, 0, st>>>(n, d_targets, ntgt, P.x, rows, P.damp, P.damp_type,
                                                                   md.excl_mode, P.exw, P.excl, chunk, out)));
-    if (ks > 1) {
-        count_launches(1);
-        k_p2p_slices<<<grid_for(ntgt * nf, 128), 128, 0, st>>>(ntgt * nf, (int)ks, out, d_field);
-    }
+    if (ks > 1) FMM_TRY(sum_slices(ntgt * nf, (int)ks, out, d_field, st));
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
@@ -375,10 +379,7 @@ int launch_p2p_f64(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
                           t, ws.sx.as<double>(), ws.sy.as<double>(), ws.sz.as<double>(), ws.sd.as<double>(), rows, n,
                           P.damp_type, md.excl_mode, P.exw, P.excl, out)));
     }
-    if (ks > 1) {
-        count_launches(1);
-        k_p2p_slices<<<grid_for(n * nf, 128), 128, 0, st>>>(n * nf, ks, out, ws.fsorted.as<double>());
-    }
+    if (ks > 1) FMM_TRY(sum_slices(n * nf, ks, out, ws.fsorted.as<double>(), st));
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }

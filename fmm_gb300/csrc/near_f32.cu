@@ -1,24 +1,29 @@
 // Mixed-precision near field (P2P): FP32 pair arithmetic with FP64 sums.
 //
 // Same pairs as particle_fields (src/fmm.F90:623-747).  Coordinates are held
-// in FP32 relative to each particle's own leaf centre; for a target leaf A and
-// a source leaf B the displacement is
-//     R = (x_t - x_s) + (c_A - c_B),
-// with the centre offset formed in FP64 once per leaf pair, so the FP32
-// rounding error scales with the leaf size and |R|, not with the distance from
-// the box origin.  Positions are double-float pairs, r^2 is compensated and
-// 1/r Newton-refined.  Contributions are summed over one source leaf in
-// compensated FP32 (TwoSum hi + lo) and the per-leaf sums are added into FP64
-// accumulators.  Excluded partners and the self pair are masked in the loop.
+// relative to the root cell's centre as double-float pairs (hi + lo, about 49
+// bits of the box), so the displacement R = (x_t - x_s)_hi + (x_t - x_s)_lo of
+// two near particles, whose hi parts subtract without rounding, carries about
+// one FP32 rounding of its own size.  r^2 is compensated and 1/r
+// Newton-refined.  Contributions are summed in compensated FP32 (TwoSum hi +
+// lo) and added into FP64 at the end.  Excluded partners and the self pair are
+// masked in the loop.
+//
+// Because positions need no leaf, the source leaves of a near list that follow
+// one another in the sorted order (most do: the list is sorted) form runs,
+// which a warp walks as one: lane groups are filled across leaf boundaries
+// (leaves of about a dozen particles leave 40% of them idle otherwise).
 //
 // The packed kernel (field orders 0 and 1, all kernels but erf) evaluates
 // each target against two sources at once in f32x2 arithmetic from a second
 // record array with even leaf starts and interleaved slot pairs, and, with
-// learned lists on AMOEBA, walks a damping-correction list after the near
-// list: far leaf pairs inside the damping range, of which only the pairs
+// learned lists on AMOEBA, a second launch walks a damping-correction list:
+// far leaf pairs inside the damping range, of which only the pairs
 // with a r below the range's cutoff are evaluated, as the difference of the
 // damped and undamped kernels (the M2L carries the undamped one).
 #include <algorithm>
+#include <climits>
+#include <cmath>
 #include <cstdlib>
 
 #include <cub/cub.cuh>
@@ -34,7 +39,7 @@ namespace {
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
-constexpr int kExwRegs = 8;  // exclusion entries held in registers per target
+constexpr int kExwRegs = 4;  // exclusion entries held in registers per target
 
 // Sub-chunks of a target leaf's last rem < 32 particles (index rem): the
 // count that minimises the lane-steps of a piece of source blocks for leaves
@@ -46,22 +51,23 @@ __constant__ int kSubChunks[32] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 2, 1, 1, 
 // Per sorted particle, one record of float4s: (x, y, z, d), (x_lo, y_lo, z_lo,
 // original index + 1 as int bits), then the FP32 scaled multipoles padded to
 // a multiple of 4 (for quadrupoles the first pad slot holds the trace of the
-// scaled second moments, used by the near-field contraction).  Positions are relative to the particle's own leaf centre
-// as double-float pairs (hi = rounded value, lo = rounded remainder), so
-// differences of positions in two leaves lose nothing beyond the final FP32
-// rounding.  A source is then read with a handful of 16-byte loads from one
-// base address.
+// scaled second moments, used by the near-field contraction).  Positions are
+// relative to the root centre (leaf: to the particle's own leaf centre, the
+// records of the selector's kernels) as double-float pairs (hi = rounded value,
+// lo = rounded remainder).  A source is then read with a handful of 16-byte
+// loads from one base address.
 __host__ __device__ constexpr int rec_vec(int dim) { return 2 + (dim + 3) / 4; }
 
-__global__ void k_gather_f32(int64_t n, int dim, const TreeDev t, const double* __restrict__ sx,
+__global__ void k_gather_f32(int64_t n, int dim, bool leaf, const TreeDev t, const double* __restrict__ sx,
                              const double* __restrict__ sy, const double* __restrict__ sz,
                              const double* __restrict__ sd, const double* __restrict__ smc,
                              float4* __restrict__ rec) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int nv = rec_vec(dim);
-    const int leaf = t.leaf_of[k];
-    const double rx = sx[k] - t.cx[leaf], ry = sy[k] - t.cy[leaf], rz = sz[k] - t.cz[leaf];
+    const int l = leaf ? t.leaf_of[k] : 0;
+    const double rx = sx[k] - (leaf ? t.cx[l] : t.root_c[0]), ry = sy[k] - (leaf ? t.cy[l] : t.root_c[1]),
+                 rz = sz[k] - (leaf ? t.cz[l] : t.root_c[2]);
     const float hx = (float)rx, hy = (float)ry, hz = (float)rz;
     float4* r = rec + (size_t)k * nv;
     r[0] = make_float4(hx, hy, hz, (float)sd[k]);
@@ -81,8 +87,8 @@ __global__ void k_gather_f32(int64_t n, int dim, const TreeDev t, const double* 
 
 // Source records of the packed near field: the sorted particles of each leaf
 // from an even slot ps[leaf] on, an odd leaf padded by one empty particle
-// (zero multipoles, 1000 bohr from its leaf centre, damping factor 1: its
-// pair terms are exactly zero); slots 2b and 2b + 1 form block b, stored
+// (zero multipoles, at least 1000 bohr from its leaf's last particle, damping
+// factor 1: its pair terms are exactly zero); slots 2b and 2b + 1 form block b, stored
 // element by element interleaved (float 2e + h of the block is element e of
 // the record of slot 2b + h), so one 16-byte shared-memory load gives two
 // elements of both particles as two packed pairs.
@@ -107,7 +113,9 @@ __global__ void k_gather_x2(int64_t n, int nv, bool q1, const TreeDev t, const i
     if (within == cnt - 1 && (cnt & 1)) {
         float* dd = d + 1;  // slot + 1: the odd half of the same block
         for (int e = 0; e < 4 * nv; ++e) dd[2 * e] = 0.0f;
-        dd[0] = 1000.0f;  // x
+        dd[0] = s[0] + fmaxf(1000.0f, fabsf(s[0]));  // x
+        dd[2] = s[1];
+        dd[4] = s[2];
         dd[2 * 3] = 1.0f; // damping factor
     }
 }
@@ -158,96 +166,44 @@ __global__ void k_node_centres_f32(int M, const TreeDev t, float4* __restrict__ 
                         (float)t.r[k]);
 }
 
-// a - b as an unevaluated pair s + e (Knuth's TwoSum with b negated).
-__device__ __forceinline__ float two_diff(float a, float b, float& e) {
-    const float s = a - b;
-    const float bb = s - a;
-    e = (a - (s - bb)) - (b + bb);
-    return s;
+// One target's position and the sorted positions (slots) that it passes over.
+struct Target {
+    float4 a, b;          // the record's first two float4s
+    int slot;             // its own slot
+    int ex[kExwRegs];     // slots of the excluded partners listed first (-1: none)
+    int lo, hi;           // range of the slots of the others
+    int orig;             // original index
+};
+
+// First block of a piece that lane group grp of ngr takes: block b of the sorted
+// slots is group b mod ngr's, so that sums do not depend on where pieces end.
+__device__ __forceinline__ int first_block(int b0, int grp, int ngr) {
+    const int d = grp - b0 % ngr;
+    return d < 0 ? d + ngr : d;
 }
 
-// FP32 field estimate at a few targets over all sources (exclusions masked),
-// from the sorted FP32 records; only a magnitude is wanted (the learned
-// selector's error budget).  Block per (target, source split); block sums
-// added into out (ntgt x nF, column-major, zeroed by the caller).
-template <int M, int F>
-__global__ void __launch_bounds__(128) k_direct_scale(const TreeDev t, const float4* __restrict__ rec,
-                                                      const float4* __restrict__ chi,
-                                                      const int64_t* __restrict__ targets, int64_t ntgt, int64_t n,
-                                                      int damp, int exw, const int32_t* __restrict__ excl,
-                                                      int64_t chunk, double* __restrict__ out) {
-    constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM);
-    __shared__ float red[NF][4];
-    const int64_t ti = blockIdx.x;
-    const int64_t i = targets[ti];
-    const int it = t.pos_of[i];
-    const float4 ta = rec[(size_t)it * NV], ca = chi[t.leaf_of[it]];
-    const float tx = ta.x + ca.x, ty = ta.y + ca.y, tz = ta.z + ca.z;
-    float acc[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0f;
-    const int64_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    for (int64_t k = j0 + threadIdx.x; k < j1; k += blockDim.x) {
-        if (k == it) continue;
-        const float4* r = rec + (size_t)k * NV;
-        const float4 sa = r[0], sb = r[1];
-        const int o = __float_as_int(sb.w);
-        bool ex = false;
-        for (int e = 0; e < exw; ++e) ex |= (excl[(size_t)e * n + i] == o);
-        if (ex) continue;
-        const float4 cb = chi[t.leaf_of[k]];
-        float mc[4 * (NV - 2)];
-#pragma unroll
-        for (int v = 0; v < NV - 2; ++v) {
-            const float4 w = r[2 + v];
-            mc[4 * v] = w.x;
-            mc[4 * v + 1] = w.y;
-            mc[4 * v + 2] = w.z;
-            mc[4 * v + 3] = w.w;
-        }
-        pair_field<M, F, float>(tx - (sa.x + cb.x), ty - (sa.y + cb.y), tz - (sa.z + cb.z), ta.w * sa.w, damp, mc,
-                                acc);
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        float v = acc[f];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[f][w] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < NF) {
-        const int f = threadIdx.x;
-        atomicAdd(&out[(size_t)f * ntgt + ti], (double)((red[f][0] + red[f][1]) + (red[f][2] + red[f][3])));
-    }
-}
-
-// Sum over the sources src[0, cnt) of one staged piece of a source leaf
-// (lane group grp of ngr) for the lane's target: compensated FP32 (TwoSum
-// hi + lo), since the per-atom terms are much larger than their neutral
-// total.  The contraction adds each pair into a plain FP32 block sum that
-// is folded into (hi, lo) every four pairs: the block sum's rounding is of
-// the order of a single pair's, and the TwoSum cost is paid once per four
-// pairs.  k0 is the sorted index of src[0].  CHECK: the piece may hold the
+// Sum over the sources src[0, cnt) of one staged piece (lane group grp of ngr)
+// for the lane's target: compensated FP32 (TwoSum hi + lo), since the per-atom
+// terms are much larger than their neutral total.  The contraction adds each
+// pair into a plain FP32 block sum (blk, of nb pairs so far, kept from piece to
+// piece) that is folded into (hi, lo) every four pairs: the block sum's
+// rounding is of the order of a single pair's, and the TwoSum cost is paid once
+// per four pairs.  k0 is the slot of src[0].  CHECK: the piece may hold the
 // target itself or one of its excluded partners.
 template <int M, int F, int DAMP, bool CHECK>
-__device__ __forceinline__ void p2p_leaf(const float4* src, int cnt, int k0, int grp, int ngr, int tgt, float xt,
-                                         float yt, float zt, float dt, float ox, float oy, float oz, float oxl,
-                                         float oyl, float ozl, const int32_t* __restrict__ excl, int exw, int64_t n,
-                                         int ot, float* hi, float* lo) {
+__device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, int grp, int ngr, const Target& T,
+                                          const int32_t* __restrict__ excl, int exw, int64_t n, float* hi, float* lo,
+                                          float* blk, int& nb) {
     constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM);
-    float blk[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) blk[f] = 0.0f;
-    int nb = 0;
-    for (int k = grp; k < cnt; k += ngr) {
+    for (int k = first_block(k0, grp, ngr); k < cnt; k += ngr) {
         const float4* r = src + k * NV;
         const float4 a = r[0], b = r[1];
         if (CHECK) {
-            if (k0 + k == tgt) continue;
             const int o = __float_as_int(b.w);
-            bool skip = false;
-            for (int e = 0; e < exw; ++e) skip |= (excl[(size_t)e * n + ot] == o);
+            bool skip = k0 + k == T.slot;
+#pragma unroll
+            for (int e = 0; e < kExwRegs; ++e) skip |= k0 + k == T.ex[e];
+            for (int e = kExwRegs; e < exw; ++e) skip |= (excl[(size_t)e * n + T.orig] == o);
             if (skip) continue;
         }
         float mc[4 * (NV - 2)];
@@ -259,10 +215,10 @@ __device__ __forceinline__ void p2p_leaf(const float4* src, int cnt, int k0, int
             mc[4 * v + 2] = w.z;
             mc[4 * v + 3] = w.w;
         }
-        const float dx = ((xt - a.x) + ox) + (oxl - b.x);
-        const float dy = ((yt - a.y) + oy) + (oyl - b.y);
-        const float dz = ((zt - a.z) + oz) + (ozl - b.z);
-        pair_field_f32acc<M, F>(dx, dy, dz, dt * a.w, DAMP, mc, blk);
+        const float dx = (T.a.x - a.x) + (T.b.x - b.x);
+        const float dy = (T.a.y - a.y) + (T.b.y - b.y);
+        const float dz = (T.a.z - a.z) + (T.b.z - b.z);
+        pair_field_f32acc<M, F>(dx, dy, dz, T.a.w * a.w, DAMP, mc, blk);
         if (++nb == 4) {
             nb = 0;
 #pragma unroll
@@ -275,42 +231,36 @@ __device__ __forceinline__ void p2p_leaf(const float4* src, int cnt, int k0, int
             }
         }
     }
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        const float s = hi[f] + blk[f];
-        const float bb = s - hi[f];
-        lo[f] += (hi[f] - (s - bb)) + (blk[f] - bb);
-        hi[f] = s;
-    }
 }
 
-// p2p_leaf on the packed records (k_gather_x2): blocks b = grp, grp + ngr,
+// p2p_piece on the packed records (k_gather_x2): blocks b = grp, grp + ngr,
 // ... of the staged piece, each the lane's target against two sources in
 // packed arithmetic.  Each half keeps its own compensated sum (H, L) over all
-// pieces of the target chunk, fed from a plain block sum B folded every four
-// blocks (four pairs per fold per half, as in the scalar loop).  The target
-// position enters as xo = x_t + (c_A - c_B)_hi per piece and the low parts as
-// oxl, so R = (xo - x_s) + (oxl - x_s,lo).  k0 is the sorted index of slot 0.
+// pieces of the target chunk, fed from a plain block sum B (of nb blocks so far)
+// folded every four blocks (four pairs per fold per half, as in the scalar
+// loop).  k0 is the slot
+// of the piece's first source.
 // CORR (a piece of a far leaf inside the damping range): only the damping
 // correction (damped minus undamped kernel) of the pairs with (a r)^2 below
 // xcut2, beyond which the damped kernel equals the undamped one to the
-// requested accuracy; a block is skipped when no lane has such a pair.
+// requested accuracy; a block is skipped when no lane has such a pair.  (A pair
+// evaluated with another lane's loses its undamped potential too, which AMOEBA
+// damping leaves undefined: which pairs those are is part of the result, so
+// correction pieces are single leaves, their blocks counted from the leaf's
+// start and their test made on leaf-relative positions, whatever the runs.)
 template <int M, int F, int DAMP, bool CHECK, bool CORR = false>
-__device__ __forceinline__ void p2p_leaf_x2(const float4* src, int nblk, int k0, int grp, int ngr, int tgt, f2 xo,
-                                            f2 yo, f2 zo, f2 dt, f2 oxl, f2 oyl, f2 ozl,
-                                            const int32_t* __restrict__ excl, int exw, int64_t n, int ot, f2* H,
-                                            f2* L, float xcut2 = 0.0f, int* ncorr = nullptr) {
+__device__ __forceinline__ void p2p_piece_x2(const float4* src, int nblk, int k0, int grp, int ngr, const Target& T,
+                                             const int32_t* __restrict__ excl, int exw, int64_t n, f2* H, f2* L,
+                                             f2* B, int& nb, float xcut2 = 0.0f, int* ncorr = nullptr) {
     constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM), NE = 4 * (NV - 2);
-    f2 B[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) B[f] = bc2(0.0f);
-    int nb = 0;
-    for (int b = grp; b < nblk; b += ngr) {
+    const f2 xt = bc2(T.a.x), yt = bc2(T.a.y), zt = bc2(T.a.z), dt = bc2(T.a.w);
+    const f2 xl = bc2(T.b.x), yl = bc2(T.b.y), zl = bc2(T.b.z);
+    for (int b = CORR ? grp : first_block(k0 >> 1, grp, ngr); b < nblk; b += ngr) {
         const ulonglong2* r = reinterpret_cast<const ulonglong2*>(src + (size_t)b * 2 * NV);
         // element pairs: (x, y), (z, d), (x_lo, y_lo), (z_lo, index), multipoles
         const ulonglong2 v0 = r[0], v1 = r[1];
         if constexpr (CORR) {
-            const f2 cx = xo - f2{v0.x}, cy = yo - f2{v0.y}, cz = zo - f2{v1.x};
+            const f2 cx = xt - f2{v0.x}, cy = yt - f2{v0.y}, cz = zt - f2{v1.x};
             const f2 aa = dt * f2{v1.y};
             const f2 tt = (aa * aa) * fma2(cx, cx, fma2(cy, cy, cz * cz));
             float t0, t1;
@@ -326,19 +276,26 @@ __device__ __forceinline__ void p2p_leaf_x2(const float4* src, int nblk, int k0,
             mc[2 * v].v = w.x;
             mc[2 * v + 1].v = w.y;
         }
-        f2 dx = (xo - f2{v0.x}) + (oxl - f2{v2.x});
-        const f2 dy = (yo - f2{v0.y}) + (oyl - f2{v2.y});
-        const f2 dz = (zo - f2{v1.x}) + (ozl - f2{v3.x});
+        f2 dx = (xt - f2{v0.x}) + (xl - f2{v2.x});
+        const f2 dy = (yt - f2{v0.y}) + (yl - f2{v2.y});
+        const f2 dz = (zt - f2{v1.x}) + (zl - f2{v3.x});
         const f2 a = dt * f2{v1.y};
         if (CHECK) {
-            float o0, o1;
-            sp2(f2{v3.y}, o0, o1);
             const int k = k0 + 2 * b;
-            bool s0 = k == tgt, s1 = k + 1 == tgt;
-            for (int e = 0; e < exw; ++e) {
-                const int x = excl[(size_t)e * n + ot];
-                s0 |= x == __float_as_int(o0);
-                s1 |= x == __float_as_int(o1);
+            bool s0 = k == T.slot, s1 = k + 1 == T.slot;
+#pragma unroll
+            for (int e = 0; e < kExwRegs; ++e) {
+                s0 |= k == T.ex[e];
+                s1 |= k + 1 == T.ex[e];
+            }
+            if (exw > kExwRegs) {
+                float o0, o1;
+                sp2(f2{v3.y}, o0, o1);
+                for (int e = kExwRegs; e < exw; ++e) {
+                    const int x = excl[(size_t)e * n + T.orig];
+                    s0 |= x == __float_as_int(o0);
+                    s1 |= x == __float_as_int(o1);
+                }
             }
             if (s0 || s1) {
                 // a skipped half gets zero multipoles at a finite distance
@@ -363,18 +320,11 @@ __device__ __forceinline__ void p2p_leaf_x2(const float4* src, int nblk, int k0,
             }
         }
     }
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        const f2 s = H[f] + B[f];
-        const f2 bb = s - H[f];
-        L[f] += (H[f] - (s - bb)) + (B[f] - bb);
-        H[f] = s;
-    }
 }
 
 // Source records are staged per warp in shared memory, double-buffered:
-// while one piece (a source leaf, or `stage` / NV of its particles when it
-// is larger) is evaluated, the next is copied with cp.async.  The staging
+// while one piece (a run of source leaves, or `stage` / NV of its particles when
+// it is longer) is evaluated, the next is copied with cp.async.  The staging
 // size (float4s per buffer) is a launch parameter (dynamic shared memory).
 constexpr int kStage = 320;  // default float4s per staging buffer
 
@@ -386,36 +336,67 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// One warp per target leaf, its particles across the lanes (for leaves of
-// fewer than 32 particles, groups of lanes split each source piece).
-// Source leaves that hold neither the target nor an excluded partner of any
-// of the warp's targets run without the exclusion test.
+// a - b as an unevaluated pair s + e (Knuth's TwoSum with b negated).
+__device__ __forceinline__ float two_diff(float a, float b, float& e) {
+    const float s = a - b;
+    const float bb = s - a;
+    e = (a - (s - bb)) - (b + bb);
+    return s;
+}
+
+// The damping-correction list's data: the targets in the selector's records
+// (positions relative to the leaf centres, as the sources' packed ones) and what
+// its leaves are passed over by.
+struct CorrArgs {
+    float xcut2;
+    unsigned long long* count;
+    float4 root;          // root centre; w: what rounding may take from a distance
+    const float4 *chi, *clo;  // node centres (hi, lo)
+    const float2* ext;    // leaf extents and smallest damping factors
+    const float4* rec;
+};
+
+// A warp's walk over a target leaf's list: 32 entries are looked up at a time,
+// one per lane, and near entries whose slots follow one another are merged into
+// runs.  All members but a, e, j are the same in every lane.
+struct RunWalk {
+    int q, qend;            // next entry, the list's end
+    int a, e, j;            // this lane's entry: first slot, end, leaf
+    unsigned starts, keep;  // lanes that start a run, lanes with an entry
+};
+
+// One warp per item, a target leaf and a slice of its near list, the leaf's
+// particles across the lanes (chunks of fewer than 32 particles run several
+// lane groups, each taking every ngr-th block of a staged piece).
+// Pieces that hold neither the target nor an excluded partner of any of the
+// warp's targets run without the exclusion test.
 // DAMP is the damping kind as a template parameter: one specialised kernel
 // per kind keeps the pair loop free of kind dispatch and its code small.
-// Work: with `next` null, warp w takes leaf t.leaves[w]; otherwise the warps
-// stay resident and take leaves order[0], order[1], ... (the target leaves
-// by decreasing pair count) from the counter `next`, so the largest leaves
-// start first and the last wave is made of the smallest.
+// Work: with `next` null, warp w takes item w; otherwise the warps stay
+// resident and take items in order from the counter `next`, the leaves by
+// decreasing pair count (order), so the largest start first and the last wave
+// is made of the smallest.  Slice s of leaf l goes to out[s][f][particle];
+// systems of few leaves are split so that the items cover the GPU several
+// times (30,000 particles, order-1 sources: 1.83 ms with an item per leaf).
 // X2: sources from the packed records `srec` (k_gather_x2, padded leaf starts
 // sstart) evaluated two at a time; otherwise srec = rec, sstart = t.start.
-// With a damping-correction list (packed kernel, AMOEBA: t.corr_off) each
-// target chunk walks it after its near list, passing over the entries whose
-// leaf bound (lext) rules out a pair inside xcut2 for every lane, and counts
-// the corrected pairs into corr_count.
-template <int M, int F, int DAMP, bool X2>
+// CORR (packed kernel, AMOEBA): the damping-correction list (t.corr_off) in
+// place of the near list, passing over the entries whose leaf bound (C.ext)
+// rules out a pair inside xcut2 for every lane, the result added to out and the
+// corrected pairs counted into C.count.  (A kernel of its own: walked after the
+// near list in one kernel it cost that one registers, and spills.)
+template <int M, int F, int DAMP, bool X2, bool CORR>
 __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float4* __restrict__ rec,
                                                     const float4* __restrict__ srec,
                                                     const int32_t* __restrict__ sstart,
-                                                    const float4* __restrict__ chi, const float4* __restrict__ clo,
                                                     const int32_t* __restrict__ excl, int exw, int64_t n,
-                                                    double* __restrict__ fs, int stage,
+                                                    double* __restrict__ out, int stage, int slices,
                                                     const int32_t* __restrict__ order, unsigned* __restrict__ next,
-                                                    float xcut2, unsigned long long* __restrict__ corr_count,
-                                                    const float2* __restrict__ lext) {
+                                                    const CorrArgs C) {
     constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM);
-    // the damping-correction list is walked after the near list (packed
-    // kernel, AMOEBA)
-    constexpr bool kCorr = X2 && DAMP == DAMP_AMOEBA;
+    static_assert(!CORR || (X2 && DAMP == DAMP_AMOEBA), "corrections: packed kernel, AMOEBA");
+    const int32_t* const list_off = CORR ? t.corr_off : t.near_off;
+    const int32_t* const list_src = CORR ? t.corr_src : t.near_src;
     extern __shared__ __align__(16) float4 sbuf_p2p[];
     const int cap = X2 ? (stage / NV) & ~1 : stage / NV;  // particles (slots) per staged piece
     const int lane = threadIdx.x & 31;
@@ -423,217 +404,238 @@ __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float
     const int w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int ncorr = 0;  // corrected pairs evaluated by this lane
     for (int round = 0;; ++round) {
-    int item;
-    if (next) {
-        unsigned v = 0;
-        if (lane == 0) v = atomicAdd(next, 1u);
-        item = (int)__shfl_sync(0xffffffffu, v, 0);
-    } else {
-        if (round > 0) break;
-        item = w0;
-    }
-    if (item >= t.num_leaves) break;
-    const int leaf = order ? order[item] : t.leaves[item];
-    const int s0 = t.start[leaf], cnt = t.count[leaf];
-    const int q0 = t.near_off[leaf], nn = t.near_off[leaf + 1] - q0;
-    const int c0 = (kCorr && t.corr_off) ? t.corr_off[leaf] : 0;
-    const int q1 = nn + ((kCorr && t.corr_off) ? t.corr_off[leaf + 1] - c0 : 0);
-    // source leaf of list entry q: near entries [0, nn), then correction entries
-    auto src_of = [&](int q) { return q < nn ? t.near_src[q0 + q] : t.corr_src[c0 + q - nn]; };
-    const float4 ca = chi[leaf], cal = clo[leaf];
-    // chunks of 32 targets, then the remaining rem < 32 in cs sub-chunks of
-    // gs targets; a chunk of g targets runs ngr = 32 / g lane groups of g
-    // lanes (any g), each taking every ngr-th block of each staged piece
-    const int full = cnt >> 5, rem = cnt & 31;
-    const int cs = rem ? kSubChunks[rem] : 0, gs = rem ? (rem + cs - 1) / cs : 1;
-    for (int ci = 0; ci < full + cs; ++ci) {
-        const int chunk = ci < full ? 32 * ci : 32 * full + (ci - full) * gs;
-        const int g = ci < full ? 32 : gs;
-        const int nt = min(g, cnt - chunk);
-        const int ngr = 32 / g;
-        const int tl = lane % g, grp = lane / g;
-        const bool valid = tl < nt && grp < ngr;
-        const int tgt = s0 + chunk + (valid ? tl : 0);
-        const float4 ta = rec[(size_t)tgt * NV], tb = rec[(size_t)tgt * NV + 1];
-        const int ot = __float_as_int(tb.w) - 1;
-        // leaves of the target's excluded partners (-1: none)
-        int exl[kExwRegs];
-#pragma unroll
-        for (int e = 0; e < kExwRegs; ++e) {
-            int o = (e < exw) ? excl[(size_t)e * n + ot] : 0;
-            exl[e] = o > 0 ? t.leaf_of[t.pos_of[o - 1]] : -1;
+        int item;
+        if (next) {
+            unsigned v = 0;
+            if (lane == 0) v = atomicAdd(next, 1u);
+            item = (int)__shfl_sync(0xffffffffu, v, 0);
+        } else {
+            if (round > 0) break;
+            item = w0;
         }
-        // per-target sums over all source leaves as double-float pairs (FP32
-        // arithmetic; the FP64 pipe is the scarce one)
-        float AH[NF], AL[NF];
-        f2 XH[NF], XL[NF];  // packed kernel: one compensated sum per half
+        if (item >= t.num_leaves * slices) break;
+        const int slice = item % slices;
+        const int leaf = order ? order[item / slices] : t.leaves[item / slices];
+        const int s0 = t.start[leaf], cnt = t.count[leaf];
+        auto part = [&](int lo, int hi, int s) { return lo + (int)((int64_t)(hi - lo) * s / slices); };
+        const int n0 = list_off[leaf], n1 = list_off[leaf + 1];
+        const int q0 = part(n0, n1, slice), q1 = part(n0, n1, slice + 1);
+        if (CORR && q0 == q1) continue;
+        // chunks of 32 targets, then the remaining rem < 32 in cs sub-chunks of
+        // gs targets; a chunk of g targets runs ngr = 32 / g lane groups of g
+        // lanes (any g), each taking every ngr-th block of each staged piece
+        const int full = cnt >> 5, rem = cnt & 31;
+        const int cs = rem ? kSubChunks[rem] : 0, gs = rem ? (rem + cs - 1) / cs : 1;
+        for (int ci = 0; ci < full + cs; ++ci) {
+            const int chunk = ci < full ? 32 * ci : 32 * full + (ci - full) * gs;
+            const int g = ci < full ? 32 : gs;
+            const int nt = min(g, cnt - chunk);
+            const int ngr = 32 / g;
+            const int tl = lane % g, grp = lane / g;
+            const bool valid = tl < nt && grp < ngr;
+            const int tgt = s0 + chunk + (valid ? tl : 0);
+            Target T;
+            T.a = rec[(size_t)tgt * NV];
+            T.b = rec[(size_t)tgt * NV + 1];
+            T.orig = __float_as_int(T.b.w) - 1;
+            T.slot = sstart[leaf] + (tgt - s0);
+            auto slot_of = [&](int o) {  // -1: unused entry
+                if (o <= 0) return -1;
+                const int pos = t.pos_of[o - 1], l = t.leaf_of[pos];
+                return sstart[l] + (pos - t.start[l]);
+            };
 #pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            AH[f] = AL[f] = 0.0f;
-            XH[f] = XL[f] = bc2(0.0f);
-        }
-        // current piece (q, off) of source leaf j = [js, js + jc); the first
-        // one is staged before the loop
-        // correction entries whose leaf cannot hold a pair that needs a
-        // correction for any of this chunk's targets are passed over without
-        // staging: for target t and leaf B, a r >= d_t dmin_B (|x_t - c_B| -
-        // extent_B) (all lanes take part)
-        auto next_entry = [&](int q) {
-            if constexpr (kCorr) {
-                const float txa = ta.x + ca.x, tya = ta.y + ca.y, tza = ta.z + ca.z;
-                while (q < q1 && q >= nn) {
-                    const int B = t.corr_src[c0 + q - nn];
-                    bool need = false;
-                    if (valid) {
-                        const float4 cb = chi[B];
-                        const float2 eb = lext[B];
-                        const float dx = txa - cb.x, dy = tya - cb.y, dz = tza - cb.z;
-                        const float rmin = fmaxf(sqrtf(dx * dx + dy * dy + dz * dz) - eb.x - 1e-2f, 0.0f);
-                        const float xm = ta.w * eb.y * rmin;
-                        need = xm * xm < xcut2;
+            for (int e = 0; e < kExwRegs; ++e) T.ex[e] = e < exw ? slot_of(excl[(size_t)e * n + T.orig]) : -1;
+            T.lo = INT_MAX;
+            T.hi = -1;
+            for (int e = kExwRegs; e < exw; ++e) {
+                const int x = slot_of(excl[(size_t)e * n + T.orig]);
+                if (x >= 0) T.lo = min(T.lo, x);
+                T.hi = max(T.hi, x);
+            }
+            // per-target sums over all source leaves as double-float pairs (FP32
+            // arithmetic; the FP64 pipe is the scarce one)
+            float AH[NF], AL[NF], AB[NF];
+            f2 XH[NF], XL[NF], XB[NF];  // packed kernel: one compensated sum per half
+            int nb = 0;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                AH[f] = AL[f] = AB[f] = 0.0f;
+                XH[f] = XL[f] = XB[f] = bc2(0.0f);
+            }
+            RunWalk W{q0, q1, 0, 0, 0, 0u, 0u};
+            // looks up the next 32 entries; false at the end of the list
+            auto load_window = [&]() -> bool {
+                while (W.q < W.qend) {
+                    const int q = W.q + lane;
+                    const bool ok = q < W.qend;
+                    W.a = W.e = W.j = 0;
+                    if (ok) {
+                        W.j = list_src[q];
+                        int c = t.count[W.j];
+                        if (X2) c += c & 1;  // padded to whole blocks
+                        W.a = sstart[W.j];
+                        W.e = W.a + c;
                     }
-                    if (__any_sync(0xffffffffu, need)) break;
-                    ++q;
+                    W.keep = __ballot_sync(0xffffffffu, ok);
+                    if constexpr (CORR) {
+                        // entries whose leaf cannot hold a pair that needs a
+                        // correction for any of this chunk's targets: for target t
+                        // and leaf B, a r >= d_t dmin_B (|x_t - c_B| - extent_B)
+                        // (all lanes take part)
+                        const int ne = __popc(W.keep);
+                        unsigned keep = 0;
+                        for (int l = 0; l < ne; ++l) {
+                            const int Bn = __shfl_sync(0xffffffffu, W.j, l);
+                            bool need = false;
+                            if (valid) {
+                                const float4 cb = C.chi[Bn];
+                                const float2 eb = C.ext[Bn];
+                                const float dx = (T.a.x + C.root.x) - cb.x, dy = (T.a.y + C.root.y) - cb.y,
+                                            dz = (T.a.z + C.root.z) - cb.z;
+                                const float rmin = fmaxf(sqrtf(dx * dx + dy * dy + dz * dz) - eb.x - C.root.w, 0.0f);
+                                const float xm = T.a.w * eb.y * rmin;
+                                need = xm * xm < C.xcut2;
+                            }
+                            if (__any_sync(0xffffffffu, need)) keep |= 1u << l;
+                        }
+                        W.keep = keep;
+                    }
+                    W.q += 32;
+                    if (!W.keep) continue;
+                    const int pe = __shfl_up_sync(0xffffffffu, W.e, 1);
+                    const bool follows = !CORR && lane > 0 && ((W.keep >> (lane - 1)) & 1u) && pe == W.a;
+                    W.starts = __ballot_sync(0xffffffffu, ((W.keep >> lane) & 1u) && !follows);
+                    return true;
                 }
-            }
-            return q;
-        };
-        int q = next_entry(0), off = 0, j = 0, js = 0, jc = 0;
-        if (q < q1) {
-            j = src_of(q);
-            js = sstart[j];
-            jc = t.count[j];
-            if (X2) jc += jc & 1;  // padded to whole blocks
-            const int pc = min(cap, jc);
-            for (int i = lane; i < pc * NV; i += 32) cp_async16(&bufs[i], srec + (size_t)js * NV + i);
-        }
-        cp_async_commit();
-        int slot = 0;
-        while (q < q1) {
-            // stage the next piece
-            int nq = q, noff = off + cap, nj = j, njs = js, njc = jc;
-            if (noff >= jc) {
-                nq = next_entry(q + 1);
-                noff = 0;
-                if (nq < q1) {
-                    nj = src_of(nq);
-                    njs = sstart[nj];
-                    njc = t.count[nj];
-                    if (X2) njc += njc & 1;
-                }
-            }
-            if (nq < q1) {
-                const int npc = min(cap, njc - noff);
-                const float4* gsrc = srec + (size_t)(njs + noff) * NV;
-                float4* dst = bufs + (slot ^ 1) * stage;
-                for (int i = lane; i < npc * NV; i += 32) cp_async16(&dst[i], gsrc + i);
+                return false;
+            };
+            // next run of slots [rs, re) (CORR: of leaf rj); false at the end of the
+            // list
+            auto next_run = [&](int& rs, int& re, int& rj) -> bool {
+                if (!W.starts && !load_window()) return false;
+                const int sl = __ffs(W.starts) - 1;
+                W.starts &= W.starts - 1;
+                const unsigned stop = (W.starts | ~W.keep) & ~((2u << sl) - 1u);
+                const int el = stop ? __ffs(stop) - 2 : 31;
+                rs = __shfl_sync(0xffffffffu, W.a, sl);
+                re = __shfl_sync(0xffffffffu, W.e, el);
+                if (CORR) rj = __shfl_sync(0xffffffffu, W.j, sl);
+                return true;
+            };
+            // current piece [ps, ps + pl) of run [.., re); the first one is staged
+            // before the loop
+            int ps = 0, re = 0, pl = 0, pj = 0;
+            bool have = next_run(ps, re, pj);
+            if (have) {
+                pl = min(cap, re - ps);
+                const float4* gsrc = srec + (size_t)ps * NV;
+                for (int i = lane; i < pl * NV; i += 32) cp_async16(&bufs[i], gsrc + i);
             }
             cp_async_commit();
-            cp_async_wait_prev();
-            __syncwarp();
-            if (valid) {
-                // leaf-centre offset c_A - c_B as hi + lo; the low parts are
-                // folded with the target's low parts
-                const float4 cb = chi[j], cbl = clo[j];
-                float ex, ey, ez;
-                const float ox = two_diff(ca.x, cb.x, ex), oy = two_diff(ca.y, cb.y, ey), oz = two_diff(ca.z, cb.z, ez);
-                const float oxl = (ex + (cal.x - cbl.x)) + tb.x, oyl = (ey + (cal.y - cbl.y)) + tb.y,
-                            ozl = (ez + (cal.z - cbl.z)) + tb.z;
-                bool need = (j == leaf) || exw > kExwRegs;
+            int slot = 0;
+            while (have) {
+                // stage the next piece
+                int nps = ps + pl, nre = re, npj = pj;
+                bool more = nps < re;
+                if (!more) more = next_run(nps, nre, npj);
+                const int npl = more ? min(cap, nre - nps) : 0;
+                if (more) {
+                    const float4* gsrc = srec + (size_t)nps * NV;
+                    float4* dst = bufs + (slot ^ 1) * stage;
+                    for (int i = lane; i < npl * NV; i += 32) cp_async16(&dst[i], gsrc + i);
+                }
+                cp_async_commit();
+                cp_async_wait_prev();
+                __syncwarp();
+                if (valid) {
+                    bool need = (unsigned)(T.slot - ps) < (unsigned)pl || (T.hi >= ps && T.lo < ps + pl);
 #pragma unroll
-                for (int e = 0; e < kExwRegs; ++e) need |= (exl[e] == j);
-                const int pc = min(cap, jc - off);
-                const float4* cur = bufs + slot * stage;
-                const int k0 = (X2 ? t.start[j] : js) + off;  // sorted index of the piece's first slot
-                if constexpr (X2) {
-                    const f2 xo = bc2(ta.x + ox), yo = bc2(ta.y + oy), zo = bc2(ta.z + oz), dt = bc2(ta.w);
-                    const f2 oxl2 = bc2(oxl), oyl2 = bc2(oyl), ozl2 = bc2(ozl);
+                    for (int e = 0; e < kExwRegs; ++e) need |= (unsigned)(T.ex[e] - ps) < (unsigned)pl;
+                    const float4* cur = bufs + slot * stage;
                     const bool anyneed = __any_sync(__activemask(), need);
-                    if (kCorr && q >= nn) {
-                        if constexpr (kCorr) {
-                            if (anyneed)
-                                p2p_leaf_x2<M, F, DAMP, true, true>(cur, pc >> 1, k0, grp, ngr, tgt, xo, yo, zo, dt,
-                                                                    oxl2, oyl2, ozl2, excl, exw, n, ot, XH, XL, xcut2,
-                                                                    &ncorr);
-                            else
-                                p2p_leaf_x2<M, F, DAMP, false, true>(cur, pc >> 1, k0, grp, ngr, tgt, xo, yo, zo, dt,
-                                                                     oxl2, oyl2, ozl2, excl, exw, n, ot, XH, XL,
-                                                                     xcut2, &ncorr);
-                        }
-                    } else if (anyneed)
-                        p2p_leaf_x2<M, F, DAMP, true>(cur, pc >> 1, k0, grp, ngr, tgt, xo, yo, zo, dt, oxl2, oyl2,
-                                                      ozl2, excl, exw, n, ot, XH, XL);
-                    else
-                        p2p_leaf_x2<M, F, DAMP, false>(cur, pc >> 1, k0, grp, ngr, tgt, xo, yo, zo, dt, oxl2, oyl2,
-                                                       ozl2, excl, exw, n, ot, XH, XL);
-                } else {
-                    float hi[NF], lo[NF];
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) hi[f] = lo[f] = 0.0f;
-                    if (__any_sync(__activemask(), need))
-                        p2p_leaf<M, F, DAMP, true>(cur, pc, k0, grp, ngr, tgt, ta.x, ta.y, ta.z, ta.w, ox, oy, oz,
-                                                   oxl, oyl, ozl, excl, exw, n, ot, hi, lo);
-                    else
-                        p2p_leaf<M, F, DAMP, false>(cur, pc, k0, grp, ngr, tgt, ta.x, ta.y, ta.z, ta.w, ox, oy, oz,
-                                                    oxl, oyl, ozl, excl, exw, n, ot, hi, lo);
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        // (AH, AL) += (hi, lo)
-                        const float sum = AH[f] + hi[f];
-                        const float bb = sum - AH[f];
-                        const float err = (AH[f] - (sum - bb)) + (hi[f] - bb);
-                        AH[f] = sum;
-                        AL[f] += err + lo[f];
+                    if constexpr (CORR) {
+                        // the target relative to the source's leaf centre: the
+                        // centres' offset hi + lo, its low part with the target's
+                        const float4 ta = C.rec[(size_t)tgt * NV], tb = C.rec[(size_t)tgt * NV + 1];
+                        const float4 ca = C.chi[leaf], cal = C.clo[leaf], cb = C.chi[pj], cbl = C.clo[pj];
+                        float ex, ey, ez;
+                        const float ox = two_diff(ca.x, cb.x, ex), oy = two_diff(ca.y, cb.y, ey),
+                                    oz = two_diff(ca.z, cb.z, ez);
+                        Target U = T;
+                        U.a = make_float4(ta.x + ox, ta.y + oy, ta.z + oz, ta.w);
+                        U.b = make_float4((ex + (cal.x - cbl.x)) + tb.x, (ey + (cal.y - cbl.y)) + tb.y,
+                                          (ez + (cal.z - cbl.z)) + tb.z, 0.0f);
+                        if (anyneed)
+                            p2p_piece_x2<M, F, DAMP, true, true>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
+                                                                 XB, nb, C.xcut2, &ncorr);
+                        else
+                            p2p_piece_x2<M, F, DAMP, false, true>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
+                                                                  XB, nb, C.xcut2, &ncorr);
+                    } else if constexpr (X2) {
+                        if (anyneed)
+                            p2p_piece_x2<M, F, DAMP, true>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
+                        else
+                            p2p_piece_x2<M, F, DAMP, false>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
+                    } else {
+                        if (anyneed)
+                            p2p_piece<M, F, DAMP, true>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
+                        else
+                            p2p_piece<M, F, DAMP, false>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
                     }
                 }
+                __syncwarp();
+                ps = nps;
+                re = nre;
+                pl = npl;
+                pj = npj;
+                have = more;
+                slot ^= 1;
             }
+            cp_async_wait_all();
             __syncwarp();
-            q = nq;
-            off = noff;
-            j = nj;
-            js = njs;
-            jc = njc;
-            slot ^= 1;
-        }
-        cp_async_wait_all();
-        __syncwarp();
-        double acc[NF];
+            double acc[NF];
 #pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            if constexpr (X2) {
-                float h0, h1, l0, l1;
-                sp2(XH[f], h0, h1);
-                sp2(XL[f], l0, l1);
-                acc[f] = ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
+            for (int f = 0; f < NF; ++f) {
+                if constexpr (X2) {
+                    float h0, h1, l0, l1;
+                    sp2(XH[f], h0, h1);
+                    sp2(XL[f], l0, l1);
+                    float b0, b1;
+                    sp2(XB[f], b0, b1);
+                    acc[f] = ((double)h0 + (double)h1) + (((double)l0 + (double)l1) + ((double)b0 + (double)b1));
+                } else {
+                    acc[f] = (double)AH[f] + ((double)AL[f] + (double)AB[f]);
+                }
+            }
+            if ((g & (g - 1)) == 0) {
+                for (int o = g; o < 32; o <<= 1) {
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], o);
+                }
             } else {
-                acc[f] = (double)AH[f] + (double)AL[f];
+                // group 0 adds groups 1 .. ngr - 1 (lanes tl + k g)
+                double part_f[NF];
+#pragma unroll
+                for (int f = 0; f < NF; ++f) part_f[f] = acc[f];
+                for (int k = 1; k < ngr; ++k) {
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) acc[f] += __shfl_sync(0xffffffffu, part_f[f], (tl + k * g) & 31);
+                }
             }
-        }
-        if ((g & (g - 1)) == 0) {
-            for (int o = g; o < 32; o <<= 1) {
+            if (grp == 0 && valid) {
 #pragma unroll
-                for (int f = 0; f < NF; ++f) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], o);
+                for (int f = 0; f < NF; ++f) {
+                    double* o = out + ((size_t)slice * NF + f) * n + tgt;
+                    *o = CORR ? *o + acc[f] : acc[f];
+                }
             }
-        } else {
-            // group 0 adds groups 1 .. ngr - 1 (lanes tl + k g)
-            double part[NF];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) part[f] = acc[f];
-            for (int k = 1; k < ngr; ++k) {
-#pragma unroll
-                for (int f = 0; f < NF; ++f) acc[f] += __shfl_sync(0xffffffffu, part[f], (tl + k * g) & 31);
-            }
-        }
-        if (grp == 0 && valid) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f) fs[(size_t)f * n + tgt] = acc[f];
         }
     }
-    }
-    if (kCorr && corr_count) {
-        // every lane of the warp is here (leaves are taken per warp)
+    if (CORR) {
+        // every lane of the warp is here (items are taken per warp)
         const int sc = __reduce_add_sync(0xffffffffu, ncorr);
-        if ((threadIdx.x & 31) == 0 && sc) atomicAdd(corr_count, (unsigned long long)sc);
+        if ((threadIdx.x & 31) == 0 && sc) atomicAdd(C.count, (unsigned long long)sc);
     }
 }
 
@@ -689,7 +691,6 @@ __global__ void __launch_bounds__(128) k_leaf_field_scale(const TreeDev t, const
             bool ex = false;
             for (int e = 0; e < exw; ++e) ex |= (excl[(size_t)e * n + ot] == o);
             if (ex) continue;
-            const float4 cb = chi[t.leaf_of[q]];
             float mc[4 * (NV - 2)];
 #pragma unroll
             for (int v = 0; v < NV - 2; ++v) {
@@ -699,6 +700,7 @@ __global__ void __launch_bounds__(128) k_leaf_field_scale(const TreeDev t, const
                 mc[4 * v + 2] = wv.z;
                 mc[4 * v + 3] = wv.w;
             }
+            const float4 cb = chi[t.leaf_of[q]];
             const float dx = tx - (sa.x + cb.x), dy = ty - (sa.y + cb.y), dz = tz - (sa.z + cb.z);
             if constexpr (M == 2) {
                 // quadrupole sources: the dot-product contraction (the record's
@@ -747,42 +749,43 @@ __global__ void k_leaf_cost(const TreeDev t, uint32_t* __restrict__ cost, int32_
 }
 
 template <int M, int F, bool X2>
-void launch_p2p_kind(unsigned blocks, int threads, size_t smem, int stage, const int32_t* order, unsigned* next,
-                     cudaStream_t st, const TreeDev& t, const float4* rec, const float4* srec, const int32_t* sstart,
-                     const float4* chi, const float4* clo, const int32_t* excl, int exw, int64_t n, int damp,
-                     double* fs, float xcut2, unsigned long long* corr_count, const float2* lext) {
+void launch_p2p_kind(unsigned blocks, int threads, size_t smem, int stage, int slices, const int32_t* order,
+                     unsigned* next, cudaStream_t st, const TreeDev& t, const float4* rec, const float4* srec,
+                     const int32_t* sstart, const int32_t* excl, int exw, int64_t n, int damp, double* out,
+                     const CorrArgs& C) {
     if constexpr (X2 && F > 1) {
         return;  // not instantiated: the packed kernel is used for field orders 0 and 1
     } else {
-    switch (damp) {
-        case DAMP_AMOEBA:
-            k_p2p_f32<M, F, DAMP_AMOEBA, X2><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, chi, clo, excl, exw,
-                                                                              n, fs, stage, order, next, xcut2, corr_count, lext);
-            break;
-        case DAMP_THOLE:
-            k_p2p_f32<M, F, DAMP_THOLE, X2><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, chi, clo, excl, exw,
-                                                                             n, fs, stage, order, next, xcut2, corr_count, lext);
-            break;
-        case DAMP_ERF:
-            k_p2p_f32<M, F, DAMP_ERF, X2><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, chi, clo, excl, exw, n,
-                                                                           fs, stage, order, next, xcut2, corr_count, lext);
-            break;
-        default:
-            k_p2p_f32<M, F, DAMP_NONE, X2><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, chi, clo, excl, exw,
-                                                                            n, fs, stage, order, next, xcut2, corr_count, lext);
-            break;
+#define FMM_P2P_KIND(D)                                                                                              \
+    k_p2p_f32<M, F, D, X2, false><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out, stage,     \
+                                                                 slices, order, next, C)
+        switch (damp) {
+            case DAMP_AMOEBA: FMM_P2P_KIND(DAMP_AMOEBA); break;
+            case DAMP_THOLE: FMM_P2P_KIND(DAMP_THOLE); break;
+            case DAMP_ERF: FMM_P2P_KIND(DAMP_ERF); break;
+            default: FMM_P2P_KIND(DAMP_NONE); break;
+        }
+#undef FMM_P2P_KIND
     }
-    }
+}
+
+template <int M, int F>
+void launch_p2p_corr(unsigned blocks, int threads, size_t smem, int stage, const int32_t* order, unsigned* next,
+                     cudaStream_t st, const TreeDev& t, const float4* rec, const float4* srec, const int32_t* sstart,
+                     const int32_t* excl, int exw, int64_t n, double* out, const CorrArgs& C) {
+    if constexpr (F <= 1)
+        k_p2p_f32<M, F, DAMP_AMOEBA, true, true><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out,
+                                                                              stage, 1, order, next, C);
 }
 
 template <int M, int F, bool X2>
 const void* p2p_kernel(int damp) {
     if constexpr (X2 && F > 1) return nullptr;
     else
-    return damp == DAMP_AMOEBA  ? (const void*)k_p2p_f32<M, F, DAMP_AMOEBA, X2>
-           : damp == DAMP_THOLE ? (const void*)k_p2p_f32<M, F, DAMP_THOLE, X2>
-           : damp == DAMP_ERF   ? (const void*)k_p2p_f32<M, F, DAMP_ERF, X2>
-                                : (const void*)k_p2p_f32<M, F, DAMP_NONE, X2>;
+    return damp == DAMP_AMOEBA  ? (const void*)k_p2p_f32<M, F, DAMP_AMOEBA, X2, false>
+           : damp == DAMP_THOLE ? (const void*)k_p2p_f32<M, F, DAMP_THOLE, X2, false>
+           : damp == DAMP_ERF   ? (const void*)k_p2p_f32<M, F, DAMP_ERF, X2, false>
+                                : (const void*)k_p2p_f32<M, F, DAMP_NONE, X2, false>;
 }
 
 template <int M, int F>
@@ -793,6 +796,9 @@ int set_p2p_smem(size_t smem) {
                           p2p_kernel<M, F, true>(DAMP_THOLE),  p2p_kernel<M, F, true>(DAMP_ERF)};
     for (const void* fn : fns)
         if (fn) FMM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (F <= 1)
+        FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_p2p_f32<M, F, DAMP_AMOEBA, true, true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return FMM_OK;
 }
 
@@ -820,14 +826,18 @@ int num_sms_f32() {
 
 }  // namespace
 
-int prepare_f32_records(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st) {
+int prepare_f32_records(Workspace& ws, const Particles& P, const TreeDev& t, bool near, bool selector,
+                        cudaStream_t st) {
     const int64_t n = P.n;
     const int nv = rec_vec(P.dim);
-    FMM_TRY(ws.f32buf.ensure(sizeof(float4) * (size_t)n * nv));
-    count_launches(1);
-    k_gather_f32<<<grid_for(n, 256), 256, 0, st>>>(n, P.dim, t, ws.sx.as<double>(), ws.sy.as<double>(),
-                                                    ws.sz.as<double>(), ws.sd.as<double>(), ws.smc.as<double>(),
-                                                    ws.f32buf.as<float4>());
+    for (int leaf = near ? 0 : 1; leaf <= (selector ? 1 : 0); ++leaf) {
+        DevBuf& b = leaf ? ws.f32sel : ws.f32buf;
+        FMM_TRY(b.ensure(sizeof(float4) * (size_t)n * nv));
+        count_launches(1);
+        k_gather_f32<<<grid_for(n, 256), 256, 0, st>>>(n, P.dim, leaf != 0, t, ws.sx.as<double>(), ws.sy.as<double>(),
+                                                        ws.sz.as<double>(), ws.sd.as<double>(), ws.smc.as<double>(),
+                                                        b.as<float4>());
+    }
     FMM_TRY(ws.f32node.ensure(sizeof(float4) * 2 * (size_t)t.num_nodes));
     float4* chi = ws.f32node.as<float4>();
     count_launches(1);
@@ -840,32 +850,15 @@ int prepare_f32_records(Workspace& ws, const Particles& P, const TreeDev& t, cud
 int launch_leaf_extent(Workspace& ws, const Particles& P, const TreeDev& t, cudaStream_t st) {
     FMM_TRY(ws.leaf_ext.ensure(sizeof(float2) * (size_t)t.num_nodes));
     count_launches(1);
-    k_leaf_extent<<<grid_for((int64_t)t.num_leaves * 32, 128), 128, 0, st>>>(rec_vec(P.dim), t, ws.f32buf.as<float4>(),
+    k_leaf_extent<<<grid_for((int64_t)t.num_leaves * 32, 128), 128, 0, st>>>(rec_vec(P.dim), t, ws.f32sel.as<float4>(),
                                                                              ws.leaf_ext.as<float2>());
-    FMM_CUDA_TRY(cudaGetLastError());
-    return FMM_OK;
-}
-
-int launch_direct_scale_f32(Workspace& ws, const Particles& P, const TreeDev& t, int field_order, double* d_out,
-                            cudaStream_t st, int64_t ntgt, const int64_t* d_targets) {
-    const int m = dim_to_order(P.dim);
-    const int nf = nT(field_order);
-    FMM_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(double) * (size_t)nf * ntgt, st));
-    int64_t ks = std::max<int64_t>(1, (16LL * 152 + ntgt - 1) / ntgt);
-    ks = std::min<int64_t>(ks, std::max<int64_t>(1, P.n / 1024));
-    const int64_t chunk = (P.n + ks - 1) / ks;
-    const float4* chi = ws.f32node.as<float4>();
-    dim3 grid((unsigned)ntgt, (unsigned)ks);
-    FMM_MF_SWITCH(m, field_order,
-                  (k_direct_scale<MM, FF><<<grid, 128, 0, st>>>(t, ws.f32buf.as<float4>(), chi, d_targets, ntgt, P.n,
-                                                                 P.damp_type, P.exw, P.excl, chunk, d_out)));
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
 
 int launch_leaf_field_scale(Workspace& ws, const Particles& P, const TreeDev& t, float* d_scale, cudaStream_t st) {
     const int m = dim_to_order(P.dim);
-    const float4* rec = ws.f32buf.as<float4>();  // prepare_f32_records
+    const float4* rec = ws.f32sel.as<float4>();  // prepare_f32_records
     const float4* chi = ws.f32node.as<float4>();
     const unsigned blocks = grid_for((int64_t)t.num_leaves * 32, 128);
     switch (m) {
@@ -901,8 +894,6 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     const int64_t n = P.n;
     const int nf = nT(field_order);
     const float4* rec = ws.f32buf.as<float4>();  // prepare_f32_records
-    const float4* chi = ws.f32node.as<float4>();
-    const float4* clo = chi + t.num_nodes;
     FMM_TRY(ws.fsorted.ensure(sizeof(double) * (size_t)n * nf));
     const P2pShape sh = ws.p2p_shape.valid() ? ws.p2p_shape : P2pShape{};
     const size_t smem = sizeof(float4) * 2 * (size_t)sh.stage * (sh.threads / 32);
@@ -921,7 +912,23 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     unsigned long long* corr_count = ws.counters.as<unsigned long long>() + 9;
     FMM_CUDA_TRY(cudaMemsetAsync(corr_count, 0, sizeof(unsigned long long), st));
     // leaf extents: computed with the lists (launch_leaf_extent)
-    const float2* lext = t.ncorr > 0 ? ws.leaf_ext.as<float2>() : nullptr;
+    const double big = std::max({std::fabs(t.root_c[0]), std::fabs(t.root_c[1]), std::fabs(t.root_c[2])}) + t.root_r;
+    CorrArgs C{ws.corr_xcut2, corr_count,
+               make_float4((float)t.root_c[0], (float)t.root_c[1], (float)t.root_c[2], (float)(1e-2 + 1e-6 * big)),
+               ws.f32node.as<float4>(), ws.f32node.as<float4>() + t.num_nodes,
+               ws.leaf_ext.as<float2>(), ws.f32sel.as<float4>()};
+    // slices of the source lists: at least four items per resident warp (about
+    // 16 an SM), while a slice keeps eight list entries
+    int64_t slices = 1;
+    if (t.num_leaves > 0) {
+        slices = (4LL * 16 * num_sms_f32() + t.num_leaves - 1) / t.num_leaves;
+        slices = std::max<int64_t>(1, std::min<int64_t>({slices, t.nnear / (8LL * t.num_leaves), 16}));
+    }
+    double* out = ws.fsorted.as<double>();
+    if (slices > 1) {
+        FMM_TRY(ws.near_part.ensure(sizeof(double) * (size_t)slices * nf * n));
+        out = ws.near_part.as<double>();
+    }
     if (x2) {
         const int nv = rec_vec(P.dim);
         const int L = t.num_leaves;
@@ -941,14 +948,18 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
             count_launches(1);
             k_leaf_pstart<<<grid_for(L, 256), 256, 0, st>>>(t, pre, ps);
         }
-        count_launches(1);
-        k_gather_x2<<<grid_for(n, 256), 256, 0, st>>>(n, nv, P.dim == 10 && field_order == 1, t,
-                                                       ws.p2p_pad.as<int32_t>(), rec,
-                                                       reinterpret_cast<float*>(ws.f32x2.as<float4>()));
+        // (with a damping-correction list, a second set from the selector's records)
+        if (t.ncorr > 0) FMM_TRY(ws.f32x2c.ensure(sizeof(float4) * (size_t)(n + L + 1) * nv));
+        for (int c = 0; c < (t.ncorr > 0 ? 2 : 1); ++c) {
+            count_launches(1);
+            k_gather_x2<<<grid_for(n, 256), 256, 0, st>>>(n, nv, P.dim == 10 && field_order == 1, t,
+                                                           ws.p2p_pad.as<int32_t>(), c ? ws.f32sel.as<float4>() : rec,
+                                                           (c ? ws.f32x2c : ws.f32x2).as<float>());
+        }
     }
     const int32_t* order = nullptr;
     unsigned* next = nullptr;
-    unsigned blocks = grid_for((int64_t)t.num_leaves * 32, sh.threads);
+    unsigned blocks = grid_for((int64_t)t.num_leaves * slices * 32, sh.threads);
     if (sh.queue && t.num_leaves > 0) {
         // target leaves by decreasing pair work (structure: kept for replays)
         FMM_TRY(ws.counters.ensure(sizeof(unsigned long long) * 32));
@@ -979,15 +990,23 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     }
     if (x2) {
         FMM_MF_SWITCH(m, field_order,
-                      (launch_p2p_kind<MM, FF, true>(blocks, sh.threads, smem, sh.stage, order, next, st, t, rec,
-                                                     ws.f32x2.as<float4>(), ws.p2p_pad.as<int32_t>(), chi, clo,
-                                                     P.excl, P.exw, n, P.damp_type, ws.fsorted.as<double>(),
-                                                     ws.corr_xcut2, corr_count, lext)));
+                      (launch_p2p_kind<MM, FF, true>(blocks, sh.threads, smem, sh.stage, (int)slices, order, next, st,
+                                                     t, rec, ws.f32x2.as<float4>(), ws.p2p_pad.as<int32_t>(), P.excl,
+                                                     P.exw, n, P.damp_type, out, C)));
     } else {
         FMM_MF_SWITCH(m, field_order,
-                      (launch_p2p_kind<MM, FF, false>(blocks, sh.threads, smem, sh.stage, order, next, st, t, rec, rec,
-                                                      t.start, chi, clo, P.excl, P.exw, n, P.damp_type,
-                                                      ws.fsorted.as<double>(), 0.0f, nullptr, nullptr)));
+                      (launch_p2p_kind<MM, FF, false>(blocks, sh.threads, smem, sh.stage, (int)slices, order, next, st,
+                                                      t, rec, rec, t.start, P.excl, P.exw, n, P.damp_type, out, C)));
+    }
+    if (slices > 1) FMM_TRY(sum_slices(n * nf, (int)slices, out, ws.fsorted.as<double>(), st));
+    if (t.ncorr > 0) {
+        if (next) FMM_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned), st));
+        const unsigned cblocks = std::min(blocks, grid_for((int64_t)t.num_leaves * 32, sh.threads));
+        FMM_MF_SWITCH(m, field_order,
+                      (launch_p2p_corr<MM, FF>(next ? cblocks : grid_for((int64_t)t.num_leaves * 32, sh.threads),
+                                               sh.threads, smem, sh.stage, order, next, st, t, rec,
+                                               ws.f32x2c.as<float4>(), ws.p2p_pad.as<int32_t>(), P.excl, P.exw, n,
+                                               ws.fsorted.as<double>(), C)));
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
