@@ -58,6 +58,7 @@ struct TreeDev {
     // range, CSR by target leaf like the near list
     int64_t ncorr = 0;
     int32_t *corr_off = nullptr, *corr_src = nullptr;
+    int src_bits = 32;  // bits of a source in the pair keys of far_sorted / near_sorted
     // periodic boxes (build_images): the node arrays hold every node nimg = 27
     // times, image a's copies from a x num_nodes on with their centres displaced
     // by its shift (image 0: the central cell, the tree itself).  Targets are

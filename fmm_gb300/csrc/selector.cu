@@ -317,11 +317,11 @@ __global__ void k_pair_feats(const TreeDev t, const float* __restrict__ lnorm, c
     for (int k = 0; k < kMlpIn; ++k) feats[(size_t)q * kMlpIn + k] = x[k];
 }
 
-__global__ void k_unpack_far(int64_t nfar, const uint64_t* __restrict__ sorted, int2* __restrict__ out) {
+__global__ void k_unpack_far(int64_t nfar, int sb, const uint64_t* __restrict__ sorted, int2* __restrict__ out) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= nfar) return;
     const uint64_t v = sorted[k];
-    out[k] = make_int2((int)(v >> 36), (int)(v & 0xffffffffull));
+    out[k] = make_int2((int)(v >> (sb + 4)), (int)(v & ((1ull << sb) - 1)));
 }
 
 // ---------------------------------------------------------------- training
@@ -522,7 +522,7 @@ int selector_pair_data(Workspace& ws, const Particles& Pt, const TreeDev& t, int
 int selector_unpack_far(Workspace& ws, const TreeDev& t, int2* d_out, cudaStream_t st) {
     if (t.nfar <= 0) return FMM_OK;
     count_launches(1);
-    k_unpack_far<<<grid_for(t.nfar, 256), 256, 0, st>>>(t.nfar, ws.far_sorted.as<uint64_t>(), d_out);
+    k_unpack_far<<<grid_for(t.nfar, 256), 256, 0, st>>>(t.nfar, t.src_bits, ws.far_sorted.as<uint64_t>(), d_out);
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }

@@ -33,7 +33,7 @@
 
 #include "internal.h"
 #include "mlp.cuh"
-#include "pair.cuh"
+#include "pair_f64.cuh"
 
 namespace fmm {
 
@@ -133,21 +133,37 @@ __global__ void k_root(double* scalars, int64_t n, int ncrit, double* bd, int32_
     bi[5 * cap] = (n < ncrit) ? 1 : 0;  // leaf
 }
 
+// Integer that orders as the double does (-0 and NaN apart: callers add +0.0,
+// and a NaN, greater than nothing, maps below everything).
+__device__ __forceinline__ long long order_bits(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+// The descent's comparisons and halvings run on integers and its additions of
+// +-r on sign bits, which leaves 3 of 10 FP64 instructions per level (300,000
+// particles: 127 us before).
 __global__ void k_keys(const double* __restrict__ X, int64_t n, const double* __restrict__ scalars,
                        uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double x = X[i], y = X[n + i], z = X[2 * n + i];
-    double cx = scalars[0], cy = scalars[1], cz = scalars[2], r = scalars[3];
+    const long long nan_key = (long long)0x8000000000000000ull;
+    const long long xb = x == x ? order_bits(x + 0.0) : nan_key, yb = y == y ? order_bits(y + 0.0) : nan_key,
+                    zb = z == z ? order_bits(z + 0.0) : nan_key;
+    double cx = scalars[0] + 0.0, cy = scalars[1] + 0.0, cz = scalars[2] + 0.0, r = scalars[3];
     uint64_t key = 0;
 #pragma unroll 1
     for (int l = 0; l < kMaxDepth; ++l) {
-        const int o = (x > cx ? 1 : 0) | (y > cy ? 2 : 0) | (z > cz ? 4 : 0);
+        const int o = (xb > order_bits(cx) ? 1 : 0) | (yb > order_bits(cy) ? 2 : 0) | (zb > order_bits(cz) ? 4 : 0);
         key = (key << 3) | (uint64_t)o;
-        r = __dmul_rn(r, 0.5);
-        cx = __dadd_rn(cx, __dmul_rn(r, (o & 1) ? 1.0 : -1.0));
-        cy = __dadd_rn(cy, __dmul_rn(r, (o & 2) ? 1.0 : -1.0));
-        cz = __dadd_rn(cz, __dmul_rn(r, (o & 4) ? 1.0 : -1.0));
+        const int e = (__double2hiint(r) >> 20) & 0x7ff;
+        r = e > 1 && e < 0x7ff ? __hiloint2double(__double2hiint(r) - (1 << 20), __double2loint(r)) : __dmul_rn(r, 0.5);
+        // a sum of -0 and anything else, and an exact cancellation, is +0 or not
+        // zero: order_bits' case apart does not arise
+        cx = __dadd_rn(cx, (o & 1) ? r : -r);
+        cy = __dadd_rn(cy, (o & 2) ? r : -r);
+        cz = __dadd_rn(cz, (o & 4) ? r : -r);
     }
     keys[i] = key;
     vals[i] = (uint32_t)i;
@@ -315,6 +331,7 @@ __device__ __forceinline__ void emit_pair(bool skip, bool accept, int order, int
                                           uint64_t* __restrict__ nearp, int64_t cap_near,
                                           unsigned long long* counters, int lane, bool corr = false,
                                           uint64_t* __restrict__ corrp = nullptr, int64_t cap_corr = 0) {
+    const int sb = t.src_bits;
     const bool isfar = !skip && accept;
     const bool isnear = !skip && !accept && li && lj && !mixed;
     const bool refine = !skip && !accept && !isnear;
@@ -336,19 +353,19 @@ __device__ __forceinline__ void emit_pair(bool skip, bool accept, int order, int
     const unsigned long long kc = warp_alloc(&counters[5], iscorr ? 1u : 0u, lane);
     if (iscorr) {
         if (kc < (unsigned long long)cap_corr)
-            corrp[kc] = ((uint64_t)(uint32_t)i << 32) | (uint32_t)j;
+            corrp[kc] = ((uint64_t)(uint32_t)i << sb) | (uint32_t)j;
         else
             counters[3] = 1;
     }
     if (isfar) {
         if (kf < (unsigned long long)cap_far)
-            far[kf] = ((uint64_t)(uint32_t)i << 36) | ((uint64_t)(order & 15) << 32) | (uint32_t)j;
+            far[kf] = ((uint64_t)(uint32_t)i << (sb + 4)) | ((uint64_t)(order & 15) << sb) | (uint32_t)j;
         else
             counters[3] = 1;
     }
     if (isnear) {
         if (kn < (unsigned long long)cap_near)
-            nearp[kn] = ((uint64_t)(uint32_t)i << 32) | (uint32_t)j;
+            nearp[kn] = ((uint64_t)(uint32_t)i << sb) | (uint32_t)j;
         else
             counters[3] = 1;
     }
@@ -379,7 +396,6 @@ __global__ void k_list_iter(const int2* __restrict__ in, int nin, int2* __restri
         const double dx = __dsub_rn(t.cx[i], t.cx[j]);
         const double dy = __dsub_rn(t.cy[i], t.cy[j]);
         const double dz = __dsub_rn(t.cz[i], t.cz[j]);
-        const double r = norm2_3(dx, dy, dz);
         ri = t.rmax[i];
         rj = t.rmax[j];
         li = t.is_leaf[i] != 0;
@@ -391,11 +407,28 @@ __global__ void k_list_iter(const int2* __restrict__ in, int nin, int2* __restri
             if (si >= 0 && sj >= 0 && si != sj) skip = true;
             mixed = si < 0 || sj < 0;
         }
-        accept = !mixed && __dmul_rn(r, theta) > __dadd_rn(ri, rj);
-        if (accept && rdamp > 0.0) {
-            // closest possible particle distance: centre distance minus the cube circumradii
-            const double gap = __dsub_rn(r, __dmul_rn(1.7320508075688772, __dadd_rn(t.r[i], t.r[j])));
-            accept = gap >= rdamp;
+        // Both tests in FP32 first: norm2_3's divisions and root are some 60
+        // FP64 instructions a candidate (they took the kernel to 1.18 ms for
+        // 6.5e6 candidates at the FP64 pipe's rate).  The FP32 values are within
+        // 1e-6; only pairs within 1e-5 of equality (the exact ties of a cell
+        // grid) need the reference's rounding.
+        const float fx = f32_bits(fabs(dx)), fy = f32_bits(fabs(dy)), fz = f32_bits(fabs(dz));
+        const float rf = sqrtf(fx * fx + fy * fy + fz * fz), sumf = f32_bits(ri) + f32_bits(rj);
+        const float lhs = rf * (float)theta;
+        const float hif = f32_bits(t.r[i]), hjf = f32_bits(t.r[j]);
+        const float gap = rf - 1.7320508f * (hif + hjf), rd = (float)rdamp;
+        const bool range = rf > 1e-15f && rf < 1e15f && sumf > 1e-15f;
+        const bool sure = range && fabsf(lhs - sumf) > 1e-5f * sumf && (rdamp <= 0.0 || fabsf(gap - rd) > 1e-5f * (rf + rd));
+        if (sure) {
+            accept = !mixed && lhs > sumf && (rdamp <= 0.0 || gap >= rd);
+        } else {
+            const double r = norm2_3(dx, dy, dz);
+            accept = !mixed && __dmul_rn(r, theta) > __dadd_rn(ri, rj);
+            if (accept && rdamp > 0.0) {
+                // closest possible particle distance: centre distance minus the cube circumradii
+                const double gap64 = __dsub_rn(r, __dmul_rn(1.7320508075688772, __dadd_rn(t.r[i], t.r[j])));
+                accept = gap64 >= rdamp;
+            }
         }
     }
     emit_pair(skip, accept, order, i, j, li, lj, mixed, ri, rj, t, out, cap_out, far, cap_far, nearp, cap_near,
@@ -499,12 +532,12 @@ __global__ void __launch_bounds__(128) k_list_iter_learned(
               counters, lane, corr, corrp, cap_corr);
 }
 
-__global__ void k_split_pairs(int64_t m, const uint64_t* __restrict__ sorted, int32_t* __restrict__ src,
+__global__ void k_split_pairs(int64_t m, int sb, const uint64_t* __restrict__ sorted, int32_t* __restrict__ src,
                               uint8_t* __restrict__ ord) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= m) return;
-    src[k] = (int32_t)(sorted[k] & 0xffffffffull);
-    if (ord) ord[k] = (uint8_t)((sorted[k] >> 32) & 15ull);
+    src[k] = (int32_t)(sorted[k] & ((1ull << sb) - 1));
+    if (ord) ord[k] = (uint8_t)((sorted[k] >> sb) & 15ull);
 }
 
 __global__ void k_csr_offsets(int M, int64_t m, const uint64_t* __restrict__ sorted, int32_t* __restrict__ off,
@@ -523,11 +556,12 @@ __global__ void k_csr_offsets(int M, int64_t m, const uint64_t* __restrict__ sor
     off[i] = (int32_t)a;
 }
 
-__global__ void k_near_pair_count(int64_t m, const uint64_t* __restrict__ sorted, const int32_t* __restrict__ count,
+__global__ void k_near_pair_count(int64_t m, int sb, const uint64_t* __restrict__ sorted,
+                                  const int32_t* __restrict__ count,
                                   unsigned long long* out) {
     unsigned long long s = 0;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(sorted[k] >> 32), j = (int)(sorted[k] & 0xffffffffull);
+        const int i = (int)(sorted[k] >> sb), j = (int)(sorted[k] & ((1ull << sb) - 1));
         s += (unsigned long long)count[i] * (unsigned long long)count[j];
     }
     typedef cub::BlockReduce<unsigned long long, 256> BR;
@@ -842,6 +876,17 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
     const bool corr = tp.sel_params && tp.corr_mode && tp.mac_mode == 1 && tp.rdamp > 0.0 && tp.corr_ext;
     int64_t cap_corr = corr ? std::max<int64_t>({4096, cap_near, (int64_t)(ws.corr_pairs.cap / sizeof(uint64_t))}) : 0;
     unsigned long long* ctr = ws.counters.as<unsigned long long>();
+    // Pair keys: target << (4 + sb) | order << sb | source (far), target << sb |
+    // source (near), sb the bits of the largest source: only the bits that carry
+    // something are sorted (a digit pass is 8 bits; 28,764 nodes: 5 passes over
+    // the far pairs and 4 over the near ones, 7 and 6 with the source in 32 bits)
+    auto bits_of = [](int64_t count) {
+        int b = 1;
+        while (b < 31 && (1ll << b) < count) ++b;
+        return b;
+    };
+    const int tb_bits = bits_of(M), sb = bits_of((int64_t)M * t.nimg);
+    t.src_bits = sb;
     for (int attempt = 0; attempt < 8; ++attempt) {
         FMM_TRY(ws.front_a.ensure(sizeof(int2) * cap_front));
         FMM_TRY(ws.front_b.ensure(sizeof(int2) * cap_front));
@@ -900,14 +945,10 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
         t.ncorr = corr ? (int64_t)h[5] : 0;
         ws.list_candidates = candidates;
         ws.list_evals = (int64_t)h[4];
-        // sort both lists by (target, source) and build CSR offsets; the keys
-        // are target << 36 (far, with the order in bits 32-35) or << 32
-        // (near), so only the bits up to the largest node index are sorted
+        // sort both lists by (target, source) and build CSR offsets
         FMM_TRY(ws.far_sorted.ensure(sizeof(uint64_t) * std::max<int64_t>(1, t.nfar)));
         FMM_TRY(ws.near_sorted.ensure(sizeof(uint64_t) * std::max<int64_t>(1, t.nnear)));
-        int nbits = 1;
-        while (nbits < 31 && (1 << nbits) < M) ++nbits;
-        const int far_bits = std::min(64, 36 + nbits), near_bits = std::min(64, 32 + nbits);
+        const int far_bits = tb_bits + 4 + sb, near_bits = tb_bits + sb;
         size_t tb = 0, tb2 = 0;
         cub::DeviceRadixSort::SortKeys(nullptr, tb, ws.far_pairs.as<uint64_t>(), ws.far_sorted.as<uint64_t>(),
                                        (int)t.nfar, 0, far_bits, st);
@@ -931,18 +972,18 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
         t.near_off = t.near_src + std::max<int64_t>(1, t.nnear);
         if (t.nfar > 0) {
             count_launches(1);
-            k_split_pairs<<<grid_for(t.nfar, 256), 256, 0, st>>>(t.nfar, ws.far_sorted.as<uint64_t>(), t.far_src,
+            k_split_pairs<<<grid_for(t.nfar, 256), 256, 0, st>>>(t.nfar, sb, ws.far_sorted.as<uint64_t>(), t.far_src,
                                                                   t.far_ord);
         }
         if (t.nnear > 0) {
             count_launches(1);
-            k_split_pairs<<<grid_for(t.nnear, 256), 256, 0, st>>>(t.nnear, ws.near_sorted.as<uint64_t>(), t.near_src,
+            k_split_pairs<<<grid_for(t.nnear, 256), 256, 0, st>>>(t.nnear, sb, ws.near_sorted.as<uint64_t>(), t.near_src,
                                                                    nullptr);
         }
         count_launches(1);
-        k_csr_offsets<<<grid_for(M + 1, 256), 256, 0, st>>>(M, t.nfar, ws.far_sorted.as<uint64_t>(), t.far_off, 36);
+        k_csr_offsets<<<grid_for(M + 1, 256), 256, 0, st>>>(M, t.nfar, ws.far_sorted.as<uint64_t>(), t.far_off, sb + 4);
         count_launches(1);
-        k_csr_offsets<<<grid_for(M + 1, 256), 256, 0, st>>>(M, t.nnear, ws.near_sorted.as<uint64_t>(), t.near_off, 32);
+        k_csr_offsets<<<grid_for(M + 1, 256), 256, 0, st>>>(M, t.nnear, ws.near_sorted.as<uint64_t>(), t.near_off, sb);
         t.corr_off = t.corr_src = nullptr;
         if (corr) {
             // damping-correction list: sorted by (target, source), CSR by target
@@ -959,19 +1000,19 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
                                                             ws.corr_sorted.as<uint64_t>(), (int)t.ncorr, 0,
                                                             near_bits, st));
                 count_launches(1);
-                k_split_pairs<<<grid_for(t.ncorr, 256), 256, 0, st>>>(t.ncorr, ws.corr_sorted.as<uint64_t>(),
+                k_split_pairs<<<grid_for(t.ncorr, 256), 256, 0, st>>>(t.ncorr, sb, ws.corr_sorted.as<uint64_t>(),
                                                                        t.corr_src, nullptr);
             }
             count_launches(1);
             k_csr_offsets<<<grid_for(M + 1, 256), 256, 0, st>>>(M, t.ncorr, ws.corr_sorted.as<uint64_t>(),
-                                                                t.corr_off, 32);
+                                                                t.corr_off, sb);
         }
         unsigned long long* pc = ctr + 4;
         FMM_CUDA_TRY(cudaMemsetAsync(pc, 0, sizeof(unsigned long long), st));
         if (t.nnear > 0) {
             count_launches(1);
             k_near_pair_count<<<std::min<int64_t>(1024, grid_for(t.nnear, 256)), 256, 0, st>>>(
-                t.nnear, ws.near_sorted.as<uint64_t>(), t.count, pc);
+                t.nnear, sb, ws.near_sorted.as<uint64_t>(), t.count, pc);
         }
         unsigned long long npp = 0;
         FMM_CUDA_TRY(cudaMemcpyAsync(&npp, pc, sizeof(npp), cudaMemcpyDeviceToHost, st));
