@@ -27,8 +27,11 @@ with the exact series coefficients a_k; centres THOLE_CENTRES in x = a r,
 AMOEBA_CENTRES in u = (a r)^3.  One table for the whole range keeps the
 lanes of a warp on one code path whichever interval each lane's pair is in.
 
+FP64 kernels take e^x from a table of 2^(j / 2^EXP_BITS), rounded to nearest.
+
 Run:  python gen_tables.py > series_tables.h
 """
+from decimal import Decimal, getcontext
 from fractions import Fraction
 from math import factorial
 
@@ -38,6 +41,7 @@ KA = 30       # AMOEBA series length (powers of u)
 NTAY = 16     # terms of each interval's expansion (a multiple of 4: rows are read as float4)
 THOLE_CENTRES = (Fraction(0), Fraction(3, 2), Fraction(5, 2))
 AMOEBA_CENTRES = (Fraction(0), Fraction(3, 2), Fraction(5, 2), Fraction(7, 2))
+EXP_BITS = 8  # 2^(j / 256), j = 0..255
 KFULL = 160   # series terms summed exactly for the re-centred coefficients
 
 
@@ -126,6 +130,14 @@ def main():
             rows = ["{" + ", ".join(fmt(b) for b in recentred(fn, j, c)) + "}" for c in cs]
             out.append("  {" + ", ".join(rows) + "}, \\")
         out.append("}")
+    getcontext().prec = 60
+    out.append(f"#define FMM_EXP_BITS {EXP_BITS}")
+    out.append("#define FMM_EXP2_INIT { \\")
+    n = 1 << EXP_BITS
+    vals = [float(Decimal(2) ** (Decimal(j) / n)).hex() for j in range(n)]
+    for j in range(0, n, 8):
+        out.append("  " + ", ".join(vals[j:j + 8]) + ", \\")
+    out.append("}")
     print("\n".join(out))
 
 

@@ -51,6 +51,64 @@ static const double hTholeSeries[FMM_SER_JMAX + 1][FMM_SER_KT + 1] = FMM_THOLE_S
 static const double hAmoebaSeries[FMM_SER_JMAX + 1][FMM_SER_KA + 1] = FMM_AMOEBA_SERIES_INIT;
 static const double hAmoebaQ[FMM_SER_JMAX + 1][FMM_SER_JMAX] = FMM_AMOEBA_Q_INIT;
 
+#ifdef __CUDACC__
+__device__ const double gExp2[1 << FMM_EXP_BITS] = FMM_EXP2_INIT;
+
+// FP32 value of a double, truncated, from its bits alone (the conversion
+// instruction runs on the FP64 pipe): 0 for magnitudes below 2^-126, 3e38 above
+// the FP32 range, NaN for infinities and NaN.
+__device__ __forceinline__ float f32_bits(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const int e = ((hi >> 20) & 0x7ff) - (1023 - 127);
+    const int m = (e << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29);
+    if (e == 2047 - (1023 - 127)) return __int_as_float(0x7fffffff);
+    const float v = e <= 0 ? 0.0f : (e >= 255 ? 3.0e38f : __int_as_float(m));
+    return __int_as_float(__float_as_int(v) | (hi & (int)0x80000000));
+}
+// The double of a normal float, from its bits (of a smaller one: below 2^-125).
+__device__ __forceinline__ double f64_bits(float x) {
+    const unsigned b = (unsigned)__float_as_int(x);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
+}
+
+// e^x for x <= 0 by table and polynomial (P. T. P. Tang, ACM Trans. Math. Softw.
+// 15, 1989): x = n ln2 / 256 + r, |r| <= ln2 / 512, e^x = 2^(n / 256) (1 + r + r^2
+// (1/2 + r t)), with n and t = 1/6 + r / 24 + r^2 / 120 (which weighs below 2^-28)
+// in FP32.  Seven FP64 instructions; the FP64 pair kernels are bound by these
+// (csrc/pair_f64.cuh).  With this and rsqrt_f64 for the library's functions:
+// 200,000 particles with Thole damping, f = 2, 128.5 -> 120.0 ms; direct
+// gradient of 20,000 particles, AMOEBA damping, 77.8 -> 73.1 ms.  Within 1 ulp
+// of the library's; 0 below -700.
+__device__ __forceinline__ double exp_nonpos(double x) {
+    const float xf = f32_bits(x);
+    if (!(xf >= -700.0f)) return x < 0.0 ? 0.0 : x;
+    const int n = __float2int_rn(xf * 369.329931f);  // 256 / ln2
+    const double nd = __hiloint2double(0x43300000, n ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
+    // ln2 / 256 in two parts, the first of 32 bits (nd times it is exact)
+    const double r = fma(nd, -0x1.a39ef35793c76p-41, fma(nd, -0x1.62e42fee00000p-9, x));
+    const float rf = f32_bits(r);
+    const double t = f64_bits(fmaf(rf, fmaf(rf, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f));
+    const double w = fma(r, t, 0.5);
+    const double p = fma(r * r, w, r);
+    const double s = gExp2[n & ((1 << FMM_EXP_BITS) - 1)];
+    const double e = fma(s, p, s);
+    return __hiloint2double(__double2hiint(e) + ((n >> FMM_EXP_BITS) << 20), __double2loint(e));
+}
+
+// 1 / sqrt(x): FP32 seed, one third-order (Halley/Householder) step y (1 + e/2 +
+// 3 e^2 / 8), e = 1 - x y^2, the last term in FP32 (e < 2^-20): four FP64
+// instructions.  Outside the FP32 range the library's.
+__device__ __forceinline__ double rsqrt_f64(double x) {
+    const float xf = f32_bits(x);
+    if (!(xf > 1e-36f && xf < 1e36f)) return ::rsqrt(x);
+    const double y = f64_bits(rsqrtf(xf));
+    const double e = fma(-(x * y), y, 1.0);
+    const float ef = f32_bits(e);
+    const double c = fma(e, 0.5, f64_bits(0.375f * ef * ef));
+    return fma(y, c, y);
+}
+#endif
+
 // Per-precision math and the switch-over points between the series and the
 // closed forms (chosen so the closed form's cancellation stays below the
 // precision's rounding; checked against high-precision values in the tests).
@@ -75,8 +133,15 @@ struct Real<double> {
         return 1.0 / ::sqrt(x);
 #endif
     }
-    __host__ __device__ static __forceinline__ double exp_(double x) { return ::exp(x); }
-    __host__ __device__ static __forceinline__ double expc_(double x) { return ::exp(x); }
+    // (arguments <= 0 here)
+    __host__ __device__ static __forceinline__ double exp_(double x) {
+#ifdef __CUDA_ARCH__
+        return exp_nonpos(x);
+#else
+        return ::exp(x);
+#endif
+    }
+    __host__ __device__ static __forceinline__ double expc_(double x) { return exp_(x); }
     __host__ __device__ static __forceinline__ double erf_(double x) { return ::erf(x); }
     __host__ __device__ static __forceinline__ double sqrt_(double x) { return ::sqrt(x); }
     __host__ __device__ static __forceinline__ double inv_odd(int i) {

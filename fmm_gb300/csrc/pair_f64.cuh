@@ -28,17 +28,6 @@ __host__ __device__ constexpr bool near_rows(int m, int f) { return m <= 2 && f 
 // Rows of source coefficients per particle.
 __host__ __device__ constexpr int near_row_count(int m, int f) { return nT(m) + (m == 2 && f <= 2 ? 1 : 0); }
 
-// FP32 value of a positive double, truncated, from its bits alone (the
-// conversion instruction runs on the FP64 pipe): 0 below 2^-126 and for
-// negative values, 3e38 above the FP32 range, NaN for infinities and NaN.
-__device__ __forceinline__ float f32_bits(double x) {
-    const int hi = __double2hiint(x), lo = __double2loint(x);
-    const int e = (hi >> 20) - (1023 - 127);
-    const float v = __int_as_float((e << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29));
-    if (e == 2047 - (1023 - 127)) return __int_as_float(0x7fffffff);
-    return e <= 0 ? 0.0f : (e >= 255 ? 3.0e38f : v);
-}
-
 // Beyond these the damped numerators round to the undamped ones for every
 // order up to 6: e^-u q_6(u) / 11!! < 2^-62 from u = (a r)^3 = 60 (AMOEBA),
 // e^-x P_6(x) / 11!! < 2^-59 from x = a r = 60 (Thole), and e^-s s^(11/2) / 11!!
@@ -132,12 +121,12 @@ __device__ __forceinline__ void pair_field_f64(double dx, double dy, double dz, 
     if constexpr (near_rows(M, F)) {
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         double g[M + F + 1];
-        radial_g_f64<M + F>(damp, r2, ::rsqrt(r2), a, g);
+        radial_g_f64<M + F>(damp, r2, rsqrt_f64(r2), a, g);
         contract_f64<M, F>(dx, dy, dz, g, mc, damp, acc);
     } else {
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         double g[M + F + 1], T[nT(M + F)];
-        radial_g_f64<M + F>(damp, r2, ::rsqrt(r2), a, g);
+        radial_g_f64<M + F>(damp, r2, rsqrt_f64(r2), a, g);
         md_tensor<M + F, double>(dx, dy, dz, g, T);
         contract<M, F, double>(T, mc, acc);
     }
