@@ -18,6 +18,12 @@
 // tensors are not harmonic: the FP64 product then runs over all Cartesian
 // components (`full`), with the reference's closed form once per group.
 //
+// The basis functions are even or odd in x, y and z, so that displacements that
+// differ in signs alone have the same operator up to the signs of its rows and
+// columns.  Where the groups are small, those of the eight octants are taken
+// together (`mirrored`): with up to eight times the pairs per operator the
+// products' columns are filled and an eighth of the operators is built.
+//
 // Units: per-node weights w'_s = w^_s / h_j^|s|, per-target locals
 // L'_f = h_i^(|f|+1) L_f, tensor T(D_c) at the displacement in units of the
 // coarser cell's half-width h_c; then G_fs = a^(|f|+1) b^|s| T_{s+f}(D_c)
@@ -26,6 +32,7 @@
 #include <algorithm>
 
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -43,10 +50,12 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 
 constexpr int kFallback = 63;            // key code of pairs without a grid displacement
 // Key layout (46 bits, so the radix sort needs 6 digit passes): level
-// difference + 31 (6 bits) | order (4) | Dx, Dy, Dz + kDOff (12 bits each).
+// difference + 31 (6 bits) | order (4) | |Dx|, |Dy|, |Dz| (11 bits each) |
+// octant (3): bit d set where D_d < 0.
 constexpr int kKeyBits = 46;
 constexpr int kKeyBitsImages = 56;       // with the target's depth and the source's image (5 bits each) above
-constexpr int64_t kDOff = 1 << 11;       // offset of the 12-bit displacement fields
+constexpr int64_t kDMax = (1 << 11) - 1;
+constexpr int kOctants = 8;
 constexpr int kTaskCols = 512;           // pairs (columns) per product block
 constexpr int kGemmThreads = 128;        // 16 row groups x 8 column groups
 constexpr int kTcRows = 128;             // tensor-core MMA M: operator rows f per half
@@ -130,25 +139,27 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
     }
     const int dl = t.depth[i] - t.depth[j];
     const int oc = (ord + oclass - 1) / oclass;  // order class: the group takes its pairs' highest order
-    const float lim = (float)(kDOff - 1);
+    const float lim = (float)kDMax;
     const bool grid = ex < tol && ey < tol && ez < tol && fabsf(rx) <= lim && fabsf(ry) <= lim && fabsf(rz) <= lim &&
                       dl > -31 && dl < 31;
     uint64_t key;
     if (grid)
-        key = ((uint64_t)(dl + 31) << 40) | ((uint64_t)oc << 36) | ((uint64_t)((int64_t)rx + kDOff) << 24) |
-              ((uint64_t)((int64_t)ry + kDOff) << 12) | (uint64_t)((int64_t)rz + kDOff) |
+        key = ((uint64_t)(dl + 31) << 40) | ((uint64_t)oc << 36) | ((uint64_t)fabsf(rx) << 25) |
+              ((uint64_t)fabsf(ry) << 14) | ((uint64_t)fabsf(rz) << 3) |
+              (uint64_t)((rx < 0.0f ? 1 : 0) | (ry < 0.0f ? 2 : 0) | (rz < 0.0f ? 4 : 0)) |
               (t.nimg > 1 ? (uint64_t)(t.depth[i] | (src_image(t, t.far_src[q]) << 5)) << kKeyBits : 0);
     else
-        key = ((uint64_t)kFallback << 40) | (uint64_t)q;
+        key = ((uint64_t)kFallback << 40) | ((uint64_t)q << 3);
     keys[q] = key;
     vals[q] = (int32_t)q;
 }
 
 // One warp per group: restricted tensor T(D_c) of orders <= 2q in FP64 by the
 // Hermite recursion (two level buffers in shared memory), stored as R, with
-// the group's order and unit ratios a, b.
+// the group's order and unit ratios a, b.  Mirrored groups: at the displacement
+// of octant 0 (skeys: the pairs' keys in group order).
 template <typename R>
-__global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_t* __restrict__ ukeys,
+__global__ void __launch_bounds__(128) k_group_tensor(int ngroups, bool mirrored, const uint64_t* __restrict__ skeys,
                                                       const int32_t* __restrict__ gstart,
                                                       const int32_t* __restrict__ svals,
                                                       const int32_t* __restrict__ tgt, const TreeDev t, int p,
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_
     __syncthreads();
     const int g = blockIdx.x * (blockDim.x >> 5) + wib;
     if (g >= ngroups) return;
-    const uint64_t key = ukeys[g];
+    const int oct = mirrored ? (int)(skeys[gstart[g]] & (kOctants - 1)) : 0;
     const int pos0 = svals[gstart[g]];
     const int i = tgt[pos0], j = t.far_src[pos0];
     // the group's order: the highest of its pairs' orders
@@ -174,7 +185,9 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, const uint64_
         q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
     for (int off = 16; off > 0; off >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, off));
     const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
-    const double X = (t.cx[i] - t.cx[j]) / hc, Y = (t.cy[i] - t.cy[j]) / hc, Z = (t.cz[i] - t.cz[j]) / hc;
+    const double X = ((oct & 1) ? -1.0 : 1.0) * (t.cx[i] - t.cx[j]) / hc,
+                 Y = ((oct & 2) ? -1.0 : 1.0) * (t.cy[i] - t.cy[j]) / hc,
+                 Z = ((oct & 4) ? -1.0 : 1.0) * (t.cz[i] - t.cz[j]) / hc;
     const int Nq = 2 * q;
     const double r2 = X * X + Y * Y + Z * Z;
     const double rinv = 1.0 / sqrt(r2), rinv2 = rinv * rinv;
@@ -491,7 +504,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_m2l_gemm(const int2* __restric
 // ---------------------------------------------------------------------------
 // Tensor-core product.  A task is up to 256 pairs of one group and one half
 // of its operator: D = G W^T with G the operator half (f x s, M = 128 rows
-// f), W the pairs' weights (pairs x s, N = 256) and K = (q+1)^2
+// f), W the pairs' weights (pairs x s, N = the pairs rounded up to 16: small
+// groups take a part of the tensor cores' time) and K = (q+1)^2
 // in chunks of 8 (one MMA K step).  Both operands are split into TF32 parts,
 // x = hi + lo, and D accumulates G_hi W_hi + G_hi W_lo + G_lo W_hi in FP32
 // (the dropped G_lo W_lo and the rounding of the parts leave about 2^-22 of
@@ -541,8 +555,17 @@ struct TcSmem {
     static constexpr size_t bytes = off_tmem + 16;
 };
 
+// Parities of component c (packed x, y, z): bit d set where the power is odd.
+// The component changes sign between octant 0 and octant o where
+// component_flips(c) & o has an odd number of bits.
+__device__ __forceinline__ int component_flips(int c) {
+    return (c & 1) | ((c >> 7) & 2) | ((c >> 14) & 4);
+}
+
 // Per-node weights as TF32 parts, chunk by chunk: [chunk][hi KC | lo KC].
-__global__ void k_split_weights(int64_t total, int nr, int ldw, int ldk, const float* __restrict__ wsc,
+// octants = 8 (mirrored groups): a copy for each octant, as its pairs' operator
+// of octant 0 wants them.
+__global__ void k_split_weights(int64_t total, int octants, int nr, int ldw, int ldk, const float* __restrict__ wsc,
                                 float* __restrict__ wsp) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t node = e / ldk;
@@ -550,9 +573,13 @@ __global__ void k_split_weights(int64_t total, int nr, int ldw, int ldk, const f
         const float v = s < nr ? wsc[node * ldw + s] : 0.0f;
         float h, l;
         umma::split_tf32(v, h, l);
-        float* o = wsp + node * 2 * ldk + (s / kTcKC) * 2 * kTcKC + (s % kTcKC);
-        o[0] = h;
-        o[kTcKC] = l;
+        float* o = wsp + node * octants * 2 * ldk + (s / kTcKC) * 2 * kTcKC + (s % kTcKC);
+        const int flips = octants > 1 && s < nr ? component_flips(qcomp(s)) : 0;
+        for (int k = 0; k < octants; ++k, o += 2 * ldk) {
+            const bool neg = __popc(flips & k) & 1;
+            o[0] = neg ? -h : h;
+            o[kTcKC] = neg ? -l : l;
+        }
     }
 }
 
@@ -575,12 +602,20 @@ __global__ void k_row_offsets(int ng, bool full, const int32_t* __restrict__ gst
     for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32) roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
 }
 
-// Source node of every far pair in group order.
-__global__ void k_pair_sources(int64_t nf, const int32_t* __restrict__ svals, const TreeDev t,
-                               int32_t* __restrict__ psrc) {
+// Source node of every far pair in group order; mirrored groups: 8 x node +
+// octant, the copy of the weights.
+__global__ void k_pair_sources(int64_t nf, bool mirrored, const uint64_t* __restrict__ skeys,
+                               const int32_t* __restrict__ svals, const TreeDev t, int32_t* __restrict__ psrc) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < nf) psrc[k] = src_node(t, t.far_src[svals[k]]);
+    if (k >= nf) return;
+    const int j = src_node(t, t.far_src[svals[k]]);
+    psrc[k] = mirrored ? kOctants * j + (int)(skeys[k] & (kOctants - 1)) : j;
 }
+
+// Key of a mirrored group: the pair key without its octant.
+struct MirroredKey {
+    __host__ __device__ __forceinline__ uint64_t operator()(uint64_t key) const { return key >> 3; }
+};
 
 // Size in floats of a group's split operator (halves x chunks x (hi + lo) x
 // 128 x KC).
@@ -648,7 +683,11 @@ __global__ void __launch_bounds__(256) k_group_operator(int ldT, const float* __
     }
 }
 
-// Source nodes of a producer thread's rows 8 (rg0 + k * producer warps) + rsub of task t.
+// Columns of a task's MMAs: its pairs rounded up to the instruction's step.
+__device__ __forceinline__ int tc_columns(int cnt) { return (cnt + 15) & ~15; }
+
+// Sources of a producer thread's rows 8 (rg0 + k * producer warps) + rsub of
+// task t (-1: none, a row of zeros).
 template <int RG>
 __device__ __forceinline__ void tc_load_rows(int t, const int2* __restrict__ tasks, const int32_t* __restrict__ gstart,
                                              const int32_t* __restrict__ psrc, int rg0, int rsub, int (&r)[RG]) {
@@ -661,7 +700,7 @@ __device__ __forceinline__ void tc_load_rows(int t, const int2* __restrict__ tas
     }
 }
 
-__global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict__ tasks, int ntasks,
+__global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict__ tasks, int ntasks, bool mirrored,
                                                          const int32_t* __restrict__ gstart,
                                                          const int32_t* __restrict__ gq,
                                                          const int64_t* __restrict__ goff, int64_t gop_base,
@@ -715,6 +754,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
         while (task < ntasks && ok) {
             const int g = tasks[task].x, q = gq[g];
             const int nch = ((q + 1) * (q + 1) + kTcKC - 1) / kTcKC;
+            const int cols = tc_columns(min(kTcPairs, gstart[g + 1] - gstart[g] - (tasks[task].y >> 1)));
             const int next = task + gridDim.x;
             if (next < ntasks) tc_load_rows<RG>(next, tasks, gstart, psrc, rg0, rsub, nrows);  // in flight
             // the task's operator half
@@ -735,11 +775,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
                 }
                 float* dst0 = Ws + part * TcSmem::w_floats + 4 * j * 8 + rsub * 4;  // tc_off(8 rg + rsub, 4 j)
                 const int coff = ch * 2 * kTcKC + part * kTcKC + 4 * j;
+                // four row groups at a time, as far as the MMAs read
+                constexpr int KB = 4;
 #pragma unroll
-                for (int k = 0; k < RG; ++k) {
-                    const int src = rows[k];
-                    const float* gsrc = src >= 0 ? wsp + (size_t)src * 2 * ldk + coff : wsp;
-                    umma::cp16_keep(dst0 + (rg0 + (kTcProducers / 32) * k) * kTcKC * 8, gsrc, src >= 0, keep);
+                for (int k0 = 0; k0 < RG; k0 += KB) {
+                    if (8 * (kTcProducers / 32) * k0 >= cols) break;
+#pragma unroll
+                    for (int k = k0; k < k0 + KB; ++k) {
+                        const int src = rows[k];
+                        const float* gsrc = src >= 0 ? wsp + (size_t)src * 2 * ldk + coff : wsp;
+                        umma::cp16_keep(dst0 + (rg0 + (kTcProducers / 32) * k) * kTcKC * 8, gsrc, src >= 0, keep);
+                    }
                 }
                 umma::cp_async_mbar_arrive(&full[st]);
             }
@@ -751,10 +797,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
         // ---- MMA issue (one thread)
         if (lane == 0) {
             uint32_t u = 0, tl = 0;
-            const uint32_t idesc = umma::idesc_tf32(kTcRows, kTcPairs);
             constexpr uint32_t LBO = 128, SBO = kTcKC / 4 * 128;
             for (int task = blockIdx.x; task < ntasks && ok; task += gridDim.x) {
                 const int g = tasks[task].x, q = gq[g];
+                const int cnt = min(kTcPairs, gstart[g + 1] - gstart[g] - (tasks[task].y >> 1));
+                const uint32_t idesc = umma::idesc_tf32(kTcRows, tc_columns(cnt));
                 const int nch = ((q + 1) * (q + 1) + kTcKC - 1) / kTcKC;
                 const int acc = (int)(tl & 1);
                 if (tl >= 2 && !umma::mbar_wait(&acc_empty[acc], ((tl >> 1) - 1) & 1, kTcWaitCycles)) {
@@ -797,6 +844,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
         constexpr int kShares = kTcEpiWarps / 4;
         const int share = (warp - 3) / 4;
         constexpr int CB = 16 * kTcEpiBatch;  // columns per wait
+        static_assert(CB == 32, "a lane per column's octant");
         uint32_t tl = 0;
         for (int task = blockIdx.x; task < ntasks && ok; task += gridDim.x) {
             const int2 tk = tasks[task];
@@ -815,13 +863,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
             // rowbase[g] x kRowUnit in group order
             const int rl = row_len(q);
             float* gout = out + ((size_t)rowbase[g] + (size_t)(tk.y >> 1) * (rl / kRowUnit)) * kRowUnit;
+            const int flips = mirrored && fr < (q + 1) * (q + 1) ? component_flips(qcomp(fr)) : 0;
             // warps whose 32 rows f lie beyond the row length have nothing to write
 #pragma unroll 1
             for (int c = share * CB; c < cnt && f0 + 32 * sp < rl; c += kShares * CB) {
                 float v[CB];
+                __syncwarp();
 #pragma unroll
                 for (int b = 0; b < kTcEpiBatch; ++b) umma::tmem_ld16(base + (uint32_t)(c + 16 * b), v + 16 * b);
                 umma::tmem_ld_wait();
+                umma::tmem_landed(v);
+                if (mirrored) {
+                    // columns (bits) in which this row changes sign
+                    const int o = c + lane < cnt ? psrc[gs + c + lane] : 0;
+                    const unsigned b0 = __ballot_sync(0xffffffffu, o & 1), b1 = __ballot_sync(0xffffffffu, o & 2),
+                                   b2 = __ballot_sync(0xffffffffu, o & 4);
+                    const unsigned neg = ((flips & 1) ? b0 : 0) ^ ((flips & 2) ? b1 : 0) ^ ((flips & 4) ? b2 : 0);
+#pragma unroll
+                    for (int jj = 0; jj < CB; ++jj)
+                        v[jj] = __uint_as_float(__float_as_uint(v[jj]) ^ ((neg >> jj) << 31));
+                }
                 // the task's rows are consecutive; streaming stores of whole lines
                 if (fr < rl) {
 #pragma unroll
@@ -923,6 +984,13 @@ constexpr double kMinGroupPairs = 16.0, kMinGroupPairs64 = 2.0;
 // by pair, which needs no rows.
 constexpr double kFullRowBytes = 64e9;
 constexpr double kOperatorBytes = 16e9;  // TF32 operator parts of one batch of groups
+// TF32 products with fewer pairs per group than this (a task's columns not
+// filled by a group) take the groups of the eight octants together, where the
+// weights' eight copies fit.  250,000 particles in clusters with learned orders
+// (4.1e6 pairs): 157,000 groups of 26 pairs become 56,000 of 72, tensors and
+// operators 18.7 -> 6.9 ms, products 12.2 -> 4.8 ms.  Where groups are large
+// there is little to gain and the copies no longer stay in the L2 cache.
+constexpr double kMirrorPairs = 256.0, kMirrorBytes = 8e9;
 
 // Split operators of the groups of one batch.
 int launch_operators(Workspace& ws, bool tc, bool full, int ldT, int ldr, const M2lBatch& b, int64_t base,
@@ -999,6 +1067,19 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         int ng = 0;
         FMM_CUDA_TRY(cudaMemcpyAsync(&ng, d_nruns, sizeof(int), cudaMemcpyDeviceToHost, st));
         FMM_CUDA_TRY(cudaStreamSynchronize(st));
+        ws.m2l_mirrored = tc && t.nimg <= 1 && (double)nf < kMirrorPairs * (double)ng &&
+                          sizeof(float) * 2.0 * kOctants * M * ldk <= kMirrorBytes;
+        if (ws.m2l_mirrored) {
+            auto mk = thrust::make_transform_iterator(ws.m2l_keys2.as<uint64_t>(), MirroredKey());
+            size_t tbm = 0;
+            cub::DeviceRunLengthEncode::Encode(nullptr, tbm, mk, ws.m2l_ukeys.as<uint64_t>(), ws.m2l_cnt.as<int32_t>(),
+                                               d_nruns, (int)nf, st);
+            FMM_TRY(ws.cub_tmp.ensure(tbm));
+            FMM_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(ws.cub_tmp.p, tbm, mk, ws.m2l_ukeys.as<uint64_t>(),
+                                                            ws.m2l_cnt.as<int32_t>(), d_nruns, (int)nf, st));
+            FMM_CUDA_TRY(cudaMemcpyAsync(&ng, d_nruns, sizeof(int), cudaMemcpyDeviceToHost, st));
+            FMM_CUDA_TRY(cudaStreamSynchronize(st));
+        }
         ws.m2l_groups = ng;
         // displacement groups of a few pairs each (irregular trees, mixed
         // orders) leave the products' columns empty and multiply the
@@ -1027,8 +1108,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             count_launches(1);
             k_group_tensor<R><<<grid_for(ng, wpb), 32 * wpb, sm, st>>>(
-                ng, ws.m2l_ukeys.as<uint64_t>(), ws.m2l_gstart.as<int32_t>(), ws.m2l_vals2.as<int32_t>(), tgt, t, p,
-                ldT, ws.m2l_T.as<R>(), ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>());
+                ng, ws.m2l_mirrored, ws.m2l_keys2.as<uint64_t>(), ws.m2l_gstart.as<int32_t>(),
+                ws.m2l_vals2.as<int32_t>(), tgt, t, p, ldT, ws.m2l_T.as<R>(), ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>());
         }
         // tasks: up to kTaskCols pairs of one group each (tensor cores: 256
         // pairs and one operator half)
@@ -1070,10 +1151,11 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
                                                         ws.m2l_toff.as<int32_t>(), ws.m2l_tasks.as<int2>());
         // source node per sorted pair (into the free unsorted-values buffer)
         count_launches(1);
-        k_pair_sources<<<grid_for(nf, 256), 256, 0, st>>>(nf, ws.m2l_vals2.as<int32_t>(), t, ws.m2l_vals.as<int32_t>());
+        k_pair_sources<<<grid_for(nf, 256), 256, 0, st>>>(nf, ws.m2l_mirrored, ws.m2l_keys2.as<uint64_t>(),
+                                                          ws.m2l_vals2.as<int32_t>(), t, ws.m2l_vals.as<int32_t>());
         if (tc || tc64) {
             // tensor-core operands: per node the weights, per group the operator
-            FMM_TRY(ws.m2l_wsplit.ensure(tc ? sizeof(float) * 2 * (size_t)M * ldk
+            FMM_TRY(ws.m2l_wsplit.ensure(tc ? sizeof(float) * 2 * (size_t)M * ldk * (ws.m2l_mirrored ? kOctants : 1)
                                             : (size_t)M * (wchunks * kDig * kD64K * 2 + sizeof(int))));
             if (tc64) FMM_TRY(ws.m2l_gexp.ensure(sizeof(int) * (size_t)ng * nr));
             FMM_TRY(ws.m2l_gopoff.ensure(sizeof(int64_t) * (ng + 1)));
@@ -1131,7 +1213,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
             count_launches(1);
             if (tc) {
                 k_split_weights<<<grid_for((int64_t)M * ldk, 256), 256, 0, st>>>(
-                    (int64_t)M * ldk, nr, ldw, ldk, reinterpret_cast<const float*>(ws.m2l_wsc.p),
+                    (int64_t)M * ldk, ws.m2l_mirrored ? kOctants : 1, nr, ldw, ldk, reinterpret_cast<const float*>(ws.m2l_wsc.p),
                     ws.m2l_wsplit.as<float>());
                 FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)TcSmem::bytes));
@@ -1159,8 +1241,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
                 count_launches(1);
                 if (tc)
                     k_m2l_tc<<<(unsigned)grid, kTcThreads, TcSmem::bytes, st>>>(
-                        ws.m2l_tasks.as<int2>() + b.t0, nt, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
-                        ws.m2l_gopoff.as<int64_t>(), many ? b.gop_base : 0, ws.m2l_gop.as<float>(),
+                        ws.m2l_tasks.as<int2>() + b.t0, nt, ws.m2l_mirrored, ws.m2l_gstart.as<int32_t>(),
+                        ws.m2l_gq.as<int32_t>(), ws.m2l_gopoff.as<int64_t>(), many ? b.gop_base : 0, ws.m2l_gop.as<float>(),
                         ws.m2l_vals.as<int32_t>(), ws.m2l_wsplit.as<float>(), ldk,
                         reinterpret_cast<float*>(ws.m2l_out.p), rowbase, d_err);
                 else

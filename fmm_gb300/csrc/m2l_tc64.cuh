@@ -427,9 +427,12 @@ __global__ void __launch_bounds__(kD64Threads, 1) k_m2l_tc64(const int2* __restr
 #pragma unroll 1
             for (int c = share * CB; c < cnt && f0 + 32 * sp < rl; c += kShares * CB) {
                 float v[kDig][CB];
+                __syncwarp();
 #pragma unroll
                 for (int d = 0; d < kDig; ++d) umma::tmem_ld8(base + (uint32_t)(d * kD64Pairs + c), v[d]);
                 umma::tmem_ld_wait();
+#pragma unroll
+                for (int d = 0; d < kDig; ++d) umma::tmem_landed(v[d]);
 #pragma unroll
                 for (int jj = 0; jj < CB; ++jj) {
                     if (c + jj < cnt) {

@@ -183,6 +183,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// The values of tensor-memory loads, once they have been waited for: the wait
+// names no registers, and without this the compiler may use them before it.
+template <int N>
+__device__ __forceinline__ void tmem_landed(float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+f"(v[i]));
+}
 
 // x = hi + lo with hi and lo exact TF32 values (10 explicit mantissa bits,
 // rounded to nearest): the pair carries about 22 bits of x.
