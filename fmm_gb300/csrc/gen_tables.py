@@ -27,6 +27,11 @@ with the exact series coefficients a_k; centres THOLE_CENTRES in x = a r,
 AMOEBA_CENTRES in u = (a r)^3.  One table for the whole range keeps the
 lanes of a warp on one code path whichever interval each lane's pair is in.
 
+FP32 kernels evaluate the Boys functions of the ERF kernel, F_n(s) = int_0^1
+t^(2n) e^(-s t^2) dt, at the highest order from polynomials of degree BOYS_N - 1
+through the Chebyshev nodes of each unit interval of s, in t = s - c - 1/2
+(relative error below 1e-9), and the lower orders by downward recursion.
+
 FP64 kernels take e^x from a table of 2^(j / 2^EXP_BITS), rounded to nearest.
 
 Run:  python gen_tables.py > series_tables.h
@@ -41,6 +46,8 @@ KA = 30       # AMOEBA series length (powers of u)
 NTAY = 16     # terms of each interval's expansion (a multiple of 4: rows are read as float4)
 THOLE_CENTRES = (Fraction(0), Fraction(3, 2), Fraction(5, 2))
 AMOEBA_CENTRES = (Fraction(0), Fraction(3, 2), Fraction(5, 2), Fraction(7, 2))
+BOYS_N = 8    # terms of a Boys interval's polynomial (a multiple of 4)
+BOYS_NC = 32  # intervals: beyond, no order's e^-s reaches FP32 precision
 EXP_BITS = 8  # 2^(j / 256), j = 0..255
 KFULL = 160   # series terms summed exactly for the re-centred coefficients
 
@@ -92,6 +99,48 @@ def recentred(fn, j, c):
     return [sum(a[k] * binom(k, n) * c ** (k - n) for k in range(n, KFULL)) for n in range(NTAY)]
 
 
+def boys(n, s):
+    """F_n(s) = e^-s sum_k (2 s)^k / ((2n+1) (2n+3) .. (2n+2k+1))."""
+    term = Decimal(1) / (2 * n + 1)
+    total, k = term, 0
+    while term > total * Decimal(10) ** -45:
+        k += 1
+        term *= 2 * s / (2 * n + 2 * k + 1)
+        total += term
+    return (-s).exp() * total
+
+
+def chebyshev_nodes(m):
+    """cos((2i + 1) pi / (2m)) / 2, by bisection of the Chebyshev polynomial."""
+    def T(x):
+        a, b = Decimal(1), x
+        for _ in range(m - 1):
+            a, b = b, 2 * x * b - a
+        return b
+    nodes, grid = [], [Decimal(2 * i - 400) / 401 for i in range(401)]
+    for lo, hi in zip(grid, grid[1:]):
+        if T(lo) * T(hi) < 0:
+            for _ in range(150):
+                mid = (lo + hi) / 2
+                lo, hi = (mid, hi) if T(lo) * T(mid) > 0 else (lo, mid)
+            nodes.append((lo + hi) / 4)
+    assert len(nodes) == m
+    return nodes
+
+
+def boys_row(n, c, nodes):
+    """Monomial coefficients in t of the interpolant (Newton's divided differences)."""
+    d = [boys(n, c + Decimal("0.5") + t) for t in nodes]
+    for j in range(1, len(nodes)):
+        for i in range(len(nodes) - 1, j - 1, -1):
+            d[i] = (d[i] - d[i - 1]) / (nodes[i] - nodes[i - j])
+    p = [Decimal(0)] * len(nodes)
+    for i in range(len(nodes) - 1, -1, -1):
+        p = [(p[k - 1] if k else Decimal(0)) - nodes[i] * p[k] for k in range(len(nodes))]
+        p[0] += d[i]
+    return p
+
+
 def fmt(fr):
     return repr(float(fr)) if fr != 0 else "0.0"
 
@@ -131,6 +180,14 @@ def main():
             out.append("  {" + ", ".join(rows) + "}, \\")
         out.append("}")
     getcontext().prec = 60
+    nodes = chebyshev_nodes(BOYS_N)
+    out.append(f"#define FMM_BOYS_N {BOYS_N}")
+    out.append(f"#define FMM_BOYS_NC {BOYS_NC}")
+    out.append("#define FMM_BOYS_INIT { \\")
+    for n in range(JMAX + 1):
+        rows = ["{" + ", ".join(repr(float(b)) for b in boys_row(n, c, nodes)) + "}" for c in range(BOYS_NC)]
+        out.append("  {" + ", ".join(rows) + "}, \\")
+    out.append("}")
     out.append(f"#define FMM_EXP_BITS {EXP_BITS}")
     out.append("#define FMM_EXP2_INIT { \\")
     n = 1 << EXP_BITS

@@ -886,7 +886,7 @@ int launch_leaf_field_scale(Workspace& ws, const Particles& P, const TreeDev& t,
 
 bool p2p_packed_enabled(const P2pShape& sh, int field_order, int damp) {
     const char* pe = std::getenv("FMM_GB300_P2P_PACKED");
-    return sh.pack && !(pe && pe[0] == '0') && field_order <= 1 && damp != DAMP_ERF;
+    return sh.pack && !(pe && pe[0] == '0') && field_order <= 1;
 }
 
 bool P2pShape::valid() const {
