@@ -203,7 +203,7 @@ class Plan:
         sizes = [np.asarray(s["coordinates"]).shape[0] for s in systems_list]
         offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
         n = int(offsets[-1])
-        X = np.asfortranarray(np.concatenate([np.asarray(s["coordinates"], dtype=np.float64) for s in systems_list]))
+        X = _stack(s["coordinates"] for s in systems_list)
         width = max(np.asarray(s["exclusions"]).reshape(sizes[k], -1).shape[1] for k, s in enumerate(systems_list))
         E = np.zeros((n, width), dtype=np.int32, order="F")
         for k, s in enumerate(systems_list):
@@ -275,6 +275,14 @@ class Plan:
         self.close()
 
 
+def _stack(arrays):
+    """Rows of all arrays in one column-major array (one copy)."""
+    a = [np.asarray(x, dtype=np.float64) for x in arrays]
+    if not a or any(x.ndim != 2 for x in a):
+        return np.asfortranarray(np.concatenate(a))
+    return np.concatenate(a, out=np.empty((sum(x.shape[0] for x in a), a[0].shape[1]), order="F"))
+
+
 def field_fmm_batched(systems_list, theta, ncrit, expansion_order, field_order, damp_type="", *, options=None):
     """Many independent systems in one call (fmm_field_fmm_batched).
 
@@ -285,8 +293,8 @@ def field_fmm_batched(systems_list, theta, ncrit, expansion_order, field_order, 
     sizes = [np.asarray(s["coordinates"]).shape[0] for s in systems_list]
     offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
     n = int(offsets[-1])
-    X = np.asfortranarray(np.concatenate([np.asarray(s["coordinates"], dtype=np.float64) for s in systems_list]))
-    M = np.asfortranarray(np.concatenate([np.asarray(s["multipoles"], dtype=np.float64) for s in systems_list]))
+    X = _stack(s["coordinates"] for s in systems_list)
+    M = _stack(s["multipoles"] for s in systems_list)
     width = max(np.asarray(s["exclusions"]).reshape(sizes[k], -1).shape[1] for k, s in enumerate(systems_list))
     E = np.zeros((n, width), dtype=np.int32, order="F")
     for k, s in enumerate(systems_list):

@@ -46,7 +46,7 @@ void Workspace::release_buffers(bool keep_selector) {
                      &far_sorted, &near_sorted, &node_dfs, &far_src,    &near_src,   &sx,         &sy,
                      &sz,        &smc,       &sd,          &fsorted,    &mom,        &loc,        &partial,
                      &term_off,  &term_abc,  &term_c, &f32buf, &f32sel, &wred, &far_ord, &sel_norms, &sel_params, &sel_scratch, &sysbuf,
-                     &m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
+                     &sys_ids, &sys_tab, &m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
                      &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &f32x2c, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
     for (DevBuf* b : all)
         if (!(keep_selector && b == &sel_params)) b->release();
@@ -617,29 +617,37 @@ struct Packed {
     int64_t min_size = 0;
 };
 
-int pack_systems(int nsys, const int64_t* offsets, const double* X, int exw, const int32_t* ex, int ncrit,
-                 Packed* out) {
+// Sizes and exclusions of the systems; the smallest size.
+int check_systems(int nsys, const int64_t* offsets, int exw, const int32_t* ex, int ncrit, int64_t* min_size) {
     const int64_t n = offsets[nsys];
-    std::vector<double> cen(3 * (size_t)nsys);
-    double hmax = 0.0;
-    int64_t min_size = n;
+    *min_size = n;
+    for (int k = 0; k < nsys; ++k) {
+        if (offsets[k + 1] - offsets[k] <= ncrit) return FMM_EINVAL;  // every system must need a tree of its own
+        *min_size = std::min(*min_size, offsets[k + 1] - offsets[k]);
+    }
     for (int k = 0; k < nsys; ++k) {
         const int64_t a = offsets[k], b = offsets[k + 1];
-        if (b - a <= ncrit) return FMM_EINVAL;  // every system must need a tree of its own
-        min_size = std::min(min_size, b - a);
-        for (int64_t i = a; i < b; ++i)
-            for (int w = 0; w < exw; ++w) {
+        bool bad = false;
+        for (int w = 0; w < exw; ++w)
+            for (int64_t i = a; i < b; ++i) {
                 const int32_t e = ex[(size_t)w * n + i];
-                if (e < 0 || e > b - a) return FMM_EINVAL;
+                bad |= e < 0 || e > b - a;
             }
+        if (bad) return FMM_EINVAL;
+    }
+    return FMM_OK;
+}
+
+// Packing box from the systems' bounds (lo x, y, z, hi x, y, z each): its
+// half-width, and per system the middle of its bounds and of its cell.
+double pack_box(int nsys, const std::vector<double>& bounds, std::vector<double>& tab) {
+    tab.resize(6 * (size_t)nsys);
+    double hmax = 0.0;
+    for (int k = 0; k < nsys; ++k) {
         double h = 0.0;
         for (int d = 0; d < 3; ++d) {
-            double lo = X[d * n + a], hi = lo;
-            for (int64_t i = a; i < b; ++i) {
-                lo = std::min(lo, X[d * n + i]);
-                hi = std::max(hi, X[d * n + i]);
-            }
-            cen[3 * (size_t)k + d] = 0.5 * (lo + hi);
+            const double lo = bounds[6 * (size_t)k + d], hi = bounds[6 * (size_t)k + 3 + d];
+            tab[6 * (size_t)k + d] = 0.5 * (lo + hi);
             h = std::max(h, 0.5 * (hi - lo));
         }
         hmax = std::max(hmax, h);
@@ -647,14 +655,37 @@ int pack_systems(int nsys, const int64_t* offsets, const double* X, int exw, con
     int G = 1;
     while ((int64_t)G * G * G < nsys) G *= 2;
     const double S = 2.0 * hmax * 1.05 + 1e-6;
+    for (int k = 0; k < nsys; ++k) {
+        const int c[3] = {k % G, (k / G) % G, k / (G * G)};
+        for (int d = 0; d < 3; ++d) tab[6 * (size_t)k + 3 + d] = (c[d] - 0.5 * (G - 1)) * S;
+    }
+    return 0.5 * G * S;
+}
+
+// On the host (plans, which keep the packed systems).
+int pack_systems(int nsys, const int64_t* offsets, const double* X, int exw, const int32_t* ex, int ncrit,
+                 Packed* out) {
+    const int64_t n = offsets[nsys];
+    FMM_TRY(check_systems(nsys, offsets, exw, ex, ncrit, &out->min_size));
+    std::vector<double> bounds(6 * (size_t)nsys), tab;
+    for (int k = 0; k < nsys; ++k)
+        for (int d = 0; d < 3; ++d) {
+            double lo = X[d * n + offsets[k]], hi = lo;
+            for (int64_t i = offsets[k]; i < offsets[k + 1]; ++i) {
+                lo = std::min(lo, X[d * n + i]);
+                hi = std::max(hi, X[d * n + i]);
+            }
+            bounds[6 * (size_t)k + d] = lo;
+            bounds[6 * (size_t)k + 3 + d] = hi;
+        }
+    out->root_r = pack_box(nsys, bounds, tab);
     out->Xp.assign((size_t)3 * n, 0.0);
     out->exg.assign((size_t)std::max(exw, 0) * n, 0);
     out->sys.assign((size_t)n, 0);
     for (int k = 0; k < nsys; ++k) {
-        const int ix = k % G, iy = (k / G) % G, iz = k / (G * G);
-        const double cc[3] = {(ix - 0.5 * (G - 1)) * S, (iy - 0.5 * (G - 1)) * S, (iz - 0.5 * (G - 1)) * S};
+        const double* c = &tab[6 * (size_t)k];
         for (int64_t i = offsets[k]; i < offsets[k + 1]; ++i) {
-            for (int d = 0; d < 3; ++d) out->Xp[d * n + i] = (X[d * n + i] - cen[3 * (size_t)k + d]) + cc[d];
+            for (int d = 0; d < 3; ++d) out->Xp[d * n + i] = (X[d * n + i] - c[d]) + c[3 + d];
             out->sys[i] = k;
             for (int w = 0; w < exw; ++w) {
                 const int32_t e = ex[(size_t)w * n + i];
@@ -662,8 +693,101 @@ int pack_systems(int nsys, const int64_t* offsets, const double* X, int exw, con
             }
         }
     }
-    out->root_r = 0.5 * G * S;
-    out->min_size = min_size;
+    return FMM_OK;
+}
+
+// Bounds of one coordinate (threadIdx.y) of chunk blockIdx.y of a system, with
+// std::min's and std::max's comparisons.
+__global__ void __launch_bounds__(3 * 256) k_system_bounds(int64_t n, const int64_t* __restrict__ offsets,
+                                                           const double* __restrict__ X,
+                                                           double* __restrict__ bounds) {
+    const int64_t a = offsets[blockIdx.x], b = offsets[blockIdx.x + 1];
+    const int d = threadIdx.y;
+    const double* x = X + (size_t)d * n;
+    double lo = x[a], hi = lo;
+    for (int64_t i = a + blockIdx.y * 256 + threadIdx.x; i < b; i += 256LL * gridDim.y) {
+        const double v = x[i];
+        lo = v < lo ? v : lo;
+        hi = hi < v ? v : hi;
+    }
+    __shared__ double slo[3][8], shi[3][8];
+    for (int o = 16; o > 0; o >>= 1) {
+        const double l = __shfl_xor_sync(0xffffffffu, lo, o), h = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = l < lo ? l : lo;
+        hi = hi < h ? h : hi;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        slo[d][threadIdx.x >> 5] = lo;
+        shi[d][threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) {
+            lo = slo[d][k] < lo ? slo[d][k] : lo;
+            hi = hi < shi[d][k] ? shi[d][k] : hi;
+        }
+        double* o = bounds + 6 * ((size_t)blockIdx.x * gridDim.y + blockIdx.y);
+        o[d] = lo;
+        o[3 + d] = hi;
+    }
+}
+
+// Moves every particle into its system's cell, makes its exclusions global
+// and notes its system.  tab: offsets (nsys + 1), then pack_box's table.
+__global__ void k_pack_systems(int64_t n, int nsys, const int64_t* __restrict__ offsets,
+                               const double* __restrict__ tab, int exw, double* __restrict__ X,
+                               int32_t* __restrict__ ex, int32_t* __restrict__ sys) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int k = 0, hi = nsys;
+    while (hi - k > 1) {
+        const int m = (k + hi) >> 1;
+        if (offsets[m] <= i) k = m;
+        else hi = m;
+    }
+    const double* c = tab + 6 * (size_t)k;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) X[(size_t)d * n + i] = (X[(size_t)d * n + i] - c[d]) + c[3 + d];
+    sys[i] = k;
+    for (int w = 0; w < exw; ++w) {
+        const int32_t e = ex[(size_t)w * n + i];
+        if (e != 0) ex[(size_t)w * n + i] = (int32_t)(e + offsets[k]);
+    }
+}
+
+// On the device, in place on the uploaded coordinates and exclusions (on the
+// host, with the copies around it, 2 of 11 ms of a call with 309,000 particles).
+int pack_systems_device(Workspace& ws, int nsys, const int64_t* offsets, int exw, double* X, int32_t* ex,
+                        double* root_r, cudaStream_t st) {
+    const int64_t n = offsets[nsys];
+    int64_t biggest = 0;
+    for (int k = 0; k < nsys; ++k) biggest = std::max(biggest, offsets[k + 1] - offsets[k]);
+    const int chunks = (int)std::min<int64_t>(64, (biggest + 8191) / 8192);
+    const size_t ob = sizeof(int64_t) * ((size_t)nsys + 1), bb = sizeof(double) * 6 * (size_t)nsys * chunks;
+    FMM_TRY(ws.sys_ids.ensure(sizeof(int32_t) * (size_t)n));
+    FMM_TRY(ws.sys_tab.ensure(ob + bb));
+    int64_t* d_off = ws.sys_tab.as<int64_t>();
+    double* d_tab = reinterpret_cast<double*>(d_off + nsys + 1);
+    FMM_CUDA_TRY(cudaMemcpyAsync(d_off, offsets, ob, cudaMemcpyHostToDevice, st));
+    count_launches(1);
+    k_system_bounds<<<dim3((unsigned)nsys, (unsigned)chunks), dim3(256, 3), 0, st>>>(n, d_off, X, d_tab);
+    std::vector<double> part(6 * (size_t)nsys * chunks), bounds(6 * (size_t)nsys), tab;
+    FMM_CUDA_TRY(cudaMemcpyAsync(part.data(), d_tab, bb, cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int k = 0; k < nsys; ++k)
+        for (int e = 0; e < 6; ++e) {
+            const double* v = &part[6 * (size_t)k * chunks + e];
+            double r = v[0];
+            for (int c = 1; c < chunks; ++c) r = e < 3 ? std::min(r, v[6 * c]) : std::max(r, v[6 * c]);
+            bounds[6 * (size_t)k + e] = r;
+        }
+    *root_r = pack_box(nsys, bounds, tab);
+    FMM_CUDA_TRY(cudaMemcpyAsync(d_tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, st));
+    count_launches(1);
+    k_pack_systems<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, nsys, d_off, d_tab, exw, X, ex,
+                                                                ws.sys_ids.as<int32_t>());
+    FMM_CUDA_TRY(cudaGetLastError());
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));  // the table's host copy
     return FMM_OK;
 }
 
@@ -1152,29 +1276,22 @@ int fmm_field_fmm_batched(int nsys, const int64_t* offsets, const double* X, int
     if (ncrit < 1 || p < 0 || !(theta > 0.0)) return FMM_EINVAL;
     if (p > kMaxP) return FMM_ENOTSUP;
     if (exw > 0 && !ex) return FMM_EINVAL;
-    Packed pk;
-    FMM_TRY(pack_systems(nsys, offsets, X, exw, ex, ncrit, &pk));
-    const std::vector<double>& Xp = pk.Xp;
-    const std::vector<int32_t>& exg = pk.exg;
-    const std::vector<int32_t>& sys = pk.sys;
-    const int64_t min_size = pk.min_size;
+    int64_t min_size = 0;
+    FMM_TRY(check_systems(nsys, offsets, exw, ex, ncrit, &min_size));
     Workspace& ws = thread_workspace();
     cudaStream_t st = o.stream;
     const int nf = nT(field_order);
     Particles P;
-    FMM_TRY(upload(ws, n, Xp.data(), mdim, mp, exw, exg.data(), dt != DAMP_NONE ? dampf : nullptr, nf, &P, st));
+    FMM_TRY(upload(ws, n, X, mdim, mp, exw, ex, dt != DAMP_NONE ? dampf : nullptr, nf, &P, st));
     P.damp_type = dt;
     FMM_TRY(ws.sysbuf.ensure(sizeof(int32_t) * (size_t)n));
-    // the node system ids reuse sysbuf after the tree is built, so keep the
-    // per-particle ids in the scalars-independent buffer below
-    DevBuf dsys;
-    FMM_TRY(dsys.ensure(sizeof(int32_t) * (size_t)n));
-    FMM_CUDA_TRY(cudaMemcpyAsync(dsys.p, sys.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
     TreeParams tp{ncrit, theta, 1, 1, {0, 0, 0}, o.mac_mode, 0.0, p};
-    tp.root_r = pk.root_r;
-    tp.d_sys = dsys.as<int32_t>();
+    FMM_TRY(pack_systems_device(ws, nsys, offsets, exw, ws.in_coords.as<double>(), ws.in_excl.as<int32_t>(),
+                                &tp.root_r, st));
+    // (the node system ids go to sysbuf once the tree is built)
+    tp.d_sys = ws.sys_ids.as<int32_t>();
     int rc = o.autotune ? run_fmm_tuned(ws, P, theta, ncrit, p, field_order, o, tp, ws.out_field.as<double>(), st,
-                                        tune_key(n, Xp.data(), mdim, field_order, p, o, dt, theta, true, pk.root_r),
+                                        tune_key(n, X, mdim, field_order, p, o, dt, theta, true, tp.root_r),
                                         min_size)
                         : run_fmm(ws, P, theta, ncrit, p, field_order, o, tp, ws.out_field.as<double>(), st);
     if (rc == FMM_OK) {
@@ -1184,7 +1301,6 @@ int fmm_field_fmm_batched(int nsys, const int64_t* offsets, const double* X, int
             rc = FMM_ECUDA;
     }
     cudaStreamSynchronize(st);
-    dsys.release();
     return rc;
 }
 
