@@ -122,16 +122,16 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
                                                  const double* __restrict__ sd, const double* __restrict__ rows,
                                                  int64_t n, int damp, int excl_mode, int exw,
                                                  const int32_t* __restrict__ excl, double* __restrict__ out) {
-    constexpr int NF = nT(F), NR = near_row_count(M, F);
+    constexpr int NF = nT(F), NA = acc_count(M, F), NR = near_row_count(M, F);
     const int64_t tgt = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (tgt >= n) return;
     const int leaf = t.leaf_of[tgt];
     const double xt = sx[tgt], yt = sy[tgt], zt = sz[tgt], dt = sd[tgt];
     const ExList ex(excl, exw, n, (int64_t)t.perm[tgt]);
-    double acc[NF];
+    double acc[NA];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+    for (int f = 0; f < NA; ++f) acc[f] = 0.0;
     const int q1 = t.near_off[leaf + 1], step = 32 * (int)gridDim.y;
     int q = t.near_off[leaf] - 1, js = 0, jc = 0, img = 0;
     for (int off = lane + 32 * (int)blockIdx.y;; off += step) {
@@ -170,7 +170,9 @@ __global__ void __launch_bounds__(128) k_p2p_f64(const TreeDev t, const double* 
         pair_field_f64<M, F>(dx, dy, dz, dt * sd[k], damp, mc, acc);
     }
     int f;
-    if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * n + tgt] = acc[0];
+    double fld[NF];
+    finish_f64<M, F>(acc, fld);
+    if (warp_totals<NF>(fld, lane, &f)) out[((size_t)blockIdx.y * NF + f) * n + tgt] = fld[0];
 }
 
 // out[e] = sum over the slices of part[slice][e].
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(128) k_direct_f64(int64_t n, const int64_t* __
                                                     const double* __restrict__ damp, int damp_type, int excl_mode,
                                                     int exw, const int32_t* __restrict__ excl, int64_t chunk,
                                                     double* __restrict__ out) {
-    constexpr int NF = nT(F), NR = near_row_count(M, F);
+    constexpr int NF = nT(F), NA = acc_count(M, F), NR = near_row_count(M, F);
     const int64_t ti = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (ti >= ntgt) return;
@@ -198,9 +200,9 @@ __global__ void __launch_bounds__(128) k_direct_f64(int64_t n, const int64_t* __
     const double xi = X[i], yi = X[n + i], zi = X[2 * n + i];
     const double di = damp ? damp[i] : 0.0;
     const ExList ex(excl, exw, n, i);
-    double acc[NF];
+    double acc[NA];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+    for (int f = 0; f < NA; ++f) acc[f] = 0.0;
     const int64_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
     for (int64_t j = j0 + lane; j < j1; j += 32) {
         double dx = xi - X[j], dy = yi - X[n + j], dz = zi - X[2 * n + j];
@@ -216,7 +218,9 @@ __global__ void __launch_bounds__(128) k_direct_f64(int64_t n, const int64_t* __
         pair_field_f64<M, F>(dx, dy, dz, di * (damp ? damp[j] : 0.0), damp_type, mc, acc);
     }
     int f;
-    if (warp_totals<NF>(acc, lane, &f)) out[((size_t)blockIdx.y * NF + f) * ntgt + ti] = acc[0];
+    double fld[NF];
+    finish_f64<M, F>(acc, fld);
+    if (warp_totals<NF>(fld, lane, &f)) out[((size_t)blockIdx.y * NF + f) * ntgt + ti] = fld[0];
 }
 
 __device__ __forceinline__ bool is_near_leaf(const int32_t* near_off, const int32_t* near_src, int li, int lj) {

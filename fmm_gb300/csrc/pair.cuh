@@ -79,8 +79,8 @@ __device__ __forceinline__ double f64_bits(float x) {
 // in FP32.  Seven FP64 instructions; the FP64 pair kernels are bound by these
 // (csrc/pair_f64.cuh).  With this and rsqrt_f64 for the library's functions:
 // 200,000 particles with Thole damping, f = 2, 128.5 -> 120.0 ms; direct
-// gradient of 20,000 particles, AMOEBA damping, 77.8 -> 73.1 ms.  Within 1 ulp
-// of the library's; 0 below -700.
+// gradient of 20,000 particles, AMOEBA damping, 77.8 -> 73.1 ms (101.2 and
+// 67.1 with what came later).  Within 1 ulp of the library's; 0 below -700.
 __device__ __forceinline__ double exp_nonpos(double x) {
     const float xf = f32_bits(x);
     if (!(xf >= -700.0f)) return x < 0.0 ? 0.0 : x;
@@ -134,6 +134,14 @@ struct Real<double> {
         return ::rsqrt(x);
 #else
         return 1.0 / ::sqrt(x);
+#endif
+    }
+    // an operand of comparisons: FP64 ones would take the FP64 pipe
+    __host__ __device__ static __forceinline__ float cmp(double x) {
+#ifdef __CUDA_ARCH__
+        return f32_bits(x);
+#else
+        return (float)x;
 #endif
     }
     // (arguments <= 0 here)
@@ -238,6 +246,7 @@ struct Real<float> {
         return 1.0f / ::sqrtf(x);
 #endif
     }
+    __host__ __device__ static __forceinline__ float cmp(float x) { return x; }
     __host__ __device__ static __forceinline__ float exp_(float x) { return ::expf(x); }
     // e^x for the closed forms of the damped numerators (x <= -3): there it
     // scales a correction of at most ~0.3 of the numerator's constant term,
@@ -300,7 +309,7 @@ __host__ __device__ __forceinline__ void radial_g(int damp, R r2, R a, R* g) {
 }
 
 // Same, with 1/r supplied by the caller (e.g. a refined FP32 value) and,
-// optionally, the relative error eps of that value (1/r = ir (1 + eps)):
+// optionally (FP32), the relative error eps of that value (1/r = ir (1 + eps)):
 // the powers r^-(2j+1) then carry the correction (2j+1) eps, which keeps the
 // error of a rounded ir from growing with the tensor order.
 template <int N, typename R>
@@ -313,8 +322,10 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
         g[0] = ir;
 #pragma unroll
         for (int j = 1; j <= N; ++j) g[j] = -(R)(2 * j - 1) * g[j - 1] * ir2;
+        if constexpr (sizeof(R) == 4) {
 #pragma unroll
-        for (int j = 0; j <= N; ++j) g[j] += g[j] * ((R)(2 * j + 1) * eps);
+            for (int j = 0; j <= N; ++j) g[j] += g[j] * ((R)(2 * j + 1) * eps);
+        }
         return;
     }
     if (damp == DAMP_ERF) {
@@ -382,7 +393,7 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
                 }
             }
         } else {
-            closed = !(x < RT::kTholeX);
+            closed = !(RT::cmp(x) < (float)RT::kTholeX);
             if (!closed) {
 #pragma unroll
                 for (int j = 0; j <= N; ++j) {
@@ -393,7 +404,7 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
                 }
             }
         }
-        if (closed && sizeof(R) == 8 && x > (R)100) {
+        if (closed && sizeof(R) == 8 && RT::cmp(x) > 100.0f) {
             // FP64, far beyond the damping range: e^{-x} P(x) is below 1e-29
             // of the undamped value, so the sum rounds to it exactly
             num[0] = (R)1;
@@ -431,7 +442,7 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
                 }
             }
         } else {
-            closed = !(u < RT::kAmoebaU);
+            closed = !(RT::cmp(u) < (float)RT::kAmoebaU);
             if (!closed) {
 #pragma unroll
                 for (int j = 1; j <= N; ++j) {
@@ -442,7 +453,7 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
                 }
             }
         }
-        if (closed && sizeof(R) == 8 && u > (R)80) {
+        if (closed && sizeof(R) == 8 && RT::cmp(u) > 80.0f) {
             // FP64, far beyond the damping range: e^{-u} q(u) is below 1e-25
             // of the undamped value, so the sum rounds to it exactly
 #pragma unroll
@@ -461,8 +472,8 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
     R irp = ir;
 #pragma unroll
     for (int j = 0; j <= N; ++j) {
-        const R v = num[j] * irp;
-        g[j] = v + v * ((R)(2 * j + 1) * eps);
+        g[j] = num[j] * irp;
+        if constexpr (sizeof(R) == 4) g[j] += g[j] * ((R)(2 * j + 1) * eps);
         irp *= ir2;
     }
 }

@@ -9,8 +9,10 @@
 // (tr = Mc_xx + Mc_yy + Mc_zz) and d g_j / d R_a = R_a g_{j+1},
 //   F_0    = S_0,                  S_k = sum_i g_{i+k} A_i
 //   F_a    = R_a S_1 + V0_a,       Vk_a = sum_i g_{i+k} dA_i / dR_a
-//   F_ab   = delta_ab S_1 + R_a R_b S_2 + R_a V1_b + R_b V1_a + W_ab,
+//   F_ab   = delta_ab S_1 + R_a U_b + R_b U_a + W_ab,  U_a = V1_a + R_a S_2 / 2,
 //   W_ab   = g_2 d^2 A_2 / dR_a dR_b.
+// The diagonal is summed as halves, R_a U_a + W_aa / 2, beside one sum of S_1
+// for all three (finish_f64).
 // Quadrupole sources come as "near rows" (near_rows below): the off-diagonal
 // second moments halved (exact) and tr as an extra row, so that with
 // h = grad A_2 / 2 the terms are A_2 = R . h and 2 g_2 h.  FP64 instructions
@@ -27,6 +29,23 @@ namespace fmm {
 __host__ __device__ constexpr bool near_rows(int m, int f) { return m <= 2 && f <= 2; }
 // Rows of source coefficients per particle.
 __host__ __device__ constexpr int near_row_count(int m, int f) { return nT(m) + (m == 2 && f <= 2 ? 1 : 0); }
+
+// Accumulators of the field: its components and, with the diagonal in halves,
+// the sum of S_1.
+__host__ __device__ constexpr int acc_count(int m, int f) { return nT(f) + (near_rows(m, f) && f == 2 ? 1 : 0); }
+
+// The field's components from the accumulators (of any part of the sum).
+template <int M, int F>
+__device__ __forceinline__ void finish_f64(const double* acc, double* fld) {
+#pragma unroll
+    for (int f = 0; f < nT(F); ++f) fld[f] = acc[f];
+    if constexpr (acc_count(M, F) > nT(F)) {
+        constexpr double w = M == 0 ? 1.0 : 2.0;
+        fld[4] = fma(w, acc[4], acc[10]);
+        fld[7] = fma(w, acc[7], acc[10]);
+        fld[9] = fma(w, acc[9], acc[10]);
+    }
+}
 
 // Beyond these the damped numerators round to the undamped ones for every
 // order up to 6: e^-u q_6(u) / 11!! < 2^-62 from u = (a r)^3 = 60 (AMOEBA),
@@ -89,32 +108,34 @@ __device__ __forceinline__ void contract_f64(double X, double Y, double Z, const
             double S2 = mc[0] * g[2];
             if constexpr (M >= 1) S2 = fma(A1, g[3], S2);
             if constexpr (M >= 2) S2 = fma(A2, g[4], S2);
-            double V1[3], U[3];
+            const double S2h = M == 0 ? S2 : 0.5 * S2;
+            double U[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 if constexpr (M == 0) {
-                    U[c] = R[c] * S2;
+                    U[c] = R[c] * S2h;  // (charges: whole components)
                 } else {
-                    V1[c] = mc[1 + c] * g[2];
-                    if constexpr (M == 2) V1[c] = fma(h[c], g[3] + g[3], V1[c]);
-                    U[c] = fma(R[c], S2, V1[c]);
+                    double v = mc[1 + c] * g[2];
+                    if constexpr (M == 2) v = fma(h[c], g[3] + g[3], v);
+                    U[c] = fma(R[c], S2h, v);
                 }
             }
+            acc[10] += S1;
             // components xx, xy, xz, yy, yz, zz
             constexpr int ca[6] = {0, 0, 0, 1, 1, 2}, cb[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
             for (int q = 0; q < 6; ++q) {
                 double v = fma(R[ca[q]], U[cb[q]], acc[4 + q]);
-                if constexpr (M >= 1) v = fma(R[cb[q]], V1[ca[q]], v);
-                if constexpr (M == 2) v = fma(mc[4 + q], g2d, v);
-                if (ca[q] == cb[q]) v += S1;
+                if (M > 0 && ca[q] != cb[q]) v = fma(R[cb[q]], U[ca[q]], v);
+                if constexpr (M == 2) v = fma(mc[4 + q], ca[q] == cb[q] ? g[2] : g2d, v);
                 acc[4 + q] = v;
             }
         }
     }
 }
 
-// Field of one source (rows mc) at displacement target - source.
+// Field of one source (rows mc) at displacement target - source, into acc_count
+// accumulators.
 template <int M, int F>
 __device__ __forceinline__ void pair_field_f64(double dx, double dy, double dz, double a, int damp, const double* mc,
                                                double* acc) {
