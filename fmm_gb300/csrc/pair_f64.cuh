@@ -16,7 +16,7 @@
 // Quadrupole sources come as "near rows" (near_rows below): the off-diagonal
 // second moments halved (exact) and tr as an extra row, so that with
 // h = grad A_2 / 2 the terms are A_2 = R . h and 2 g_2 h.  FP64 instructions
-// per undamped pair (m = 2): 50 at f = 1 and 80 at f = 2, against 126 and
+// per undamped pair (m = 2): 47 at f = 1 and 74 at f = 2, against 126 and
 // about 240 of the tensor recursion and full contraction (which orders above
 // 2 keep, pair.cuh).
 #pragma once

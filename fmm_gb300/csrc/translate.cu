@@ -139,8 +139,9 @@ __constant__ float2 cInvIntF[kMaxP + 1] = {
 
 // e[a] = d^a / a!, a = 0..p
 __device__ __forceinline__ void scaled_powers(double d, int p, double* e) {
-    e[0] = 1.0;
-    for (int a = 1; a <= p; ++a) e[a] = e[a - 1] * d * cInvInt[a];
+    double v = 1.0;
+    e[0] = v;
+    for (int a = 1; a <= p; ++a) e[a] = v *= d * cInvInt[a];
 }
 
 // Product of two double-float pairs (hi, lo), renormalised.
@@ -455,22 +456,25 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_p2m(const TreeDev t, const dou
 // (a (p+1) + b) (p+1) + c for the component (a, b, c): C(p+4,4) terms per
 // shift instead of the C(p+6,6) of the direct sum, and no output of a shift
 // has more than p+1 terms, so the block's outputs finish together.  A block
-// per parent node takes its children one after another.
-constexpr int kXThreads = 512;  // one output per thread up to order 12: a shift waits for at most p+1 terms
-constexpr int kXOut = (nT(kMaxP) + kXThreads - 1) / kXThreads;  // outputs per thread
+// per parent node takes its children NG at a time, each by a group of kXThreads
+// / NG threads with one output per thread: a level is a chain of dependent
+// shifts, and with a whole block per child (NG = 1, which orders above 9 need)
+// low orders leave most of its threads idle.  30,000 dipoles at p = 6, four
+// levels up and down, 153 of 865 us: the call 896 -> 834 us.
+constexpr int kXThreads = 512;
+static_assert(nT(kMaxP) <= kXThreads, "one output per thread");
+int x_groups(int p) { return nT(p) <= kXThreads / 4 ? 4 : (nT(p) <= kXThreads / 2 ? 2 : 1); }
 
 __device__ __forceinline__ int d3(int a, int b, int c, int P1) { return (a * P1 + b) * P1 + c; }
 
 // Children of a node (ch[0..7], count in ch[8]) and the scaled powers
 // d^a / a! of their offsets d = c_child - c_node, e[(k * 3 + axis) * (p+1) + a].
 __device__ __forceinline__ void child_offsets(const TreeDev& t, int node, int p, int* ch, double* e) {
-    if (threadIdx.x == 0) {
-        int k = 0;
-        for (int o = 0; o < 8; ++o) {
-            const int c = t.child[8 * node + o];
-            if (c >= 0) ch[k++] = c;
-        }
-        ch[8] = k;
+    if (threadIdx.x < 32) {
+        const int c = threadIdx.x < 8 ? t.child[8 * node + threadIdx.x] : -1;
+        const unsigned has = __ballot_sync(0xffffffffu, c >= 0);
+        if (c >= 0) ch[__popc(has & ((1u << threadIdx.x) - 1))] = c;
+        if (threadIdx.x == 0) ch[8] = __popc(has);
     }
     __syncthreads();
     const int P1 = p + 1;
@@ -486,18 +490,19 @@ __device__ __forceinline__ void child_offsets(const TreeDev& t, int node, int p,
 // as shifts along z (Y from X), y (X from Y) and x (into the accumulator of
 // the thread's output), each visiting its outputs sorted by the number of
 // terms; the next child's moments are loaded during the current child's
-// shifts.  Writes the result unless *big was raised.
-template <bool DF>
+// shifts.  The groups' sums are added in order at the end.  Writes the result
+// unless *big was raised.
+template <bool DF, int NG>
 __device__ __forceinline__ void m2m_node(int node, int p, int nq, const int* comp, const int* byz, const int* byy,
                                          const int* byx, const int* ch, const double* e, void* buf, int* big,
                                          double* __restrict__ mom) {
-    static_assert(kXOut == 1, "one output per thread");
     using O = XOps<DF>;
     using V = typename O::V;
-    const int P1 = p + 1, n3 = P1 * P1 * P1, q = threadIdx.x;
-    V* X = reinterpret_cast<V*>(buf);
+    constexpr int GT = kXThreads / NG;
+    const int P1 = p + 1, n3 = P1 * P1 * P1, q = threadIdx.x % GT, grp = threadIdx.x / GT;
+    V* X = reinterpret_cast<V*>(buf) + 2 * grp * n3;
     V* Y = X + n3;
-    V* E = Y + n3;  // [8][3][p+1]
+    V* E = reinterpret_cast<V*>(buf) + 2 * NG * n3;  // [8][3][p+1]
     const int nch = ch[8];
     for (int k = threadIdx.x; k < nch * 3 * P1; k += blockDim.x) E[k] = O::in(e[k], big);
     int cz = 0, cy = 0, cx = 0, xo = 0;
@@ -507,45 +512,55 @@ __device__ __forceinline__ void m2m_node(int node, int p, int nq, const int* com
         cx = byx[q];
         xo = pk_index(cx & 0xff, (cx >> 8) & 0xff, cx >> 16);
     }
-    double mnext = (q < nq && nch > 0) ? mom[(size_t)ch[0] * nq + q] : 0.0;
+    double mnext = (q < nq && grp < nch) ? mom[(size_t)ch[grp] * nq + q] : 0.0;
     typename O::Acc acc;
-    for (int b = 0; b < nch; ++b) {
-        if (q < nq) {
+    for (int b0 = 0; b0 < nch; b0 += NG) {
+        const int b = b0 + grp;
+        const bool on = q < nq && b < nch;
+        if (on) {
             const int cc = comp[q];
             X[d3(cc & 0xff, (cc >> 8) & 0xff, cc >> 16, P1)] = O::in(mnext, big);
         }
         __syncthreads();
-        if (b + 1 < nch && q < nq) mnext = mom[(size_t)ch[b + 1] * nq + q];  // in flight during the shifts
+        if (q < nq && b + NG < nch) mnext = mom[(size_t)ch[b + NG] * nq + q];  // in flight during the shifts
         const V* ex = E + b * 3 * P1;
         const V* ey = ex + P1;
         const V* ez = ey + P1;
-        if (q < nq) {
+        if (on) {
             const int x = cz & 0xff, y = (cz >> 8) & 0xff, z = cz >> 16;
             typename O::Acc s;
             for (int u = 0; u <= z; ++u) s.mac(ez[u], X[d3(x, y, z - u, P1)]);
             Y[d3(x, y, z, P1)] = s.val();
         }
         __syncthreads();
-        if (q < nq) {
+        if (on) {
             const int x = cy & 0xff, y = (cy >> 8) & 0xff, z = cy >> 16;
             typename O::Acc s;
             for (int u = 0; u <= y; ++u) s.mac(ey[u], Y[d3(x, y - u, z, P1)]);
             X[d3(x, y, z, P1)] = s.val();
         }
         __syncthreads();
-        if (q < nq) {
+        if (on) {
             const int x = cx & 0xff, y = (cx >> 8) & 0xff, z = cx >> 16;
             for (int u = 0; u <= x; ++u) acc.mac(ex[u], X[d3(x - u, y, z, P1)]);
         }
         __syncthreads();  // X is the next child's
     }
+    if constexpr (NG > 1) {
+        if (grp > 0 && q < nq) X[q] = acc.val();  // (nq <= n3)
+        __syncthreads();
+        if (grp == 0 && q < nq) {
+#pragma unroll
+            for (int k = 1; k < NG; ++k) acc.add(X[2 * k * n3 + q]);
+        }
+    }
     if (DF && *big) return;
-    if (q < nq) mom[(size_t)node * nq + xo] = O::out(acc.val());
+    if (grp == 0 && q < nq) mom[(size_t)node * nq + xo] = O::out(acc.val());
 }
 
 // DF: double-float shifts, FP64 again for the blocks whose powers or moments
 // leave the range where FP32 exponents suffice.
-template <bool DF>
+template <bool DF, int NG>
 __global__ void __launch_bounds__(kXThreads) k_m2m(const TreeDev t, const int32_t* __restrict__ nodes, int p,
                                                    const int* __restrict__ tab, TabView v, double* __restrict__ mom) {
     extern __shared__ __align__(16) double sm_m2m[];
@@ -559,67 +574,64 @@ __global__ void __launch_bounds__(kXThreads) k_m2m(const TreeDev t, const int32_
     copy_ints(comp, tab + v.comp, 4 * nq);
     if (threadIdx.x == 0) big = 0;
     child_offsets(t, node, p, ch, e);
-    m2m_node<DF>(node, p, nq, comp, comp + nq, comp + 2 * nq, comp + 3 * nq, ch, e, buf, &big, mom);
+    m2m_node<DF, NG>(node, p, nq, comp, comp + nq, comp + 2 * nq, comp + 3 * nq, ch, e, buf, &big, mom);
     if (DF) {
         __syncthreads();
-        if (big) m2m_node<false>(node, p, nq, comp, comp + nq, comp + 2 * nq, comp + 3 * nq, ch, e, buf, &big, mom);
+        if (big) m2m_node<false, NG>(node, p, nq, comp, comp + nq, comp + 2 * nq, comp + 3 * nq, ch, e, buf, &big, mom);
     }
 }
 
 // L2L of one parent into each child: L_t(child) += sum_u L_{t+u}(parent)
 // d^u/u! (|t + u| <= p) as shifts along z (Y from X, the parent's
 // expansion), y (Z from Y) and x (into the child's expansion).
-template <bool DF>
+template <bool DF, int NG>
 __device__ __forceinline__ void l2l_node(int node, int p, int nq, const int* comp, const int* ch, const double* e,
                                          void* buf, int* big, double* __restrict__ loc) {
-    static_assert(kXOut == 1, "one output per thread");
     using O = XOps<DF>;
     using V = typename O::V;
-    const int P1 = p + 1, n3 = P1 * P1 * P1;
+    constexpr int GT = kXThreads / NG;
+    const int P1 = p + 1, n3 = P1 * P1 * P1, q = threadIdx.x % GT, grp = threadIdx.x / GT;
     V* X = reinterpret_cast<V*>(buf);
-    V* Y = X + n3;
+    V* Y = X + (1 + 2 * grp) * n3;
     V* Z = Y + n3;
-    V* E = Z + n3;  // [8][3][p+1]
+    V* E = X + (1 + 2 * NG) * n3;  // [8][3][p+1]
     const int nch = ch[8];
     for (int k = threadIdx.x; k < nch * 3 * P1; k += blockDim.x) E[k] = O::in(e[k], big);
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-        const int cc = comp[q];
-        X[d3(cc & 0xff, (cc >> 8) & 0xff, cc >> 16, P1)] = O::in(loc[(size_t)node * nq + q], big);
-    }
+    const int cc = q < nq ? comp[q] : 0, x = cc & 0xff, y = (cc >> 8) & 0xff, z = cc >> 16;
+    if (grp == 0 && q < nq) X[d3(x, y, z, P1)] = O::in(loc[(size_t)node * nq + q], big);
     __syncthreads();
     if (DF && *big) return;  // every thread sees the flag after the barrier
-    for (int b = 0; b < nch; ++b) {
+    for (int b0 = 0; b0 < nch; b0 += NG) {
+        const int b = b0 + grp;
+        const bool on = q < nq && b < nch;
         const V* ex = E + b * 3 * P1;
         const V* ey = ex + P1;
         const V* ez = ey + P1;
         // the child's own expansion, in flight during the shifts
-        double* lc = loc + (size_t)ch[b] * nq;
-        const double lprev = threadIdx.x < nq ? lc[threadIdx.x] : 0.0;
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            const int cc = comp[q], x = cc & 0xff, y = (cc >> 8) & 0xff, z = cc >> 16;
+        double* lc = on ? loc + (size_t)ch[b] * nq + q : nullptr;
+        const double lprev = on ? *lc : 0.0;
+        if (on) {
             typename O::Acc s;
             for (int u = 0; u <= p - x - y - z; ++u) s.mac(ez[u], X[d3(x, y, z + u, P1)]);
             Y[d3(x, y, z, P1)] = s.val();
         }
         __syncthreads();
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            const int cc = comp[q], x = cc & 0xff, y = (cc >> 8) & 0xff, z = cc >> 16;
+        if (on) {
             typename O::Acc s;
             for (int u = 0; u <= p - x - y - z; ++u) s.mac(ey[u], Y[d3(x, y + u, z, P1)]);
             Z[d3(x, y, z, P1)] = s.val();
         }
         __syncthreads();
-        if (threadIdx.x < nq) {  // one output per thread
-            const int q = threadIdx.x, cc = comp[q], x = cc & 0xff, y = (cc >> 8) & 0xff, z = cc >> 16;
+        if (on) {
             typename O::Acc s;
             for (int u = 0; u <= p - x - y - z; ++u) s.mac(ex[u], Z[d3(x + u, y, z, P1)]);
-            lc[q] = lprev + O::out(s.val());
+            *lc = lprev + O::out(s.val());
         }
         __syncthreads();  // Y and Z are the next child's
     }
 }
 
-template <bool DF>
+template <bool DF, int NG>
 __global__ void __launch_bounds__(kXThreads) k_l2l(const TreeDev t, const int32_t* __restrict__ nodes, int p,
                                                    const int* __restrict__ tab, TabView v, double* __restrict__ loc) {
     extern __shared__ __align__(16) double sm_l2l[];
@@ -633,10 +645,10 @@ __global__ void __launch_bounds__(kXThreads) k_l2l(const TreeDev t, const int32_
     copy_ints(comp, tab + v.comp, nq);
     if (threadIdx.x == 0) big = 0;
     child_offsets(t, node, p, ch, e);
-    l2l_node<DF>(node, p, nq, comp, ch, e, buf, &big, loc);
+    l2l_node<DF, NG>(node, p, nq, comp, ch, e, buf, &big, loc);
     if (DF && big) {
         __syncthreads();
-        l2l_node<false>(node, p, nq, comp, ch, e, buf, &big, loc);
+        l2l_node<false, NG>(node, p, nq, comp, ch, e, buf, &big, loc);
     }
 }
 
@@ -762,19 +774,16 @@ int launch_p2m_m2m(Workspace& ws, const Particles& P, const TreeDev& t, int p, c
             else return FMM_ENOTSUP;
         }
     }
-    {
-        const size_t sm = xlate_smem(p, 2, 4);
-        FMM_TRY(set_smem((const void*)k_m2m<false>, sm));
-        FMM_TRY(set_smem((const void*)k_m2m<true>, sm));
-        for (int d = t.max_depth - 1; d >= 1; --d) {
-            const int lo = t.level_start[d], hi = t.level_start[d + 1];
-            if (hi <= lo) continue;
-            count_launches(1);
-            if (df)
-                k_m2m<true><<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, mom);
-            else
-                k_m2m<false><<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, mom);
-        }
+    const int ng = x_groups(p);
+    const size_t sm = xlate_smem(p, 2 * ng, 4);
+    auto kernel = df ? (ng == 4 ? k_m2m<true, 4> : (ng == 2 ? k_m2m<true, 2> : k_m2m<true, 1>))
+                     : (ng == 4 ? k_m2m<false, 4> : (ng == 2 ? k_m2m<false, 2> : k_m2m<false, 1>));
+    FMM_TRY(set_smem((const void*)kernel, sm));
+    for (int d = t.max_depth - 1; d >= 1; --d) {
+        const int lo = t.level_start[d], hi = t.level_start[d + 1];
+        if (hi <= lo) continue;
+        count_launches(1);
+        kernel<<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, mom);
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -787,19 +796,16 @@ int launch_l2l_l2p(Workspace& ws, const Particles& P, const TreeDev& t, int p, i
     FMM_TRY(ensure_tables(ws, p, &v, st));
     const int* tab = ws.xlate.as<int>();
     double* loc = ws.loc.as<double>();
-    {
-        const size_t sm = xlate_smem(p, 3, 1);
-        FMM_TRY(set_smem((const void*)k_l2l<false>, sm));
-        FMM_TRY(set_smem((const void*)k_l2l<true>, sm));
-        for (int d = 1; d < t.max_depth; ++d) {
-            const int lo = t.level_start[d], hi = t.level_start[d + 1];
-            if (hi <= lo) continue;
-            count_launches(1);
-            if (fp32)
-                k_l2l<true><<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, loc);
-            else
-                k_l2l<false><<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, loc);
-        }
+    const int ng = x_groups(p);
+    const size_t sm = xlate_smem(p, 1 + 2 * ng, 1);
+    auto kernel = fp32 ? (ng == 4 ? k_l2l<true, 4> : (ng == 2 ? k_l2l<true, 2> : k_l2l<true, 1>))
+                       : (ng == 4 ? k_l2l<false, 4> : (ng == 2 ? k_l2l<false, 2> : k_l2l<false, 1>));
+    FMM_TRY(set_smem((const void*)kernel, sm));
+    for (int d = 1; d < t.max_depth; ++d) {
+        const int lo = t.level_start[d], hi = t.level_start[d + 1];
+        if (hi <= lo) continue;
+        count_launches(1);
+        kernel<<<(unsigned)(hi - lo), kXThreads, sm, st>>>(t, t.level_nodes + lo, p, tab, v, loc);
     }
     if (t.num_leaves > 0) {
         L2pTab lv;
