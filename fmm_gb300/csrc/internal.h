@@ -204,6 +204,7 @@ struct Workspace {
     DevBuf p2p_order;    // target leaves by decreasing pair work (queue mode), and scratch
     float corr_xcut2 = 0.0f;  // damping correction: (a r)^2 beyond which a pair needs none
     DevBuf leaf_ext;          // damping correction: per leaf (particle extent, smallest damping factor)
+    DevBuf list_cnt;  // list construction: pair counts and frontier sizes
     DevBuf sys_ids, sys_tab;  // packed systems: system of each particle; offsets, bounds and cells of the systems
     DevBuf p2p_pad;      // packed near field: padded leaf starts (node-indexed), odd-leaf flags and their scan
     DevBuf f32x2;        // packed near field: interleaved source records of padded leaves

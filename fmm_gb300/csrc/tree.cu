@@ -396,7 +396,8 @@ __global__ void k_pos_of(int64_t n, const uint32_t* __restrict__ perm, int32_t* 
     if (k < n) pos_of[perm[k]] = (int32_t)k;
 }
 
-// counters: [0] next frontier size, [1] far count, [2] near count, [3] overflow flag
+// front: [0] the frontier's size, [1] the next one's.  counters: [1] far count,
+// [2] near count, [3] overflow flag, [4] network evaluations, [5] corrections
 // Slots for this lane's `cnt` entries in a list shared by the whole grid: one
 // atomic per warp (warp-wide inclusive scan of the counts); every lane of
 // the warp must call it.  Returns the first slot of the lane's entries.
@@ -425,7 +426,8 @@ __device__ __forceinline__ void emit_pair(bool skip, bool accept, int order, int
                                           bool mixed, RR ri, RR rj, const TreeDev& t, int2* __restrict__ out,
                                           int64_t cap_out, uint64_t* __restrict__ far, int64_t cap_far,
                                           uint64_t* __restrict__ nearp, int64_t cap_near,
-                                          unsigned long long* counters, int lane, bool corr = false,
+                                          unsigned long long* front, unsigned long long* counters, int lane,
+                                          bool corr = false,
                                           uint64_t* __restrict__ corrp = nullptr, int64_t cap_corr = 0) {
     const int sb = t.src_bits;
     const bool isfar = !skip && accept;
@@ -445,7 +447,7 @@ __device__ __forceinline__ void emit_pair(bool skip, bool accept, int order, int
     }
     const unsigned long long kf = warp_alloc(&counters[1], isfar ? 1u : 0u, lane);
     const unsigned long long kn = warp_alloc(&counters[2], isnear ? 1u : 0u, lane);
-    const unsigned long long kr = warp_alloc(&counters[0], (unsigned)nc, lane);
+    const unsigned long long kr = warp_alloc(front, (unsigned)nc, lane);
     const unsigned long long kc = warp_alloc(&counters[5], iscorr ? 1u : 0u, lane);
     if (iscorr) {
         if (kc < (unsigned long long)cap_corr)
@@ -474,61 +476,65 @@ __device__ __forceinline__ void emit_pair(bool skip, bool accept, int order, int
     }
 }
 
-__global__ void k_list_iter(const int2* __restrict__ in, int nin, int2* __restrict__ out, int64_t cap_out,
-                            uint64_t* __restrict__ far, int64_t cap_far, uint64_t* __restrict__ nearp,
+__global__ void k_list_iter(const int2* __restrict__ in, unsigned long long* front, int2* __restrict__ out,
+                            int64_t cap_out, uint64_t* __restrict__ far, int64_t cap_far, uint64_t* __restrict__ nearp,
                             int64_t cap_near, const TreeDev t, double theta, double rdamp, int order,
                             unsigned long long* counters) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    bool skip = q >= nin;
-    int i = 0, j = 0;
-    double ri = 0.0, rj = 0.0;
-    bool li = false, lj = false, mixed = false, accept = false;
-    if (!skip) {
-        i = in[q].x;
-        j = in[q].y;
-        // delta = c_i - (c_j + displacement) (fmm.F90:357-358); a periodic
-        // image's nodes hold the displaced centre
-        const double dx = __dsub_rn(t.cx[i], t.cx[j]);
-        const double dy = __dsub_rn(t.cy[i], t.cy[j]);
-        const double dz = __dsub_rn(t.cz[i], t.cz[j]);
-        ri = t.rmax[i];
-        rj = t.rmax[j];
-        li = t.is_leaf[i] != 0;
-        lj = t.is_leaf[j] != 0;
-        // batched systems: no pairs across systems; nodes spanning several
-        // systems are always refined
-        if (t.sysid) {
-            const int si = t.sysid[i], sj = t.sysid[j];
-            if (si >= 0 && sj >= 0 && si != sj) skip = true;
-            mixed = si < 0 || sj < 0;
-        }
-        // Both tests in FP32 first: norm2_3's divisions and root are some 60
-        // FP64 instructions a candidate (they took the kernel to 1.18 ms for
-        // 6.5e6 candidates at the FP64 pipe's rate).  The FP32 values are within
-        // 1e-6; only pairs within 1e-5 of equality (the exact ties of a cell
-        // grid) need the reference's rounding.
-        const float fx = f32_bits(fabs(dx)), fy = f32_bits(fabs(dy)), fz = f32_bits(fabs(dz));
-        const float rf = sqrtf(fx * fx + fy * fy + fz * fz), sumf = f32_bits(ri) + f32_bits(rj);
-        const float lhs = rf * (float)theta;
-        const float hif = f32_bits(t.r[i]), hjf = f32_bits(t.r[j]);
-        const float gap = rf - 1.7320508f * (hif + hjf), rd = (float)rdamp;
-        const bool range = rf > 1e-15f && rf < 1e15f && sumf > 1e-15f;
-        const bool sure = range && fabsf(lhs - sumf) > 1e-5f * sumf && (rdamp <= 0.0 || fabsf(gap - rd) > 1e-5f * (rf + rd));
-        if (sure) {
-            accept = !mixed && lhs > sumf && (rdamp <= 0.0 || gap >= rd);
-        } else {
-            const double r = norm2_3(dx, dy, dz);
-            accept = !mixed && __dmul_rn(r, theta) > __dadd_rn(ri, rj);
-            if (accept && rdamp > 0.0) {
-                // closest possible particle distance: centre distance minus the cube circumradii
-                const double gap64 = __dsub_rn(r, __dmul_rn(1.7320508075688772, __dadd_rn(t.r[i], t.r[j])));
-                accept = gap64 >= rdamp;
+    // the pairs, the same number in the whole warp; an overflow ends the expansion
+    const int64_t nin = __shfl_sync(0xffffffffu, counters[3] ? 0ll : (long long)front[0], 0);
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < nin; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t q = base + threadIdx.x;
+        bool skip = q >= nin;
+        int i = 0, j = 0;
+        double ri = 0.0, rj = 0.0;
+        bool li = false, lj = false, mixed = false, accept = false;
+        if (!skip) {
+            i = in[q].x;
+            j = in[q].y;
+            // delta = c_i - (c_j + displacement) (fmm.F90:357-358); a periodic
+            // image's nodes hold the displaced centre
+            const double dx = __dsub_rn(t.cx[i], t.cx[j]);
+            const double dy = __dsub_rn(t.cy[i], t.cy[j]);
+            const double dz = __dsub_rn(t.cz[i], t.cz[j]);
+            ri = t.rmax[i];
+            rj = t.rmax[j];
+            li = t.is_leaf[i] != 0;
+            lj = t.is_leaf[j] != 0;
+            // batched systems: no pairs across systems; nodes spanning several
+            // systems are always refined
+            if (t.sysid) {
+                const int si = t.sysid[i], sj = t.sysid[j];
+                if (si >= 0 && sj >= 0 && si != sj) skip = true;
+                mixed = si < 0 || sj < 0;
+            }
+            // Both tests in FP32 first: norm2_3's divisions and root are some 60
+            // FP64 instructions a candidate (they took the kernel to 1.18 ms for
+            // 6.5e6 candidates at the FP64 pipe's rate).  The FP32 values are within
+            // 1e-6; only pairs within 1e-5 of equality (the exact ties of a cell
+            // grid) need the reference's rounding.
+            const float fx = f32_bits(fabs(dx)), fy = f32_bits(fabs(dy)), fz = f32_bits(fabs(dz));
+            const float rf = sqrtf(fx * fx + fy * fy + fz * fz), sumf = f32_bits(ri) + f32_bits(rj);
+            const float lhs = rf * (float)theta;
+            const float hif = f32_bits(t.r[i]), hjf = f32_bits(t.r[j]);
+            const float gap = rf - 1.7320508f * (hif + hjf), rd = (float)rdamp;
+            const bool range = rf > 1e-15f && rf < 1e15f && sumf > 1e-15f;
+            const bool sure = range && fabsf(lhs - sumf) > 1e-5f * sumf && (rdamp <= 0.0 || fabsf(gap - rd) > 1e-5f * (rf + rd));
+            if (sure) {
+                accept = !mixed && lhs > sumf && (rdamp <= 0.0 || gap >= rd);
+            } else {
+                const double r = norm2_3(dx, dy, dz);
+                accept = !mixed && __dmul_rn(r, theta) > __dadd_rn(ri, rj);
+                if (accept && rdamp > 0.0) {
+                    // closest possible particle distance: centre distance minus the cube circumradii
+                    const double gap64 = __dsub_rn(r, __dmul_rn(1.7320508075688772, __dadd_rn(t.r[i], t.r[j])));
+                    accept = gap64 >= rdamp;
+                }
             }
         }
+        emit_pair(skip, accept, order, i, j, li, lj, mixed, ri, rj, t, out, cap_out, far, cap_far, nearp, cap_near,
+                  &front[1], counters, lane);
     }
-    emit_pair(skip, accept, order, i, j, li, lj, mixed, ri, rj, t, out, cap_out, far, cap_far, nearp, cap_near,
-              counters, lane);
 }
 
 // Learned acceptance (selector): a pair that passes the loose geometric test
@@ -542,7 +548,8 @@ __global__ void k_list_iter(const int2* __restrict__ in, int nin, int2* __restri
 // the near-field kernel (the difference of the damped and undamped
 // kernels), and listed in corrp.
 __global__ void __launch_bounds__(128) k_list_iter_learned(
-    const int2* __restrict__ in, int nin, int2* __restrict__ out, int64_t cap_out, uint64_t* __restrict__ far,
+    const int2* __restrict__ in, unsigned long long* front, int2* __restrict__ out, int64_t cap_out,
+    uint64_t* __restrict__ far,
     int64_t cap_far, uint64_t* __restrict__ nearp, int64_t cap_near, const TreeDev t, float theta_loose, float rdamp,
     int qmax, const float* __restrict__ params, const float* __restrict__ lnorm, const float* __restrict__ dmin,
     int P, const float* __restrict__ log_budget, const float4* __restrict__ chi, const float4* __restrict__ clo,
@@ -553,79 +560,83 @@ __global__ void __launch_bounds__(128) k_list_iter_learned(
     float* X = sm_sel + wib * kWarpTcFloats;  // this warp's network scratch
     float* Y = X + 32 * kMlpInP;
     const float* S = params + kMlpInfOff;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    bool skip = q >= nin;
-    int i = 0, j = 0;
-    float ri = 0.0f, rj = 0.0f;  // FP32 node data throughout: the FP64 pipe is the scarce one
-    bool li = false, lj = false, mixed = false, accept = false, corr = false, ingap = false;
-    float4 ci = make_float4(0.f, 0.f, 0.f, 0.f), cj = ci, oi = ci, oj = ci;
-    if (!skip) {
-        i = in[q].x;
-        j = in[q].y;
-        ci = chi[i];
-        cj = chi[j];
-        oi = clo[i];
-        oj = clo[j];
-        ri = ci.w;
-        rj = cj.w;
-        li = t.is_leaf[i] != 0;
-        lj = t.is_leaf[j] != 0;
-        // batched systems: no pairs across systems; nodes spanning several
-        // systems are always refined
-        if (t.sysid) {
-            const int si = t.sysid[i], sj = t.sysid[j];
-            if (si >= 0 && sj >= 0 && si != sj) skip = true;
-            mixed = si < 0 || sj < 0;
-        }
-        // loose geometric gate in FP32 (the network decides; no parity with
-        // the reference's rule is involved here)
-        const float dx = (ci.x - cj.x) + (oi.x - oj.x), dy = (ci.y - cj.y) + (oi.y - oj.y),
-                    dz = (ci.z - cj.z) + (oi.z - oj.z);
-        const float r = sqrtf(dx * dx + dy * dy + dz * dz);
-        accept = !skip && !mixed && r * theta_loose > ri + rj;
-        if (accept && rdamp > 0.0f) {
-            const float gap = r - 1.7320508f * (oi.w + oj.w);
-            if (gap < rdamp) {
-                if (corr_mode && li && lj) {
-                    // listed for the correction unless no particle pair of the
-                    // two leaves can have a r below the cutoff: a r >= dmin_i
-                    // dmin_j (r - extent_i - extent_j)
-                    ingap = true;
-                    const float2 ea = lext[i], eb = lext[j];
-                    const float xm = ea.y * eb.y * fmaxf(r - ea.x - eb.x - 1e-2f, 0.0f);
-                    corr = xm * xm < xcut2;
-                } else {
-                    accept = false;
+    const int64_t nin = __shfl_sync(0xffffffffu, counters[3] ? 0ll : (long long)front[0], 0);
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < nin; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t q = base + threadIdx.x;
+        bool skip = q >= nin;
+        int i = 0, j = 0;
+        float ri = 0.0f, rj = 0.0f;  // FP32 node data throughout: the FP64 pipe is the scarce one
+        bool li = false, lj = false, mixed = false, accept = false, corr = false, ingap = false;
+        float4 ci = make_float4(0.f, 0.f, 0.f, 0.f), cj = ci, oi = ci, oj = ci;
+        if (!skip) {
+            i = in[q].x;
+            j = in[q].y;
+            ci = chi[i];
+            cj = chi[j];
+            oi = clo[i];
+            oj = clo[j];
+            ri = ci.w;
+            rj = cj.w;
+            li = t.is_leaf[i] != 0;
+            lj = t.is_leaf[j] != 0;
+            // batched systems: no pairs across systems; nodes spanning several
+            // systems are always refined
+            if (t.sysid) {
+                const int si = t.sysid[i], sj = t.sysid[j];
+                if (si >= 0 && sj >= 0 && si != sj) skip = true;
+                mixed = si < 0 || sj < 0;
+            }
+            // loose geometric gate in FP32 (the network decides; no parity with
+            // the reference's rule is involved here)
+            const float dx = (ci.x - cj.x) + (oi.x - oj.x), dy = (ci.y - cj.y) + (oi.y - oj.y),
+                        dz = (ci.z - cj.z) + (oi.z - oj.z);
+            const float r = sqrtf(dx * dx + dy * dy + dz * dz);
+            accept = !skip && !mixed && r * theta_loose > ri + rj;
+            if (accept && rdamp > 0.0f) {
+                const float gap = r - 1.7320508f * (oi.w + oj.w);
+                if (gap < rdamp) {
+                    if (corr_mode && li && lj) {
+                        // listed for the correction unless no particle pair of the
+                        // two leaves can have a r below the cutoff: a r >= dmin_i
+                        // dmin_j (r - extent_i - extent_j)
+                        ingap = true;
+                        const float2 ea = lext[i], eb = lext[j];
+                        const float xm = ea.y * eb.y * fmaxf(r - ea.x - eb.x - 1e-2f, 0.0f);
+                        corr = xm * xm < xcut2;
+                    } else {
+                        accept = false;
+                    }
                 }
             }
         }
-    }
-    // the network runs once per warp on the pairs that passed the loose test
-    const unsigned need = __ballot_sync(0xffffffffu, accept);
-    if (need && lane == 0) atomicAdd(&counters[4], (unsigned long long)__popc(need));
-    int order = 0;
-    if (need) {
-        const int slot = __popc(need & ((1u << lane) - 1u));
-        if (accept) {
-            float x[kMlpIn];
-            selector_features_f32(chi, clo, t.count, lnorm, dmin, P, i, j, x);
-            if (ingap) x[16] = 1.0f;  // the M2L carries the undamped kernel; the damping is corrected pairwise
-            mlp_input(S, x, X + slot * kMlpInP);
+        // the network runs once per warp on the pairs that passed the loose test
+        const unsigned need = __ballot_sync(0xffffffffu, accept);
+        if (need && lane == 0) atomicAdd(&counters[4], (unsigned long long)__popc(need));
+        int order = 0;
+        if (need) {
+            const int slot = __popc(need & ((1u << lane) - 1u));
+            if (accept) {
+                float x[kMlpIn];
+                selector_features_f32(chi, clo, t.count, lnorm, dmin, P, i, j, x);
+                if (ingap) x[16] = 1.0f;  // the M2L carries the undamped kernel; the damping is corrected pairwise
+                mlp_input(S, x, X + slot * kMlpInP);
+            }
+            __syncwarp();
+            warp_mlp_tc(params, X, Y, __popc(need), lane);
+            if (accept) {
+                const float b = log_budget[i];  // the target node's budget
+                for (int o = kQmin; o <= qmax; ++o)
+                    if (Y[slot * kMlpOutP + (o - kQmin)] <= b) {
+                        order = o;
+                        break;
+                    }
+                accept = order > 0;
+            }
         }
-        __syncwarp();
-        warp_mlp_tc(params, X, Y, __popc(need), lane);
-        if (accept) {
-            const float b = log_budget[i];  // the target node's budget
-            for (int o = kQmin; o <= qmax; ++o)
-                if (Y[slot * kMlpOutP + (o - kQmin)] <= b) {
-                    order = o;
-                    break;
-                }
-            accept = order > 0;
-        }
+        emit_pair(skip, accept, order, i, j, li, lj, mixed, ri, rj, t, out, cap_out, far, cap_far, nearp, cap_near,
+                  &front[1], counters, lane, corr, corrp, cap_corr);
+        __syncwarp();  // the scratch is the next pairs'
     }
-    emit_pair(skip, accept, order, i, j, li, lj, mixed, ri, rj, t, out, cap_out, far, cap_far, nearp, cap_near,
-              counters, lane, corr, corrp, cap_corr);
 }
 
 __global__ void k_split_pairs(int64_t m, int sb, const uint64_t* __restrict__ sorted, int32_t* __restrict__ src,
@@ -958,6 +969,8 @@ int build_images(Workspace& ws, const TreeDev& t, const Box9& H, TreeDev* out, c
     return FMM_OK;
 }
 
+constexpr int kListSteps = 2 * kMaxDepth + 4, kListCounts = 8 + kListSteps + 1;
+
 int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st) {
     const int M = t.num_nodes;
     // capacities: pair counts grow like theta^-3; never below what the
@@ -972,6 +985,11 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
     const bool corr = tp.sel_params && tp.corr_mode && tp.mac_mode == 1 && tp.rdamp > 0.0 && tp.corr_ext;
     int64_t cap_corr = corr ? std::max<int64_t>({4096, cap_near, (int64_t)(ws.corr_pairs.cap / sizeof(uint64_t))}) : 0;
     unsigned long long* ctr = ws.counters.as<unsigned long long>();
+    FMM_TRY(ws.list_cnt.ensure(sizeof(unsigned long long) * kListCounts));
+    unsigned long long* lc = ws.list_cnt.as<unsigned long long>();
+    int sms = 0, dev = 0;
+    FMM_CUDA_TRY(cudaGetDevice(&dev));
+    FMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // Pair keys: target << (4 + sb) | order << sb | source (far), target << sb |
     // source (near), sb the bits of the largest source: only the bits that carry
     // something are sorted (a digit pass is 8 bits; 28,764 nodes: 5 passes over
@@ -992,42 +1010,52 @@ int build_lists(Workspace& ws, TreeDev& t, const TreeParams& tp, cudaStream_t st
         int2 root[27];
         for (int a = 0; a < t.nimg; ++a) root[a] = make_int2(0, a * M);
         FMM_CUDA_TRY(cudaMemcpyAsync(ws.front_a.p, root, sizeof(int2) * t.nimg, cudaMemcpyHostToDevice, st));
-        // frontier, far, near, overflow flag, network evaluations, correction pairs
-        unsigned long long h[6] = {0, 0, 0, 0, 0, 0};
-        FMM_CUDA_TRY(cudaMemcpyAsync(ctr, h, sizeof(h), cudaMemcpyHostToDevice, st));
-        int64_t nin = t.nimg;
-        int64_t candidates = 0;
+        // [1..5]: far, near, overflow flag, network evaluations, correction
+        // pairs; [8 ..]: the frontiers' sizes
+        unsigned long long h[kListCounts] = {};
+        h[8] = (unsigned long long)t.nimg;
+        FMM_CUDA_TRY(cudaMemcpyAsync(lc, h, sizeof(h), cudaMemcpyHostToDevice, st));
+        // Each step descends one side of every pair, and the deepest leaf's
+        // self pair is never accepted: 2 max_depth + 1 steps empty the frontier.
+        // They are launched without reading the sizes in between (15 us a step
+        // for the host's round trip); the kernels take them from the device.
         int2* fin = ws.front_a.as<int2>();
         int2* fout = ws.front_b.as<int2>();
-        bool overflow = false;
-        while (nin > 0) {
-            candidates += nin;
-            FMM_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st));
-            count_launches(1);
-            if (tp.sel_params) {
-                const size_t smem = sizeof(float) * 4 * (size_t)kWarpTcFloats;
-                FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_list_iter_learned,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                k_list_iter_learned<<<grid_for(nin, 128), 128, smem, st>>>(
-                    fin, (int)nin, fout, cap_front, ws.far_pairs.as<uint64_t>(), cap_far, ws.near_pairs.as<uint64_t>(),
-                    cap_near, t, (float)tp.sel_theta, tp.mac_mode == 1 ? (float)tp.rdamp : 0.0f, tp.order,
-                    tp.sel_params, tp.sel_lnorm, tp.sel_dmin, tp.sel_P, tp.sel_budget, tp.sel_chi, tp.sel_clo,
-                    ctr, corr ? 1 : 0, corr ? ws.corr_pairs.as<uint64_t>() : nullptr, cap_corr, tp.corr_ext,
-                    tp.corr_xcut2);
-            } else
-            k_list_iter<<<grid_for(nin, 256), 256, 0, st>>>(fin, (int)nin, fout, cap_front,
-                                                             ws.far_pairs.as<uint64_t>(), cap_far,
-                                                             ws.near_pairs.as<uint64_t>(), cap_near, t, tp.theta,
-                                                             tp.mac_mode == 1 ? tp.rdamp : 0.0, tp.order, ctr);
-            FMM_CUDA_TRY(cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, st));
-            FMM_CUDA_TRY(cudaStreamSynchronize(st));
-            if (h[3]) {
-                overflow = true;
-                break;
+        int steps = 0, want = std::min(2 * t.max_depth + 1, kListSteps);
+        int64_t bound = t.nimg;
+        do {
+            for (; steps < want; ++steps, std::swap(fin, fout)) {
+                unsigned long long* front = lc + 8 + steps;
+                count_launches(1);
+                if (tp.sel_params) {
+                    const size_t smem = sizeof(float) * 4 * (size_t)kWarpTcFloats;
+                    FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_list_iter_learned,
+                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    k_list_iter_learned<<<std::min<unsigned>(grid_for(bound, 128), 16 * sms), 128, smem, st>>>(
+                        fin, front, fout, cap_front, ws.far_pairs.as<uint64_t>(), cap_far,
+                        ws.near_pairs.as<uint64_t>(), cap_near, t, (float)tp.sel_theta,
+                        tp.mac_mode == 1 ? (float)tp.rdamp : 0.0f, tp.order, tp.sel_params, tp.sel_lnorm, tp.sel_dmin,
+                        tp.sel_P, tp.sel_budget, tp.sel_chi, tp.sel_clo, lc, corr ? 1 : 0,
+                        corr ? ws.corr_pairs.as<uint64_t>() : nullptr, cap_corr, tp.corr_ext, tp.corr_xcut2);
+                } else {
+                    k_list_iter<<<std::min<unsigned>(grid_for(bound, 256), 16 * sms), 256, 0, st>>>(
+                        fin, front, fout, cap_front, ws.far_pairs.as<uint64_t>(), cap_far,
+                        ws.near_pairs.as<uint64_t>(), cap_near, t, tp.theta, tp.mac_mode == 1 ? tp.rdamp : 0.0,
+                        tp.order, lc);
+                }
+                bound = std::min<int64_t>(8 * bound, cap_front);  // a pair has at most eight successors
             }
-            nin = (int64_t)h[0];
-            std::swap(fin, fout);
+            FMM_CUDA_TRY(cudaMemcpyAsync(h, lc, sizeof(h), cudaMemcpyDeviceToHost, st));
+            FMM_CUDA_TRY(cudaStreamSynchronize(st));
+            want = steps + 1;
+        } while (!h[3] && h[8 + steps] > 0 && want <= kListSteps);
+        if (!h[3] && h[8 + steps] > 0) return FMM_EINVAL;  // (deeper than any tree)
+        int64_t candidates = 0;
+        for (int k = 0; k <= steps; ++k) {
+            candidates += (int64_t)h[8 + k];
+            h[0] = std::max(h[0], h[8 + k]);
         }
+        const bool overflow = h[3] != 0;
         if (overflow) {
             if ((int64_t)h[0] > cap_front) cap_front = 2 * (int64_t)h[0];
             if ((int64_t)h[1] > cap_far) cap_far = 2 * (int64_t)h[1];
