@@ -154,11 +154,34 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
     vals[q] = (int32_t)q;
 }
 
+// A group's order: the highest of its pairs' orders (gq starts at zero).  Warp
+// per group and slice of its pairs (blockIdx.y), for large groups: the
+// displacements of the deepest level have as many pairs as there are leaves, and
+// a warp that reads them all keeps the tensors waiting (300,000 particles, 3,400
+// pairs a group: a call 8.23 -> 8.14 ms, with sliced row offsets).  With few
+// slices the extra launch costs more than it saves.
+__global__ void k_group_orders(int ng, const int32_t* __restrict__ gstart, const int32_t* __restrict__ svals,
+                               const TreeDev t, int p, int32_t* __restrict__ gq) {
+    const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (g >= ng) return;
+    int q = 0;
+    for (int k = gstart[g] + 32 * blockIdx.y + lane; k < gstart[g + 1]; k += 32 * gridDim.y)
+        q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
+    q = __reduce_max_sync(0xffffffffu, q);
+    if (lane == 0 && q > 0) atomicMax(&gq[g], q);
+}
+
+// Slices of the groups' pairs for the kernels with a warp per group: some eight
+// steps of a warp each at the mean.
+inline unsigned group_slices(int64_t nf, int ng) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(64, nf / ng / 256));
+}
+
 // One warp per group: restricted tensor T(D_c) of orders <= 2q in FP64 by the
 // Hermite recursion (two level buffers in shared memory), stored as R, with
-// the group's order and unit ratios a, b.  Mirrored groups: at the displacement
+// the group's unit ratios a, b.  Mirrored groups: at the displacement
 // of octant 0 (skeys: the pairs' keys in group order).
-template <typename R>
+template <typename R, bool HAVE_Q>
 __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, bool mirrored, const uint64_t* __restrict__ skeys,
                                                       const int32_t* __restrict__ gstart,
                                                       const int32_t* __restrict__ svals,
@@ -179,11 +202,14 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, bool mirrored
     const int oct = mirrored ? (int)(skeys[gstart[g]] & (kOctants - 1)) : 0;
     const int pos0 = svals[gstart[g]];
     const int i = tgt[pos0], j = t.far_src[pos0];
-    // the group's order: the highest of its pairs' orders
     int q = 0;
-    for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32)
-        q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
-    for (int off = 16; off > 0; off >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, off));
+    if (HAVE_Q) {  // (k_group_orders)
+        q = gq[g];
+    } else {
+        for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32)
+            q = max(q, t.far_ord ? min((int)t.far_ord[svals[k]], p) : p);
+        for (int off = 16; off > 0; off >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, off));
+    }
     const double hi = t.r[i], hj = t.r[j], hc = fmax(hi, hj);
     const double X = ((oct & 1) ? -1.0 : 1.0) * (t.cx[i] - t.cx[j]) / hc,
                  Y = ((oct & 2) ? -1.0 : 1.0) * (t.cy[i] - t.cy[j]) / hc,
@@ -227,7 +253,7 @@ __global__ void __launch_bounds__(128) k_group_tensor(int ngroups, bool mirrored
     R* out = gT + (size_t)g * ldT;
     for (int e = lane; e < rbase(Nq + 1); e += 32) out[e] = (R)A[e];
     if (lane == 0) {
-        gq[g] = q;
+        if (!HAVE_Q) gq[g] = q;
         gab[g] = make_float2((float)(hi / hc), (float)(hj / hc));
     }
 }
@@ -592,14 +618,16 @@ __global__ void k_row_sizes(int ng, bool full, const int32_t* __restrict__ gstar
 }
 
 // Row of every far pair, indexed in target order (svals maps group order to
-// target order), in units of kRowUnit entries.  Warp per group.
+// target order), in units of kRowUnit entries.  Warp per group and slice of its
+// pairs (blockIdx.y).
 __global__ void k_row_offsets(int ng, bool full, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
                               const int32_t* __restrict__ rowbase, const int32_t* __restrict__ svals,
                               int32_t* __restrict__ roff) {
     const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= ng) return;
     const int lane = threadIdx.x & 31, u = row_len(gq[g], full) / kRowUnit;
-    for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32) roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
+    for (int k = gstart[g] + 32 * blockIdx.y + lane; k < gstart[g + 1]; k += 32 * gridDim.y)
+        roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
 }
 
 // Source node of every far pair in group order; mirrored groups: 8 x node +
@@ -1095,6 +1123,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws.cub_tmp.p, tb4, ws.m2l_cnt.as<int32_t>(),
                                                    ws.m2l_gstart.as<int32_t>(), ng + 1, st));
         // per-group tensors
+        const unsigned slices = group_slices(nf, ng);
         FMM_TRY(ws.m2l_T.ensure(sizeof(R) * (size_t)ng * ldT));
         FMM_TRY(ws.m2l_gq.ensure(sizeof(int32_t) * ng));
         FMM_TRY(ws.m2l_gab.ensure(sizeof(float2) * ng));
@@ -1103,13 +1132,22 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         } else {
             const int wpb = 4;
             const size_t sm = sizeof(double) * (nTr + (size_t)wpb * (2 * nTr + N + 1));
+            const bool have_q = slices > 4;
+            auto kernel = have_q ? k_group_tensor<R, true> : k_group_tensor<R, false>;
             if (sm > 48 * 1024)
-                FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_group_tensor<R>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                FMM_CUDA_TRY(
+                    cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            if (have_q) {
+                count_launches(1);
+                FMM_CUDA_TRY(cudaMemsetAsync(ws.m2l_gq.p, 0, sizeof(int32_t) * ng, st));
+                k_group_orders<<<dim3(grid_for(ng, 8), slices), 256, 0, st>>>(
+                    ng, ws.m2l_gstart.as<int32_t>(), ws.m2l_vals2.as<int32_t>(), t, p, ws.m2l_gq.as<int32_t>());
+            }
             count_launches(1);
-            k_group_tensor<R><<<grid_for(ng, wpb), 32 * wpb, sm, st>>>(
+            kernel<<<grid_for(ng, wpb), 32 * wpb, sm, st>>>(
                 ng, ws.m2l_mirrored, ws.m2l_keys2.as<uint64_t>(), ws.m2l_gstart.as<int32_t>(),
-                ws.m2l_vals2.as<int32_t>(), tgt, t, p, ldT, ws.m2l_T.as<R>(), ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>());
+                ws.m2l_vals2.as<int32_t>(), tgt, t, p, ldT, ws.m2l_T.as<R>(), ws.m2l_gq.as<int32_t>(),
+                ws.m2l_gab.as<float2>());
         }
         // tasks: up to kTaskCols pairs of one group each (tensor cores: 256
         // pairs and one operator half)
@@ -1136,9 +1174,9 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         FMM_TRY(ws.cub_tmp.ensure(tb7));
         FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws.cub_tmp.p, tb7, rowbase, rowbase, ng + 1, st));
         count_launches(1);
-        k_row_offsets<<<grid_for(ng, 8), 256, 0, st>>>(ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
-                                                        rowbase, ws.m2l_vals2.as<int32_t>(),
-                                                        reinterpret_cast<int32_t*>(ws.m2l_keys.p));
+        k_row_offsets<<<dim3(grid_for(ng, 8), slices), 256, 0, st>>>(
+            ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(), rowbase, ws.m2l_vals2.as<int32_t>(),
+            reinterpret_cast<int32_t*>(ws.m2l_keys.p));
         int hcnt[2] = {0, 0};  // tasks, rows (units of 32 entries)
         FMM_CUDA_TRY(cudaMemcpyAsync(&hcnt[0], ws.m2l_toff.as<int32_t>() + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
         FMM_CUDA_TRY(cudaMemcpyAsync(&hcnt[1], rowbase + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
