@@ -417,7 +417,7 @@ int run_fmm(Workspace& ws, const Particles& P, double theta, int ncrit, int p, i
         // demote them)
         const char* ce = std::getenv("FMM_GB300_DAMP_CORR");
         if (learned && (md.precision == 1 || md.precision == 2) && tpl.rdamp > 0.0 && P.damp_type == DAMP_AMOEBA &&
-            p2p_packed_enabled(ws.p2p_shape.valid() ? ws.p2p_shape : P2pShape{}, f, P.damp_type) && !(ce && ce[0] == '0')) {
+            p2p_packed_enabled(ws.p2p_shape.valid() ? ws.p2p_shape : P2pShape{}, f) && !(ce && ce[0] == '0')) {
             tpl.corr_mode = 1;
             // AMOEBA depends on a r only: the range at a = 1 is the cutoff of a r
             const double xc = damping_range(P.damp_type, 1.0, dim_to_order(P.dim) + f, 0.1 * o.target);

@@ -137,9 +137,9 @@ struct P2pShape {
     int pack = 1;  // sources two at a time in packed FP32 (Blackwell f32x2 instructions)
     bool valid() const;
 };
-// Whether the FP32 near field runs the packed kernel for this shape, field
-// order and damping kind.
-bool p2p_packed_enabled(const P2pShape& sh, int field_order, int damp);
+// Whether the FP32 near field runs the packed kernel for this shape and field
+// order.
+bool p2p_packed_enabled(const P2pShape& sh, int field_order);
 
 struct Workspace {
     // inputs on device (host entry points copy here)

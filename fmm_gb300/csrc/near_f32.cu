@@ -14,7 +14,7 @@
 // which a warp walks as one: lane groups are filled across leaf boundaries
 // (leaves of about a dozen particles leave 40% of them idle otherwise).
 //
-// The packed kernel (field orders 0 and 1, all kernels but erf) evaluates
+// The packed kernel (field orders 0 and 1) evaluates
 // each target against two sources at once in f32x2 arithmetic from a second
 // record array with even leaf starts and interleaved slot pairs, and, with
 // learned lists on AMOEBA, a second launch walks a damping-correction list:
@@ -884,7 +884,7 @@ int launch_leaf_field_scale(Workspace& ws, const Particles& P, const TreeDev& t,
     return FMM_OK;
 }
 
-bool p2p_packed_enabled(const P2pShape& sh, int field_order, int damp) {
+bool p2p_packed_enabled(const P2pShape& sh, int field_order) {
     const char* pe = std::getenv("FMM_GB300_P2P_PACKED");
     return sh.pack && !(pe && pe[0] == '0') && field_order <= 1;
 }
@@ -905,10 +905,8 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     if (rec_vec(P.dim) > sh.stage) return FMM_EINVAL;
     // packed kernel: sources two at a time from the padded, interleaved
     // records, for field orders 0 and 1 (at order 2 the packed registers do
-    // not fit) and all kernels but erf (whose Boys series, at a r^2 < 6 for
-    // much of an erf near field, runs per half: measured slower than the
-    // one-source kernel); FMM_GB300_P2P_PACKED=0 selects the one-source kernel
-    const bool x2 = p2p_packed_enabled(sh, field_order, P.damp_type) && t.num_leaves > 0 &&
+    // not fit); FMM_GB300_P2P_PACKED=0 selects the one-source kernel
+    const bool x2 = p2p_packed_enabled(sh, field_order) && t.num_leaves > 0 &&
                     n + (int64_t)t.num_leaves < (int64_t)INT32_MAX;
     // a damping-correction list is walked by the packed kernel only; the
     // pairs it corrects are counted in counter 9
