@@ -92,8 +92,9 @@ __global__ void k_gather_f32(int64_t n, int dim, bool leaf, const TreeDev t, con
 
 // Source records of the packed near field: the sorted particles of each leaf
 // from an even slot ps[leaf] on, an odd leaf padded by one empty particle
-// (zero multipoles, at least 1000 bohr from its leaf's last particle, damping
-// factor 1: its pair terms are exactly zero); slots 2b and 2b + 1 form block b, stored
+// (zero multipoles, damping factor 1, outside the root cell by its width and
+// 1000 bohr: no target is there, whose field would be 0 x infinity, and the pair
+// terms are exactly zero); slots 2b and 2b + 1 form block b, stored
 // element by element interleaved (float 2e + h of the block is element e of
 // the record of slot 2b + h), so one 16-byte shared-memory load gives two
 // elements of both particles as two packed pairs.
@@ -118,9 +119,9 @@ __global__ void k_gather_x2(int64_t n, int nv, bool q1, const TreeDev t, const i
     if (within == cnt - 1 && (cnt & 1)) {
         float* dd = d + 1;  // slot + 1: the odd half of the same block
         for (int e = 0; e < 4 * nv; ++e) dd[2 * e] = 0.0f;
-        dd[0] = s[0] + fmaxf(1000.0f, fabsf(s[0]));  // x
-        dd[2] = s[1];
-        dd[4] = s[2];
+        // positions are relative to the root's or a leaf's centre, so a target is
+        // within 2 root_r of the origin along each axis
+        dd[0] = 4.0f * (float)t.root_r + 1000.0f;  // x
         dd[2 * 3] = 1.0f; // damping factor
     }
 }
