@@ -54,28 +54,49 @@ __global__ void k_centroid_lanes(const double* __restrict__ X, int64_t n, double
 
 // Sequential sums in parallel, rounding for rounding.  While a running sum s =
 // k 2^(e - 52), 2^52 <= |k| < 2^53, keeps its binade, adding x moves k by x
-// 2^(52 - e) rounded to the nearest integer, whatever k is, unless that is a
-// tie (which goes to the even sum).  So a block takes a tile of terms' integer
-// steps, scans them, accepts the terms before the first one that ties or leaves
-// the binade, adds that one in FP64 and goes on behind it.  Binade changes and
-// ties are few: a tile of 4,096 terms takes 1 us, where the chain of FP64
-// additions takes 38 ns a term: 7.6 -> 0.2 ms for 200,000 particles.
-struct SeqTerm {
-    long long k;  // integer step
-    bool bad;     // tie, or larger than the sum's binade
+// 2^(52 - e) rounded to the nearest integer, whatever k is; a tie goes to the
+// even sum, so its step depends on whether k is even.  A term is therefore a
+// pair of steps, and pairs compose: a block takes a tile of terms, scans their
+// pairs and accepts the terms before the first one that leaves the binade.  That
+// one is added in FP64.  Where few terms pass (sums around zero change binade
+// some thousand times in 200,000 terms), the tile is taken in units of its
+// terms' last bit, if its sums have no more than 53 bits of them (lattices,
+// coordinates of a file's digits in FP32): then nothing rounds.  Otherwise a warp
+// goes on in windows of 128 terms (seq_tail).
+// Trees of 200,000 particles, FP64 additions one by one / this: in a box from
+// zero on 7.4 / 0.7 ms, uniform or normal around zero 7.4 / 3.8 to 5.5, a lattice
+// around zero 7.4 / 0.8.
+struct SeqSteps {
+    unsigned long long a0, a1;  // integer steps of an even and an odd sum
 };
-// Step of the term with bits b at a sum of biased exponent es (0: the sum is
+// b after a.
+__host__ __device__ __forceinline__ SeqSteps seq_then(const SeqSteps& a, const SeqSteps& b) {
+    return {a.a0 + (a.a0 & 1 ? b.a1 : b.a0), a.a1 + (a.a1 & 1 ? b.a0 : b.a1)};
+}
+__host__ __device__ __forceinline__ long long seq_apply(long long k, const SeqSteps& a) {
+    return (long long)((unsigned long long)k + (k & 1 ? a.a1 : a.a0));
+}
+struct SeqTerm {
+    SeqSteps k;
+    bool bad;  // larger than the sum's binade
+};
+// Steps of the term with bits b at a sum of biased exponent es (0: the sum is
 // zero, which zeros leave).
 __host__ __device__ __forceinline__ SeqTerm seq_term(long long b, int es) {
-    if (es == 0) return {0, (b << 1) != 0};
+    if (es == 0) return {{0, 0}, (b << 1) != 0};
     const int ex = (int)(b >> 52) & 0x7ff;
     const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
     const int sh = es - (ex ? ex : 1);
-    if (sh < 0) return {0, true};
-    if (sh > 54) return {0, false};  // less than a quarter
+    if (sh < 0) return {{0, 0}, true};
+    if (sh > 54) return {{0, 0}, false};  // less than a quarter
     const long long half = sh ? 1ll << (sh - 1) : 0, rem = m & ((1ll << sh) - 1);
-    const long long k = (m >> sh) + (sh && rem > half ? 1 : 0);
-    return {b < 0 ? -k : k, sh && rem == half};
+    if (sh && rem == half) {
+        const long long f = b < 0 ? -(m >> sh) - 1 : m >> sh;  // the lower neighbour's step
+        return {{(unsigned long long)(f + (f & 1)), (unsigned long long)(f + 1 - (f & 1))}, false};
+    }
+    long long k = (m >> sh) + (sh && rem > half ? 1 : 0);
+    if (b < 0) k = -k;
+    return {{(unsigned long long)k, (unsigned long long)k}, false};
 }
 // Whether the sum k is inside its binade, clear of the ends.
 __host__ __device__ __forceinline__ bool seq_inside(long long k) {
@@ -91,83 +112,221 @@ __host__ __device__ __forceinline__ long long seq_bits(long long k, int es) {
     return ((k < 0 ? -k : k) & 0xfffffffffffffll) | ((long long)es << 52) | (k < 0 ? (long long)(1ull << 63) : 0ll);
 }
 
-// Terms added one by one at a time at most, where sums change binade all the
-// time (terms of both signs): there the parallel attempts cost a tenth more
-// than the chain alone; a longer limit costs more at the start of a sum.
-constexpr int kSeqThreads = 1024, kSeqPer = 4, kSeqSerial = 128;
+constexpr int kSeqThreads = 1024, kSeqPer = 4, kSeqTile = kSeqThreads * kSeqPer;
+// Terms that a tile must pass to be worth its time and barriers, and a window
+// (1.1 us, that of as many FP64 additions); the most terms added one by one
+// before the next window.
+constexpr int kSeqWorthTile = 512, kSeqWorth = 28, kSeqSerial = 1024;
+
+// Composition of the lanes' steps up to and including this lane's.
+__device__ __forceinline__ SeqSteps seq_scan(SeqSteps inc, int lane) {
+    if (__all_sync(0xffffffffu, inc.a0 == inc.a1)) {  // no tie: sums
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, inc.a0, o);
+            if (lane >= o) inc.a0 += u;
+        }
+        return {inc.a0, inc.a0};
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const SeqSteps u{__shfl_up_sync(0xffffffffu, inc.a0, o), __shfl_up_sync(0xffffffffu, inc.a1, o)};
+        if (lane >= o) inc = seq_then(u, inc);
+    }
+    return inc;
+}
+// The previous lane's (none: no step).
+__device__ __forceinline__ SeqSteps seq_before(const SeqSteps& inc, int lane) {
+    const SeqSteps u{__shfl_up_sync(0xffffffffu, inc.a0, 1), __shfl_up_sync(0xffffffffu, inc.a1, 1)};
+    return lane ? u : SeqSteps{0, 0};
+}
+
+// s + tile[i] + .. + tile[cnt - 1], in order; by a warp (every lane gets the
+// sum).  Where windows pass few terms, the terms are added one by one, in
+// stretches that grow.
+__device__ double seq_tail(const double* tile, int i, int cnt, double s, int& stretch, int lane) {
+    while (i < cnt) {
+        const long long sb = __double_as_longlong(s);
+        const int es = (int)(sb >> 52) & 0x7ff;
+        int ok = 0;  // accepted terms
+        if (s == 0.0 || (es != 0 && es != 0x7ff)) {
+            SeqSteps k[kSeqPer];
+            int f = kSeqPer;  // first of the lane's terms that does not pass
+#pragma unroll
+            for (int j = 0; j < kSeqPer; ++j) {
+                const int e = i + kSeqPer * lane + j;
+                const SeqTerm t = e < cnt ? seq_term(__double_as_longlong(tile[e]), es) : SeqTerm{{0, 0}, true};
+                // (steps wrap beyond the first term that does not pass: not used)
+                k[j] = j ? seq_then(k[j ? j - 1 : 0], t.k) : t.k;
+                if (t.bad) f = min(f, j);
+            }
+            const long long base = seq_apply(seq_mantissa(sb), seq_before(seq_scan(k[kSeqPer - 1], lane), lane));
+            long long sum[kSeqPer];
+#pragma unroll
+            for (int j = 0; j < kSeqPer; ++j) {
+                sum[j] = seq_apply(base, k[j]);
+                if (es != 0 && !seq_inside(sum[j])) f = min(f, j);
+            }
+            const unsigned stop = __ballot_sync(0xffffffffu, f < kSeqPer);
+            const int first = stop ? __ffs(stop) - 1 : 31;
+            ok = kSeqPer * first + __shfl_sync(0xffffffffu, f, first);
+            long long last = 0;
+#pragma unroll
+            for (int j = 0; j < kSeqPer; ++j)
+                if (j == ((ok - 1) & (kSeqPer - 1))) last = sum[j];
+            last = __shfl_sync(0xffffffffu, last, ok > 0 ? (ok - 1) / kSeqPer : 0);
+            if (ok > 0) s = es ? __longlong_as_double(seq_bits(last, es)) : 0.0;
+            i += ok;
+        }
+        stretch = ok < kSeqWorth ? min(max(16, 2 * stretch), kSeqSerial) : 0;
+        const int end = min(cnt, i + (ok < 32 * kSeqPer ? 1 : 0) + stretch);
+        if (lane == 0) {
+#pragma unroll 4
+            for (int e = i; e < end; ++e) s = __dadd_rn(s, tile[e]);
+        }
+        i = end;
+        s = __shfl_sync(0xffffffffu, s, 0);
+    }
+    return s;
+}
+
+struct SeqShared {
+    double tile[kSeqTile];
+    SeqSteps steps[kSeqThreads / 32];
+    long long last;
+    double s;
+    int first, unit[kSeqThreads / 32];
+};
+
+// The tile's sums from k0 on, by a block (k: the thread's terms; bad: a bit for
+// each that does not pass whatever the sum).  Returns the number of terms before
+// the first one that does not pass or whose sum is not inside(); *last: the sum
+// after them.
+template <typename Inside>
+__device__ int seq_block(SeqSteps (&k)[kSeqPer], unsigned bad, long long k0, int cnt, SeqShared& sh,
+                         const Inside& inside, long long* last) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // (steps wrap beyond the first term that does not pass: not used)
+#pragma unroll
+    for (int j = 1; j < kSeqPer; ++j) k[j] = seq_then(k[j - 1], k[j]);
+    const SeqSteps inc = seq_scan(k[kSeqPer - 1], lane);
+    if (lane == 31) sh.steps[warp] = inc;
+    if (tid == 0) sh.first = cnt;
+    __syncthreads();
+    const SeqSteps w = seq_scan(sh.steps[lane], lane);
+    const int pw = warp ? warp - 1 : 0;
+    SeqSteps before{__shfl_sync(0xffffffffu, w.a0, pw), __shfl_sync(0xffffffffu, w.a1, pw)};
+    if (warp == 0) before = {0, 0};
+    const long long base = seq_apply(seq_apply(k0, before), seq_before(inc, lane));
+    int f = kSeqTile;
+    long long sum[kSeqPer];
+#pragma unroll
+    for (int j = kSeqPer - 1; j >= 0; --j) {
+        sum[j] = seq_apply(base, k[j]);
+        if ((bad >> j & 1) || !inside(sum[j])) f = kSeqPer * tid + j;
+    }
+    if (f < cnt) atomicMin(&sh.first, f);
+    __syncthreads();
+    const int ok = sh.first;
+#pragma unroll
+    for (int j = 0; j < kSeqPer; ++j)
+        if (kSeqPer * tid + j == ok - 1) sh.last = sum[j];
+    __syncthreads();
+    *last = sh.last;
+    return ok;
+}
+
+constexpr long long kSeqOver = 0x7fffffffffffffffll;
+
+// Exponent of the last set bit of a number (biased as its exponent is, less
+// 52), -1 for infinities and NaN, a large one for zero.
+__device__ __forceinline__ int seq_unit(long long b) {
+    const int ex = (int)(b >> 52) & 0x7ff;
+    const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
+    return ex == 0x7ff ? -1 : (m ? max(ex, 1) + __ffsll(m) - 1 : 1 << 20);
+}
+// The number in units of that bit of weight u; 2^53 or more: kSeqOver.
+__device__ __forceinline__ long long seq_units(long long b, int u) {
+    const int ex = (int)(b >> 52) & 0x7ff;
+    const long long m = (b & 0xfffffffffffffll) | (ex ? 0x10000000000000ll : 0ll);
+    const int sh = max(ex, 1) - u;
+    if (m == 0) return 0;
+    if (sh > 0 && (sh >= 53 || (m >> (53 - sh)) != 0)) return kSeqOver;
+    const long long k = sh > 0 ? m << sh : m >> -sh;
+    return b < 0 ? -k : k;
+}
 
 // The sum of v[0..n), as one thread adding in order would get it; by a block.
 __device__ double seq_sum(const double* __restrict__ v, int64_t n) {
-    constexpr int kTile = kSeqThreads * kSeqPer;
-    __shared__ long long wsum[kSeqThreads / 32];
-    __shared__ double sh_s;
-    __shared__ int first;
+    __shared__ SeqShared sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double s = 0.0;
-    int serial = 1;  // terms added one by one where the tile's first terms do not pass
+    int tail = kSeqWorthTile, stretch = 0;  // terms given to the windows, to the chain
     for (int64_t pos = 0; pos < n;) {
         const long long sb = __double_as_longlong(s);
         const int es = (int)(sb >> 52) & 0x7ff;
-        const int cnt = (int)min((int64_t)kTile, n - pos);
+        const int cnt = (int)min((int64_t)kSeqTile, n - pos);
+        long long x[kSeqPer], last;
+#pragma unroll
+        for (int j = 0; j < kSeqPer; ++j) {
+            const int i = kSeqPer * tid + j;
+            x[j] = i < cnt ? __double_as_longlong(v[pos + i]) : 0;
+        }
         int ok = 0;  // accepted terms
+        SeqSteps k[kSeqPer];
         if (s == 0.0 || (es != 0 && es != 0x7ff)) {
-            long long k[kSeqPer];
-            bool bad[kSeqPer];
-            long long sum = 0;
+            unsigned bad = 0;
 #pragma unroll
             for (int j = 0; j < kSeqPer; ++j) {
-                const int i = kSeqPer * tid + j;
-                const SeqTerm t = i < cnt ? seq_term(__double_as_longlong(v[pos + i]), es) : SeqTerm{0, true};
-                // (sums wrap beyond the first term that does not pass: not used)
-                sum = (long long)((unsigned long long)sum + (unsigned long long)t.k);
-                k[j] = sum;
-                bad[j] = t.bad;
+                const SeqTerm t = seq_term(x[j], es);
+                k[j] = t.k;
+                bad |= (unsigned)t.bad << j;
             }
-            unsigned long long inc = (unsigned long long)sum;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long u = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += u;
-            }
-            if (lane == 31) wsum[warp] = (long long)inc;
-            if (tid == 0) first = cnt;
-            __syncthreads();
-            unsigned long long w = lane < warp ? (unsigned long long)wsum[lane] : 0ull;
-            for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-            const unsigned long long base = (unsigned long long)seq_mantissa(sb) + w + (inc - (unsigned long long)sum);
-            int f = kTile;
-#pragma unroll
-            for (int j = kSeqPer - 1; j >= 0; --j) {
-                k[j] = (long long)(base + (unsigned long long)k[j]);
-                if (bad[j] || (es != 0 && !seq_inside(k[j]))) f = kSeqPer * tid + j;
-            }
-            if (f < cnt) atomicMin(&first, f);
-            __syncthreads();
-            ok = first;
-#pragma unroll
-            for (int j = 0; j < kSeqPer; ++j)
-                if (kSeqPer * tid + j == ok - 1) sh_s = es ? __longlong_as_double(seq_bits(k[j], es)) : 0.0;
-            if (ok > 0) {
-                __syncthreads();
-                s = sh_s;
-            }
-        } else {
-            serial = max(serial, 8);
+            ok = seq_block(k, bad, seq_mantissa(sb), cnt, sh, [&](long long m) { return es == 0 || seq_inside(m); },
+                           &last);
+            if (ok > 0 && es != 0) s = __longlong_as_double(seq_bits(last, es));
         }
-        pos += ok;
+        if (ok < kSeqWorthTile && ok < cnt) {
+            int u = seq_unit(sb);
+#pragma unroll
+            for (int j = 0; j < kSeqPer; ++j) u = min(u, seq_unit(x[j]));
+            u = __reduce_min_sync(0xffffffffu, u);
+            if (lane == 0) sh.unit[warp] = u;
+            __syncthreads();
+            u = __reduce_min_sync(0xffffffffu, sh.unit[lane]);
+            if (u >= 0) {
+                unsigned bad = 0;
+#pragma unroll
+                for (int j = 0; j < kSeqPer; ++j) {
+                    const long long m = seq_units(x[j], u);
+                    k[j] = {(unsigned long long)m, (unsigned long long)m};
+                    bad |= (unsigned)(m == kSeqOver) << j;
+                }
+                const long long k0 = seq_units(sb, u);
+                const int oke = seq_block(
+                    k, bad, k0, cnt, sh,
+                    [&](long long m) { return k0 != kSeqOver && m >= -(1ll << 53) && m <= (1ll << 53); }, &last);
+                if (oke > ok) {
+                    ok = oke;
+                    s = scalbn((double)last, u - 1075);
+                }
+            }
+        }
+        int done = ok;
         if (ok < cnt) {
-            // one by one: the term that did not pass, and twice as many as the
-            // last time where few terms passed since
-            serial = ok < serial ? min(2 * serial, kSeqSerial) : 1;
-            if (tid == 0) {
-                const int m = (int)min((int64_t)serial, n - pos);
-#pragma unroll 4
-                for (int i = 0; i < m; ++i) s = __dadd_rn(s, v[pos + i]);
-                sh_s = s;
+            tail = ok < kSeqWorthTile ? min(2 * tail, kSeqTile) : kSeqWorthTile;
+            done = ok < kSeqWorthTile ? min(cnt, ok + tail) : ok + 1;
+#pragma unroll
+            for (int j = 0; j < kSeqPer; ++j) sh.tile[kSeqPer * tid + j] = __longlong_as_double(x[j]);
+            __syncthreads();
+            if (warp == 0) {
+                s = ok < kSeqWorthTile ? seq_tail(sh.tile, ok, done, s, stretch, lane) : __dadd_rn(s, sh.tile[ok]);
+                if (lane == 0) sh.s = s;
             }
             __syncthreads();
-            s = sh_s;
-            pos += min((int64_t)serial, n - pos);
+            s = sh.s;
         }
+        pos += done;
         __syncthreads();
     }
     return s;
