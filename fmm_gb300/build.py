@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libfmm_gb300.so")
 SOURCES = ["api.cu", "tree.cu", "near.cu", "near_f32.cu", "expansions.cu", "translate.cu", "m2l.cu", "m2l_gemm.cu", "diag.cu", "noalloc.cu", "selector.cu", "qmmm.cu"]
-HEADERS = ["common.cuh", "m2l_basis.cuh", "pair.cuh", "pair_f64.cuh", "dispatch.cuh", "mlp.cuh", "m2l_tc64.cuh", "umma.cuh", "pair_x2.cuh", "internal.h", "series_tables.h", os.path.join("..", "..", "include", "fmm_gpu.h")]
+HEADERS = ["common.cuh", "m2l_basis.cuh", "pair.cuh", "pair_f64.cuh", "dispatch.cuh", "mlp.cuh", "m2l_tc64.cuh", "m2l_size.h", "umma.cuh", "pair_x2.cuh", "internal.h", "series_tables.h", os.path.join("..", "..", "include", "fmm_gpu.h")]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",

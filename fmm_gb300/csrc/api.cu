@@ -38,6 +38,13 @@ void DevBuf::release() {
     cap = 0;
 }
 
+void Workspace::release_grouped() {
+    for (DevBuf* b : {&m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
+                      &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit,
+                      &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp})
+        b->release();
+}
+
 void Workspace::release_buffers(bool keep_selector) {
     DevBuf* all[] = {&in_coords, &in_mp,     &in_excl,     &in_damp,    &out_field,  &keys_a,     &keys_b,
                      &vals_a,    &vals_b,    &cub_tmp,     &perm,       &pos_of,     &leaf_of,    &node_d,

@@ -348,11 +348,10 @@ static int launch_m2l_pairwise(Workspace& ws, const TreeDev& t, int p, const Mod
 int launch_m2l(Workspace& ws, const TreeDev& t, int p, const Modes& md, cudaStream_t st) {
     int rc;
     if (md.coef_mode != 0 || 2 * p <= kExactRefOrder) {
-        rc = launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, st);
+        rc = launch_m2l_reduced(ws, t, p, md.precision == 1 || md.precision == 3, md.coef_mode == 0 || t.nimg > 1, st);
     } else {
         FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)t.num_nodes * nT(p)));
-        rc = (ws.reuse_structure && ws.m2l_pairwise) ? FMM_ENOTSUP
-                                                     : launch_m2l_grouped(ws, t, p, false, st, true);
+        rc = launch_m2l_grouped(ws, t, p, false, st, true, true);
     }
     return rc == FMM_ENOTSUP ? launch_m2l_pairwise(ws, t, p, md, st) : rc;
 }

@@ -221,6 +221,7 @@ struct Workspace {
     // Frees every device buffer (keep_selector: except the loaded selector
     // network) and forgets the tables cached in them.
     void release_buffers(bool keep_selector);
+    void release_grouped();  // the grouped M2L's
 };
 
 Workspace& thread_workspace();
@@ -278,8 +279,8 @@ int launch_group_tensor_ref(Workspace& ws, const TreeDev& t, int ng, const int32
 // *d_levels receives the number of lattice levels used.
 int launch_periodic_lattice(Workspace& ws, const TreeDev& t, int p, int f, const Modes& md, const Box9& H,
                             double* d_fs, int* d_levels, cudaStream_t st);
-int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st);
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full = false);
+int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, bool bounded, cudaStream_t st);
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full, bool bounded);
 int launch_reduce_moments(Workspace& ws, const TreeDev& t, int p, cudaStream_t st);
 // selector.cu
 int selector_node_norms(Workspace& ws, const TreeDev& t, int P, const double* d_sorted_damp, cudaStream_t st);

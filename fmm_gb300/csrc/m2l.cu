@@ -304,16 +304,13 @@ int launch_reduce_moments(Workspace& ws, const TreeDev& t, int p, cudaStream_t s
 }
 
 // Exact-tensor M2L: reduced moments, reduced M2L (FP32 or FP64), completion of
-// the local expansions.  Where the pairs go one by one and the sources are
+// the local expansions.  bounded: see launch_m2l_grouped.  Where the pairs go one by one and the sources are
 // periodic images, returns FMM_ENOTSUP: the general per-pair kernel takes those.
-int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st) {
+int launch_m2l_reduced(Workspace& ws, const TreeDev& t, int p, bool fp32, bool bounded, cudaStream_t st) {
     const int M = t.num_nodes, nq = nT(p);
     FMM_TRY(ws.loc.ensure(sizeof(double) * (size_t)M * nq));
     if (ws.wred_p != p) FMM_TRY(launch_reduce_moments(ws, t, p, st));  // not yet reduced from this call's moments
-    // (replays keep the choice between grouped products and the per-pair
-    // kernel made when the structure was built)
-    const int gst = (ws.reuse_structure && ws.m2l_pairwise) ? FMM_ENOTSUP
-                                                            : launch_m2l_grouped(ws, t, p, fp32, st);
+    const int gst = launch_m2l_grouped(ws, t, p, fp32, st, false, bounded);
     if (gst == FMM_ENOTSUP) {
         if (t.nimg > 1) return FMM_ENOTSUP;
         // per-pair kernel (FP64 operator too large for shared memory, or

@@ -39,6 +39,7 @@
 
 #include "internal.h"
 #include "m2l_basis.cuh"
+#include "m2l_size.h"
 #include "m2l_tc64.cuh"
 #include "umma.cuh"
 
@@ -467,9 +468,7 @@ __device__ __forceinline__ void gemm_task(const GemmSmem<R, CPT>& L, char* sm, i
 }
 
 // Result rows: group g's rows start at rowbase[g] x kRowUnit entries, one
-// row of (q+1)^2 rounded up to kRowUnit entries (32 bytes in FP32, one DRAM
-// sector) per pair in group order.
-constexpr int kRowUnit = 8;
+// row of (q+1)^2 rounded up to kRowUnit entries per pair in group order.
 __host__ __device__ __forceinline__ int row_len(int q, bool full = false) {
     return (d64_rows(q, full) + kRowUnit - 1) / kRowUnit * kRowUnit;
 }
@@ -484,7 +483,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_m2l_gemm(const int2* __restric
                                                            const float2* __restrict__ gab, const R* __restrict__ gT,
                                                            int ldT, const int32_t* __restrict__ psrc,
                                                            const R* __restrict__ wsc, R* __restrict__ out,
-                                                           const int32_t* __restrict__ rowbase) {
+                                                           const int64_t* __restrict__ rowbase) {
     extern __shared__ __align__(16) char sm_gemm[];
     const GemmSmem<R, CPT> L(p);
     const int nr = (p + 1) * (p + 1);
@@ -619,23 +618,23 @@ __global__ void k_split_weights(int64_t total, int octants, int nr, int ldw, int
 
 // Rows of each group in units of kRowUnit entries (scanned into rowbase).
 __global__ void k_row_sizes(int ng, bool full, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
-                            int32_t* __restrict__ rsz) {
+                            int64_t* __restrict__ rsz) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g > ng) return;
-    rsz[g] = g < ng ? (gstart[g + 1] - gstart[g]) * (row_len(gq[g], full) / kRowUnit) : 0;
+    rsz[g] = g < ng ? (int64_t)(gstart[g + 1] - gstart[g]) * (row_len(gq[g], full) / kRowUnit) : 0;
 }
 
 // Row of every far pair, indexed in target order (svals maps group order to
 // target order), in units of kRowUnit entries.  Warp per group and slice of its
 // pairs (blockIdx.y).
 __global__ void k_row_offsets(int ng, bool full, const int32_t* __restrict__ gstart, const int32_t* __restrict__ gq,
-                              const int32_t* __restrict__ rowbase, const int32_t* __restrict__ svals,
+                              const int64_t* __restrict__ rowbase, const int32_t* __restrict__ svals,
                               int32_t* __restrict__ roff) {
     const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= ng) return;
     const int lane = threadIdx.x & 31, u = row_len(gq[g], full) / kRowUnit;
     for (int k = gstart[g] + 32 * blockIdx.y + lane; k < gstart[g + 1]; k += 32 * gridDim.y)
-        roff[svals[k]] = rowbase[g] + (k - gstart[g]) * u;
+        roff[svals[k]] = (int32_t)(rowbase[g] + (int64_t)(k - gstart[g]) * u);  // (m2l_rows_fit)
 }
 
 // Source node of every far pair in group order; mirrored groups: 8 x node +
@@ -744,7 +743,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_m2l_tc(const int2* __restrict
                                                          const int32_t* __restrict__ psrc,
                                                          const float* __restrict__ wsp, int ldk,
                                                          float* __restrict__ out,
-                                                         const int32_t* __restrict__ rowbase,
+                                                         const int64_t* __restrict__ rowbase,
                                                          int* __restrict__ err) {
     extern __shared__ __align__(1024) char sm_tc[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1016,10 +1015,12 @@ constexpr int kOrderClass = 2;
 // tensor-core product of one group costs about what the per-pair kernel takes
 // for one or two pairs (order 10: 33 ns against 44 ns a pair at the FP64 peak).
 constexpr double kMinGroupPairs = 16.0, kMinGroupPairs64 = 2.0;
-// Result rows of the full basis: above this the reference-mode M2L runs pair
-// by pair, which needs no rows.
-constexpr double kFullRowBytes = 64e9;
-constexpr double kOperatorBytes = 16e9;  // TF32 operator parts of one batch of groups
+// Memory limit of the calls that need not take the grouped products
+// (FMM_GB300_M2L_BYTES; read at every call).
+double grouped_bytes() {
+    const char* e = std::getenv("FMM_GB300_M2L_BYTES");
+    return e ? std::atof(e) : kGroupedBytes;
+}
 // TF32 products with fewer pairs per group than this (a task's columns not
 // filled by a group) take the groups of the eight octants together, where the
 // weights' eight copies fit.  250,000 particles in clusters with learned orders
@@ -1045,8 +1046,10 @@ int launch_operators(Workspace& ws, bool tc, bool full, int ldT, int ldr, const 
     return FMM_OK;
 }
 
+// bounded: the memory is limited to grouped_bytes().  FMM_ENOTSUP: the pairs should
+// go one by one.
 template <typename R, int CPT>
-int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) {
+int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, bool bounded) {
     const int M = t.num_nodes, nr = d64_rows(p, full), N = 2 * p, nTr = full ? nT(N) : rbase(N + 1);
     const bool tc = sizeof(R) == 4 && !product_on_cuda_cores();
     const bool tc64 = sizeof(R) == 8 && (full || !product_on_cuda_cores());
@@ -1056,15 +1059,14 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
     const int ldk = (nr + 15) / 16 * 16;
     const int ldT = nTr;
     const int wchunks = d64_chunks(p, full);
-    const int32_t* roff = nullptr;  // row of each far pair (target order), units of 32 entries
+    const int32_t* roff = nullptr;  // row of each far pair (target order), units of kRowUnit entries
     if (nf > 0 && !ws.reuse_structure) {
         // structure: displacement groups, their tensors and operators, tasks
         // and result rows (geometry only; kept for replays)
-        ws.m2l_pairwise = false;
-        if (full && (double)nf * row_len(p, true) * sizeof(R) > kFullRowBytes) {
-            ws.m2l_pairwise = true;
-            return FMM_ENOTSUP;
-        }
+        M2lSize size{nf, 1, row_len(p, full), ldT, 0, (int)sizeof(R)};
+        if (tc64) size.operator_bytes = (int64_t)d64_parts(p, full) * wchunks * D64Smem::g_bytes + sizeof(int) * (int64_t)nr;
+        if (tc) size.operator_bytes = (int64_t)tc_halves(p) * ((nr + kTcKC - 1) / kTcKC) * kTcRows * kTcKC * 2 * sizeof(float);
+        if (bounded && m2l_bytes(size) > grouped_bytes()) return FMM_ENOTSUP;
         FMM_TRY(ws.m2l_tgt.ensure(sizeof(int32_t) * nf));
         FMM_TRY(ws.m2l_keys.ensure(sizeof(uint64_t) * nf));
         FMM_TRY(ws.m2l_keys2.ensure(sizeof(uint64_t) * nf));
@@ -1120,10 +1122,10 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         // displacement groups of a few pairs each (irregular trees, mixed
         // orders) leave the products' columns empty and multiply the
         // per-group operators: the per-pair kernel is then the faster one
-        if ((double)nf < (tc64 ? kMinGroupPairs64 : kMinGroupPairs) * (double)ng) {
-            ws.m2l_pairwise = true;
+        if ((double)nf < (tc64 ? kMinGroupPairs64 : kMinGroupPairs) * (double)ng) return FMM_ENOTSUP;
+        size.groups = ng;
+        if ((bounded || (double)nf < kMinGroupPairs * (double)ng) && m2l_bytes(size) > grouped_bytes())
             return FMM_ENOTSUP;
-        }
         FMM_CUDA_TRY(cudaMemsetAsync(ws.m2l_cnt.as<int32_t>() + ng, 0, sizeof(int32_t), st));
         size_t tb4 = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tb4, ws.m2l_cnt.as<int32_t>(), ws.m2l_gstart.as<int32_t>(), ng + 1, st);
@@ -1172,8 +1174,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         // result rows in group order, (q+1)^2 rounded up to kRowUnit entries per
         // pair; the per-target sum finds them through roff (in the free
         // unsorted-keys buffer)
-        FMM_TRY(ws.m2l_rowbase.ensure(sizeof(int32_t) * (ng + 1)));
-        int32_t* rowbase = ws.m2l_rowbase.as<int32_t>();
+        FMM_TRY(ws.m2l_rowbase.ensure(sizeof(int64_t) * (ng + 1)));
+        int64_t* rowbase = ws.m2l_rowbase.as<int64_t>();
         count_launches(1);
         k_row_sizes<<<grid_for(ng + 1, 256), 256, 0, st>>>(ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
                                                             rowbase);
@@ -1181,16 +1183,17 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
         cub::DeviceScan::ExclusiveSum(nullptr, tb7, rowbase, rowbase, ng + 1, st);
         FMM_TRY(ws.cub_tmp.ensure(tb7));
         FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws.cub_tmp.p, tb7, rowbase, rowbase, ng + 1, st));
+        int ntasks = 0;
+        int64_t rows = 0;  // in units of kRowUnit entries
+        FMM_CUDA_TRY(cudaMemcpyAsync(&ntasks, ws.m2l_toff.as<int32_t>() + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
+        FMM_CUDA_TRY(cudaMemcpyAsync(&rows, rowbase + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        FMM_CUDA_TRY(cudaStreamSynchronize(st));
+        if (!m2l_rows_fit(rows)) return FMM_ENOTSUP;
         count_launches(1);
         k_row_offsets<<<dim3(grid_for(ng, 8), slices), 256, 0, st>>>(
             ng, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(), rowbase, ws.m2l_vals2.as<int32_t>(),
             reinterpret_cast<int32_t*>(ws.m2l_keys.p));
-        int hcnt[2] = {0, 0};  // tasks, rows (units of 32 entries)
-        FMM_CUDA_TRY(cudaMemcpyAsync(&hcnt[0], ws.m2l_toff.as<int32_t>() + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
-        FMM_CUDA_TRY(cudaMemcpyAsync(&hcnt[1], rowbase + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
-        FMM_CUDA_TRY(cudaStreamSynchronize(st));
-        const int ntasks = hcnt[0];
-        FMM_TRY(ws.m2l_out.ensure(sizeof(R) * kRowUnit * (size_t)std::max(1, hcnt[1])));
+        FMM_TRY(ws.m2l_out.ensure(sizeof(R) * kRowUnit * (size_t)std::max<int64_t>(1, rows)));
         FMM_TRY(ws.m2l_tasks.ensure(sizeof(int2) * std::max(1, ntasks)));
         count_launches(1);
         k_fill_tasks<<<grid_for(ng, 256), 256, 0, st>>>(ng, cols, ws.m2l_gq.as<int32_t>(), ws.m2l_gstart.as<int32_t>(),
@@ -1245,7 +1248,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
     if (nf > 0) {
         // numeric: scaled weights, the product, (below) the per-target sums
         const int ntasks = ws.m2l_ntasks;
-        const int32_t* rowbase = ws.m2l_rowbase.as<int32_t>();
+        const int64_t* rowbase = ws.m2l_rowbase.as<int64_t>();
         roff = reinterpret_cast<const int32_t*>(ws.m2l_keys.p);
         if (!tc64) {
             count_launches(1);
@@ -1336,11 +1339,24 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full) 
 // Grouped M2L into the local expansions ws.loc: the reduced components from the
 // weights ws.wred (which must be current), in FP32 products for `fp32`, else
 // FP64; or (full) all Cartesian components in FP64 with the reference's wrapped
-// tensors.  Returns FMM_ENOTSUP where the pairs should be evaluated one by one.
-int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full) {
-    if (fp32) return grouped<float, 8>(ws, t, p, st, false);
-    if (!full && product_on_cuda_cores() && GemmSmem<double, 4>(p).bytes > 227 * 1024) return FMM_ENOTSUP;
-    return grouped<double, 4>(ws, t, p, st, full);
+// tensors.  Returns FMM_ENOTSUP where the pairs should be evaluated one by one,
+// which replays keep (ws.m2l_pairwise): small groups, more rows than their
+// 32-bit numbers reach, or memory that is not there (the per-pair kernels need
+// none per pair) or, bounded, not for these products to take.
+int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full, bool bounded) {
+    if (ws.reuse_structure && ws.m2l_pairwise) return FMM_ENOTSUP;
+    int rc = FMM_ENOTSUP;
+    if (fp32)
+        rc = grouped<float, 8>(ws, t, p, st, false, bounded);
+    else if (full || !product_on_cuda_cores() || GemmSmem<double, 4>(p).bytes <= 227 * 1024)
+        rc = grouped<double, 4>(ws, t, p, st, full, bounded);
+    if (ws.reuse_structure) return rc;
+    if (rc == FMM_ENOMEM) {
+        ws.release_grouped();
+        rc = FMM_ENOTSUP;
+    }
+    ws.m2l_pairwise = rc == FMM_ENOTSUP;
+    return rc;
 }
 
 }  // namespace fmm

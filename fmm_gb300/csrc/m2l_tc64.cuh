@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kD64Threads, 1) k_m2l_tc64(const int2* __restr
                                                             const int32_t* __restrict__ psrc,
                                                             const uint4* __restrict__ wdig, int wchunks,
                                                             const int* __restrict__ wexp, double* __restrict__ out,
-                                                            const int32_t* __restrict__ rowbase, int row_unit,
+                                                            const int64_t* __restrict__ rowbase, int row_unit,
                                                             int* __restrict__ err) {
     extern __shared__ __align__(1024) char sm_d64[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
