@@ -317,7 +317,7 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
     using RT = Real<R>;
     const R ir2 = ir * ir;
     bool plain = damp == DAMP_NONE;
-    if constexpr (RT::kTay) plain = plain || (damp == DAMP_ERF && !(a * r2 < erf_far(N)));
+    if constexpr (RT::kTay) plain = plain || (damp == DAMP_ERF && a * r2 >= erf_far(N));
     if (plain) {
         g[0] = ir;
 #pragma unroll
@@ -339,7 +339,8 @@ __host__ __device__ __forceinline__ void radial_g_ir(int damp, R r2, R ir, R a, 
             // terms beside erf and divisions, and half the near field's time
             // (48 systems of 1,000 to 30,000 charges and dipoles: 5.35 ->
             // 2.98 ms, with the packed pairs that it makes worth while)
-            const int c = (int)s;
+            // (s < 0, factors of both signs, and NaN give NaN: the row only has to be there)
+            const int c = s > (R)0 ? (int)s : 0;
             const R t = s - ((R)c + (R)0.5);
             R b[FMM_BOYS_N];
             RT::boys_row(N, c, b);

@@ -117,7 +117,7 @@ __device__ __forceinline__ void radial_g_x2(int damp, f2 r2, f2 ir, f2 a, f2 eps
         const f2 s = a * r2;
         float s0, s1;
         sp2(s, s0, s1);
-        packed = !(s0 < erf_far(N)) && !(s1 < erf_far(N));
+        packed = s0 >= erf_far(N) && s1 >= erf_far(N);
         if (packed) {
 #pragma unroll
             for (int j = 0; j <= N; ++j) num[j] = bc2((float)((j % 2 ? -1.0 : 1.0) * dfact_odd(j)));
