@@ -79,3 +79,15 @@ def test_in_range(program, n):
     rows = [r for r in rows if r[2] > 0.0]
     for (g, row) in zip(evaluate(program, rows), rows):
         assert np.all(np.abs(g[:, 0] - g[:, 1]) <= 1e-6 * np.abs(g[:, 1])), (row, g)
+
+
+@pytest.mark.parametrize("n,bars", [(1, [9.5e-8, 1.22e-7]), (2, [9.4e-8, 1.16e-7, 1.20e-7]),
+                                    (4, [9.3e-8, 1.15e-7, 1.15e-7, 1.38e-7, 1.33e-7])])
+def test_accuracy(program, n, bars):
+    """rms errors: the bars are those of the plain series and error function."""
+    rng = np.random.default_rng(0)
+    s = np.exp(rng.uniform(np.log(1e-3), np.log(40.0), 6000))
+    a = rng.uniform(0.09, 0.64, 6000)
+    v = np.array(evaluate(program, [(n, x / b, b) for x, b in zip(s, a)]))
+    rms = np.sqrt(np.mean((v[:, :, 0] / v[:, :, 1] - 1.0) ** 2, axis=0))
+    assert np.all(rms <= bars), rms
