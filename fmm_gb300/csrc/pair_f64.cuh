@@ -90,7 +90,8 @@ __device__ __forceinline__ void contract_f64(double X, double Y, double Z, const
         A2 = fma(X, h[0], fma(Y, h[1], Z * h[2]));
         g2d = g[2] + g[2];
     }
-    if (damp != DAMP_AMOEBA) acc[0] = fma(mc[0], g[0], acc[0]);  // AMOEBA: g_0 = 0
+    // AMOEBA: g_0 = 0, which leaves NaN of infinite charges and NaN
+    if (damp != DAMP_AMOEBA || (__double2hiint(mc[0]) & 0x7ff00000) == 0x7ff00000) acc[0] = fma(mc[0], g[0], acc[0]);
     if constexpr (M >= 1) acc[0] = fma(A1, g[1], acc[0]);
     if constexpr (M >= 2) acc[0] = fma(A2, g[2], acc[0]);
     if constexpr (F >= 1) {
