@@ -6,11 +6,16 @@
 // Oishi, Rump, Numer. Algorithms 59, 2012): every row of G and every column of
 // W gets a power-of-two scale, its entries become 62-bit integers, and those
 // eight signed base-256 digits each, which FP16 holds exactly.  Digit products
-// of equal weight 256^-(i+j) are accumulated by the tensor cores in one FP32
-// accumulator per weight, exactly (at most 2^24: K <= 464 products of 2^14, the
-// leading digits being at most 64), and the eight sums are put together in
-// 64-bit integers and rounded once to FP64.  Digit products below 256^-7 are
-// left out: 36 of 64 remain.  The result is within 2^-60 K of the row scale
+// of equal weight 256^-d, d = i + j, are accumulated by the tensor cores in one
+// FP32 accumulator per weight, and the eight sums are put together in 64-bit
+// integers and rounded once to FP64.  The leading digits being at most 64, an
+// accumulator holds at most max(d, 1/4) K 2^14, and sums to 2^24 are exact: K is
+// taken in segments of kD64Segment chunks (176 components), each of which ends
+// in the rounded sum, so that every weight to 256^-5 is exact whatever the digits.
+// (256^-6 and 256^-7 could reach 1.03 and 1.2 times 2^24 if all digits were
+// extreme and of one sign; 37 and 238 additions would then round by a unit at
+// most, which is below an eighth of what the products left out can be.)  Digit
+// products below 256^-7 are left out: 36 of 64 remain.  The result is within 2^-60 K of the row scale
 // times the column scale, where an FP64 sum rounds K times at 2^-53 of its
 // partial sums.  So that a scale fits all the entries it covers, component s is
 // weighted by 2^sigma(|s|) ~ |s|! / 3^(|s|/2) in W and the inverse in G: tensors
@@ -46,6 +51,7 @@ constexpr int kD64Rows = 128;      // operator rows per part (MMA M)
 constexpr int kD64Pairs = 64;      // pairs per task (MMA N)
 constexpr int kD64K = 16;          // components per chunk (MMA K)
 constexpr int kD64Stages = 4;
+constexpr int kD64Segment = 11;    // chunks per accumulation (reduced basis: all, to order 12)
 constexpr int kD64Producers = 64;  // warps 0-1
 constexpr int kD64MmaWarp = 2;
 constexpr int kD64EpiWarps = 16;
@@ -371,35 +377,37 @@ __global__ void __launch_bounds__(kD64Threads, 1) k_m2l_tc64(const int2* __restr
             constexpr uint32_t LBO = 128, SBO = 256;
             for (int task = blockIdx.x; task < ntasks && ok; task += gridDim.x) {
                 const int nch = d64_chunks(gq[tasks[task].x], full);
-                if (tl >= 1 && !umma::mbar_wait(acc_empty, (tl - 1) & 1, kD64WaitCycles)) {
-                    ok = false;
-                    break;
-                }
-                umma::fence_after_sync();
-                for (int ch = 0; ch < nch; ++ch, ++u) {
-                    const int st = (int)(u % kD64Stages);
-                    if (!umma::mbar_wait(&fullb[st], (u / kD64Stages) & 1, kD64WaitCycles)) {
+                for (int c0 = 0; c0 < nch && ok; c0 += kD64Segment) {
+                    if (tl >= 1 && !umma::mbar_wait(acc_empty, (tl - 1) & 1, kD64WaitCycles)) {
                         ok = false;
                         break;
                     }
-                    umma::fence_proxy_async();
                     umma::fence_after_sync();
-                    const char* Gs = sm_d64 + (size_t)st * D64Smem::stage_bytes;
-                    const char* Ws = Gs + D64Smem::g_bytes;
+                    for (int ch = c0; ch < min(nch, c0 + kD64Segment); ++ch, ++u) {
+                        const int st = (int)(u % kD64Stages);
+                        if (!umma::mbar_wait(&fullb[st], (u / kD64Stages) & 1, kD64WaitCycles)) {
+                            ok = false;
+                            break;
+                        }
+                        umma::fence_proxy_async();
+                        umma::fence_after_sync();
+                        const char* Gs = sm_d64 + (size_t)st * D64Smem::stage_bytes;
+                        const char* Ws = Gs + D64Smem::g_bytes;
 #pragma unroll 1
-                    for (int i = 0; i < kDig; ++i) {
-                        const uint64_t a = umma::smem_desc(Gs + i * (kD64Rows * kD64K * 2), LBO, SBO);
+                        for (int i = 0; i < kDig; ++i) {
+                            const uint64_t a = umma::smem_desc(Gs + i * (kD64Rows * kD64K * 2), LBO, SBO);
 #pragma unroll 1
-                        for (int k = 0; k < kDig - i; ++k)
-                            umma::mma_f16(tmem + (uint32_t)((i + k) * kD64Pairs), a,
-                                          umma::smem_desc(Ws + k * (kD64Pairs * kD64K * 2), LBO, SBO), idesc,
-                                          (ch > 0 || i > 0) ? 1u : 0u);
+                            for (int k = 0; k < kDig - i; ++k)
+                                umma::mma_f16(tmem + (uint32_t)((i + k) * kD64Pairs), a,
+                                              umma::smem_desc(Ws + k * (kD64Pairs * kD64K * 2), LBO, SBO), idesc,
+                                              (ch > c0 || i > 0) ? 1u : 0u);
+                        }
+                        umma::commit(&empty[st]);
                     }
-                    umma::commit(&empty[st]);
+                    if (!ok) break;
+                    umma::commit(acc_full);
+                    ++tl;
                 }
-                if (!ok) break;
-                umma::commit(acc_full);
-                ++tl;
             }
         }
         __syncwarp();
@@ -418,44 +426,51 @@ __global__ void __launch_bounds__(kD64Threads, 1) k_m2l_tc64(const int2* __restr
             const int K = d64_rows(q, full), rl = (K + row_unit - 1) / row_unit * row_unit;
             const int ef = f < K ? gexp[(size_t)g * ldr + f] : 0;
             double* gout = out + (size_t)rowbase[g] * row_unit + (size_t)first * rl;
-            if (!umma::mbar_wait(acc_full, tl & 1, kD64WaitCycles)) {
-                ok = false;
-                break;
-            }
-            umma::fence_after_sync();
+            const int nch = d64_chunks(q, full);
             const uint32_t base = tmem + ((uint32_t)(32 * sp) << 16);
+            for (int c0 = 0; c0 < nch; c0 += kD64Segment, ++tl) {
+                if (!umma::mbar_wait(acc_full, tl & 1, kD64WaitCycles)) {
+                    ok = false;
+                    break;
+                }
+                umma::fence_after_sync();
 #pragma unroll 1
-            for (int c = share * CB; c < cnt && f0 + 32 * sp < rl; c += kShares * CB) {
-                float v[kDig][CB];
-                __syncwarp();
+                for (int c = share * CB; c < cnt && f0 + 32 * sp < rl; c += kShares * CB) {
+                    float v[kDig][CB];
+                    __syncwarp();
 #pragma unroll
-                for (int d = 0; d < kDig; ++d) umma::tmem_ld8(base + (uint32_t)(d * kD64Pairs + c), v[d]);
-                umma::tmem_ld_wait();
+                    for (int d = 0; d < kDig; ++d) umma::tmem_ld8(base + (uint32_t)(d * kD64Pairs + c), v[d]);
+                    umma::tmem_ld_wait();
 #pragma unroll
-                for (int d = 0; d < kDig; ++d) umma::tmem_landed(v[d]);
+                    for (int d = 0; d < kDig; ++d) umma::tmem_landed(v[d]);
 #pragma unroll
-                for (int jj = 0; jj < CB; ++jj) {
-                    if (c + jj < cnt) {
-                        // sum of the accumulators 256^-d: (hi 2^32 + lo) units of
-                        // 2^(ef + ew - 68)
-                        const int ew = wexp[psrc[gs + c + jj]];
-                        long long hi = 0, lo = 0;
+                    for (int jj = 0; jj < CB; ++jj) {
+                        if (c + jj < cnt) {
+                            // sum of the accumulators 256^-d: (hi 2^32 + lo) units of
+                            // 2^(ef + ew - 68)
+                            const int ew = wexp[psrc[gs + c + jj]];
+                            long long hi = 0, lo = 0;
 #pragma unroll
-                        for (int d = 0; d < 4; ++d) hi = (hi << 8) + (long long)__float2int_rn(v[d][jj]);
+                            for (int d = 0; d < 4; ++d) hi = (hi << 8) + (long long)__float2int_rn(v[d][jj]);
 #pragma unroll
-                        for (int d = 4; d < 8; ++d) lo = (lo << 8) + (long long)__float2int_rn(v[d][jj]);
-                        // as many bits of lo as hi leaves room for (|hi| < 2^46)
-                        const int up = min(32, __clzll(hi < 0 ? ~hi : hi) - 2);
-                        double r = d64_round((hi << up) + (lo >> (32 - up)), ef + ew - 36 - up);
-                        if (ew >= kD64BadExp) r = __longlong_as_double(0x7ff8000000000000ll);
-                        if (f < rl) __stcs(gout + (size_t)(c + jj) * rl + f, f < K ? r : 0.0);
+                            for (int d = 4; d < 8; ++d) lo = (lo << 8) + (long long)__float2int_rn(v[d][jj]);
+                            // as many bits of lo as hi leaves room for (|hi| < 2^46)
+                            const int up = min(32, __clzll(hi < 0 ? ~hi : hi) - 2);
+                            double r = d64_round((hi << up) + (lo >> (32 - up)), ef + ew - 36 - up);
+                            if (ew >= kD64BadExp) r = __longlong_as_double(0x7ff8000000000000ll);
+                            double* o = gout + (size_t)(c + jj) * rl + f;
+                            if (c0 == 0) {
+                                if (f < rl) __stcs(o, f < K ? r : 0.0);
+                            } else if (f < K) {
+                                *o += r;  // (this thread's, of the segments before)
+                            }
+                        }
                     }
                 }
+                umma::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) umma::mbar_arrive(acc_empty);
             }
-            umma::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) umma::mbar_arrive(acc_empty);
-            ++tl;
         }
     }
     if (!ok) atomicExch(err, 1);
