@@ -41,7 +41,7 @@ void DevBuf::release() {
 void Workspace::release_grouped() {
     for (DevBuf* b : {&m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
                       &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit,
-                      &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp})
+                      &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &m2l_gord})
         b->release();
 }
 
@@ -54,7 +54,7 @@ void Workspace::release_buffers(bool keep_selector) {
                      &sz,        &smc,       &sd,          &fsorted,    &mom,        &loc,        &partial,
                      &term_off,  &term_abc,  &term_c, &f32buf, &f32sel, &wred, &far_ord, &sel_norms, &sel_params, &sel_scratch, &sysbuf,
                      &list_cnt, &sys_ids, &sys_tab, &m2l_tgt, &m2l_keys, &m2l_keys2, &m2l_vals, &m2l_vals2, &m2l_ukeys, &m2l_cnt, &m2l_gstart,
-                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &f32x2c, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
+                     &m2l_tcnt, &m2l_toff, &m2l_tasks, &m2l_T, &m2l_gq, &m2l_gab, &m2l_wsc, &m2l_out, &m2l_wsplit, &m2l_gop, &m2l_gopoff, &m2l_rowbase, &m2l_gexp, &m2l_gord, &xlate, &l2pt, &dsmc, &f32node, &lattice, &p2p_order, &p2p_pad, &f32x2, &f32x2c, &sel_budget, &corr_pairs, &corr_sorted, &corr_src, &leaf_ext, &near_rows, &near_part, &images};
     for (DevBuf* b : all)
         if (!(keep_selector && b == &sel_params)) b->release();
     if (!keep_selector) sel_ready = false;

@@ -1040,7 +1040,8 @@ int launch_operators(Workspace& ws, bool tc, bool full, int ldT, int ldr, const 
     } else {
         k_operator64<<<(unsigned)(b.g1 - b.g0), 256, sizeof(double) * ldT, st>>>(
             full, ldT, ws.m2l_T.as<double>(), ws.m2l_gq.as<int32_t>(), ws.m2l_gab.as<float2>(),
-            ws.m2l_gopoff.as<int64_t>(), b.g0, base, ldr, ws.m2l_gop.as<uint4>(), ws.m2l_gexp.as<int>());
+            ws.m2l_gopoff.as<int64_t>(), b.g0, base, ldr, ws.m2l_gop.as<uint4>(), ws.m2l_gexp.as<int>(),
+            ws.m2l_gord.as<short>());
     }
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
@@ -1205,8 +1206,11 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         if (tc || tc64) {
             // tensor-core operands: per node the weights, per group the operator
             FMM_TRY(ws.m2l_wsplit.ensure(tc ? sizeof(float) * 2 * (size_t)M * ldk * (ws.m2l_mirrored ? kOctants : 1)
-                                            : (size_t)M * (wchunks * kDig * kD64K * 2 + sizeof(int))));
-            if (tc64) FMM_TRY(ws.m2l_gexp.ensure(sizeof(int) * (size_t)ng * nr));
+                                            : (size_t)M * (wchunks * kDig * kD64K * 2 + sizeof(int) + sizeof(short) * kD64Orders)));
+            if (tc64) {
+                FMM_TRY(ws.m2l_gexp.ensure(sizeof(int) * (size_t)ng * nr));
+                FMM_TRY(ws.m2l_gord.ensure(sizeof(short) * kD64Orders * (size_t)ng));
+            }
             FMM_TRY(ws.m2l_gopoff.ensure(sizeof(int64_t) * (ng + 1)));
             int64_t* goff = ws.m2l_gopoff.as<int64_t>();
             count_launches(1);
@@ -1259,6 +1263,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         if (tc || tc64) {
             // TF32 parts or digits of the weights (per node)
             int* wexp = nullptr;
+            short* word = nullptr;
             count_launches(1);
             if (tc) {
                 k_split_weights<<<grid_for((int64_t)M * ldk, 256), 256, 0, st>>>(
@@ -1267,9 +1272,10 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
                 FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)TcSmem::bytes));
             } else {
-                wexp = reinterpret_cast<int*>(ws.m2l_wsplit.as<uint4>() + (size_t)M * wchunks * kDig * 2);
+                word = reinterpret_cast<short*>(ws.m2l_wsplit.as<uint4>() + (size_t)M * wchunks * kDig * 2);
+                wexp = reinterpret_cast<int*>(word + (size_t)M * kD64Orders);
                 k_weights64<<<grid_for(M, 4), 128, 0, st>>>(M, p, full, full ? ws.mom.as<double>() : ws.wred.as<double>(),
-                                                            t.r, ws.m2l_wsplit.as<uint4>(), wexp);
+                                                            t.r, ws.m2l_wsplit.as<uint4>(), wexp, word);
                 FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)D64Smem::bytes));
             }
@@ -1301,6 +1307,17 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
                         ws.m2l_gop.as<uint4>(), nr, ws.m2l_gexp.as<int>(), ws.m2l_vals.as<int32_t>(),
                         ws.m2l_wsplit.as<uint4>(), wchunks, wexp, reinterpret_cast<double*>(ws.m2l_out.p), rowbase,
                         kRowUnit, d_err);
+            }
+            if (tc64 && ntasks > 0) {
+                const size_t sm = sizeof(double) * ((size_t)ldT + 4 * nr);
+                FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_m2l_pairs64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)sm));
+                count_launches(1);
+                k_m2l_pairs64<<<(unsigned)std::min(ntasks, 8 * sms), 128, sm, st>>>(
+                    ws.m2l_tasks.as<int2>(), ntasks, full, ws.m2l_gstart.as<int32_t>(), ws.m2l_gq.as<int32_t>(),
+                    ws.m2l_gab.as<float2>(), ws.m2l_T.as<double>(), ldT, ws.m2l_gord.as<short>(),
+                    ws.m2l_vals.as<int32_t>(), full ? ws.mom.as<double>() : ws.wred.as<double>(), nr, t.r, word, wexp,
+                    reinterpret_cast<double*>(ws.m2l_out.p), rowbase, kRowUnit);
             }
             if (ws.product_timed) cudaEventRecord(ws.ev[9], st);
             // the product's error flag is read with the call's final copies

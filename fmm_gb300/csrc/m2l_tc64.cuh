@@ -58,6 +58,12 @@ constexpr int kD64EpiWarps = 16;
 constexpr int kD64Threads = 32 * (3 + kD64EpiWarps);
 constexpr int kD64BadExp = 1 << 20;  // column exponent of non-finite weights: their products are NaN
 constexpr long long kD64WaitCycles = 4000000000LL;
+// Exponents per order of a node's weights and of a group's first row, and (the
+// last) the group's scale: 32 bytes each.
+constexpr int kD64Orders = 16;
+constexpr int kD64NoExp = -32000;  // no such entry
+// Bits by which a pair's scales may exceed its largest term (k_m2l_pairs64).
+constexpr int kD64Loss = 6;
 
 // Operator rows (and columns) of order q: the reduced basis, or all Cartesian
 // components (full).
@@ -144,13 +150,17 @@ __device__ __forceinline__ double d64_round(long long v, int e) {
 }
 
 // Digits of every node's weights w'_s = w_s / h^|s|, node by node and chunk by
-// chunk ([chunk][digit][16]), and the node's exponent.  w is the reduced
-// weights, or (full) (-1)^(|s|+1) M'_s of the moments.  Warp per node.
+// chunk ([chunk][digit][16]), the node's exponent and those of its orders.  w is
+// the reduced weights, or (full) (-1)^(|s|+1) M'_s of the moments.  Warp per node.
 __global__ void __launch_bounds__(128) k_weights64(int M, int p, bool full, const double* __restrict__ w,
                                                    const double* __restrict__ h, uint4* __restrict__ dig,
-                                                   int* __restrict__ wexp) {
+                                                   int* __restrict__ wexp, short* __restrict__ word) {
+    __shared__ int eord[4][kD64Orders];
     const int node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (node >= M) return;
+    int* eo = eord[threadIdx.x >> 5];
+    if (lane < kD64Orders) eo[lane] = kD64NoExp;
+    __syncwarp();
     const int K = d64_rows(p, full), pieces = 2 * d64_chunks(p, full);
     const double ih = 1.0 / h[node];
     double pw = 1.0;  // lane j: ih^j
@@ -175,7 +185,9 @@ __global__ void __launch_bounds__(128) k_weights64(int M, int p, bool full, cons
                 const int x = d64_sigma(o);
                 if (pass == 0) {
                     const bool bad = ((__double2hiint(v) >> 20) & 0x7ff) == 0x7ff;
-                    emax = max(emax, bad ? kD64BadExp : d64_exp(v, x));
+                    const int e = d64_exp(v, x);
+                    emax = max(emax, bad ? kD64BadExp : e);
+                    if (s < K && e > kD64NoExp) atomicMax(&eo[o], e);
                 } else {
                     q[k] = emax >= kD64BadExp ? 0 : d64_fix(v, x, emax + 1);
                 }
@@ -193,6 +205,7 @@ __global__ void __launch_bounds__(128) k_weights64(int M, int p, bool full, cons
             for (int off = 16; off > 0; off >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, off));
     }
     if (lane == 0) wexp[node] = emax >= kD64BadExp ? kD64BadExp : emax + 1;
+    if (lane < kD64Orders) word[(size_t)node * kD64Orders + lane] = (short)eo[lane];
 }
 
 // Bytes / 16 of a group's operator digits.
@@ -204,13 +217,15 @@ __global__ void k_op64_sizes(int ng, bool full, const int32_t* __restrict__ gq, 
 
 // Block per group: the digits of G_fs = a^(|f|+1) b^|s| T_{f+s}(D_c)
 // 2^-sigma(|s|), part by part and chunk by chunk ([digit][128 x 16] in the
-// operand layout), and the exponent of every row f.  a and b are powers of two
-// and only move exponents.
+// operand layout), the exponent of every row f, and (gord) those of the first
+// row's orders and the largest of 2^-sigma(|f|) G_f, which is what row f weighs in
+// the target's potential.  a and b are powers of two and only move exponents.
 __global__ void __launch_bounds__(256) k_operator64(bool full, int ldT, const double* __restrict__ gT,
                                                     const int32_t* __restrict__ gq, const float2* __restrict__ gab,
                                                     const int64_t* __restrict__ goff, int g0, int64_t gop_base, int ldr,
-                                                    uint4* __restrict__ gop, int* __restrict__ gexp) {
-    __shared__ int dec[nT(kMaxP)], rexp[kD64MaxRows];
+                                                    uint4* __restrict__ gop, int* __restrict__ gexp,
+                                                    short* __restrict__ gord) {
+    __shared__ int dec[nT(kMaxP)], rexp[kD64MaxRows], eord[kD64Orders];
     extern __shared__ double Tsh[];
     const int g = g0 + blockIdx.x, q = gq[g];
     const int K = d64_rows(q, full), nch = d64_chunks(q, full), nrow = d64_parts(q, full) * kD64Rows;
@@ -219,6 +234,7 @@ __global__ void __launch_bounds__(256) k_operator64(bool full, int ldT, const do
     for (int e = threadIdx.x; e < nTq; e += blockDim.x) Tsh[e] = gT[(size_t)g * ldT + e];
     const float2 ab = gab[g];
     const int ea = ((__float_as_int(ab.x) >> 23) & 255) - 127, eb = ((__float_as_int(ab.y) >> 23) & 255) - 127;
+    if (threadIdx.x < kD64Orders) eord[threadIdx.x] = kD64NoExp;
     __syncthreads();
     auto entry = [&](int cf, int cs, int* x) {
         const int tx = (cs & 0xff) + (cf & 0xff), ty = ((cs >> 8) & 0xff) + ((cf >> 8) & 0xff),
@@ -233,15 +249,19 @@ __global__ void __launch_bounds__(256) k_operator64(bool full, int ldT, const do
             for (int s = lane; s < K; s += 32) {
                 int x;
                 const double v = entry(dec[f], dec[s], &x);
-                emax = max(emax, d64_exp(v, x));
+                const int e = d64_exp(v, x);
+                emax = max(emax, e);
+                if (f == 0 && e > kD64NoExp) atomicMax(&eord[dec[s] >> 24], e);
             }
         for (int off = 16; off > 0; off >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, off));
         if (lane == 0) {
             rexp[f] = emax + 1;
             if (f < ldr) gexp[(size_t)g * ldr + f] = emax + 1;
+            if (f < K) atomicMax(&eord[kD64Orders - 1], emax - d64_sigma(dec[f] >> 24));
         }
     }
     __syncthreads();
+    if (threadIdx.x < kD64Orders) gord[(size_t)g * kD64Orders + threadIdx.x] = (short)eord[threadIdx.x];
     uint4* out = gop + (goff[g] - gop_base);
     for (int it = threadIdx.x; it < nrow * nch * 2; it += blockDim.x) {
         // consecutive threads: consecutive rows of one (part, chunk, half of K)
@@ -477,6 +497,93 @@ __global__ void __launch_bounds__(kD64Threads, 1) k_m2l_tc64(const int2* __restr
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, kDig * kD64Pairs);
+}
+
+// Pairs whose scales exceed their terms: FP64 sums in place of the products.  The
+// products' error follows the row's scale times the column's, which can lie far
+// above the largest term: quadrupoles without charges in a fine cell meet the
+// row's third order, (h_j / D)^2 below its first.  With the exponents e_k of the
+// node's orders, r_k of the group's first row (which is of the potential's size)
+// and S of all rows, S + max e - max (r_k + e_k) bits are lost.  Emulated against
+// long double at orders 5 to 12, D from 1.3 to 20 half-widths, level differences
+// to 4, charges, dipoles, quadrupoles and all of them, the products' error is 0.1 to
+// 0.65 of an FP64 sum's to 6 bits, as large at 7, and then doubles with each.
+// A thread checks a pair, a warp sums one (a task's first part does the whole row).
+__global__ void __launch_bounds__(128) k_m2l_pairs64(const int2* __restrict__ tasks, int ntasks, bool full,
+                                                     const int32_t* __restrict__ gstart,
+                                                     const int32_t* __restrict__ gq, const float2* __restrict__ gab,
+                                                     const double* __restrict__ gT, int ldT,
+                                                     const short* __restrict__ gord, const int32_t* __restrict__ psrc,
+                                                     const double* __restrict__ w, int ldw,
+                                                     const double* __restrict__ h, const short* __restrict__ word,
+                                                     const int* __restrict__ wexp, double* __restrict__ out,
+                                                     const int64_t* __restrict__ rowbase, int row_unit) {
+    extern __shared__ double sm_pairs64[];
+    __shared__ int list[kD64Pairs], count, dec[nT(kMaxP)];
+    static_assert(kD64Pairs <= 128, "a thread per pair");
+    double* T = sm_pairs64;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double* ws = T + ldT + warp * ldw;
+    if (tid == 0) count = 0;
+    __syncthreads();
+    for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+        const int2 tk = tasks[task];
+        if ((tk.y & 3) != 0) continue;
+        const int g = tk.x, first = tk.y >> 2, gs = gstart[g] + first, cnt = min(kD64Pairs, gstart[g + 1] - gs);
+        bool lossy = false;
+        if (tid < cnt) {
+            const int src = psrc[gs + tid];
+            const uint4* ep = reinterpret_cast<const uint4*>(word) + 2 * (size_t)src;
+            const uint4* rp = reinterpret_cast<const uint4*>(gord) + 2 * (size_t)g;
+            const uint4 e0 = ep[0], e1 = ep[1], r0 = rp[0], r1 = rp[1];
+            const unsigned ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+            const unsigned rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+            auto at = [](const unsigned (&v)[8], int k) { return (int)(short)(v[k >> 1] >> (16 * (k & 1))); };
+            int emax = kD64NoExp, term = 2 * kD64NoExp;
+#pragma unroll
+            for (int k = 0; k <= kMaxP; ++k) {
+                emax = max(emax, at(ev, k));
+                term = max(term, at(ev, k) + at(rv, k));
+            }
+            lossy = emax > kD64NoExp && at(rv, kD64Orders - 1) + emax - term > kD64Loss && wexp[src] < kD64BadExp;
+            if (lossy) list[atomicAdd(&count, 1)] = tid;
+        }
+        const int n = __syncthreads_count(lossy);
+        if (n == 0) continue;
+        const int q = gq[g], K = d64_rows(q, full), rl = (K + row_unit - 1) / row_unit * row_unit;
+        for (int e = tid; e < (full ? nT(2 * q) : rbase(2 * q + 1)); e += blockDim.x) T[e] = gT[(size_t)g * ldT + e];
+        for (int e = tid; e < K; e += blockDim.x) dec[e] = d64_comp(e, full);
+        __syncthreads();
+        const double a = gab[g].x, b = gab[g].y;
+        for (int l = warp; l < n; l += 4) {
+            const int pr = list[l], src = psrc[gs + pr];
+            const double bh = b / h[src];
+            for (int s = lane; s < K; s += 32) {
+                const int o = dec[s] >> 24;
+                double v = w[(size_t)src * ldw + s];
+                for (int k = 0; k < o; ++k) v *= bh;
+                ws[s] = full && (o & 1) == 0 ? -v : v;
+            }
+            __syncwarp();
+            double* row = out + (size_t)rowbase[g] * row_unit + (size_t)(first + pr) * rl;
+            for (int f = lane; f < rl; f += 32) {
+                double v = 0.0;
+                if (f < K) {
+                    const int cf = dec[f];
+                    for (int s = 0; s < K; ++s) {
+                        const int c = cf + dec[s], x = c & 0xff, y = (c >> 8) & 0xff, z = (c >> 16) & 0xff;
+                        v = fma(T[full ? pidx(x, y, z) : ridx(x, y, z)], ws[s], v);
+                    }
+                    for (int k = 0; k <= (cf >> 24); ++k) v *= a;
+                }
+                row[f] = v;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        if (tid == 0) count = 0;
+        __syncthreads();
+    }
 }
 
 }  // namespace
