@@ -211,6 +211,7 @@ struct Workspace {
     DevBuf f32x2c;       // the damping-correction list's
     int m2l_ng = 0, m2l_ntasks = 0;  // grouped M2L structure of the last evaluation
     bool m2l_mirrored = false;       // its groups join the eight octants' displacements
+    bool m2l_fp64 = false;           // its products are FP64
     bool m2l_pairwise = false;       // the last structure chose the per-pair M2L kernel
     std::vector<M2lBatch> m2l_batches;  // operator batches of the last structure
     int64_t list_candidates = 0; // cell pairs examined by the last list build

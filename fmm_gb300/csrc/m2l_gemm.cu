@@ -1106,6 +1106,13 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         int ng = 0;
         FMM_CUDA_TRY(cudaMemcpyAsync(&ng, d_nruns, sizeof(int), cudaMemcpyDeviceToHost, st));
         FMM_CUDA_TRY(cudaStreamSynchronize(st));
+        // displacement groups of a few pairs each (irregular trees, mixed orders)
+        // leave the products' columns empty and multiply the per-group operators.
+        // Counted before the octants are joined: what is below the line is summed in
+        // FP64 (launch_m2l_grouped) or pair by pair, both more accurate than TF32
+        // parts (3,001 clustered particles, 13 pairs a group, far field at order 12:
+        // 2e-10 against 4.6e-9)
+        const bool few = (double)nf < (tc64 ? kMinGroupPairs64 : kMinGroupPairs) * (double)ng;
         ws.m2l_mirrored = tc && t.nimg <= 1 && (double)nf < kMirrorPairs * (double)ng &&
                           sizeof(float) * 2.0 * kOctants * M * ldk <= kMirrorBytes;
         if (ws.m2l_mirrored) {
@@ -1120,10 +1127,7 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
             FMM_CUDA_TRY(cudaStreamSynchronize(st));
         }
         ws.m2l_groups = ng;
-        // displacement groups of a few pairs each (irregular trees, mixed
-        // orders) leave the products' columns empty and multiply the
-        // per-group operators: the per-pair kernel is then the faster one
-        if ((double)nf < (tc64 ? kMinGroupPairs64 : kMinGroupPairs) * (double)ng) return FMM_ENOTSUP;
+        if (few) return FMM_ENOTSUP;
         size.groups = ng;
         if ((bounded || (double)nf < kMinGroupPairs * (double)ng) && m2l_bytes(size) > grouped_bytes())
             return FMM_ENOTSUP;
@@ -1356,16 +1360,25 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
 // Grouped M2L into the local expansions ws.loc: the reduced components from the
 // weights ws.wred (which must be current), in FP32 products for `fp32`, else
 // FP64; or (full) all Cartesian components in FP64 with the reference's wrapped
-// tensors.  Returns FMM_ENOTSUP where the pairs should be evaluated one by one,
+// tensors.  Groups too small for the FP32 products take the FP64 ones where they
+// hold two pairs or more (3,001 clustered particles, 13 pairs a group: the M2L at
+// orders 4 / 8 / 12 0.7 / 1.1 / 2.7 ms, pair by pair 0.8 / 2.6 / 15.6).  Returns FMM_ENOTSUP where the pairs should be evaluated one by one,
 // which replays keep (ws.m2l_pairwise): small groups, more rows than their
 // 32-bit numbers reach, or memory that is not there (the per-pair kernels need
 // none per pair) or, bounded, not for these products to take.
 int launch_m2l_grouped(Workspace& ws, const TreeDev& t, int p, bool fp32, cudaStream_t st, bool full, bool bounded) {
     if (ws.reuse_structure && ws.m2l_pairwise) return FMM_ENOTSUP;
     int rc = FMM_ENOTSUP;
-    if (fp32)
+    if (!ws.reuse_structure) ws.m2l_fp64 = !fp32;
+    if (!ws.m2l_fp64) {
         rc = grouped<float, 8>(ws, t, p, st, false, bounded);
-    else if (full || !product_on_cuda_cores() || GemmSmem<double, 4>(p).bytes <= 227 * 1024)
+        if (rc == FMM_ENOTSUP && !product_on_cuda_cores()) {
+            const int64_t groups = ws.m2l_groups;  // (the octants' joined, as the statistics count them)
+            ws.m2l_fp64 = true;
+            rc = grouped<double, 4>(ws, t, p, st, false, true);
+            ws.m2l_groups = groups;
+        }
+    } else if (full || !product_on_cuda_cores() || GemmSmem<double, 4>(p).bytes <= 227 * 1024)
         rc = grouped<double, 4>(ws, t, p, st, full, bounded);
     if (ws.reuse_structure) return rc;
     if (rc == FMM_ENOMEM) {
