@@ -44,7 +44,12 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 // four, water with Thole damping (60,000 sites) is 1.31e-6 off the FP64 near
 // field, at three 1.27e-6, as with the folds at every leaf end before.
 constexpr int kFold = 3;
-constexpr int kExwRegs = 4;  // exclusion entries held in registers per target
+// Exclusion entries held in registers per target; for the others a piece is
+// checked by the range of their slots.  Eight cost the kernels 3 to 7%, so longer
+// lists than four have kernels of their own (WIDE).  240,000 particles in
+// molecules of eight, near field with four / eight: charges 2.0 / 1.4 ms, dipoles with
+// field gradients 3.5 / 2.8.
+__host__ __device__ constexpr int exw_regs(bool wide) { return wide ? 8 : 4; }
 
 // Sub-chunks of a target leaf's last rem < 32 particles (index rem): the
 // count that minimises the lane-steps of a piece of source blocks for leaves
@@ -173,10 +178,11 @@ __global__ void k_node_centres_f32(int M, const TreeDev t, float4* __restrict__ 
 }
 
 // One target's position and the sorted positions (slots) that it passes over.
+template <bool WIDE>
 struct Target {
     float4 a, b;          // the record's first two float4s
     int slot;             // its own slot
-    int ex[kExwRegs];     // slots of the excluded partners listed first (-1: none)
+    int ex[exw_regs(WIDE)];  // slots of the excluded partners listed first (-1: none)
     int lo, hi;           // range of the slots of the others
     int orig;             // original index
 };
@@ -196,8 +202,8 @@ __device__ __forceinline__ int first_block(int b0, int grp, int ngr) {
 // rounding is of the order of a single pair's, and the TwoSum cost is paid once
 // per fold.  k0 is the slot of src[0].  CHECK: the piece may hold the
 // target itself or one of its excluded partners.
-template <int M, int F, int DAMP, bool CHECK>
-__device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, int grp, int ngr, const Target& T,
+template <int M, int F, int DAMP, bool CHECK, bool WIDE>
+__device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, int grp, int ngr, const Target<WIDE>& T,
                                           const int32_t* __restrict__ excl, int exw, int64_t n, float* hi, float* lo,
                                           float* blk, int& nb) {
     constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM);
@@ -208,8 +214,8 @@ __device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, in
             const int o = __float_as_int(b.w);
             bool skip = k0 + k == T.slot;
 #pragma unroll
-            for (int e = 0; e < kExwRegs; ++e) skip |= k0 + k == T.ex[e];
-            for (int e = kExwRegs; e < exw; ++e) skip |= (excl[(size_t)e * n + T.orig] == o);
+            for (int e = 0; e < exw_regs(WIDE); ++e) skip |= k0 + k == T.ex[e];
+            for (int e = exw_regs(WIDE); e < exw; ++e) skip |= (excl[(size_t)e * n + T.orig] == o);
             if (skip) continue;
         }
         float mc[4 * (NV - 2)];
@@ -254,8 +260,8 @@ __device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, in
 // damping leaves undefined: which pairs those are is part of the result, so
 // correction pieces are single leaves, their blocks counted from the leaf's
 // start and their test made on leaf-relative positions, whatever the runs.)
-template <int M, int F, int DAMP, bool CHECK, bool CORR = false>
-__device__ __forceinline__ void p2p_piece_x2(const float4* src, int nblk, int k0, int grp, int ngr, const Target& T,
+template <int M, int F, int DAMP, bool CHECK, bool CORR, bool WIDE>
+__device__ __forceinline__ void p2p_piece_x2(const float4* src, int nblk, int k0, int grp, int ngr, const Target<WIDE>& T,
                                              const int32_t* __restrict__ excl, int exw, int64_t n, f2* H, f2* L,
                                              f2* B, int& nb, float xcut2 = 0.0f, int* ncorr = nullptr) {
     constexpr int NF = nT(F), NM = nT(M), NV = rec_vec(NM), NE = 4 * (NV - 2);
@@ -290,14 +296,14 @@ __device__ __forceinline__ void p2p_piece_x2(const float4* src, int nblk, int k0
             const int k = k0 + 2 * b;
             bool s0 = k == T.slot, s1 = k + 1 == T.slot;
 #pragma unroll
-            for (int e = 0; e < kExwRegs; ++e) {
+            for (int e = 0; e < exw_regs(WIDE); ++e) {
                 s0 |= k == T.ex[e];
                 s1 |= k + 1 == T.ex[e];
             }
-            if (exw > kExwRegs) {
+            if (exw > exw_regs(WIDE)) {
                 float o0, o1;
                 sp2(f2{v3.y}, o0, o1);
-                for (int e = kExwRegs; e < exw; ++e) {
+                for (int e = exw_regs(WIDE); e < exw; ++e) {
                     const int x = excl[(size_t)e * n + T.orig];
                     s0 |= x == __float_as_int(o0);
                     s1 |= x == __float_as_int(o1);
@@ -391,7 +397,7 @@ struct RunWalk {
 // rules out a pair inside xcut2 for every lane, the result added to out and the
 // corrected pairs counted into C.count.  (A kernel of its own: walked after the
 // near list in one kernel it cost that one registers, and spills.)
-template <int M, int F, int DAMP, bool X2, bool CORR>
+template <int M, int F, int DAMP, bool X2, bool CORR, bool WIDE>
 __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float4* __restrict__ rec,
                                                     const float4* __restrict__ srec,
                                                     const int32_t* __restrict__ sstart,
@@ -440,7 +446,7 @@ __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float
             const int tl = lane % g, grp = lane / g;
             const bool valid = tl < nt && grp < ngr;
             const int tgt = s0 + chunk + (valid ? tl : 0);
-            Target T;
+            Target<WIDE> T;
             T.a = rec[(size_t)tgt * NV];
             T.b = rec[(size_t)tgt * NV + 1];
             T.orig = __float_as_int(T.b.w) - 1;
@@ -451,10 +457,10 @@ __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float
                 return sstart[l] + (pos - t.start[l]);
             };
 #pragma unroll
-            for (int e = 0; e < kExwRegs; ++e) T.ex[e] = e < exw ? slot_of(excl[(size_t)e * n + T.orig]) : -1;
+            for (int e = 0; e < exw_regs(WIDE); ++e) T.ex[e] = e < exw ? slot_of(excl[(size_t)e * n + T.orig]) : -1;
             T.lo = INT_MAX;
             T.hi = -1;
-            for (int e = kExwRegs; e < exw; ++e) {
+            for (int e = exw_regs(WIDE); e < exw; ++e) {
                 const int x = slot_of(excl[(size_t)e * n + T.orig]);
                 if (x >= 0) T.lo = min(T.lo, x);
                 T.hi = max(T.hi, x);
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float
                 if (valid) {
                     bool need = (unsigned)(T.slot - ps) < (unsigned)pl || (T.hi >= ps && T.lo < ps + pl);
 #pragma unroll
-                    for (int e = 0; e < kExwRegs; ++e) need |= (unsigned)(T.ex[e] - ps) < (unsigned)pl;
+                    for (int e = 0; e < exw_regs(WIDE); ++e) need |= (unsigned)(T.ex[e] - ps) < (unsigned)pl;
                     const float4* cur = bufs + slot * stage;
                     const bool anyneed = __any_sync(__activemask(), need);
                     if constexpr (CORR) {
@@ -568,26 +574,26 @@ __global__ void __launch_bounds__(256, 2) k_p2p_f32(const TreeDev t, const float
                         float ex, ey, ez;
                         const float ox = two_diff(ca.x, cb.x, ex), oy = two_diff(ca.y, cb.y, ey),
                                     oz = two_diff(ca.z, cb.z, ez);
-                        Target U = T;
+                        Target<WIDE> U = T;
                         U.a = make_float4(ta.x + ox, ta.y + oy, ta.z + oz, ta.w);
                         U.b = make_float4((ex + (cal.x - cbl.x)) + tb.x, (ey + (cal.y - cbl.y)) + tb.y,
                                           (ez + (cal.z - cbl.z)) + tb.z, 0.0f);
                         if (anyneed)
-                            p2p_piece_x2<M, F, DAMP, true, true>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
+                            p2p_piece_x2<M, F, DAMP, true, true, WIDE>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
                                                                  XB, nb, C.xcut2, &ncorr);
                         else
-                            p2p_piece_x2<M, F, DAMP, false, true>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
+                            p2p_piece_x2<M, F, DAMP, false, true, WIDE>(cur, pl >> 1, ps, grp, ngr, U, excl, exw, n, XH, XL,
                                                                   XB, nb, C.xcut2, &ncorr);
                     } else if constexpr (X2) {
                         if (anyneed)
-                            p2p_piece_x2<M, F, DAMP, true>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
+                            p2p_piece_x2<M, F, DAMP, true, false, WIDE>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
                         else
-                            p2p_piece_x2<M, F, DAMP, false>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
+                            p2p_piece_x2<M, F, DAMP, false, false, WIDE>(cur, pl >> 1, ps, grp, ngr, T, excl, exw, n, XH, XL, XB, nb);
                     } else {
                         if (anyneed)
-                            p2p_piece<M, F, DAMP, true>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
+                            p2p_piece<M, F, DAMP, true, WIDE>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
                         else
-                            p2p_piece<M, F, DAMP, false>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
+                            p2p_piece<M, F, DAMP, false, WIDE>(cur, pl, ps, grp, ngr, T, excl, exw, n, AH, AL, AB, nb);
                     }
                 }
                 __syncwarp();
@@ -754,7 +760,7 @@ __global__ void k_leaf_cost(const TreeDev t, uint32_t* __restrict__ cost, int32_
     }
 }
 
-template <int M, int F, bool X2>
+template <int M, int F, bool X2, bool WIDE>
 void launch_p2p_kind(unsigned blocks, int threads, size_t smem, int stage, int slices, const int32_t* order,
                      unsigned* next, cudaStream_t st, const TreeDev& t, const float4* rec, const float4* srec,
                      const int32_t* sstart, const int32_t* excl, int exw, int64_t n, int damp, double* out,
@@ -763,7 +769,7 @@ void launch_p2p_kind(unsigned blocks, int threads, size_t smem, int stage, int s
         return;  // not instantiated: the packed kernel is used for field orders 0 and 1
     } else {
 #define FMM_P2P_KIND(D)                                                                                              \
-    k_p2p_f32<M, F, D, X2, false><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out, stage,     \
+    k_p2p_f32<M, F, D, X2, false, WIDE><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out, stage,     \
                                                                  slices, order, next, C)
         switch (damp) {
             case DAMP_AMOEBA: FMM_P2P_KIND(DAMP_AMOEBA); break;
@@ -780,38 +786,40 @@ void launch_p2p_corr(unsigned blocks, int threads, size_t smem, int stage, const
                      cudaStream_t st, const TreeDev& t, const float4* rec, const float4* srec, const int32_t* sstart,
                      const int32_t* excl, int exw, int64_t n, double* out, const CorrArgs& C) {
     if constexpr (F <= 1)
-        k_p2p_f32<M, F, DAMP_AMOEBA, true, true><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out,
+        k_p2p_f32<M, F, DAMP_AMOEBA, true, true, false><<<blocks, threads, smem, st>>>(t, rec, srec, sstart, excl, exw, n, out,
                                                                               stage, 1, order, next, C);
 }
 
-template <int M, int F, bool X2>
+template <int M, int F, bool X2, bool WIDE>
 const void* p2p_kernel(int damp) {
     if constexpr (X2 && F > 1) return nullptr;
     else
-    return damp == DAMP_AMOEBA  ? (const void*)k_p2p_f32<M, F, DAMP_AMOEBA, X2, false>
-           : damp == DAMP_THOLE ? (const void*)k_p2p_f32<M, F, DAMP_THOLE, X2, false>
-           : damp == DAMP_ERF   ? (const void*)k_p2p_f32<M, F, DAMP_ERF, X2, false>
-                                : (const void*)k_p2p_f32<M, F, DAMP_NONE, X2, false>;
+    return damp == DAMP_AMOEBA  ? (const void*)k_p2p_f32<M, F, DAMP_AMOEBA, X2, false, WIDE>
+           : damp == DAMP_THOLE ? (const void*)k_p2p_f32<M, F, DAMP_THOLE, X2, false, WIDE>
+           : damp == DAMP_ERF   ? (const void*)k_p2p_f32<M, F, DAMP_ERF, X2, false, WIDE>
+                                : (const void*)k_p2p_f32<M, F, DAMP_NONE, X2, false, WIDE>;
 }
 
 template <int M, int F>
-int set_p2p_smem(size_t smem) {
-    const void* fns[8] = {p2p_kernel<M, F, false>(DAMP_NONE), p2p_kernel<M, F, false>(DAMP_AMOEBA),
-                          p2p_kernel<M, F, false>(DAMP_THOLE), p2p_kernel<M, F, false>(DAMP_ERF),
-                          p2p_kernel<M, F, true>(DAMP_NONE),  p2p_kernel<M, F, true>(DAMP_AMOEBA),
-                          p2p_kernel<M, F, true>(DAMP_THOLE),  p2p_kernel<M, F, true>(DAMP_ERF)};
-    for (const void* fn : fns)
-        if (fn) FMM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+const void* p2p_kernel(int damp, bool x2, bool wide) {
+    return x2 ? (wide ? p2p_kernel<M, F, true, true>(damp) : p2p_kernel<M, F, true, false>(damp))
+              : (wide ? p2p_kernel<M, F, false, true>(damp) : p2p_kernel<M, F, false, false>(damp));
+}
+
+template <int M, int F>
+int set_p2p_smem(int damp, bool x2, bool wide, size_t smem) {
+    FMM_CUDA_TRY(cudaFuncSetAttribute(p2p_kernel<M, F>(damp, x2, wide), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
     if constexpr (F <= 1)
-        FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_p2p_f32<M, F, DAMP_AMOEBA, true, true>,
+        FMM_CUDA_TRY(cudaFuncSetAttribute((const void*)k_p2p_f32<M, F, DAMP_AMOEBA, true, true, false>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return FMM_OK;
 }
 
 template <int M, int F>
-int p2p_blocks_per_sm(int damp, bool x2, int threads, size_t smem) {
+int p2p_blocks_per_sm(int damp, bool x2, bool wide, int threads, size_t smem) {
     int nb = 0;
-    const void* fn = x2 ? p2p_kernel<M, F, true>(damp) : p2p_kernel<M, F, false>(damp);
+    const void* fn = p2p_kernel<M, F>(damp, x2, wide);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 1;
@@ -909,6 +917,7 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
     // not fit); FMM_GB300_P2P_PACKED=0 selects the one-source kernel
     const bool x2 = p2p_packed_enabled(sh, field_order) && t.num_leaves > 0 &&
                     n + (int64_t)t.num_leaves < (int64_t)INT32_MAX;
+    const bool wide = P.exw > exw_regs(false);
     // a damping-correction list is walked by the packed kernel only; the
     // pairs it corrects are counted in counter 9
     if (t.ncorr > 0 && !(x2 && P.damp_type == DAMP_AMOEBA)) return FMM_ENOTSUP;
@@ -986,22 +995,26 @@ int launch_p2p_f32(Workspace& ws, const Particles& P, const TreeDev& t, int fiel
         order = ws.p2p_order.as<int32_t>();
         FMM_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned), st));
         int bps = 1;
-        FMM_MF_SWITCH(m, field_order, (bps = p2p_blocks_per_sm<MM, FF>(P.damp_type, x2, sh.threads, smem)));
+        FMM_MF_SWITCH(m, field_order, (bps = p2p_blocks_per_sm<MM, FF>(P.damp_type, x2, wide, sh.threads, smem)));
         blocks = (unsigned)std::min<int64_t>(blocks, (int64_t)bps * num_sms_f32());
     }
     if (smem > 48 * 1024) {
-        FMM_MF_SWITCH(m, field_order, FMM_TRY((set_p2p_smem<MM, FF>(smem))));
+        FMM_MF_SWITCH(m, field_order, FMM_TRY((set_p2p_smem<MM, FF>(P.damp_type, x2, wide, smem))));
     }
-    if (x2) {
-        FMM_MF_SWITCH(m, field_order,
-                      (launch_p2p_kind<MM, FF, true>(blocks, sh.threads, smem, sh.stage, (int)slices, order, next, st,
-                                                     t, rec, ws.f32x2.as<float4>(), ws.p2p_pad.as<int32_t>(), P.excl,
-                                                     P.exw, n, P.damp_type, out, C)));
+#define FMM_P2P_LAUNCH(X2, WIDE, SREC, SSTART)                                                                       \
+    FMM_MF_SWITCH(m, field_order,                                                                                    \
+                  (launch_p2p_kind<MM, FF, X2, WIDE>(blocks, sh.threads, smem, sh.stage, (int)slices, order, next, st, \
+                                                     t, rec, SREC, SSTART, P.excl, P.exw, n, P.damp_type, out, C)))
+    if (x2 && wide) {
+        FMM_P2P_LAUNCH(true, true, ws.f32x2.as<float4>(), ws.p2p_pad.as<int32_t>());
+    } else if (x2) {
+        FMM_P2P_LAUNCH(true, false, ws.f32x2.as<float4>(), ws.p2p_pad.as<int32_t>());
+    } else if (wide) {
+        FMM_P2P_LAUNCH(false, true, rec, t.start);
     } else {
-        FMM_MF_SWITCH(m, field_order,
-                      (launch_p2p_kind<MM, FF, false>(blocks, sh.threads, smem, sh.stage, (int)slices, order, next, st,
-                                                      t, rec, rec, t.start, P.excl, P.exw, n, P.damp_type, out, C)));
+        FMM_P2P_LAUNCH(false, false, rec, t.start);
     }
+#undef FMM_P2P_LAUNCH
     if (slices > 1) FMM_TRY(sum_slices(n * nf, (int)slices, out, ws.fsorted.as<double>(), st));
     if (t.ncorr > 0) {
         if (next) FMM_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned), st));
