@@ -1,8 +1,9 @@
-"""The sequential root centre (csrc/tree.cu seq_sum) where its sum
-changes binade all the time: coordinates around zero.  One FP64 addition after
-the other, 200,000 particles take 7.4 ms (and a parallel form with a block's attempt
-at each change 8.5 to 12.5); the whole tree is to stay below the chain.  And the bits
-of the result there: ties, sums that nowhere round."""
+"""The sequential root centre (csrc/tree.cu seq_sum) where its sum changes
+binade all the time: coordinates around zero.  One FP64 addition after the other,
+200,000 particles take 7.4 ms; a parallel form with a block's attempt at each
+change took 8.5 to 12.5 ms, with a tree of 0.7 ms where the sum grows steadily; the
+whole tree is to stay below ten times that.  And the bits of the result there:
+ties, sums that nowhere round."""
 import numpy as np
 import pytest
 import torch
@@ -15,24 +16,28 @@ pytestmark = pytest.mark.gpu
 N = 199998
 
 
-@pytest.mark.parametrize("kind", ["box", "centred", "gauss", "lattice"])
+def _tree_time(X):
+    n = len(X)
+    put = lambda a: torch.from_numpy(np.ascontiguousarray(a.T)).cuda().t()  # noqa: E731
+    M = np.random.default_rng(1).normal(size=(n, 1))
+    dev = put(X), put(M), put(np.arange(1, n + 1, dtype=np.int32)[:, None])
+    F = torch.zeros((1, n), dtype=torch.float64, device="cuda").t()
+    times = []
+    for _ in range(4):
+        fmm_gb300.field_fmm_device(*dev, 0.9, 512, 2, 0, F, options=Options())
+        times.append(fmm_gb300.last_stats()["t_tree"])
+    return min(times)
+
+
+@pytest.mark.parametrize("kind", ["centred", "gauss", "lattice"])
 def test_tree_time(kind):
     rng = np.random.default_rng(4)
     if kind == "lattice":
         g = 2.5 * np.arange(-29, 30)
         X = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)[:N]
     else:
-        X = {"box": lambda: rng.uniform(0.0, 146.0, (N, 3)), "centred": lambda: rng.uniform(-73.0, 73.0, (N, 3)),
-             "gauss": lambda: 40.0 * rng.normal(size=(N, 3))}[kind]()
-    n = X.shape[0]
-    put = lambda a: torch.from_numpy(np.ascontiguousarray(a.T)).cuda().t()  # noqa: E731
-    dev = put(X), put(rng.normal(size=(n, 1))), put(np.arange(1, n + 1, dtype=np.int32)[:, None])
-    F = torch.zeros((1, n), dtype=torch.float64, device="cuda").t()
-    times = []
-    for _ in range(4):
-        fmm_gb300.field_fmm_device(*dev, 0.9, 512, 2, 0, F, options=Options())
-        times.append(fmm_gb300.last_stats()["t_tree"])
-    assert min(times) < 37e-6 * n, times
+        X = {"centred": lambda: rng.uniform(-73.0, 73.0, (N, 3)), "gauss": lambda: 40.0 * rng.normal(size=(N, 3))}[kind]()
+    assert _tree_time(X) < 10.0 * _tree_time(rng.uniform(0.0, 146.0, (N, 3)))
 
 
 def _values(kind, n, rng):
