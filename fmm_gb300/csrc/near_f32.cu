@@ -43,7 +43,10 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 // compensated one.  A fold is 24 packed operations of about 140 a block; at
 // four, water with Thole damping (60,000 sites) is 1.31e-6 off the FP64 near
 // field, at three 1.27e-6, as with the folds at every leaf end before.
-constexpr int kFold = 3;
+// Potentials alone (F = 0), of which every one is a sum of charges' and multipoles'
+// large terms, fold at two: dipoles and quadrupoles with Thole damping 2.99e-7 off
+// (700 points, box of 20), at three 3.27e-7; 1 to 3% of the kernel's time.
+__host__ __device__ constexpr int fold_of(int f) { return f == 0 ? 2 : 3; }
 // Exclusion entries held in registers per target; for the others a piece is
 // checked by the range of their slots.  Eight cost the kernels 3 to 7%, so longer
 // lists than four have kernels of their own (WIDE).  240,000 particles in
@@ -198,7 +201,7 @@ __device__ __forceinline__ int first_block(int b0, int grp, int ngr) {
 // for the lane's target: compensated FP32 (TwoSum hi + lo), since the per-atom
 // terms are much larger than their neutral total.  The contraction adds each
 // pair into a plain FP32 block sum (blk, of nb pairs so far, kept from piece to
-// piece) that is folded into (hi, lo) every kFold pairs: the block sum's
+// piece) that is folded into (hi, lo) every fold_of(F) pairs: the block sum's
 // rounding is of the order of a single pair's, and the TwoSum cost is paid once
 // per fold.  k0 is the slot of src[0].  CHECK: the piece may hold the
 // target itself or one of its excluded partners.
@@ -231,7 +234,7 @@ __device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, in
         const float dy = (T.a.y - a.y) + (T.b.y - b.y);
         const float dz = (T.a.z - a.z) + (T.b.z - b.z);
         pair_field_f32acc<M, F>(dx, dy, dz, T.a.w * a.w, DAMP, mc, blk);
-        if (++nb == kFold) {
+        if (++nb == fold_of(F)) {
             nb = 0;
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
@@ -249,7 +252,7 @@ __device__ __forceinline__ void p2p_piece(const float4* src, int cnt, int k0, in
 // ... of the staged piece, each the lane's target against two sources in
 // packed arithmetic.  Each half keeps its own compensated sum (H, L) over all
 // pieces of the target chunk, fed from a plain block sum B (of nb blocks so far)
-// folded every kFold blocks (as many pairs per fold and half as in the scalar
+// folded every fold_of(F) blocks (as many pairs per fold and half as in the scalar
 // loop).  k0 is the slot
 // of the piece's first source.
 // CORR (a piece of a far leaf inside the damping range): only the damping
@@ -320,7 +323,7 @@ __device__ __forceinline__ void p2p_piece_x2(const float4* src, int nblk, int k0
             }
         }
         pair_field_x2<M, F, CORR>(dx, dy, dz, a, DAMP, mc, B);
-        if (++nb == kFold) {
+        if (++nb == fold_of(F)) {
             nb = 0;
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
