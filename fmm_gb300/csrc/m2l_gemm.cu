@@ -101,12 +101,15 @@ __global__ void k_scale_weights(int M, int nr, int ld, const double* __restrict_
 // pipe; its error (a few 1e-8 relative of the displacement, up to ~1e-4 cell
 // units at the largest encodable displacement) stays far below the 1e-3
 // tolerance of the integer test.  Without them, FP64 with a 1e-6 tolerance.
+// Cell centres are rounded, so pairs of a group differ from its displacement by
+// some 1e-16 of the coordinates (dev: the largest difference, in units of the
+// smaller half-width, where FP64 pairs are asked for it).
 // Sources in periodic images are displaced by their image's shift, the same in
 // bohr but not in units of their cells: only pairs of one image and one level
 // share an operator.
 __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restrict__ tgt, int p, int oclass,
                            const float4* __restrict__ chi, const float4* __restrict__ clo,
-                           uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+                           uint64_t* __restrict__ keys, int32_t* __restrict__ vals, int* __restrict__ dev) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= nfar) return;
     const int i = tgt[q], j = src_node(t, t.far_src[q]);
@@ -153,6 +156,10 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
         key = ((uint64_t)kFallback << 40) | ((uint64_t)q << 3);
     keys[q] = key;
     vals[q] = (int32_t)q;
+    if (dev) {  // largest deviation from the grid, as the bits of a float >= 0
+        const int e = __reduce_max_sync(__activemask(), grid ? __float_as_int(fmaxf(ex, fmaxf(ey, ez))) : 0);
+        if ((threadIdx.x & 31) == 0 && e > *(volatile int*)dev) atomicMax(dev, e);
+    }
 }
 
 // A group's order: the highest of its pairs' orders (gq starts at zero).  Warp
@@ -1015,6 +1022,12 @@ constexpr int kOrderClass = 2;
 // tensor-core product of one group costs about what the per-pair kernel takes
 // for one or two pairs (order 10: 33 ns against 44 ns a pair at the FP64 peak).
 constexpr double kMinGroupPairs = 16.0, kMinGroupPairs64 = 2.0;
+// Where the per-pair kernels are an alternative of the same kind, pairs may be
+// off their group's displacement by this much (half-widths): they take each
+// pair's own.  60,000 particles in a box of 98 with its corner at 0 are 7e-15 off,
+// at 1,000 1.2e-13; 1,500 in a box of 3 6e-15 at 0, 6e-14 at 30 (their field 5e-14),
+// 2e-12 at 1,000 (above 1e-12).
+constexpr float kGroupDeviation = 1e-13f;
 // Memory limit of the calls that need not take the grouped products
 // (FMM_GB300_M2L_BYTES; read at every call).
 double grouped_bytes() {
@@ -1085,8 +1098,10 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         // FP32 node data where the mixed path prepared it
         const float4* chi = (sizeof(R) == 4 && ws.f32node_ok) ? ws.f32node.as<float4>() : nullptr;
         const int kbits = t.nimg > 1 ? kKeyBitsImages : kKeyBits;
+        int* d_dev = sizeof(R) == 8 ? reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 10) : nullptr;
+        if (d_dev) FMM_CUDA_TRY(cudaMemsetAsync(d_dev, 0, sizeof(int), st));
         k_m2l_keys<<<grid_for(nf, 256), 256, 0, st>>>(nf, t, tgt, p, kOrderClass, chi, chi ? chi + M : nullptr,
-                                                       ws.m2l_keys.as<uint64_t>(), ws.m2l_vals.as<int32_t>());
+                                                       ws.m2l_keys.as<uint64_t>(), ws.m2l_vals.as<int32_t>(), d_dev);
         // sort by key, run-length encode into groups
         int* d_nruns = reinterpret_cast<int*>(ws.counters.as<unsigned long long>() + 14);
         size_t tb1 = 0, tb2 = 0, tb3 = 0;
@@ -1104,7 +1119,9 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
                                                         ws.m2l_ukeys.as<uint64_t>(), ws.m2l_cnt.as<int32_t>(),
                                                         d_nruns, (int)nf, st));
         int ng = 0;
+        float dev = 0.0f;
         FMM_CUDA_TRY(cudaMemcpyAsync(&ng, d_nruns, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (d_dev) FMM_CUDA_TRY(cudaMemcpyAsync(&dev, d_dev, sizeof(float), cudaMemcpyDeviceToHost, st));
         FMM_CUDA_TRY(cudaStreamSynchronize(st));
         // displacement groups of a few pairs each (irregular trees, mixed orders)
         // leave the products' columns empty and multiply the per-group operators.
@@ -1129,7 +1146,8 @@ int grouped(Workspace& ws, const TreeDev& t, int p, cudaStream_t st, bool full, 
         ws.m2l_groups = ng;
         if (few) return FMM_ENOTSUP;
         size.groups = ng;
-        if ((bounded || (double)nf < kMinGroupPairs * (double)ng) && m2l_bytes(size) > grouped_bytes())
+        if ((bounded || (double)nf < kMinGroupPairs * (double)ng) &&
+            (m2l_bytes(size) > grouped_bytes() || dev > kGroupDeviation))
             return FMM_ENOTSUP;
         FMM_CUDA_TRY(cudaMemsetAsync(ws.m2l_cnt.as<int32_t>() + ng, 0, sizeof(int32_t), st));
         size_t tb4 = 0;
