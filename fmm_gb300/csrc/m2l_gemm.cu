@@ -111,6 +111,7 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
                            const float4* __restrict__ chi, const float4* __restrict__ clo,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ vals, int* __restrict__ dev) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const unsigned warp = __ballot_sync(0xffffffffu, q < nfar);  // whole warps are launched
     if (q >= nfar) return;
     const int i = tgt[q], j = src_node(t, t.far_src[q]);
     const int ord = t.far_ord ? min((int)t.far_ord[q], p) : p;
@@ -157,7 +158,7 @@ __global__ void k_m2l_keys(int64_t nfar, const TreeDev t, const int32_t* __restr
     keys[q] = key;
     vals[q] = (int32_t)q;
     if (dev) {  // largest deviation from the grid, as the bits of a float >= 0
-        const int e = __reduce_max_sync(__activemask(), grid ? __float_as_int(fmaxf(ex, fmaxf(ey, ez))) : 0);
+        const int e = __reduce_max_sync(warp, grid ? __float_as_int(fmaxf(ex, fmaxf(ey, ez))) : 0);
         if ((threadIdx.x & 31) == 0 && e > *(volatile int*)dev) atomicMax(dev, e);
     }
 }
